@@ -1612,92 +1612,113 @@ namespace lst {
 
   // Duplicate removal among the T5s of one module (SDL/Kernels.h:202-249).
   // Every pair (i < j) of a module is independent and only ever sets isDup
-  // bit 1, so the pairs are spread over a block: a chunk of 32 entries of the
-  // eligible-module list is scanned for modules holding two or more T5s, and each such module's
-  // T5s are staged in shared memory (eta, phi, score, hits) and its n x n pair
-  // square is shared out among the block's threads.  The largest modules hold
-  // a few hundred T5s, whose pairs would otherwise run on one warp.
-  constexpr int kT5DedupThreads = 128;
-  constexpr unsigned int kT5DedupStage = 256;
+  // bit 1, so the pairs are dealt out in tiles of 32 x 32 to all warps of the
+  // event: a module may hold a few hundred T5s (of about 1300 in the event),
+  // nearly all of them within the eta / phi windows of one another, and one
+  // block working through such a module's pairs took 1.3 ms.  Each block scans
+  // the eligible modules' counts itself (a few microseconds, in place of a
+  // list made by another launch), numbers the tile pairs (ti <= tj) of the
+  // modules with two or more T5s, and takes the tile pairs of its warps: a
+  // lane holds one T5 of tile tj in registers, and the T5s of tile ti, one per
+  // lane, are broadcast in turn, so that the ten-by-ten hit comparison reads
+  // no memory.  Bound by the comparisons' issue slots.
+  constexpr int kT5DedupThreads = 256;
+  constexpr unsigned int kT5DedupPerThread = 8;
+  constexpr unsigned int kT5DedupChunk = kT5DedupThreads * kT5DedupPerThread;  // eligible modules scanned at a time
   __global__ void __launch_bounds__(kT5DedupThreads) kT5DedupAfterBuild(DeviceES es, const EventView* evs) {
-    __shared__ float sEta[kT5DedupStage], sPhi[kT5DedupStage], sScore[kT5DedupStage];
-    __shared__ unsigned int sHits[kT5DedupStage * 10];
-    __shared__ uint16_t sMods[32];
-    __shared__ unsigned int sNMods;
+    __shared__ unsigned int sPre[kT5DedupChunk + 1];  // first tile pair of each listed module
+    __shared__ uint16_t sMods[kT5DedupChunk];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nElig = *ev.rg.nEligibleT5Modules;
+    const unsigned int lane = laneId();
     Quintuplets q = ev.t5;
-    // chunks of 32 eligible modules: the first warp picks those with two or more T5s
-    for (unsigned int c0 = blockIdx.x * 32; c0 < nElig; c0 += gridDim.x * 32) {
-      if (threadIdx.x < 32) {
-        const unsigned int e = c0 + threadIdx.x;
-        uint16_t lmLoad = 0;
-        unsigned int nLoad = 0;
-        if (e < nElig) {
-          lmLoad = ev.rg.indicesOfEligibleT5Modules[e];
-          nLoad = q.nQuintuplets[lmLoad];
-        }
-        unsigned int tot;
-        const unsigned int slot = warpRank(nLoad >= 2, tot);
-        if (nLoad >= 2)
-          sMods[slot] = lmLoad;
-        if (threadIdx.x == 0)
-          sNMods = tot;
+    for (unsigned int c0 = 0; c0 < nElig; c0 += kT5DedupChunk) {
+      uint16_t mods[kT5DedupPerThread];
+      unsigned int pairs[kT5DedupPerThread];
+      unsigned int myMods = 0, myPairs = 0;
+#pragma unroll
+      for (unsigned int k = 0; k < kT5DedupPerThread; ++k) {
+        const unsigned int e = c0 + threadIdx.x * kT5DedupPerThread + k;
+        mods[k] = e < nElig ? ev.rg.indicesOfEligibleT5Modules[e] : 0;
       }
+#pragma unroll
+      for (unsigned int k = 0; k < kT5DedupPerThread; ++k) {
+        const unsigned int e = c0 + threadIdx.x * kT5DedupPerThread + k;
+        const unsigned int n = e < nElig ? q.nQuintuplets[mods[k]] : 0u;
+        const unsigned int tiles = (n + 31u) >> 5;
+        pairs[k] = n >= 2 ? tiles * (tiles + 1) / 2 : 0u;
+        myMods += pairs[k] ? 1u : 0u;
+        myPairs += pairs[k];
+      }
+      unsigned int nMods, nPairs;
+      unsigned int slot = blockExclusiveScan(myMods, nMods);
+      unsigned int first = blockExclusiveScan(myPairs, nPairs);
+#pragma unroll
+      for (unsigned int k = 0; k < kT5DedupPerThread; ++k) {
+        if (pairs[k] == 0)
+          continue;
+        sMods[slot] = mods[k];
+        sPre[slot++] = first;
+        first += pairs[k];
+      }
+      if (threadIdx.x == 0)
+        sPre[nMods] = nPairs;
       __syncthreads();
-      const unsigned int nMods = sNMods;
-      for (unsigned int k = 0; k < nMods; ++k) {
+      const unsigned int wpb = kT5DedupThreads / 32;
+      for (unsigned int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < nPairs; t += gridDim.x * wpb) {
+        const int k = findSlot(sPre, int(nMods), t);
         const uint16_t lm = sMods[k];
         const unsigned int n = q.nQuintuplets[lm];
         const unsigned int base = ev.rg.quintupletModuleIndices[lm];
-        const bool staged = n <= kT5DedupStage && !ev.forceWalk;
-        if (staged) {
-          for (unsigned int t = threadIdx.x; t < n; t += blockDim.x) {
-            sEta[t] = q.eta[base + t];
-            sPhi[t] = q.phi[base + t];
-            sScore[t] = q.score_rphisum[base + t];
-          }
-          for (unsigned int t = threadIdx.x; t < 10 * n; t += blockDim.x)
-            sHits[t] = q.hitIndices[10 * base + t];
+        const unsigned int local = t - sPre[k];
+        unsigned int tj = 0;
+        while ((tj + 1) * (tj + 2) / 2 <= local)
+          ++tj;
+        const unsigned int ti = local - tj * (tj + 1) / 2;
+        const unsigned int i = 32 * ti + lane, j = 32 * tj + lane;
+        const unsigned int ix = base + min(i, n - 1), jx = base + min(j, n - 1);
+        const float etaI = q.eta[ix], phiI = q.phi[ix], scoreI = q.score_rphisum[ix];
+        const float etaJ = q.eta[jx], phiJ = q.phi[jx], scoreJ = q.score_rphisum[jx];
+        unsigned int hitI[10], hitJ[10];
+        // (40 bytes per T5: the ten indices lie on an 8-byte boundary)
+        const uint2* hI = reinterpret_cast<const uint2*>(q.hitIndices + 10 * size_t(ix));
+        const uint2* hJ = reinterpret_cast<const uint2*>(q.hitIndices + 10 * size_t(jx));
+#pragma unroll
+        for (int a = 0; a < 5; ++a) {
+          const uint2 u = hI[a], v = hJ[a];
+          hitI[2 * a] = u.x;
+          hitI[2 * a + 1] = u.y;
+          hitJ[2 * a] = v.x;
+          hitJ[2 * a + 1] = v.y;
         }
-        __syncthreads();
-        for (unsigned int pr = threadIdx.x; pr < n * n; pr += blockDim.x) {
-          const unsigned int i = pr / n, j = pr - i * n;
-          if (j <= i)
-            continue;
-          const unsigned int ix = base + i, jx = base + j;
-          const float eta1 = staged ? sEta[i] : q.eta[ix], phi1 = staged ? sPhi[i] : q.phi[ix];
-          const float eta2 = staged ? sEta[j] : q.eta[jx], phi2 = staged ? sPhi[j] : q.phi[jx];
-          const float dEta = fabs_(eta1 - eta2);
-          const float dPhi = wrapDPhi(phi1, phi2);
-          if (dEta > 0.1f)
-            continue;
-          if (fabs_(dPhi) > 0.1f)
+        const unsigned int rows = min(n - 32 * ti, 32u);
+        for (unsigned int r = 0; r < rows; ++r) {
+          const float eta1 = __shfl_sync(kFullMask, etaI, r), phi1 = __shfl_sync(kFullMask, phiI, r);
+          const float dEta = fabs_(eta1 - etaJ);
+          const float dPhi = wrapDPhi(phi1, phiJ);
+          const bool near = j < n && j > 32 * ti + r && !(dEta > 0.1f) && !(fabs_(dPhi) > 0.1f);
+          if (!__any_sync(kFullMask, near))
             continue;
           int nMatched = 0;
-          if (staged) {
-            for (int a = 0; a < 10; a++) {
-              const unsigned int h = sHits[10 * i + a];
-              bool matched = false;
-              for (int b = 0; b < 10; b++)
-                matched |= h == sHits[10 * j + b];
-              nMatched += matched ? 1 : 0;
-            }
-          } else {
-            nMatched = sharedHitsT5(q, ix, jx);
+#pragma unroll
+          for (int a = 0; a < 10; ++a) {
+            const unsigned int h = __shfl_sync(kFullMask, hitI[a], r);
+            bool matched = false;
+#pragma unroll
+            for (int b = 0; b < 10; ++b)
+              matched |= h == hitJ[b];
+            nMatched += matched ? 1 : 0;
           }
-          if (nMatched >= 7) {
-            const float score1 = staged ? sScore[i] : q.score_rphisum[ix];
-            const float score2 = staged ? sScore[j] : q.score_rphisum[jx];
-            if (score1 >= score2)
-              q.isDup[ix] = 1;
+          const float score1 = __shfl_sync(kFullMask, scoreI, r);
+          if (near && nMatched >= 7) {
+            if (score1 >= scoreJ)
+              q.isDup[base + 32 * ti + r] = 1;
             else
               q.isDup[jx] = 1;
           }
         }
-        __syncthreads();
       }
-      __syncthreads();  // sMods / sNMods are rewritten for the next chunk
+      __syncthreads();  // sMods / sPre are rewritten for the next chunk
     }
   }
 
