@@ -60,17 +60,16 @@ namespace lst {
     unsigned int t5CandTotal;     // quintuplet candidates of the event
     unsigned int t5CandOverflow;  // more candidates than the flag buffer holds
     unsigned int t5PassCount;     // passing candidates found by kT5Eval
-    unsigned int pixCandTotal;    // pT5 / pT3 candidates of the current pixel stage
     unsigned int pixPassCount;    // passing candidates found by kPixEval
+    unsigned int pixOverflow;     // a pLS has more candidates than a key can number
     unsigned int pixFallback;     // the pixel stage overflowed the staging: walk instead
-    unsigned int pixQueueCount;   // candidates passing the pixel pre-selection
+    unsigned int pixQueueCount;   // pixel candidates passing the radius criterion and the first tracklet
     unsigned int t5QueueCount;    // candidates passing the quintuplet pre-selection
-    unsigned int pixQueueBack;    // pixel candidates queued from the back (endcap tracklet algorithm)
     unsigned int t5QueueBack;     // quintuplet candidates queued from the back (modules not all barrel)
-    unsigned int pixQueue2Count;  // pixel candidates passing the first pixel tracklet as well
     unsigned int t5SortCount;     // quintuplets binned by eta for the cross-module cleaning
     unsigned int mdNext;          // next task for kCreateMD's warps
     unsigned int lsNext;          // next lower module for kCreateLS's warps
+    unsigned int pixNext; // next task (a few pLS) for kPixMid's warps
     unsigned int t3Next;          // next lower module for kCreateT3's warps
   };
 
@@ -93,9 +92,8 @@ namespace lst {
     unsigned int* plsHit2;
     unsigned int* plsHit3;
     float* plsDPhiChange;
+    float* plsPhiP;  // phi of the pLS momentum (px, py), for the pixel tracklets
     // scratch
-    unsigned int* plsConnIndex;
-    unsigned int* plsConnSize;
     unsigned int* plsCount;
     unsigned int* plsOffset;
     unsigned int* moduleCount;
@@ -120,12 +118,8 @@ namespace lst {
     unsigned int* t5PassC;      //   and their candidate index
     float* t5DnnFeat;           // candidates staged for the classifier (kT5Eval): 38 inputs each
     struct T5DnnSlotG* t5DnnSlot;  //   and their selection state
-    unsigned int* plsModPre;    // per pLS: candidate prefix over its connected modules (41 entries)
-    unsigned int* plsCand;      // per pLS: candidates
-    unsigned int* plsCandOff;   // per pLS: first candidate (nPLS + 1 entries)
-    unsigned int* pixPassC;     // passing candidates: candidate index
+    unsigned int* pixPassC;     // passing candidates: key
     unsigned int* pixPassObj;   //   the T5 / T3 index
-    unsigned int* pixPassPLS;   //   the pLS index
     float* pixPassV;            //   the selection values (8 per candidate)
     float* hitMiniSlope;        // per hit: the slope term of the mini-doublet dphi threshold
     float* hitShiftXa;          // per hit moved by the strip shift: its moved point and z
@@ -134,8 +128,8 @@ namespace lst {
     unsigned int* t5Order;      // quintuplets sorted by eta bin (their index)
     uint16_t* t5OrderPos;       //   and their module's position in the eligible-module list
     unsigned int* t5BinStart;   // start of each eta bin in t5Order (bins + 2 entries)
+    unsigned int* candQueueObj; // and the object of a queued pixel candidate
     unsigned int* candQueue;    // candidates passing a pre-selection (T5, then pT5 / pT3), any order
-    unsigned int* pixChunkPLS;  // per 32 pT5 / pT3 candidates: the pLS of the first one
     unsigned int* t5ChunkMod;   // per 32 T5 candidates: the eligible module of the first one
     struct TCCleanInfo* tcCleanInfo;  // per track candidate: the pLS cross-cleaning record
     struct PLSRec* plsRec;      // pass-2 pLS records sorted by eta bin

@@ -545,10 +545,7 @@ namespace {
         LST_LAUNCH(lst::kPLSCleanHits, dim3(blocksFor(P, count), count), kThreads, d, v, false);
         break;
       case LST_STAGE_PIXEL_QUINTUPLETS:
-        LST_LAUNCH(lst::kPixelConnect, dim3(blocksFor(P, count), count), kThreads, d, v);
-        LST_LAUNCH(lst::kPixPrefix<5>, warpGrid(P, 8, count), 256, d, v);
-        LST_LAUNCH(lst::kPixScan, one, 1024, d, v);
-        LST_LAUNCH(lst::kPixPre<5>, dim3(blocksFor(size_t(1) << 20, count), count), kThreads, d, v);
+        LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kPixMid<5>, tunedFlatGrid(ev, kTuMid5, count), tunedThreads(ev, kTuMid5), d, v);
         LST_LAUNCH(lst::kPixEval<5>, tunedFlatGrid(ev, kTuPix5, count), tunedThreads(ev, kTuPix5), d, v);
         LST_LAUNCH(lst::kPixRankEmit<5>, one, 1024, d, v);
@@ -561,10 +558,7 @@ namespace {
         LST_LAUNCH(lst::kAddPT5TC, one, 1024, d, v);
         break;
       case LST_STAGE_PIXEL_TRIPLETS:
-        LST_LAUNCH(lst::kPixelConnect, dim3(blocksFor(P, count), count), kThreads, d, v);
-        LST_LAUNCH(lst::kPixPrefix<3>, warpGrid(P, 8, count), 256, d, v);
-        LST_LAUNCH(lst::kPixScan, one, 1024, d, v);
-        LST_LAUNCH(lst::kPixPre<3>, dim3(blocksFor(size_t(1) << 20, count), count), kThreads, d, v);
+        LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kPixMid<3>, tunedFlatGrid(ev, kTuMid3, count), tunedThreads(ev, kTuMid3), d, v);
         LST_LAUNCH(lst::kPixEval<3>, tunedFlatGrid(ev, kTuPix3, count), tunedThreads(ev, kTuPix3), d, v);
         LST_LAUNCH(lst::kPixRankEmit<3>, one, 1024, d, v);
@@ -684,16 +678,10 @@ namespace {
         {"kPLSCleanHits", (const void*)lst::kPLSCleanHits},
         {"kPLSCleanNear", (const void*)lst::kPLSCleanNear},
         {"kMergePLSFlag", (const void*)lst::kMergePLSFlag},
-        {"kPixelConnect", (const void*)lst::kPixelConnect},
-        {"kPixPrefix<5>", (const void*)lst::kPixPrefix<5>},
-        {"kPixPrefix<3>", (const void*)lst::kPixPrefix<3>},
-        {"kPixScan", (const void*)lst::kPixScan},
         {"kPixEval<5>", (const void*)lst::kPixEval<5>},
-        {"kPixPre<5>", (const void*)lst::kPixPre<5>},
         {"kT5Pre", (const void*)lst::kT5Pre},
         {"kPixMid<5>", (const void*)lst::kPixMid<5>},
         {"kPixMid<3>", (const void*)lst::kPixMid<3>},
-        {"kPixPre<3>", (const void*)lst::kPixPre<3>},
         {"kPixEval<3>", (const void*)lst::kPixEval<3>},
         {"kPixRankEmit<5>", (const void*)lst::kPixRankEmit<5>},
         {"kPixRankEmit<3>", (const void*)lst::kPixRankEmit<3>},

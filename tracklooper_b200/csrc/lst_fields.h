@@ -215,8 +215,7 @@
   X(plsHit2, unsigned int, P)                         \
   X(plsHit3, unsigned int, P)                         \
   X(plsDPhiChange, float, P)                          \
-  X(plsConnIndex, unsigned int, P)                    \
-  X(plsConnSize, unsigned int, P)                     \
+  X(plsPhiP, float, P)                                \
   X(plsCount, unsigned int, P)                        \
   X(plsOffset, unsigned int, P)                       \
   X(moduleCount, unsigned int, L + 1)                 \
@@ -239,15 +238,11 @@
   X(t5PassC, unsigned int, lst::kT5PassCap)           \
   X(t5DnnFeat, float, 38 * lst::kT5DnnCap)            \
   X(t5DnnSlot, lst::T5DnnSlotG, lst::kT5DnnCap)      \
-  X(plsModPre, unsigned int, P * (lst::kMaxConnectedModules + 1)) \
-  X(plsCand, unsigned int, P)                         \
-  X(plsCandOff, unsigned int, P + 1)                  \
   X(pixPassC, unsigned int, lst::kPixPassCap)         \
   X(pixPassObj, unsigned int, lst::kPixPassCap)       \
-  X(pixPassPLS, unsigned int, lst::kPixPassCap)       \
   X(pixPassV, float, 8 * lst::kPixPassCap)            \
   X(candQueue, unsigned int, lst::kCandQueueCap)        \
-  X(pixChunkPLS, unsigned int, lst::kPixChunkCap)       \
+  X(candQueueObj, unsigned int, lst::kCandQueueCap)     \
   X(t5ChunkMod, unsigned int, lst::kT5CandCap / 32)     \
   X(hitMiniSlope, float, H)                           \
   X(t5Order, unsigned int, lst::kT5SortCap)           \

@@ -314,6 +314,7 @@ namespace lst {
       storePixelSegment(
           es.m, ev.hits, md, ls, pix, mdBase, lsBase, tid, hit[0], hit[1], hit[2], hit[3], ev.plsDPhiChange[tid]);
       ls.partOfPT5[tid] = 0;
+      ev.plsPhiP[tid] = phiOf(ls.px[tid], ls.py[tid]);
       for (unsigned int slot = 0; slot < 4; ++slot) {
         const unsigned int e = 4 * tid + slot;
         ev.plsHitNext[e] = atomicExch(&ev.plsHitHead[plsHitBucket(ls.pLSHitsIdxs[e])], e);
@@ -329,14 +330,18 @@ namespace lst {
 
   // Work counters of the kernels whose warps take their next task from the
   // event's counter (kCreateMD, kCreateLS, kCreateT3), so that a warp that
-  // drew light tasks takes more: the work per module is very uneven.  Zeroed
-  // before each of those kernels runs.
+  // drew light tasks takes more: the work per module is very uneven; and the
+  // list lengths of the pixel stages.  Zeroed before each of those kernels runs.
   __global__ void kTaskCountersReset(const EventView* evs) {
     if (threadIdx.x == 0) {
       EventScalars* sc = evs[blockIdx.y].sc;
       sc->mdNext = 0;
       sc->lsNext = 0;
       sc->t3Next = 0;
+      sc->pixNext = 0;
+      sc->pixQueueCount = 0;
+      sc->pixPassCount = 0;
+      sc->pixOverflow = 0;
     }
   }
   // The next task of the calling warp from counter *next (the same value on
@@ -463,7 +468,7 @@ namespace lst {
 #define LST_LB_T5EVAL_B 8
 #endif
 #ifndef LST_LB_PIXMID_B
-#define LST_LB_PIXMID_B 12
+#define LST_LB_PIXMID_B 10
 #endif
 #define LST_LB_MD 256, LST_LB_MD_B
 #define LST_LB_LS 128, LST_LB_LS_B
@@ -1110,7 +1115,6 @@ namespace lst {
   // candidates than the flag buffer holds take the walk instead.
   constexpr unsigned int kT5CandCap = 1u << 21;  // candidates per event
   constexpr unsigned int kCandQueueCap = 1u << 18;  // pre-selected candidates per event (T5, pT5, pT3)
-  constexpr unsigned int kPixChunkCap = 1u << 16;   // 32-candidate chunks of the pT5 / pT3 chunk table
   constexpr unsigned int kT5SortCap = 1u << 15;     // quintuplets per event sorted by eta for the TC cleaning
   constexpr unsigned int kT5PassCap = 1u << 16;  // passing candidates per event whose values are kept
 
@@ -1969,28 +1973,25 @@ namespace lst {
   }
 
   // ============================================ pixel-map slices per pLS
-  // SDL/Event.cc:1055-1080
-  __global__ void kPixelConnect(DeviceES es, const EventView* evs) {
-    const EventView& ev = evs[blockIdx.y];
-    const unsigned int nPLS = ev.ls.nSegments[es.pixelModule];
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < nPLS; i += gridDim.x * blockDim.x) {
-      int8_t pixelType = ev.ls.pixelType[i];
-      int superbin = ev.ls.superbin[i];
-      unsigned int size = 0, index = 0;
-      if (!((superbin < 0) or (superbin >= int(kSizeSuperbins)) or (pixelType > 2) or (pixelType < 0))) {
-        if (pixelType == 0) {
-          size = es.cpSizes[superbin];
-          index = es.cpIndex[superbin];
-        } else if (pixelType == 1) {
-          size = es.cpSizesPos[superbin];
-          index = es.cpIndexPos[superbin] + es.pixelIndexOffsetPos;
-        } else {
-          size = es.cpSizesNeg[superbin];
-          index = es.cpIndexNeg[superbin] + es.pixelIndexOffsetNeg;
-        }
-      }
-      ev.plsConnSize[i] = size;
-      ev.plsConnIndex[i] = index;
+  // The connected modules of pLS i: es.m.connectedPixels[index .. index + size)
+  // (SDL/Event.cc:1055-1080).
+  __device__ __forceinline__ void pixelSlice(DeviceES const& es, const EventView& ev, unsigned int i, unsigned int& size,
+                                             unsigned int& index) {
+    const int8_t pixelType = ev.ls.pixelType[i];
+    const int superbin = ev.ls.superbin[i];
+    size = 0;
+    index = 0;
+    if ((superbin < 0) or (superbin >= int(kSizeSuperbins)) or (pixelType > 2) or (pixelType < 0))
+      return;
+    if (pixelType == 0) {
+      size = es.cpSizes[superbin];
+      index = es.cpIndex[superbin];
+    } else if (pixelType == 1) {
+      size = es.cpSizesPos[superbin];
+      index = es.cpIndexPos[superbin] + es.pixelIndexOffsetPos;
+    } else {
+      size = es.cpSizesNeg[superbin];
+      index = es.cpIndexNeg[superbin] + es.pixelIndexOffsetNeg;
     }
   }
 
@@ -2012,8 +2013,8 @@ namespace lst {
                                           uint16_t* mods) {
     if (ev.ls.isDup[iPLS])
       return;
-    const unsigned int nConn = ev.plsConnSize[iPLS];
-    const unsigned int cidx = ev.plsConnIndex[iPLS];
+    unsigned int nConn, cidx;
+    pixelSlice(es, ev, iPLS, nConn, cidx);
     for (unsigned int k = laneId(); k < nConn; k += 32)
       mods[k] = static_cast<uint16_t>(es.m.connectedPixels[cidx + k]);
     __syncwarp();
@@ -2341,8 +2342,8 @@ namespace lst {
                                           uint16_t* mods) {
     if (ev.ls.isDup[iPLS] || ev.ls.partOfPT5[iPLS])
       return;
-    const unsigned int nConn = ev.plsConnSize[iPLS];
-    const unsigned int cidx = ev.plsConnIndex[iPLS];
+    unsigned int nConn, cidx;
+    pixelSlice(es, ev, iPLS, nConn, cidx);
     for (unsigned int k = laneId(); k < nConn; k += 32)
       mods[k] = static_cast<uint16_t>(es.m.connectedPixels[cidx + k]);
     __syncwarp();
@@ -2417,16 +2418,19 @@ namespace lst {
   }
 
   // ------------------------------------- pT5 / pT3 as candidate lists
-  // Candidate c of the event is the c-th (pLS, connected module, object) of
-  // the reference's loop nest (SDL/PixelTriplet.h:1043-1158, :2697-2786), so
-  // the global rank of a passing candidate is the number of passing
-  // candidates with a smaller c.  Every candidate is evaluated on its own
-  // thread; the passing ones are appended with their values and one block
-  // per event ranks them by c and stores the first 15000 (pT5) / 5000 (pT3).
-  // Events with more passing candidates than the staging holds take the
-  // per-pLS count/emit walk instead.
+  // The candidates of a pLS are its (connected module, object) pairs in the
+  // reference's loop order (SDL/PixelTriplet.h:1043-1158, :2697-2786).  A
+  // candidate's key is its pLS (16 bits) and its number f within the pLS (16
+  // bits), so that keys ascend in the order of the reference's loop nest, and
+  // the global rank of a passing candidate is the number of passing candidates
+  // with a smaller key.  kPixMid walks all candidates and queues those that
+  // pass the opening tests, kPixEval runs the rest of the selection on them,
+  // and one block per event ranks the passing ones and stores the first 15000
+  // (pT5) / 5000 (pT3).  Events that overflow the lists (or a pLS with more
+  // than 2^16 candidates) take the per-pLS count/emit walk instead.
   constexpr unsigned int kPixPassCap = 8192;
-  constexpr int kConnStride = kMaxConnectedModules + 1;
+  constexpr unsigned int kPixKeyCandidates = 1u << 16;  // candidates of one pLS that a key can number
+  static_assert(kMaxPixelSegments <= (1u << 16), "a key holds a pLS in 16 bits");
 
   template <int K>
   __device__ __forceinline__ unsigned int pixModuleCount(DeviceES const& es, const EventView& ev, uint16_t mod) {
@@ -2438,224 +2442,202 @@ namespace lst {
     return K == 5 ? (ev.ls.isDup[i] != 0) : (ev.ls.isDup[i] || ev.ls.partOfPT5[i]);
   }
 
-  template <int K>
-  __global__ void kPixPrefix(DeviceES es, const EventView* evs) {
-    const EventView& ev = evs[blockIdx.y];
-    const int wpb = blockDim.x >> 5;
-    const unsigned int nPLS = ev.ls.nSegments[es.pixelModule];
-    for (unsigned int i = blockIdx.x * wpb + (threadIdx.x >> 5); i < nPLS; i += gridDim.x * wpb) {
-      unsigned int carry = 0;
-      unsigned int* pre = ev.plsModPre + size_t(i) * kConnStride;
-      if (!pixSkipPLS<K>(ev, i)) {
-        const unsigned int nConn = ev.plsConnSize[i];
-        const unsigned int cidx = ev.plsConnIndex[i];
-        for (unsigned int b = 0; b < nConn; b += 32) {
-          const unsigned int k = b + laneId();
-          const unsigned int c =
-              k < nConn ? pixModuleCount<K>(es, ev, static_cast<uint16_t>(es.m.connectedPixels[cidx + k])) : 0u;
-          unsigned int incl = c;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            unsigned int y = __shfl_up_sync(kFullMask, incl, o);
-            if (int(laneId()) >= o)
-              incl += y;
-          }
-          if (k < nConn)
-            pre[k] = carry + incl - c;
-          carry += __shfl_sync(kFullMask, incl, 31);
-        }
-      }
-      if (laneId() == 0)
-        ev.plsCand[i] = carry;
-    }
-  }
-
-  __global__ void __launch_bounds__(1024) kPixScan(DeviceES es, const EventView* evs) {
-    const EventView& ev = evs[blockIdx.y];
-    const unsigned int n = ev.ls.nSegments[es.pixelModule];
-    unsigned int carry = 0;
-    for (unsigned int base = 0; base < n; base += blockDim.x) {
-      unsigned int i = base + threadIdx.x;
-      unsigned int c = i < n ? ev.plsCand[i] : 0u;
-      unsigned int tot;
-      unsigned int ex = blockExclusiveScan(c, tot);
-      if (i < n)
-        ev.plsCandOff[i] = carry + ex;
-      carry += tot;
-    }
-    if (threadIdx.x == 0) {
-      ev.plsCandOff[n] = carry;
-      ev.sc->pixCandTotal = carry;
-      ev.sc->pixPassCount = 0;
-      ev.sc->pixQueueCount = 0;
-      ev.sc->pixQueueBack = 0;
-      ev.sc->pixQueue2Count = 0;
-    }
-    // The chunk table: candidate 32 j lies in pLS pixChunkPLS[j].
-    if (carry > 32u * kPixChunkCap)
-      return;
-    __syncthreads();
-    for (unsigned int i = threadIdx.x; i < n; i += blockDim.x) {
-      const unsigned int a = ev.plsCandOff[i], b = ev.plsCandOff[i + 1];
-      for (unsigned int j = (a + 31u) >> 5; j < ((b + 31u) >> 5); ++j)
-        ev.pixChunkPLS[j] = i;
-    }
-  }
-
-  // (pLS, object) of candidate c.
-  template <int K>
-  __device__ __forceinline__ void pixCandidate(DeviceES const& es, const EventView& ev, unsigned int c, unsigned int& iPLS,
-                                               unsigned int& obj, uint16_t& mod) {
-    const unsigned int nPLS = ev.ls.nSegments[es.pixelModule];
-    const unsigned int* off = ev.plsCandOff;
-    // The last pLS whose first candidate is at most c: from the chunk table
-    // and a short walk (pLS without candidates are stepped over), or by a
-    // binary search when the candidates outnumber the table.
-    int lo = 0;
-    if (ev.sc->pixCandTotal <= 32u * kPixChunkCap) {
-      lo = static_cast<int>(ev.pixChunkPLS[c >> 5]);
-      while (off[lo + 1] <= c)
-        ++lo;
-    } else {
-      int hi = int(nPLS);
-      while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (off[mid] <= c)
-          lo = mid;
-        else
-          hi = mid;
-      }
-    }
-    iPLS = lo;
-    const unsigned int f = c - off[lo];
-    const unsigned int* pre = ev.plsModPre + size_t(lo) * kConnStride;
-    int klo = 0, khi = int(ev.plsConnSize[lo]);
-    while (khi - klo > 1) {
-      int mid = (klo + khi) >> 1;
-      if (pre[mid] <= f)
-        klo = mid;
-      else
-        khi = mid;
-    }
-    mod = static_cast<uint16_t>(es.m.connectedPixels[ev.plsConnIndex[lo] + klo]);
-    obj = (K == 5 ? static_cast<unsigned int>(ev.rg.quintupletModuleIndices[mod])
-                  : static_cast<unsigned int>(ev.rg.tripletModuleIndices[mod])) +
-          (f - pre[klo]);
-  }
-
-  // Pre-selection of the pT5 / pT3 candidates: the tests that come first in
-  // kPixEval (object not removed or used, the pLS-triplet radius criterion),
-  // which most candidates fail.  The survivors are queued in any order, so
-  // that kPixEval runs its long selection with all lanes of a warp busy; the
-  // outcome of a candidate does not depend on which thread evaluates it, and
-  // the passing ones are ranked by candidate index afterwards.  Candidates
-  // whose first pixel tracklet takes the barrel algorithm fill the queue from
-  // the front, the endcap ones from the back, so that a warp mostly runs one
-  // of the two.  A full queue makes kPixEval evaluate every candidate instead.
-  template <int K>
-  __global__ void __launch_bounds__(256) kPixPre(DeviceES es, const EventView* evs) {
-    const EventView& ev = evs[blockIdx.y];
-    const unsigned int total = ev.sc->pixCandTotal;
-    const unsigned int plsBase = es.lsOffset[es.nLowerModules];
-    const unsigned int stride = gridDim.x * blockDim.x;
-    for (unsigned int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-      const unsigned int c = base + laneId();
-      bool pass = false, endcap = false;
-      if (c < total) {
-        unsigned int iPLS, obj;
-        uint16_t mod;
-        pixCandidate<K>(es, ev, c, iPLS, obj, mod);
-        const unsigned int t3 = K == 5 ? ev.t5.tripletIndices[2 * obj] : obj;
-        if (K == 5)
-          pass = !ev.t5.isDup[obj] && pt3RadiusPass(es.m, ev.rg, ev.ls, ev.t3, plsBase + iPLS, t3);
-        else
-          pass = es.m.moduleType[ev.t3.lowerModuleIndices[3 * obj + 1]] != TwoS && !ev.t3.partOfPT5[obj] &&
-                 pt3RadiusPass(es.m, ev.rg, ev.ls, ev.t3, plsBase + iPLS, obj);
-        endcap = es.m.subdets[ev.t3.lowerModuleIndices[3 * t3]] == Endcap;
-      }
-      const unsigned int maskF = __ballot_sync(kFullMask, pass && !endcap);
-      const unsigned int maskB = __ballot_sync(kFullMask, pass && endcap);
-      if ((maskF | maskB) == 0u)
-        continue;
-      unsigned int startF = 0, startB = 0;
-      if (laneId() == 0) {
-        if (maskF)
-          startF = atomicAdd(&ev.sc->pixQueueCount, __popc(maskF));
-        if (maskB)
-          startB = atomicAdd(&ev.sc->pixQueueBack, __popc(maskB));
-      }
-      startF = __shfl_sync(kFullMask, startF, 0);
-      startB = __shfl_sync(kFullMask, startB, 0);
-      if (pass) {
-        const unsigned int k = endcap ? startB + __popc(maskB & lanesBelowMask())
-                                      : startF + __popc(maskF & lanesBelowMask());
-        if (k < kCandQueueCap)
-          ev.candQueue[endcap ? kCandQueueCap - 1 - k : k] = c;
-      }
-    }
-  }
-
-  // Second pre-selection stage: the first pixel tracklet algorithm (of the
-  // pLS with the triplet's, or the quintuplet's inner triplet's, inner
-  // segment), the long test that few queued candidates pass.  Its survivors
-  // are queued again, between the two ends of the first queue; without room
-  // there, kPixEval takes the first queue instead.
+  // The opening tests of the pT5 / pT3 selection: the object's flags and the
+  // pLS-triplet radius criterion, which most candidates fail, then the first
+  // pixel tracklet algorithm (of the pLS with the triplet's, or the
+  // quintuplet's inner triplet's, inner segment), a long test that few of the
+  // others pass.  A warp takes a few consecutive pLS (their flags and pixel-map
+  // slices fetched by its lanes together), deals their (pLS, connected module)
+  // pairs to its lanes and keeps the pairs that have candidates in shared memory,
+  // with their running count, so that a candidate finds its pLS and object there
+  // and the lanes are filled across pLS.  Survivors of the flags and the radius
+  // criterion wait in the warp's own queue in shared memory until there is a warp
+  // full of them for the tracklet's opening windows; those of the windows (half)
+  // wait likewise for the rest of it, and what passes that goes to the event's
+  // queue in any order.
+  // A candidate's outcome does not depend on which thread evaluates it, and the
+  // passing ones are ranked by key afterwards.
+  //
+  // Bound by the latency of dependent gathers.  A list of candidates numbered
+  // over the event (a prefix kernel, a scan, and per candidate a chunk table,
+  // a walk over the pLS offsets and a binary search in the pLS's prefix: about
+  // 16 dependent loads), with the radius survivors in a queue in memory between
+  // two kernels, took 1.59 ms (pT3) and 0.56 ms (pT5) for 64 PU200 events, this
+  // with kPixEval 1.40 and 0.45 ms.  PU250 and pt0.6 events also
+  // overflowed that queue's 2^18 entries, and every candidate took the whole
+  // selection (3.5 ms for the pT3s of 16 pt0.6 events, now 0.97); here only
+  // candidates that pass the tracklet are queued, a thirtieth of them.  The
+  // scratch is kept at 9 KB a block: with 18 KB too little of the L1 was left
+  // (pT3 1.57 ms).
+  constexpr int kPixMidWarps = 4;
+  constexpr unsigned int kPixPairs = 128;  // (pLS, connected module) pairs of one group, at least a row of the pixel map
+  static_assert(kPixPairs >= kMaxConnectedModules, "a pLS's connected modules fit a group");
+  struct PixScratch {
+    unsigned int pre[kPixPairs + 1];  // per pair with candidates: its first candidate within the group
+    unsigned int obj[kPixPairs];      //   its first object
+    uint8_t owner[kPixPairs];         //   and the lane of its pLS
+    unsigned int first[32];           // per lane's pLS: its first candidate within the group
+    // candidates waiting for the tracklet's windows [0] and its long part [1]
+    unsigned int qKey[2][64], qObj[2][64];
+  };
   template <int K>
   __global__ void __launch_bounds__(LST_LB_PIXMID) kPixMid(DeviceES es, const EventView* evs) {
+    __shared__ PixScratch sScratch[kPixMidWarps];
     const EventView& ev = evs[blockIdx.y];
-    const unsigned int front = ev.sc->pixQueueCount, back = ev.sc->pixQueueBack;
-    if (!(front <= kCandQueueCap && back <= kCandQueueCap - front))
-      return;
-    const unsigned int n = front + back, room = kCandQueueCap - n;
+    PixScratch& sc = sScratch[threadIdx.x >> 5];
+    const unsigned int nPLS = ev.ls.nSegments[es.pixelModule];
     const unsigned int plsBase = es.lsOffset[es.nLowerModules];
-    const unsigned int stride = gridDim.x * blockDim.x;
-    for (unsigned int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-      const unsigned int q = base + laneId();
-      bool pass = false;
-      unsigned int c = 0;
-      if (q < n) {
-        c = ev.candQueue[q < front ? q : kCandQueueCap - 1 - (q - front)];
-        unsigned int iPLS, obj;
-        uint16_t mod;
-        pixCandidate<K>(es, ev, c, iPLS, obj, mod);
-        const unsigned int t3 = K == 5 ? ev.t5.tripletIndices[2 * obj] : obj;
-        pass = pt3FirstTracklet(es.m, ev.rg, ev.md, ev.ls, ev.t3, plsBase + iPLS, t3);
+    const unsigned int lane = laneId();
+    const unsigned int nWarps = gridDim.x * (blockDim.x >> 5);
+    const unsigned int perTask = min(32u, max(1u, nPLS / (2u * nWarps)));
+    bool more = true;                  // the event may have tasks left
+    unsigned int task = 0, left = 0;   // the current task's first pLS and the lanes of those not yet grouped
+    unsigned int size = 0, index = 0;  // this lane's pLS of the task: its pixel-map slice
+    unsigned int f0 = 0, total = 0;    // the current group's candidates from f0 on
+    int nPairs = 0;                    //   and its pairs that have any
+    unsigned int fill[2] = {0, 0};
+    // the triplet (a quintuplet's inner one) that the opening tests take
+    auto tripletOf = [&](unsigned int obj) { return K == 5 ? ev.t5.tripletIndices[2 * obj] : obj; };
+    auto push = [&](int level, bool pass, unsigned int key, unsigned int obj) {
+      const unsigned int ok = __ballot_sync(kFullMask, pass);
+      if (pass) {
+        const unsigned int k = fill[level] + __popc(ok & lanesBelowMask());
+        sc.qKey[level][k] = key;
+        sc.qObj[level][k] = obj;
       }
-      const unsigned int mask = __ballot_sync(kFullMask, pass);
-      if (mask == 0u)
+      fill[level] += __popc(ok);
+      __syncwarp();
+    };
+    // up to 32 entries off the queue; false on the lanes without one
+    auto pop = [&](int level, unsigned int& key, unsigned int& obj) {
+      const unsigned int take = min(fill[level], 32u);
+      fill[level] -= take;
+      const bool have = lane < take;
+      if (have) {
+        key = sc.qKey[level][fill[level] + lane];
+        obj = sc.qObj[level][fill[level] + lane];
+      }
+      __syncwarp();  // the entries have been read
+      return have;
+    };
+    while (true) {
+      while (fill[1] < 32u) {
+        while (fill[0] < 32u) {
+          if (f0 < total) {
+            const unsigned int f = f0 + lane;
+            f0 += 32u;
+            bool pass = false;
+            unsigned int obj = 0, key = 0;
+            if (f < total) {
+              const int k = findSlot(sc.pre, nPairs, f);
+              const unsigned int iPLS = task + sc.owner[k], number = f - sc.first[sc.owner[k]];
+              obj = sc.obj[k] + (f - sc.pre[k]);
+              key = (iPLS << 16) | number;
+              if (number >= kPixKeyCandidates)
+                ev.sc->pixOverflow = 1;
+              else if (K == 5)
+                pass = !ev.t5.isDup[obj];
+              else
+                pass = es.m.moduleType[ev.t3.lowerModuleIndices[3 * obj + 1]] != TwoS && !ev.t3.partOfPT5[obj];
+              if (pass)
+                pass = pt3RadiusPass(es.m, ev.rg, ev.ls, ev.t3, plsBase + iPLS, tripletOf(obj));
+            }
+            push(0, pass, key, obj);
+          } else if (left != 0) {
+            // the next group: the pLS left, as long as their pairs fit
+            const unsigned int mine = (left >> lane) & 1u ? size : 0u;
+            const unsigned int incl = laneInclusiveSum(mine);
+            const unsigned int fits = __ballot_sync(kFullMask, mine != 0 && incl <= kPixPairs);
+            const unsigned int pairs = __shfl_sync(kFullMask, incl, 31 - __clz(fits));
+            left &= ~fits;
+            __syncwarp();  // the previous group's scratch has been read
+            nPairs = 0;
+            total = 0;
+            for (unsigned int p0 = 0; p0 < pairs; p0 += 32) {
+              const unsigned int p = p0 + lane;
+              const int o = laneOwner(incl, p);
+              const unsigned int k = p - (__shfl_sync(kFullMask, incl, o) - __shfl_sync(kFullMask, size, o));
+              const unsigned int slice = __shfl_sync(kFullMask, index, o);
+              unsigned int n = 0, obj = 0;
+              if (p < pairs) {
+                const uint16_t mod = static_cast<uint16_t>(es.m.connectedPixels[slice + k]);
+                n = pixModuleCount<K>(es, ev, mod);
+                if (n != 0)
+                  obj = static_cast<unsigned int>(K == 5 ? ev.rg.quintupletModuleIndices[mod]
+                                                         : ev.rg.tripletModuleIndices[mod]);
+              }
+              const unsigned int upTo = total + laneInclusiveSum(n);
+              const unsigned int has = __ballot_sync(kFullMask, n != 0);
+              if (p < pairs && k == 0)
+                sc.first[o] = upTo - n;
+              if (n != 0) {
+                const int e = nPairs + __popc(has & lanesBelowMask());
+                sc.pre[e] = upTo - n;
+                sc.obj[e] = obj;
+                sc.owner[e] = static_cast<uint8_t>(o);
+              }
+              nPairs += __popc(has);
+              total = __shfl_sync(kFullMask, upTo, 31);
+            }
+            __syncwarp();
+            f0 = 0;
+          } else if (more) {
+            task = warpNextTask(&ev.sc->pixNext) * perTask;
+            more = task < nPLS;
+            const unsigned int i = task + lane;
+            size = 0;
+            if (lane < perTask && i < nPLS && !pixSkipPLS<K>(ev, i))
+              pixelSlice(es, ev, i, size, index);
+            left = __ballot_sync(kFullMask, size != 0);
+          } else {
+            break;
+          }
+        }
+        if (fill[0] == 0)
+          break;
+        unsigned int key = 0, obj = 0;
+        bool pass = pop(0, key, obj);
+        if (pass)
+          pass = pt3FirstWindows(es.m, ev.rg, ev.md, ev.ls, ev.t3, plsBase + (key >> 16), tripletOf(obj));
+        push(1, pass, key, obj);
+      }
+      if (fill[1] == 0)
+        break;
+      unsigned int key = 0, obj = 0;
+      bool pass = pop(1, key, obj);
+      if (pass)
+        pass = pt3FirstBeta(es.m, ev.rg, ev.md, ev.ls, ev.t3, plsBase + (key >> 16), tripletOf(obj),
+                            ev.plsPhiP[key >> 16]);
+      const unsigned int ok = __ballot_sync(kFullMask, pass);
+      if (ok == 0u)
         continue;
       unsigned int start = 0;
-      if (laneId() == 0)
-        start = atomicAdd(&ev.sc->pixQueue2Count, __popc(mask));
+      if (lane == 0)
+        start = atomicAdd(&ev.sc->pixQueueCount, __popc(ok));
       start = __shfl_sync(kFullMask, start, 0);
-      const unsigned int k = start + __popc(mask & lanesBelowMask());
-      if (pass && k < room)
-        ev.candQueue[front + k] = c;
+      const unsigned int k = start + __popc(ok & lanesBelowMask());
+      if (pass && k < kCandQueueCap) {
+        ev.candQueue[k] = key;
+        ev.candQueueObj[k] = obj;
+      }
     }
   }
 
+  // The rest of the selection for the queued candidates.
   template <int K>
   __global__ void __launch_bounds__(LST_LB_EVAL) kPixEval(DeviceES es, const EventView* evs) {
     const EventView& ev = evs[blockIdx.y];
-    const unsigned int total = ev.sc->pixCandTotal;
-    const unsigned int front = ev.sc->pixQueueCount, back = ev.sc->pixQueueBack;
-    const bool fromQueue = front <= kCandQueueCap && back <= kCandQueueCap - front;
-    const unsigned int n2 = ev.sc->pixQueue2Count;
-    const bool fromQueue2 = fromQueue && n2 <= kCandQueueCap - front - back;
-    const unsigned int n = fromQueue2 ? n2 : (fromQueue ? front + back : total);
+    const unsigned int n = ev.sc->pixQueueCount;
+    if (n > kCandQueueCap)
+      return;  // the event takes the walk (kPixRankEmit)
     const unsigned int plsBase = es.lsOffset[es.nLowerModules];
     for (unsigned int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-      const unsigned int c = fromQueue2  ? ev.candQueue[front + q]
-                             : fromQueue ? ev.candQueue[q < front ? q : kCandQueueCap - 1 - (q - front)]
-                                         : q;
-      unsigned int iPLS, obj;
-      uint16_t mod;
-      pixCandidate<K>(es, ev, c, iPLS, obj, mod);
+      const unsigned int c = ev.candQueue[q], iPLS = c >> 16, obj = ev.candQueueObj[q];
       float vals[8];
       bool ok;
       if (K == 5) {
         PT5Values v;
-        ok = !ev.t5.isDup[obj] && pt5Select(es.m, ev.rg, ev.md, ev.ls, ev.t3, ev.t5, plsBase + iPLS, obj, iPLS, v);
+        ok = pt5Select(es.m, ev.rg, ev.md, ev.ls, ev.t3, ev.t5, plsBase + iPLS, obj, iPLS, v, true);
         vals[0] = v.rzChiSquared;
         vals[1] = v.rPhiChiSquared;
         vals[2] = v.rPhiChiSquaredInwards;
@@ -2666,8 +2648,7 @@ namespace lst {
         vals[7] = 0.f;
       } else {
         PT3Values v;
-        ok = es.m.moduleType[ev.t3.lowerModuleIndices[3 * obj + 1]] != TwoS && !ev.t3.partOfPT5[obj] &&
-             pt3Select(es.m, ev.rg, ev.md, ev.ls, ev.t3, plsBase + iPLS, obj, true, v);
+        ok = pt3Select(es.m, ev.rg, ev.md, ev.ls, ev.t3, plsBase + iPLS, obj, true, v, true);
         vals[0] = v.pixelRadius;
         vals[1] = v.pixelRadiusError;
         vals[2] = v.tripletRadius;
@@ -2682,7 +2663,6 @@ namespace lst {
         if (slot < kPixPassCap) {
           ev.pixPassC[slot] = c;
           ev.pixPassObj[slot] = obj;
-          ev.pixPassPLS[slot] = iPLS;
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             ev.pixPassV[8 * slot + k] = vals[k];
@@ -2691,14 +2671,14 @@ namespace lst {
     }
   }
 
-  // Ranks the passing candidates by c and stores them; one block per event.
+  // Ranks the passing candidates by key and stores them; one block per event.
   template <int K>
   __global__ void __launch_bounds__(1024) kPixRankEmit(DeviceES es, const EventView* evs) {
     __shared__ unsigned int sKey[kPixPassCap];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.sc->pixPassCount;
     const unsigned int capOut = K == 5 ? kMaxPixelQuintuplets : kMaxPixelTriplets;
-    if (n > kPixPassCap || ev.forceWalk) {
+    if (n > kPixPassCap || ev.sc->pixQueueCount > kCandQueueCap || ev.sc->pixOverflow || ev.forceWalk) {
       if (threadIdx.x == 0)
         ev.sc->pixFallback = 1;
       return;
@@ -2718,7 +2698,7 @@ namespace lst {
       if (rank >= capOut)
         continue;
       const unsigned int obj = ev.pixPassObj[sIdx];
-      const unsigned int iPLS = ev.pixPassPLS[sIdx];
+      const unsigned int iPLS = key >> 16;
       const float* vals = ev.pixPassV + 8 * sIdx;
       if (K == 5) {
         PT5Values v;

@@ -12,302 +12,236 @@ namespace lst {
     return m.layers[i] + 6 * (m.subdets[i] == Endcap) + 5 * (m.subdets[i] == Endcap and m.moduleType[i] == TwoS);
   }
 
-  // Pixel segment against a pair of outer-tracker mini-doublets, barrel outer
-  // modules (SDL/PixelTriplet.h:1264-1553).
-  LST_HD_BIG bool ptPPBB(const Modules& m,
-                     const Ranges& rg,
-                     const MiniDoublets& md,
-                     const Segments& s,
-                     uint16_t pixelModule,
-                     uint16_t lmOI,
-                     uint16_t lmOO,
-                     unsigned int innerSeg,
-                     unsigned int outerSeg,
-                     unsigned int md1,
-                     unsigned int md2,
-                     unsigned int md3,
-                     unsigned int md4) {
-    bool isPS_OutLo = (m.moduleType[lmOI] == PS);
-    float rt_InLo = md.anchorPos[md1].rt, rt_InUp = md.anchorPos[md2].rt, rt_OutLo = md.anchorPos[md3].rt, rt_OutUp = md.anchorPos[md4].rt;
-    float z_InUp = md.anchorPos[md2].z, z_OutLo = md.anchorPos[md3].z;
-    float x_InLo = md.anchorPos[md1].x, x_InUp = md.anchorPos[md2].x, x_OutLo = md.anchorPos[md3].x, x_OutUp = md.anchorPos[md4].x;
-    float y_InLo = md.anchorPos[md1].y, y_InUp = md.anchorPos[md2].y, y_OutLo = md.anchorPos[md3].y, y_OutUp = md.anchorPos[md4].y;
-    float rt_InOut = rt_InUp;
-    // deltaPhi of two anchor hits, from their stored phi (hits.phis is phi()
-    // of the same coordinates, so the value is identical)
-    if (!(fabs_(phiMpiPi(md.anchorPhi[md3] - md.anchorPhi[md2])) <= 0.5f * float(M_PI)))
-      return false;
+  // Pixel segment against a pair of outer-tracker mini-doublets: inner module of
+  // the pair in the barrel (SDL/PixelTriplet.h:1264-1553) or both in the endcap
+  // (:1555-1862).  The two algorithms differ in their opening windows (z against
+  // r) and are the same from the dPhi cut on, so they share one body: half the
+  // code, and warps with both kinds of candidates run the long part together.
+  struct PtTracklet {
+    bool endcap;
+    uint16_t lmOI, lmOO;  // the pair's modules
+    unsigned int pls;     // the pixel segment's number
+    unsigned int innerSeg, outerSeg;
+    unsigned int md1, md2, md3, md4;
+  };
 
-    unsigned int pls = innerSeg - rg.segmentModuleIndices[pixelModule];
+  // The pair and its kind (SDL/PixelTriplet.h:206-314); false for a pair that
+  // neither algorithm takes.
+  LST_HD bool ptSetup(const Modules& m, const Ranges& rg, const Segments& s, uint16_t pixelModule, uint16_t lmOI,
+                      uint16_t lmOO, unsigned int innerSeg, unsigned int outerSeg, PtTracklet& q) {
+    const short sOI = m.subdets[lmOI], sOO = m.subdets[lmOO];
+    q.endcap = sOI == Endcap and sOO == Endcap;
+    q.lmOI = lmOI;
+    q.lmOO = lmOO;
+    q.pls = innerSeg - rg.segmentModuleIndices[pixelModule];
+    q.innerSeg = innerSeg;
+    q.outerSeg = outerSeg;
+    q.md1 = s.mdIndices[2 * innerSeg];
+    q.md2 = s.mdIndices[2 * innerSeg + 1];
+    q.md3 = s.mdIndices[2 * outerSeg];
+    q.md4 = s.mdIndices[2 * outerSeg + 1];
+    return q.endcap or (sOI == Barrel and (sOO == Barrel or sOO == Endcap));
+  }
+
+  LST_HD float ptThetaMuls(float rt_InUp, float z_InUp, float rt_OutLo) {
+    const float r3_InUp = fsqrt(z_InUp * z_InUp + rt_InUp * rt_InUp);
+    return 0.015f * fsqrt(0.1f + 0.2f * (rt_OutLo - rt_InUp) / 50.f) * fsqrt(r3_InUp / rt_InUp);
+  }
+
+  // The opening windows.
+  LST_HD_BIG bool ptWindows(const Modules& m, const MiniDoublets& md, const Segments& s, const PtTracklet& q) {
+    const bool endcap = q.endcap;
+    const unsigned int pls = q.pls;
+    const MDRec& rec1 = md.rec[q.md1];
+    const MDRec& rec2 = md.rec[q.md2];
+    const MDRec& rec3 = md.rec[q.md3];
+    bool isPS_OutLo = (m.moduleType[q.lmOI] == PS);
+    float z_InUp = rec2.z, z_OutLo = rec3.z;
+    if (endcap) {
+      if (!(z_InUp * z_OutLo > 0))
+        return false;
+    } else {
+      // deltaPhi of two anchor hits, from their stored phi (hits.phis is phi()
+      // of the same coordinates, so the value is identical)
+      if (!(fabs_(phiMpiPi(rec3.phi - rec2.phi)) <= 0.5f * float(M_PI)))
+        return false;
+    }
+    float rt_InLo = rec1.rt, rt_InUp = rec2.rt, rt_OutLo = rec3.rt;
     float ptIn = s.ptIn[pls];
-    float px = s.px[pls], py = s.py[pls], pz = s.pz[pls];
+    float pz = s.pz[pls];
     float etaErr = s.etaErr[pls];
 
-    float alpha1GeV_OutLo = md.slope[md3];
-    const float rtRatio_OutLoInOut = rt_OutLo / rt_InOut;
-    float dzDrtScale = md.tanSlope[md3] / alpha1GeV_OutLo;
+    float alpha1GeV_OutLo = rec3.slope;
+    const float dzDrtScale = rec3.tanSlope / alpha1GeV_OutLo;
     const float zpitch_InLo = 0.05f;
     const float zpitch_InOut = 0.05f;
     float zpitch_OutLo = (isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch);
     float zGeom = zpitch_InLo + zpitch_OutLo;
-    float zHi = z_InUp + (z_InUp + kDeltaZLum) * (rtRatio_OutLoInOut - 1.f) * (z_InUp < 0.f ? 1.f : dzDrtScale) +
-                (zpitch_InOut + zpitch_OutLo);
-    float zLo = z_InUp + (z_InUp - kDeltaZLum) * (rtRatio_OutLoInOut - 1.f) * (z_InUp > 0.f ? 1.f : dzDrtScale) -
-                (zpitch_InOut + zpitch_OutLo);
-    if (!((z_OutLo >= zLo) && (z_OutLo <= zHi)))
-      return false;
+    const float rtGeom1 = isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch;
+    if (endcap) {
+      const float dLum = signTransfer(kDeltaZLum, z_InUp);
+      const float zGeom1 = signTransfer(zGeom, z_InUp);
+      float rtLo = rt_InUp * (1.f + (z_OutLo - z_InUp - zGeom1) / (z_InUp + zGeom1 + dLum) / dzDrtScale) - rtGeom1;
+      float zInForHi = z_InUp - zGeom1 - dLum;
+      if (zInForHi * z_InUp < 0)
+        zInForHi = signTransfer(0.1f, z_InUp);
+      float rtHi = rt_InUp * (1.f + (z_OutLo - z_InUp + zGeom1) / zInForHi) + rtGeom1;
+      if (!((rt_OutLo >= rtLo) && (rt_OutLo <= rtHi)))
+        return false;
+    } else {
+      const float rtRatio_OutLoInOut = rt_OutLo / rt_InUp;
+      float zHi = z_InUp + (z_InUp + kDeltaZLum) * (rtRatio_OutLoInOut - 1.f) * (z_InUp < 0.f ? 1.f : dzDrtScale) +
+                  (zpitch_InOut + zpitch_OutLo);
+      float zLo = z_InUp + (z_InUp - kDeltaZLum) * (rtRatio_OutLoInOut - 1.f) * (z_InUp > 0.f ? 1.f : dzDrtScale) -
+                  (zpitch_InOut + zpitch_OutLo);
+      if (!((z_OutLo >= zLo) && (z_OutLo <= zHi)))
+        return false;
+    }
 
     const float coshEta = fsqrt(ptIn * ptIn + pz * pz) / ptIn;
     const float drt_OutLo_InUp = (rt_OutLo - rt_InUp);
-    const float r3_InUp = fsqrt(z_InUp * z_InUp + rt_InUp * rt_InUp);
-    float drt_InSeg = rt_InOut - rt_InLo;
-    const float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rt_OutLo - rt_InUp) / 50.f) * fsqrt(r3_InUp / rt_InUp);
-    const float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    float dzErr = drt_OutLo_InUp * etaErr * coshEta;
-    dzErr *= dzErr;
-    dzErr += 0.03f * 0.03f;
-    dzErr *= 9.f;
-    dzErr += sdlMuls * sdlMuls * drt_OutLo_InUp * drt_OutLo_InUp / 3.f * coshEta * coshEta;
-    dzErr += zGeom * zGeom;
-    dzErr = fsqrt(dzErr);
-    const float dzDrIn = pz / ptIn;
-    const float zWindow = dzErr / drt_InSeg * drt_OutLo_InUp + zGeom;
-    const float dzMean =
-        dzDrIn * drt_OutLo_InUp *
-        (1.f + drt_OutLo_InUp * drt_OutLo_InUp * 4 * k2Rinv1GeVf * k2Rinv1GeVf / ptIn / ptIn / 24.f);
-    float zLoPointed = z_InUp + dzMean - zWindow;
-    float zHiPointed = z_InUp + dzMean + zWindow;
-    if (!((z_OutLo >= zLoPointed) && (z_OutLo <= zHiPointed)))
-      return false;
-
-    const float sdlPVoff = 0.1f / rt_OutLo;
-    float sdlCut = alpha1GeV_OutLo + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
-    float midPointX = 0.5f * (x_InLo + x_OutLo);
-    float midPointY = 0.5f * (y_InLo + y_OutLo);
-    float diffX = x_OutLo - x_InLo;
-    float diffY = y_OutLo - y_InLo;
-    float dPhi = deltaPhi(midPointX, midPointY, diffX, diffY);
-    if (!(fabs_(dPhi) <= sdlCut))
-      return false;
-
-    float alpha_InLo = s.dPhiChanges[innerSeg];
-    float alpha_OutLo = s.dPhiChanges[outerSeg];
-    bool isEC_lastLayer = m.subdets[lmOO] == Endcap and m.moduleType[lmOO] == TwoS;
-    float alpha_OutUp = phiMpiPi(phiOf(x_OutUp - x_OutLo, y_OutUp - y_OutLo) - md.anchorPhi[md4]);
-    float tl_axis_x = x_OutUp - x_InUp;
-    float tl_axis_y = y_OutUp - y_InUp;
-    const float phiTlAxis = phiOf(tl_axis_x, tl_axis_y);
-    float betaIn = -phiMpiPi(phiTlAxis - phiOf(px, py));
-    float betaInRHmin = betaIn;
-    float betaInRHmax = betaIn;
-    float betaOut = -alpha_OutUp + phiMpiPi(phiTlAxis - md.anchorPhi[md4]);
-    float betaOutRHmin = betaOut;
-    float betaOutRHmax = betaOut;
-    if (isEC_lastLayer) {
-      float hx = md.anchorHighEdgeX[md4], hy = md.anchorHighEdgeY[md4];
-      float lx = md.anchorLowEdgeX[md4], ly = md.anchorLowEdgeY[md4];
-      float alpha_OutUp_highEdge = deltaPhi(hx, hy, hx - x_OutLo, hy - y_OutLo);
-      float alpha_OutUp_lowEdge = deltaPhi(lx, ly, lx - x_OutLo, ly - y_OutLo);
-      float tl_axis_highEdge_x = hx - x_InUp;
-      float tl_axis_highEdge_y = hy - y_InUp;
-      float tl_axis_lowEdge_x = lx - x_InUp;
-      float tl_axis_lowEdge_y = ly - y_InUp;
-      betaOutRHmin = -alpha_OutUp_highEdge + deltaPhi(hx, hy, tl_axis_highEdge_x, tl_axis_highEdge_y);
-      betaOutRHmax = -alpha_OutUp_lowEdge + deltaPhi(lx, ly, tl_axis_lowEdge_x, tl_axis_lowEdge_y);
+    const float sdlMuls = ptThetaMuls(rt_InUp, z_InUp, rt_OutLo) * 3.f / m.ptCut * 4.f;
+    if (endcap) {
+      const float dzOutInAbs = fabs_(z_OutLo - z_InUp);
+      const float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
+      float drtErr = etaErr * multDzDr;
+      drtErr *= drtErr;
+      drtErr += 0.03f * 0.03f;
+      drtErr *= 9.f;
+      drtErr += sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta;
+      drtErr = fsqrt(drtErr);
+      const float drtDzIn = fabs_(ptIn / pz);
+      const float rtWindow = drtErr + rtGeom1;
+      const float drtMean =
+          drtDzIn * dzOutInAbs *
+          (1.f - drt_OutLo_InUp * drt_OutLo_InUp * 4 * k2Rinv1GeVf * k2Rinv1GeVf / ptIn / ptIn / 24.f);
+      const float rtLo_point = rt_InUp + drtMean - rtWindow;
+      const float rtHi_point = rt_InUp + drtMean + rtWindow;
+      if (!((rt_OutLo >= rtLo_point) && (rt_OutLo <= rtHi_point)))
+        return false;
+    } else {
+      float dzErr = drt_OutLo_InUp * etaErr * coshEta;
+      dzErr *= dzErr;
+      dzErr += 0.03f * 0.03f;
+      dzErr *= 9.f;
+      dzErr += sdlMuls * sdlMuls * drt_OutLo_InUp * drt_OutLo_InUp / 3.f * coshEta * coshEta;
+      dzErr += zGeom * zGeom;
+      dzErr = fsqrt(dzErr);
+      const float dzDrIn = pz / ptIn;
+      float drt_InSeg = rt_InUp - rt_InLo;
+      const float zWindow = dzErr / drt_InSeg * drt_OutLo_InUp + zGeom;
+      const float dzMean =
+          dzDrIn * drt_OutLo_InUp *
+          (1.f + drt_OutLo_InUp * drt_OutLo_InUp * 4 * k2Rinv1GeVf * k2Rinv1GeVf / ptIn / ptIn / 24.f);
+      float zLoPointed = z_InUp + dzMean - zWindow;
+      float zHiPointed = z_InUp + dzMean + zWindow;
+      if (!((z_OutLo >= zLoPointed) && (z_OutLo <= zHiPointed)))
+        return false;
     }
 
-    float drt_tl_axis = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    const float rt_InSeg = fsqrt((x_InUp - x_InLo) * (x_InUp - x_InLo) + (y_InUp - y_InLo) * (y_InUp - y_InLo));
-    float betaAv = 0.5f * (betaIn + betaOut);
-    float pt_beta = ptIn;
-    int lIn = 0;
-    int lOut = isEC_lastLayer ? 11 : 5;
-    float sdOut_dr = fsqrt((x_OutUp - x_OutLo) * (x_OutUp - x_OutLo) + (y_OutUp - y_OutLo) * (y_OutUp - y_OutLo));
-    float sdOut_d = rt_OutUp - rt_OutLo;
-    deltaBetaIterations(betaIn, betaOut, betaAv, pt_beta, rt_InSeg, sdOut_dr, drt_tl_axis, lIn);
-
-    const float betaInMMSF =
-        (fabs_(betaInRHmin + betaInRHmax) > 0) ? (2.f * betaIn / fabs_(betaInRHmin + betaInRHmax)) : 0.f;
-    const float betaOutMMSF =
-        (fabs_(betaOutRHmin + betaOutRHmax) > 0) ? (2.f * betaOut / fabs_(betaOutRHmin + betaOutRHmax)) : 0.f;
-    betaInRHmin *= betaInMMSF;
-    betaInRHmax *= betaInMMSF;
-    betaOutRHmin *= betaOutMMSF;
-    betaOutRHmax *= betaOutMMSF;
-
-    const float dBetaMuls = sdlThetaMulsF * 4.f / fmin_(fabs_(pt_beta), kPtBetaMax);
-    const float alphaInAbsReg = fmax_(fabs_(alpha_InLo), md.slope3[md2]);
-    const float alphaOutAbsReg = fmax_(fabs_(alpha_OutLo), md.slope3[md3]);
-    const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InUp);
-    const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
-    const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);
-    const float sinDPhi = fsin(dPhi);
-    const float dBetaRIn2 = 0;
-    float dBetaROut = 0;
-    if (isEC_lastLayer) {
-      dBetaROut = (fsqrt(md.anchorHighEdgeX[md4] * md.anchorHighEdgeX[md4] + md.anchorHighEdgeY[md4] * md.anchorHighEdgeY[md4]) -
-                   fsqrt(md.anchorLowEdgeX[md4] * md.anchorLowEdgeX[md4] + md.anchorLowEdgeY[md4] * md.anchorLowEdgeY[md4])) *
-                  sinDPhi / drt_tl_axis;
-    }
-    const float dBetaROut2 = dBetaROut * dBetaROut;
-    float betaOutCut = fasin(fmin_(drt_tl_axis * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdOut_d) +
-                       fsqrt(dBetaLum2 + dBetaMuls * dBetaMuls);
-    if (!(fabs_(betaOut) < betaOutCut))
-      return false;
-    const float dBetaRes = 0.02f / fmin_(sdOut_d, drt_InSeg);
-    return betaDifferenceCut(betaIn, betaOut, betaInRHmin, betaInRHmax, betaOutRHmin, betaOutRHmax, dBetaRes, dBetaMuls,
-                             dBetaLum2, dBetaRIn2, dBetaROut2);
+    return true;
   }
 
-  // Pixel segment against an endcap pair (SDL/PixelTriplet.h:1555-1862).
-  LST_HD_BIG bool ptPPEE(const Modules& m,
-                     const Ranges& rg,
-                     const MiniDoublets& md,
-                     const Segments& s,
-                     uint16_t pixelModule,
-                     uint16_t lmOI,
-                     uint16_t lmOO,
-                     unsigned int innerSeg,
-                     unsigned int outerSeg,
-                     unsigned int md1,
-                     unsigned int md2,
-                     unsigned int md3,
-                     unsigned int md4) {
-    bool isPS_OutLo = (m.moduleType[lmOI] == PS);
-    float z_InUp = md.anchorPos[md2].z;
-    float z_OutLo = md.anchorPos[md3].z;
-    if (!(z_InUp * z_OutLo > 0))
-      return false;
-    float rt_InLo = md.anchorPos[md1].rt, rt_InUp = md.anchorPos[md2].rt, rt_OutLo = md.anchorPos[md3].rt, rt_OutUp = md.anchorPos[md4].rt;
-    float x_InLo = md.anchorPos[md1].x, x_InUp = md.anchorPos[md2].x, x_OutLo = md.anchorPos[md3].x, x_OutUp = md.anchorPos[md4].x;
-    float y_InLo = md.anchorPos[md1].y, y_InUp = md.anchorPos[md2].y, y_OutLo = md.anchorPos[md3].y, y_OutUp = md.anchorPos[md4].y;
-    unsigned int pls = innerSeg - rg.segmentModuleIndices[pixelModule];
-    float ptIn = s.ptIn[pls];
-    float px = s.px[pls], py = s.py[pls], pz = s.pz[pls];
-    float etaErr = s.etaErr[pls];
-
-    const float zpitch_InLo = 0.05f;
-    float zpitch_OutLo = (isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch);
-    float zGeom = zpitch_InLo + zpitch_OutLo;
-    const float sdlSlope = md.slope[md3];
-    const float dzDrtScale = md.tanSlope[md3] / sdlSlope;
-    const float dLum = signTransfer(kDeltaZLum, z_InUp);
-    bool isOutSgInnerMDPS = m.moduleType[lmOI] == PS;
-    const float rtGeom1 = isOutSgInnerMDPS ? kPixelPSZpitch : kStrip2SZpitch;
-    const float zGeom1 = signTransfer(zGeom, z_InUp);
-    float rtLo = rt_InUp * (1.f + (z_OutLo - z_InUp - zGeom1) / (z_InUp + zGeom1 + dLum) / dzDrtScale) - rtGeom1;
-    float zInForHi = z_InUp - zGeom1 - dLum;
-    if (zInForHi * z_InUp < 0)
-      zInForHi = signTransfer(0.1f, z_InUp);
-    float rtHi = rt_InUp * (1.f + (z_OutLo - z_InUp + zGeom1) / zInForHi) + rtGeom1;
-    if (!((rt_OutLo >= rtLo) && (rt_OutLo <= rtHi)))
-      return false;
-
-    const float dzOutInAbs = fabs_(z_OutLo - z_InUp);
-    const float coshEta = fsqrt(ptIn * ptIn + pz * pz) / ptIn;
-    const float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
-    const float r3_InUp = fsqrt(z_InUp * z_InUp + rt_InUp * rt_InUp);
-    const float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rt_OutLo - rt_InUp) / 50.f) * fsqrt(r3_InUp / rt_InUp);
-    const float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    float drtErr = etaErr * multDzDr;
-    drtErr *= drtErr;
-    drtErr += 0.03f * 0.03f;
-    drtErr *= 9.f;
-    drtErr += sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta;
-    drtErr = fsqrt(drtErr);
-    const float drtDzIn = fabs_(ptIn / pz);
-    const float drt_OutLo_InUp = (rt_OutLo - rt_InUp);
-    const float rtWindow = drtErr + rtGeom1;
-    const float drtMean =
-        drtDzIn * dzOutInAbs *
-        (1.f - drt_OutLo_InUp * drt_OutLo_InUp * 4 * k2Rinv1GeVf * k2Rinv1GeVf / ptIn / ptIn / 24.f);
-    const float rtLo_point = rt_InUp + drtMean - rtWindow;
-    const float rtHi_point = rt_InUp + drtMean + rtWindow;
-    if (!((rt_OutLo >= rtLo_point) && (rt_OutLo <= rtHi_point)))
-      return false;
-
-    const float alpha1GeV_OutLo = md.slope[md3];
-    const float sdlPVoff = 0.1f / rt_OutLo;
-    float sdlCut = alpha1GeV_OutLo + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
-    float midPointX = 0.5f * (x_InLo + x_OutLo);
-    float midPointY = 0.5f * (y_InLo + y_OutLo);
-    float diffX = x_OutLo - x_InLo;
-    float diffY = y_OutLo - y_InLo;
-    float dPhi = deltaPhi(midPointX, midPointY, diffX, diffY);
-    if (!(fabs_(dPhi) <= sdlCut))
-      return false;
-
-    float alpha_InLo = s.dPhiChanges[innerSeg];
-    float alpha_OutLo = s.dPhiChanges[outerSeg];
-    bool isEC_lastLayer = m.subdets[lmOO] == Endcap and m.moduleType[lmOO] == TwoS;
-    float alpha_OutUp = phiMpiPi(phiOf(x_OutUp - x_OutLo, y_OutUp - y_OutLo) - md.anchorPhi[md4]);
-    float tl_axis_x = x_OutUp - x_InUp;
-    float tl_axis_y = y_OutUp - y_InUp;
-    const float phiTlAxis = phiOf(tl_axis_x, tl_axis_y);
-    float betaIn = -phiMpiPi(phiTlAxis - phiOf(px, py));
-    float betaInRHmin = betaIn;
-    float betaInRHmax = betaIn;
-    float betaOut = -alpha_OutUp + phiMpiPi(phiTlAxis - md.anchorPhi[md4]);
-    float betaOutRHmin = betaOut;
-    float betaOutRHmax = betaOut;
-    if (isEC_lastLayer) {
-      float hx = md.anchorHighEdgeX[md4], hy = md.anchorHighEdgeY[md4];
-      float lx = md.anchorLowEdgeX[md4], ly = md.anchorLowEdgeY[md4];
-      float alpha_OutUp_highEdge = deltaPhi(hx, hy, hx - x_OutLo, hy - y_OutLo);
-      float alpha_OutUp_lowEdge = deltaPhi(lx, ly, lx - x_OutLo, ly - y_OutLo);
-      float tl_axis_highEdge_x = hx - x_InUp;
-      float tl_axis_highEdge_y = hy - y_InUp;
-      float tl_axis_lowEdge_x = lx - x_InUp;
-      float tl_axis_lowEdge_y = ly - y_InUp;
-      betaOutRHmin = -alpha_OutUp_highEdge + deltaPhi(hx, hy, tl_axis_highEdge_x, tl_axis_highEdge_y);
-      betaOutRHmax = -alpha_OutUp_lowEdge + deltaPhi(lx, ly, tl_axis_lowEdge_x, tl_axis_lowEdge_y);
-    }
-
-    float drt_tl_axis = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    const float rt_InSeg = fsqrt((x_InUp - x_InLo) * (x_InUp - x_InLo) + (y_InUp - y_InLo) * (y_InUp - y_InLo));
-    float betaAv = 0.5f * (betaIn + betaOut);
-    float pt_beta = ptIn;
-    int lIn = 0;
-    int lOut = isEC_lastLayer ? 11 : 5;
-    float sdOut_dr = fsqrt((x_OutUp - x_OutLo) * (x_OutUp - x_OutLo) + (y_OutUp - y_OutLo) * (y_OutUp - y_OutLo));
-    float sdOut_d = rt_OutUp - rt_OutLo;
-    deltaBetaIterations(betaIn, betaOut, betaAv, pt_beta, rt_InSeg, sdOut_dr, drt_tl_axis, lIn);
-
-    const float betaInMMSF =
-        (fabs_(betaInRHmin + betaInRHmax) > 0) ? (2.f * betaIn / fabs_(betaInRHmin + betaInRHmax)) : 0.f;
-    const float betaOutMMSF =
-        (fabs_(betaOutRHmin + betaOutRHmax) > 0) ? (2.f * betaOut / fabs_(betaOutRHmin + betaOutRHmax)) : 0.f;
-    betaInRHmin *= betaInMMSF;
-    betaInRHmax *= betaInMMSF;
-    betaOutRHmin *= betaOutMMSF;
-    betaOutRHmax *= betaOutMMSF;
-
-    const float dBetaMuls = sdlThetaMulsF * 4.f / fmin_(fabs_(pt_beta), kPtBetaMax);
-    const float alphaInAbsReg = fmax_(fabs_(alpha_InLo), md.slope3[md2]);
-    const float alphaOutAbsReg = fmax_(fabs_(alpha_OutLo), md.slope3[md3]);
-    const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InUp);
-    const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
-    const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);
-    const float sinDPhi = fsin(dPhi);
-    const float dBetaRIn2 = 0;
-    float dBetaROut = 0;
-    if (isEC_lastLayer) {
-      dBetaROut = (fsqrt(md.anchorHighEdgeX[md4] * md.anchorHighEdgeX[md4] + md.anchorHighEdgeY[md4] * md.anchorHighEdgeY[md4]) -
-                   fsqrt(md.anchorLowEdgeX[md4] * md.anchorLowEdgeX[md4] + md.anchorLowEdgeY[md4] * md.anchorLowEdgeY[md4])) *
-                  sinDPhi / drt_tl_axis;
-    }
-    const float dBetaROut2 = dBetaROut * dBetaROut;
-    float betaOutCut = fasin(fmin_(drt_tl_axis * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdOut_d) +
-                       fsqrt(dBetaLum2 + dBetaMuls * dBetaMuls);
-    if (!(fabs_(betaOut) < betaOutCut))
-      return false;
+  // The cuts after the windows.  phiP: phi of the pixel segment's momentum.
+  // Every test is a pure function of the pair and all must pass, so they run in
+  // the order that rejects soonest: the beta difference leaves a tenth of the
+  // pairs that get here (PU200), the dPhi and betaOut cuts, which the reference
+  // tests before it and which hardly ever reject, come after it.
+  LST_HD_BIG bool ptBeta(const Modules& m, const MiniDoublets& md, const Segments& s, const PtTracklet& q, float phiP) {
+    const uint16_t lmOO = q.lmOO;
+    const unsigned int innerSeg = q.innerSeg, outerSeg = q.outerSeg, md2 = q.md2, md3 = q.md3, md4 = q.md4;
+    const MDRec& rec1 = md.rec[q.md1];
+    const MDRec& rec2 = md.rec[md2];
+    const MDRec& rec3 = md.rec[md3];
+    const MDRec& rec4 = md.rec[md4];
+    float rt_InLo = rec1.rt, rt_InUp = rec2.rt, rt_OutLo = rec3.rt;
+    float z_InUp = rec2.z, z_OutLo = rec3.z;
+    float ptIn = s.ptIn[q.pls];
+    const float sdlThetaMulsF = ptThetaMuls(rt_InUp, z_InUp, rt_OutLo);
     float drt_InSeg = rt_InUp - rt_InLo;
+    float x_InLo = rec1.x, x_InUp = rec2.x, x_OutLo = rec3.x, x_OutUp = rec4.x;
+    float y_InLo = rec1.y, y_InUp = rec2.y, y_OutLo = rec3.y, y_OutUp = rec4.y;
+    float alpha_InLo = s.dPhiChanges[innerSeg];
+    float alpha_OutLo = s.dPhiChanges[outerSeg];
+    bool isEC_lastLayer = m.subdets[lmOO] == Endcap and m.moduleType[lmOO] == TwoS;
+    float alpha_OutUp = phiMpiPi(phiOf(x_OutUp - x_OutLo, y_OutUp - y_OutLo) - rec4.phi);
+    float tl_axis_x = x_OutUp - x_InUp;
+    float tl_axis_y = y_OutUp - y_InUp;
+    const float phiTlAxis = phiOf(tl_axis_x, tl_axis_y);
+    float betaIn = -phiMpiPi(phiTlAxis - phiP);
+    float betaInRHmin = betaIn;
+    float betaInRHmax = betaIn;
+    float betaOut = -alpha_OutUp + phiMpiPi(phiTlAxis - rec4.phi);
+    float betaOutRHmin = betaOut;
+    float betaOutRHmax = betaOut;
+    if (isEC_lastLayer) {
+      float hx = md.anchorHighEdgeX[md4], hy = md.anchorHighEdgeY[md4];
+      float lx = md.anchorLowEdgeX[md4], ly = md.anchorLowEdgeY[md4];
+      float alpha_OutUp_highEdge = deltaPhi(hx, hy, hx - x_OutLo, hy - y_OutLo);
+      float alpha_OutUp_lowEdge = deltaPhi(lx, ly, lx - x_OutLo, ly - y_OutLo);
+      float tl_axis_highEdge_x = hx - x_InUp;
+      float tl_axis_highEdge_y = hy - y_InUp;
+      float tl_axis_lowEdge_x = lx - x_InUp;
+      float tl_axis_lowEdge_y = ly - y_InUp;
+      betaOutRHmin = -alpha_OutUp_highEdge + deltaPhi(hx, hy, tl_axis_highEdge_x, tl_axis_highEdge_y);
+      betaOutRHmax = -alpha_OutUp_lowEdge + deltaPhi(lx, ly, tl_axis_lowEdge_x, tl_axis_lowEdge_y);
+    }
+
+    float drt_tl_axis = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
+    const float rt_InSeg = fsqrt((x_InUp - x_InLo) * (x_InUp - x_InLo) + (y_InUp - y_InLo) * (y_InUp - y_InLo));
+    float betaAv = 0.5f * (betaIn + betaOut);
+    float pt_beta = ptIn;
+    int lIn = 0;
+    int lOut = isEC_lastLayer ? 11 : 5;
+    float sdOut_dr = fsqrt((x_OutUp - x_OutLo) * (x_OutUp - x_OutLo) + (y_OutUp - y_OutLo) * (y_OutUp - y_OutLo));
+    float sdOut_d = rec4.rt - rt_OutLo;
+    deltaBetaIterations(betaIn, betaOut, betaAv, pt_beta, rt_InSeg, sdOut_dr, drt_tl_axis, lIn);
+
+    const float betaInMMSF =
+        (fabs_(betaInRHmin + betaInRHmax) > 0) ? (2.f * betaIn / fabs_(betaInRHmin + betaInRHmax)) : 0.f;
+    const float betaOutMMSF =
+        (fabs_(betaOutRHmin + betaOutRHmax) > 0) ? (2.f * betaOut / fabs_(betaOutRHmin + betaOutRHmax)) : 0.f;
+    betaInRHmin *= betaInMMSF;
+    betaInRHmax *= betaInMMSF;
+    betaOutRHmin *= betaOutMMSF;
+    betaOutRHmax *= betaOutMMSF;
+
+    const float dBetaMuls = sdlThetaMulsF * 4.f / fmin_(fabs_(pt_beta), kPtBetaMax);
+    const float alphaInAbsReg = fmax_(fabs_(alpha_InLo), md.slope3[md2]);
+    const float alphaOutAbsReg = fmax_(fabs_(alpha_OutLo), md.slope3[md3]);
+    const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InUp);
+    const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
+    const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);
+    const float dBetaRIn2 = 0;
+    float dBetaROut = 0;
+    auto midPointDPhi = [&]() {
+      return deltaPhi(0.5f * (x_InLo + x_OutLo), 0.5f * (y_InLo + y_OutLo), x_OutLo - x_InLo, y_OutLo - y_InLo);
+    };
+    float dPhi = 0;
+    if (isEC_lastLayer) {
+      dPhi = midPointDPhi();
+      const float sinDPhi = fsin(dPhi);
+      dBetaROut = (fsqrt(md.anchorHighEdgeX[md4] * md.anchorHighEdgeX[md4] + md.anchorHighEdgeY[md4] * md.anchorHighEdgeY[md4]) -
+                   fsqrt(md.anchorLowEdgeX[md4] * md.anchorLowEdgeX[md4] + md.anchorLowEdgeY[md4] * md.anchorLowEdgeY[md4])) *
+                  sinDPhi / drt_tl_axis;
+    }
+    const float dBetaROut2 = dBetaROut * dBetaROut;
     const float dBetaRes = 0.02f / fmin_(sdOut_d, drt_InSeg);
-    return betaDifferenceCut(betaIn, betaOut, betaInRHmin, betaInRHmax, betaOutRHmin, betaOutRHmax, dBetaRes, dBetaMuls,
-                             dBetaLum2, dBetaRIn2, dBetaROut2);
+    if (!betaDifferenceCut(betaIn, betaOut, betaInRHmin, betaInRHmax, betaOutRHmin, betaOutRHmax, dBetaRes, dBetaMuls,
+                           dBetaLum2, dBetaRIn2, dBetaROut2))
+      return false;
+    float betaOutCut = fasin(fmin_(drt_tl_axis * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdOut_d) +
+                       fsqrt(dBetaLum2 + dBetaMuls * dBetaMuls);
+    if (!(fabs_(betaOut) < betaOutCut))
+      return false;
+    const float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
+    const float sdlPVoff = 0.1f / rt_OutLo;
+    float sdlCut = rec3.slope + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
+    if (!isEC_lastLayer)
+      dPhi = midPointDPhi();
+    return fabs_(dPhi) <= sdlCut;
   }
 
-  // Dispatch (SDL/PixelTriplet.h:206-314).
   LST_HD bool ptPixelTracklet(const Modules& m,
                               const Ranges& rg,
                               const MiniDoublets& md,
@@ -316,15 +250,11 @@ namespace lst {
                               uint16_t lmOI,
                               uint16_t lmOO,
                               unsigned int innerSeg,
-                              unsigned int outerSeg) {
-    short sOI = m.subdets[lmOI], sOO = m.subdets[lmOO];
-    unsigned int md1 = s.mdIndices[2 * innerSeg], md2 = s.mdIndices[2 * innerSeg + 1];
-    unsigned int md3 = s.mdIndices[2 * outerSeg], md4 = s.mdIndices[2 * outerSeg + 1];
-    if (sOI == Barrel and (sOO == Barrel or sOO == Endcap))
-      return ptPPBB(m, rg, md, s, pixelModule, lmOI, lmOO, innerSeg, outerSeg, md1, md2, md3, md4);
-    if (sOI == Endcap and sOO == Endcap)
-      return ptPPEE(m, rg, md, s, pixelModule, lmOI, lmOO, innerSeg, outerSeg, md1, md2, md3, md4);
-    return false;
+                              unsigned int outerSeg,
+                              float phiP) {
+    PtTracklet q;
+    return ptSetup(m, rg, s, pixelModule, lmOI, lmOO, innerSeg, outerSeg, q) && ptWindows(m, md, s, q) &&
+           ptBeta(m, md, s, q, phiP);
   }
 
   // ------------------------------------------------------------- pT3 cuts
@@ -544,16 +474,27 @@ namespace lst {
     return pt3RadiusCriterion(kind, pixelRadius, pixelRadiusError, t.circleRadius[t3]);
   }
 
-  // The second test of pt3Select below, alone: the pixel tracklet algorithm
-  // of the pLS with the triplet's inner segment.
-  LST_HD bool pt3FirstTracklet(const Modules& m, const Ranges& rg, const MiniDoublets& md, const Segments& s,
-                               const Triplets& t, unsigned int plsIndex, unsigned int t3) {
-    const uint16_t pixelModule = s.innerLowerModuleIndices[plsIndex];
-    return ptPixelTracklet(m, rg, md, s, pixelModule, t.lowerModuleIndices[3 * t3], t.lowerModuleIndices[3 * t3 + 1],
-                           plsIndex, t.segmentIndices[2 * t3]);
+  // The second test of pt3Select below in two parts: the pixel tracklet
+  // algorithm of the pLS with the triplet's inner segment.
+  LST_HD bool pt3FirstSetup(const Modules& m, const Ranges& rg, const Segments& s, const Triplets& t,
+                            unsigned int plsIndex, unsigned int t3, PtTracklet& q) {
+    return ptSetup(m, rg, s, s.innerLowerModuleIndices[plsIndex], t.lowerModuleIndices[3 * t3],
+                   t.lowerModuleIndices[3 * t3 + 1], plsIndex, t.segmentIndices[2 * t3], q);
+  }
+  LST_HD bool pt3FirstWindows(const Modules& m, const Ranges& rg, const MiniDoublets& md, const Segments& s,
+                              const Triplets& t, unsigned int plsIndex, unsigned int t3) {
+    PtTracklet q;
+    return pt3FirstSetup(m, rg, s, t, plsIndex, t3, q) && ptWindows(m, md, s, q);
+  }
+  LST_HD bool pt3FirstBeta(const Modules& m, const Ranges& rg, const MiniDoublets& md, const Segments& s,
+                           const Triplets& t, unsigned int plsIndex, unsigned int t3, float phiP) {
+    PtTracklet q;
+    pt3FirstSetup(m, rg, s, t, plsIndex, t3, q);
+    return ptBeta(m, md, s, q, phiP);
   }
 
-  // pLS x T3 selection (SDL/PixelTriplet.h:826-1023).
+  // pLS x T3 selection (SDL/PixelTriplet.h:826-1023).  opened: the pair is known
+  // to pass the radius criterion and the first tracklet (kPixMid).
   LST_HD bool pt3Select(const Modules& m,
                         const Ranges& rg,
                         const MiniDoublets& md,
@@ -562,7 +503,8 @@ namespace lst {
                         unsigned int plsIndex,
                         unsigned int t3,
                         bool runChiSquaredCuts,
-                        PT3Values& v) {
+                        PT3Values& v,
+                        bool opened = false) {
     uint16_t pixelModule = s.innerLowerModuleIndices[plsIndex];
     uint16_t lmL = t.lowerModuleIndices[3 * t3], lmM = t.lowerModuleIndices[3 * t3 + 1],
              lmU = t.lowerModuleIndices[3 * t3 + 2];
@@ -576,12 +518,18 @@ namespace lst {
     // a pure function of the pair, so testing this cheap one first changes no
     // outcome and skips the two tracklet algorithms for most pairs.
     int kind = (m.subdets[lmL] == Endcap) ? 3 : (m.subdets[lmM] == Endcap) ? 2 : (m.subdets[lmU] == Endcap) ? 1 : 0;
-    if (!pt3RadiusCriterion(kind, v.pixelRadius, v.pixelRadiusError, v.tripletRadius))
+    if (!opened && !pt3RadiusCriterion(kind, v.pixelRadius, v.pixelRadiusError, v.tripletRadius))
       return false;
-    if (!ptPixelTracklet(m, rg, md, s, pixelModule, lmL, lmM, plsIndex, t.segmentIndices[2 * t3]))
-      return false;
-    if (!ptPixelTracklet(m, rg, md, s, pixelModule, lmM, lmU, plsIndex, t.segmentIndices[2 * t3 + 1]))
-      return false;
+    const float phiP = phiOf(s.px[pls], s.py[pls]);
+    // The tracklets of the inner and the outer segment: one copy of the code
+    // (an unrolled pair costs more in instruction fetches than it saves).
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int k = opened ? 1 : 0; k < 2; ++k)
+      if (!ptPixelTracklet(m, rg, md, s, pixelModule, k == 0 ? lmL : lmM, k == 0 ? lmM : lmU, plsIndex,
+                           t.segmentIndices[2 * t3 + k], phiP))
+        return false;
 
     float pixelG = s.circleCenterX[pls];
     float pixelF = s.circleCenterY[pls];
@@ -899,11 +847,12 @@ namespace lst {
                         unsigned int plsIndex,
                         unsigned int t5,
                         unsigned int pls,
-                        PT5Values& v) {
+                        PT5Values& v,
+                        bool opened = false) {
     unsigned int innerT3 = q.tripletIndices[2 * t5];
     unsigned int outerT3 = q.tripletIndices[2 * t5 + 1];
     PT3Values tmp;
-    if (!pt3Select(m, rg, md, s, t, plsIndex, innerT3, false, tmp))
+    if (!pt3Select(m, rg, md, s, t, plsIndex, innerT3, false, tmp, opened))
       return false;
     unsigned int seg1 = t.segmentIndices[2 * innerT3], seg2 = t.segmentIndices[2 * innerT3 + 1];
     unsigned int seg3 = t.segmentIndices[2 * outerT3], seg4 = t.segmentIndices[2 * outerT3 + 1];
