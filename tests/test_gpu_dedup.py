@@ -58,3 +58,26 @@ def test_module_quintuplet_duplicates(es, config, index, pileup):
         keep_second = sc[:, None] >= sc[None, :]  # the first of the pair goes
         expected = (pair & keep_second).any(axis=1) | (pair & ~keep_second).any(axis=0)
         assert np.array_equal(is_dup[o] != 0, expected), f"module {m} with {n_t5[m]} quintuplets"
+
+
+@pytest.mark.parametrize("config,index,pileup", EVENTS)
+def test_pt5_duplicates(es, config, index, pileup):
+    inp = gen.generate_event(config, index, pileup)
+    s = lst.EventSet(es, 1, inp.n_hits + 1024)
+    try:
+        s.add_inputs(0, inp)
+        for st in ("md", "ls", "t3", "t5", "pls_clean", "pt5"):
+            s.run_stage(0, st)
+        n = int(s.field(0, "pt5.nPixelQuintuplets")[0])
+        score, is_dup = (s.field(0, f"pt5.{f}", n) for f in ("score", "isDup"))
+        hits = s.field(0, "pt5.hitIndices", 14 * n).reshape(-1, 14)
+    finally:
+        s.close()
+    if pileup > 300:
+        assert n > 1170
+    i = np.arange(n)
+    for a0 in range(0, n, 64):
+        a = i[a0:a0 + 64]
+        worse = (score[a][:, None] > score[None, :]) | ((score[a][:, None] == score[None, :]) & (a[:, None] > i[None, :]))
+        expected = (worse & (matched(hits[a], hits) >= 7)).any(axis=1)
+        assert np.array_equal(is_dup[a] != 0, expected), f"pT5s {a0}.. of {n}"

@@ -135,6 +135,8 @@ namespace lst {
     struct PLSRec* plsRec;      // pass-2 pLS records sorted by eta bin
     unsigned int* plsHitHead;   // hit -> pLS index of the pLS cleaning: chain head per bucket
     unsigned int* plsHitNext;   //   and the next entry (4 pLS + hit slot) per entry
+    unsigned int* pt5HitHead;   // hit -> (pT5, slot) chains of the pT5 duplicate removal
+    unsigned int* pt5HitNext;
     unsigned int* plsBinStart;  // start of each eta bin in plsRec (bins + 2 entries)
     unsigned int maxHits;
     unsigned int forceWalk;  // take the fallback paths (walks, pair-by-pair tests) for testing them

@@ -2120,84 +2120,65 @@ namespace lst {
   // pT5 duplicate removal (SDL/Kernels.h:356-382): pT5 ix is removed if some
   // jx shares at least 7 of its 14 hit slots and has a lower score (ties: the
   // higher index goes).  The outcome is an OR over jx, and a pair sharing 7
-  // slots shares at least one hit, so only pairs that meet in some hit need the
-  // full test.  kPT5DedupHashed (kPT5DedupBlocks blocks per event) chains the
-  // event's (hit, pT5) entries by hit in a shared-memory hash table (a head
-  // per bucket, a next index per entry, filled by one atomicExch per entry),
-  // each block on its own, and tests its share of the entries against the
-  // other entries of the same hit (the marks are only ever set, so the
-  // blocks' marks combine and the walking order does not matter); an event
-  // with more than kPT5DedupMaxN pT5s is left to kPT5Dedup, which tests every
-  // pair in shared-memory tiles.
-  constexpr unsigned int kPT5DedupBlocks = 2;
-  constexpr unsigned int kPT5DedupMaxEntries = 16384;
-  constexpr unsigned int kPT5DedupMaxN = kPT5DedupMaxEntries / 14;
-  constexpr unsigned int kPT5DedupBucketBits = 13;
-  constexpr unsigned int kPT5DedupBuckets = 1u << kPT5DedupBucketBits;
-  constexpr unsigned int kPT5DedupNone = 0xffffffffu;
-  constexpr size_t kPT5DedupSmem = kPT5DedupBuckets * sizeof(unsigned int) +
-                                   2 * kPT5DedupMaxEntries * sizeof(unsigned int) +
-                                   kPT5DedupMaxN * sizeof(float) + kPT5DedupMaxN;
-  LST_DEV unsigned int pt5HitBucket(unsigned int h) { return (h * 2654435761u) >> (32 - kPT5DedupBucketBits); }
+  // slots shares one of any 8 of them, so only pairs that meet in one of ix's
+  // first 8 slots need the full test.  kPixRankEmit<5> chains the event's (slot,
+  // pT5) entries e = 14 pT5 + slot by hit as it stores the pT5s, in a hash table
+  // in memory (a head per bucket, emptied by kPixEval<5>, and a next index per
+  // entry), and kPT5DedupHits gives each of the first 8 slots of each pT5 a
+  // thread that walks its hit's chain.  Bound by the latency of the walks.
+  // Tables in shared memory, built by each of two blocks per event, held 1170
+  // pT5s, and a denser event of a batch (PU250, pt0.6) took the tiles below:
+  // 738 + 71 us for 13 PU250 events, now 22 here and 28 more in kPixRankEmit<5>.
+  // Events whose pT5s the walk stored take the tiles.
+  constexpr unsigned int kPT5HitBucketBits = 15;
+  constexpr unsigned int kPT5HitBuckets = 1u << kPT5HitBucketBits;
+  constexpr unsigned int kPT5HitNone = 0xffffffffu;
+  constexpr unsigned int kPT5DedupSlots = 8;
+  LST_DEV unsigned int pt5HitBucket(unsigned int h) { return (h * 2654435761u) >> (32 - kPT5HitBucketBits); }
 
-  __global__ void __launch_bounds__(1024) kPT5DedupHashed(DeviceES es, const EventView* evs) {
-    extern __shared__ __align__(16) unsigned char psm[];
-    unsigned int* sHead = reinterpret_cast<unsigned int*>(psm);
-    unsigned int* sNext = sHead + kPT5DedupBuckets;
-    unsigned int* sHits = sNext + kPT5DedupMaxEntries;
-    float* sScore = reinterpret_cast<float*>(sHits + kPT5DedupMaxEntries);
-    unsigned char* sDup = reinterpret_cast<unsigned char*>(sScore + kPT5DedupMaxN);
+  __global__ void kPT5DedupHits(DeviceES es, const EventView* evs) {
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.pt5.nPixelQuintuplets;
-    if (n < 2 || n > kPT5DedupMaxN || ev.forceWalk)
+    if (ev.sc->pixFallback)
       return;
     PixelQuintuplets p = ev.pt5;
-    const unsigned int E = 14 * n;
-    for (unsigned int t = threadIdx.x; t < kPT5DedupBuckets; t += blockDim.x)
-      sHead[t] = kPT5DedupNone;
-    for (unsigned int t = threadIdx.x; t < n; t += blockDim.x) {
-      sScore[t] = p.score[t];
-      sDup[t] = 0;
-    }
-    __syncthreads();
-    for (unsigned int t = threadIdx.x; t < E; t += blockDim.x) {
-      const unsigned int h = p.hitIndices[t];
-      sHits[t] = h;
-      sNext[t] = atomicExch(&sHead[pt5HitBucket(h)], t);
-    }
-    __syncthreads();
-    for (unsigned int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x) {
-      const unsigned int a = e / 14;
-      const unsigned int h = sHits[e];
-      const float score1 = sScore[a];
-      for (unsigned int q = sHead[pt5HitBucket(h)]; q != kPT5DedupNone; q = sNext[q]) {
-        if (sDup[a])
-          break;
-        if (sHits[q] != h)
-          continue;
+    for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < kPT5DedupSlots * n;
+         t += gridDim.x * blockDim.x) {
+      const unsigned int a = t / kPT5DedupSlots;
+      const unsigned int h = p.hitIndices[14 * a + t % kPT5DedupSlots];
+      const float score1 = p.score[a];
+      for (unsigned int q = ev.pt5HitHead[pt5HitBucket(h)]; q != kPT5HitNone; q = ev.pt5HitNext[q]) {
         const unsigned int b = q / 14;
-        if (b == a)
+        if (p.hitIndices[q] != h || b == a)
           continue;
-        const float score2 = sScore[b];
+        const float score2 = p.score[b];
         if (!(score1 > score2 or ((score1 == score2) and (a > b))))
           continue;
-        const unsigned int* mine = sHits + 14 * a;
-        const unsigned int* other = sHits + 14 * b;
+        // (56 bytes per pT5: the fourteen indices lie on an 8-byte boundary)
+        const uint2* mine = reinterpret_cast<const uint2*>(p.hitIndices + 14 * size_t(a));
+        const uint2* other = reinterpret_cast<const uint2*>(p.hitIndices + 14 * size_t(b));
+        uint2 o[7];
+#pragma unroll
+        for (int j = 0; j < 7; ++j)
+          o[j] = other[j];
         int nMatched = 0;
-        for (int i = 0; i < 14; ++i) {
-          bool matched = false;
-          for (int j = 0; j < 14; ++j)
-            matched |= (mine[i] == other[j]);
-          nMatched += matched ? 1 : 0;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+          const uint2 m = mine[i];
+          bool mx = false, my = false;
+#pragma unroll
+          for (int j = 0; j < 7; ++j) {
+            mx |= m.x == o[j].x || m.x == o[j].y;
+            my |= m.y == o[j].x || m.y == o[j].y;
+          }
+          nMatched += (mx ? 1 : 0) + (my ? 1 : 0);
         }
-        if (nMatched >= 7)
-          sDup[a] = 1;
+        if (nMatched >= 7) {
+          p.isDup[a] = 1;
+          break;
+        }
       }
     }
-    __syncthreads();
-    for (unsigned int t = threadIdx.x; t < n; t += blockDim.x)
-      if (sDup[t])
-        p.isDup[t] = 1;
   }
 
   constexpr int kDedupTile = 128;
@@ -2206,8 +2187,8 @@ namespace lst {
     __shared__ float sScore[kDedupTile];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.pt5.nPixelQuintuplets;
-    if (n <= kPT5DedupMaxN && !ev.forceWalk)
-      return;  // kPT5DedupHashed has done this event
+    if (!ev.sc->pixFallback)
+      return;  // kPT5DedupHits has done this event
     PixelQuintuplets p = ev.pt5;
     for (unsigned int ixBase = blockIdx.x * kDedupTile; ixBase < n; ixBase += gridDim.x * kDedupTile) {
       const unsigned int ix = ixBase + threadIdx.x;
@@ -2627,6 +2608,9 @@ namespace lst {
   template <int K>
   __global__ void __launch_bounds__(LST_LB_EVAL) kPixEval(DeviceES es, const EventView* evs) {
     const EventView& ev = evs[blockIdx.y];
+    if (K == 5)
+      for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < kPT5HitBuckets; i += gridDim.x * blockDim.x)
+        ev.pt5HitHead[i] = kPT5HitNone;
     const unsigned int n = ev.sc->pixQueueCount;
     if (n > kCandQueueCap)
       return;  // the event takes the walk (kPixRankEmit)
@@ -2711,6 +2695,8 @@ namespace lst {
         v.centerY = vals[6];
         PixelQuintuplets pt5 = ev.pt5;
         storePT5(ev.md, ls, t3, t5, pt5, plsBase + iPLS, iPLS, obj, v, rank);
+        for (unsigned int e = 14 * rank; e < 14 * rank + 14; ++e)
+          ev.pt5HitNext[e] = atomicExch(&ev.pt5HitHead[pt5HitBucket(pt5.hitIndices[e])], e);
       } else {
         PT3Values v;
         v.pixelRadius = vals[0];
