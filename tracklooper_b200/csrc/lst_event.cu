@@ -493,6 +493,8 @@ namespace {
     const size_t nLower = d.nLowerModules;
     const size_t P = lst::kMaxPixelSegments;
     const dim3 one(1, count);
+    // pT5 / pT3 ranking: up to 16 blocks (2048 threads) per event
+    const dim3 rankGrid(std::min(16u, ceilDiv(kResidentBlocks, count)), count);
     switch (stage) {
       case LST_STAGE_MINI_DOUBLETS: {
         // modules per warp task: 8 from 4 events per launch, 4 for fewer, so
@@ -548,7 +550,7 @@ namespace {
         LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kPixMid<5>, tunedFlatGrid(ev, kTuMid5, count), tunedThreads(ev, kTuMid5), d, v);
         LST_LAUNCH(lst::kPixEval<5>, tunedFlatGrid(ev, kTuPix5, count), tunedThreads(ev, kTuPix5), d, v);
-        LST_LAUNCH(lst::kPixRankEmit<5>, one, 1024, d, v);
+        LST_LAUNCH(lst::kPixRankEmit<5>, rankGrid, lst::kPixRankThreads, d, v);
         LST_LAUNCH(lst::kPT5Count, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
         LST_LAUNCH(lst::kPLSScan, one, 1024, d, v, 0);
         LST_LAUNCH(lst::kPT5Emit, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
@@ -561,7 +563,7 @@ namespace {
         LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kPixMid<3>, tunedFlatGrid(ev, kTuMid3, count), tunedThreads(ev, kTuMid3), d, v);
         LST_LAUNCH(lst::kPixEval<3>, tunedFlatGrid(ev, kTuPix3, count), tunedThreads(ev, kTuPix3), d, v);
-        LST_LAUNCH(lst::kPixRankEmit<3>, one, 1024, d, v);
+        LST_LAUNCH(lst::kPixRankEmit<3>, rankGrid, lst::kPixRankThreads, d, v);
         LST_LAUNCH(lst::kPT3Count, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
         LST_LAUNCH(lst::kPLSScan, one, 1024, d, v, 1);
         LST_LAUNCH(lst::kPT3Emit, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
