@@ -210,12 +210,14 @@ namespace lst {
                       uint16_t outerLM,
                       const LSValues& v,
                       unsigned int idx) {
+    // (loads before stores, as in storeMD)
+    const unsigned int innerHit = md.anchorHitIndices[innerMD], outerHit = md.anchorHitIndices[outerMD];
     s.mdIndices[idx * 2] = innerMD;
     s.mdIndices[idx * 2 + 1] = outerMD;
     s.innerLowerModuleIndices[idx] = innerLM;
     s.outerLowerModuleIndices[idx] = outerLM;
-    s.innerMiniDoubletAnchorHitIndices[idx] = md.anchorHitIndices[innerMD];
-    s.outerMiniDoubletAnchorHitIndices[idx] = md.anchorHitIndices[outerMD];
+    s.innerMiniDoubletAnchorHitIndices[idx] = innerHit;
+    s.outerMiniDoubletAnchorHitIndices[idx] = outerHit;
     s.dPhis[idx] = v.dPhi;
     s.dPhiMins[idx] = v.dPhiMin;
     s.dPhiMaxs[idx] = v.dPhiMax;
@@ -243,12 +245,9 @@ namespace lst {
     unsigned int innerMD = mdBase + 2 * tid;
     unsigned int outerMD = mdBase + 2 * tid + 1;
     unsigned int pls = lsBase + tid;
-    MDValues zero{0, 0, 0, 0, 0, 0, 0, 0, 0};
-    storeMD(m, h, md, hit0, hit1, pixelModule, zero, innerMD);
-    storeMD(m, h, md, hit2, hit3, pixelModule, zero, outerMD);
-    // The anchor and outer hits storeMD has just stored (its rule), so that
-    // the values below are read from the hits directly rather than back
-    // through the stored mini-doublets.
+    // The anchor and outer hits of the two mini-doublets (storeMD's rule), so
+    // that the values below are read from the hits directly, and before the
+    // stores (as in storeMD).
     const bool swap = m.moduleType[pixelModule] == PS and m.moduleLayerType[pixelModule] == Strip;
     const unsigned int inAnchor = swap ? hit1 : hit0, inOuter = swap ? hit0 : hit1;
     const unsigned int outAnchor = swap ? hit3 : hit2, outOuter = swap ? hit2 : hit3;
@@ -258,20 +257,8 @@ namespace lst {
     float score_lsq = (h.rts[outAnchor] * slope + intercept) - (h.zs[outAnchor]);
     score_lsq = score_lsq * score_lsq;
 
-    s.mdIndices[pls * 2] = innerMD;
-    s.mdIndices[pls * 2 + 1] = outerMD;
-    s.innerLowerModuleIndices[pls] = pixelModule;
-    s.outerLowerModuleIndices[pls] = pixelModule;
-    s.innerMiniDoubletAnchorHitIndices[pls] = hit0;
-    s.outerMiniDoubletAnchorHitIndices[pls] = hit2;
-    s.dPhiChanges[pls] = dPhiChange;
-    s.isDup[tid] = 0;
-    s.score[tid] = score_lsq;
-    s.pLSHitsIdxs[4 * tid + 0] = h.idxs[inAnchor];
-    s.pLSHitsIdxs[4 * tid + 1] = h.idxs[outAnchor];
-    s.pLSHitsIdxs[4 * tid + 2] = h.idxs[inOuter];
-    s.pLSHitsIdxs[4 * tid + 3] = h.idxs[outOuter];
-
+    const unsigned int idxInAnchor = h.idxs[inAnchor], idxOutAnchor = h.idxs[outAnchor];
+    const unsigned int idxInOuter = h.idxs[inOuter], idxOutOuter = h.idxs[outOuter];
     float circleRadius = h.xs[inOuter] / (2 * k2Rinv1GeVf);
     float circlePhi = h.zs[inOuter];
     const float inAnchorX = h.xs[inAnchor], inAnchorY = h.ys[inAnchor];
@@ -289,6 +276,22 @@ namespace lst {
         bestIndex = i;
       }
     }
+    MDValues zero{0, 0, 0, 0, 0, 0, 0, 0, 0};
+    storeMD(m, h, md, hit0, hit1, pixelModule, zero, innerMD);
+    storeMD(m, h, md, hit2, hit3, pixelModule, zero, outerMD);
+    s.mdIndices[pls * 2] = innerMD;
+    s.mdIndices[pls * 2 + 1] = outerMD;
+    s.innerLowerModuleIndices[pls] = pixelModule;
+    s.outerLowerModuleIndices[pls] = pixelModule;
+    s.innerMiniDoubletAnchorHitIndices[pls] = hit0;
+    s.outerMiniDoubletAnchorHitIndices[pls] = hit2;
+    s.dPhiChanges[pls] = dPhiChange;
+    s.isDup[tid] = 0;
+    s.score[tid] = score_lsq;
+    s.pLSHitsIdxs[4 * tid + 0] = idxInAnchor;
+    s.pLSHitsIdxs[4 * tid + 1] = idxOutAnchor;
+    s.pLSHitsIdxs[4 * tid + 2] = idxInOuter;
+    s.pLSHitsIdxs[4 * tid + 3] = idxOutOuter;
     s.circleCenterX[tid] = candidateCenterXs[bestIndex];
     s.circleCenterY[tid] = candidateCenterYs[bestIndex];
     s.circleRadius[tid] = circleRadius;

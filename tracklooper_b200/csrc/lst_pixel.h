@@ -590,39 +590,40 @@ namespace lst {
                        short layer2_adjustment,
                        const PT3Values& v,
                        unsigned int idx) {
-    unsigned int etaMD = s.mdIndices[2 * t.segmentIndices[2 * t3] + layer2_adjustment];
+    // (loads before stores, as in storeMD)
+    const unsigned int etaMD = s.mdIndices[2 * t.segmentIndices[2 * t3] + layer2_adjustment];
+    const unsigned int pixelInnerMD = s.mdIndices[2 * plsIndex];
+    const unsigned int pixelOuterMD = s.mdIndices[2 * plsIndex + 1];
+    const float pt = s.ptIn[pls], etaPix = s.eta[pls], phiPix = s.phi[pls];
+    const uint16_t modules[5] = {s.innerLowerModuleIndices[plsIndex], s.outerLowerModuleIndices[plsIndex],
+                                 t.lowerModuleIndices[3 * t3], t.lowerModuleIndices[3 * t3 + 1],
+                                 t.lowerModuleIndices[3 * t3 + 2]};
+    const uint8_t layers[5] = {0, 0, t.logicalLayers[t3 * 3], t.logicalLayers[t3 * 3 + 1], t.logicalLayers[t3 * 3 + 2]};
+    const float eta = md.anchorEta[etaMD], phi = md.anchorPhi[etaMD];
+    unsigned int hits[10] = {md.anchorHitIndices[pixelInnerMD], md.outerHitIndices[pixelInnerMD],
+                             md.anchorHitIndices[pixelOuterMD], md.outerHitIndices[pixelOuterMD]};
+    for (int i = 0; i < 6; ++i)
+      hits[4 + i] = t.hitIndices[6 * t3 + i];
     p.pixelSegmentIndices[idx] = plsIndex;
     p.tripletIndices[idx] = t3;
     p.pixelRadius[idx] = v.pixelRadius;
     p.tripletRadius[idx] = v.tripletRadius;
-    p.pt[idx] = s.ptIn[pls];
-    p.eta[idx] = md.anchorEta[etaMD];
-    p.phi[idx] = md.anchorPhi[etaMD];
-    p.eta_pix[idx] = s.eta[pls];
-    p.phi_pix[idx] = s.phi[pls];
+    p.pt[idx] = pt;
+    p.eta[idx] = eta;
+    p.phi[idx] = phi;
+    p.eta_pix[idx] = etaPix;
+    p.phi_pix[idx] = phiPix;
     p.isDup[idx] = 0;
     p.partOfPT5[idx] = 0;
     p.score[idx] = v.rPhiChiSquared + v.rPhiChiSquaredInwards;
     p.centerX[idx] = v.centerX;
     p.centerY[idx] = v.centerY;
-    p.logicalLayers[5 * idx] = 0;
-    p.logicalLayers[5 * idx + 1] = 0;
-    p.logicalLayers[5 * idx + 2] = t.logicalLayers[t3 * 3];
-    p.logicalLayers[5 * idx + 3] = t.logicalLayers[t3 * 3 + 1];
-    p.logicalLayers[5 * idx + 4] = t.logicalLayers[t3 * 3 + 2];
-    p.lowerModuleIndices[5 * idx] = s.innerLowerModuleIndices[plsIndex];
-    p.lowerModuleIndices[5 * idx + 1] = s.outerLowerModuleIndices[plsIndex];
-    p.lowerModuleIndices[5 * idx + 2] = t.lowerModuleIndices[3 * t3];
-    p.lowerModuleIndices[5 * idx + 3] = t.lowerModuleIndices[3 * t3 + 1];
-    p.lowerModuleIndices[5 * idx + 4] = t.lowerModuleIndices[3 * t3 + 2];
-    unsigned int pixelInnerMD = s.mdIndices[2 * plsIndex];
-    unsigned int pixelOuterMD = s.mdIndices[2 * plsIndex + 1];
-    p.hitIndices[10 * idx] = md.anchorHitIndices[pixelInnerMD];
-    p.hitIndices[10 * idx + 1] = md.outerHitIndices[pixelInnerMD];
-    p.hitIndices[10 * idx + 2] = md.anchorHitIndices[pixelOuterMD];
-    p.hitIndices[10 * idx + 3] = md.outerHitIndices[pixelOuterMD];
-    for (int i = 0; i < 6; ++i)
-      p.hitIndices[10 * idx + 4 + i] = t.hitIndices[6 * t3 + i];
+    for (int i = 0; i < 5; ++i) {
+      p.logicalLayers[5 * idx + i] = layers[i];
+      p.lowerModuleIndices[5 * idx + i] = modules[i];
+    }
+    for (int i = 0; i < 10; ++i)
+      p.hitIndices[10 * idx + i] = hits[i];
     p.pixelRadiusError[idx] = v.pixelRadiusError;
     p.rPhiChiSquared[idx] = v.rPhiChiSquared;
     p.rPhiChiSquaredInwards[idx] = v.rPhiChiSquaredInwards;
@@ -915,37 +916,42 @@ namespace lst {
                        unsigned int t5,
                        const PT5Values& v,
                        unsigned int idx) {
+    // (loads before stores, as in storeMD)
+    const unsigned int pixelInnerMD = s.mdIndices[2 * plsIndex];
+    const unsigned int pixelOuterMD = s.mdIndices[2 * plsIndex + 1];
+    const unsigned int innerT3 = q.tripletIndices[2 * t5], outerT3 = q.tripletIndices[2 * t5 + 1];
+    const float eta = q.eta[t5], phi = q.phi[t5];
+    uint8_t layers[7] = {0, 0};
+    uint16_t modules[7] = {s.innerLowerModuleIndices[plsIndex], s.outerLowerModuleIndices[plsIndex]};
+    for (int i = 0; i < 5; ++i) {
+      layers[2 + i] = q.logicalLayers[t5 * 5 + i];
+      modules[2 + i] = q.lowerModuleIndices[t5 * 5 + i];
+    }
+    unsigned int hits[14] = {md.anchorHitIndices[pixelInnerMD], md.outerHitIndices[pixelInnerMD],
+                             md.anchorHitIndices[pixelOuterMD], md.outerHitIndices[pixelOuterMD]};
+    for (int i = 0; i < 10; ++i)
+      hits[4 + i] = q.hitIndices[10 * t5 + i];
     p.pixelIndices[idx] = plsIndex;
     p.T5Indices[idx] = t5;
     p.isDup[idx] = 0;
     p.score[idx] = v.rPhiChiSquared;
-    p.eta[idx] = q.eta[t5];
-    p.phi[idx] = q.phi[t5];
+    p.eta[idx] = eta;
+    p.phi[idx] = phi;
     p.pixelRadius[idx] = v.pixelRadius;
     p.quintupletRadius[idx] = v.quintupletRadius;
     p.centerX[idx] = v.centerX;
     p.centerY[idx] = v.centerY;
-    p.logicalLayers[7 * idx] = 0;
-    p.logicalLayers[7 * idx + 1] = 0;
-    for (int i = 0; i < 5; ++i)
-      p.logicalLayers[7 * idx + 2 + i] = q.logicalLayers[t5 * 5 + i];
-    p.lowerModuleIndices[7 * idx] = s.innerLowerModuleIndices[plsIndex];
-    p.lowerModuleIndices[7 * idx + 1] = s.outerLowerModuleIndices[plsIndex];
-    for (int i = 0; i < 5; ++i)
-      p.lowerModuleIndices[7 * idx + 2 + i] = q.lowerModuleIndices[t5 * 5 + i];
-    unsigned int pixelInnerMD = s.mdIndices[2 * plsIndex];
-    unsigned int pixelOuterMD = s.mdIndices[2 * plsIndex + 1];
-    p.hitIndices[14 * idx] = md.anchorHitIndices[pixelInnerMD];
-    p.hitIndices[14 * idx + 1] = md.outerHitIndices[pixelInnerMD];
-    p.hitIndices[14 * idx + 2] = md.anchorHitIndices[pixelOuterMD];
-    p.hitIndices[14 * idx + 3] = md.outerHitIndices[pixelOuterMD];
-    for (int i = 0; i < 10; ++i)
-      p.hitIndices[14 * idx + 4 + i] = q.hitIndices[10 * t5 + i];
+    for (int i = 0; i < 7; ++i) {
+      p.logicalLayers[7 * idx + i] = layers[i];
+      p.lowerModuleIndices[7 * idx + i] = modules[i];
+    }
+    for (int i = 0; i < 14; ++i)
+      p.hitIndices[14 * idx + i] = hits[i];
     p.rzChiSquared[idx] = v.rzChiSquared;
     p.rPhiChiSquared[idx] = v.rPhiChiSquared;
     p.rPhiChiSquaredInwards[idx] = v.rPhiChiSquaredInwards;
-    t.partOfPT5[q.tripletIndices[2 * t5]] = 1;
-    t.partOfPT5[q.tripletIndices[2 * t5 + 1]] = 1;
+    t.partOfPT5[innerT3] = 1;
+    t.partOfPT5[outerT3] = 1;
     s.partOfPT5[pls] = 1;
     q.partOfPT5[t5] = 1;
   }

@@ -332,6 +332,15 @@ namespace lst {
                       uint16_t lm3,
                       const T3Values& v,
                       unsigned int idx) {
+    // (loads before stores, as in storeMD)
+    const unsigned int md1 = s.mdIndices[2 * innerSeg];
+    const unsigned int md2 = s.mdIndices[2 * innerSeg + 1];
+    const unsigned int md3 = s.mdIndices[2 * outerSeg + 1];
+    const uint8_t layer1 = m.layers[lm1] + (m.subdets[lm1] == 4) * 6;
+    const uint8_t layer2 = m.layers[lm2] + (m.subdets[lm2] == 4) * 6;
+    const uint8_t layer3 = m.layers[lm3] + (m.subdets[lm3] == 4) * 6;
+    const unsigned int hits[6] = {md.anchorHitIndices[md1], md.outerHitIndices[md1], md.anchorHitIndices[md2],
+                                  md.outerHitIndices[md2],  md.anchorHitIndices[md3], md.outerHitIndices[md3]};
     t.segmentIndices[idx * 2] = innerSeg;
     t.segmentIndices[idx * 2 + 1] = outerSeg;
     t.lowerModuleIndices[idx * 3] = lm1;
@@ -341,18 +350,11 @@ namespace lst {
     t.circleRadius[idx] = v.circleRadius;
     t.circleCenterX[idx] = v.circleCenterX;
     t.circleCenterY[idx] = v.circleCenterY;
-    t.logicalLayers[idx * 3] = m.layers[lm1] + (m.subdets[lm1] == 4) * 6;
-    t.logicalLayers[idx * 3 + 1] = m.layers[lm2] + (m.subdets[lm2] == 4) * 6;
-    t.logicalLayers[idx * 3 + 2] = m.layers[lm3] + (m.subdets[lm3] == 4) * 6;
-    unsigned int md1 = s.mdIndices[2 * innerSeg];
-    unsigned int md2 = s.mdIndices[2 * innerSeg + 1];
-    unsigned int md3 = s.mdIndices[2 * outerSeg + 1];
-    t.hitIndices[idx * 6] = md.anchorHitIndices[md1];
-    t.hitIndices[idx * 6 + 1] = md.outerHitIndices[md1];
-    t.hitIndices[idx * 6 + 2] = md.anchorHitIndices[md2];
-    t.hitIndices[idx * 6 + 3] = md.outerHitIndices[md2];
-    t.hitIndices[idx * 6 + 4] = md.anchorHitIndices[md3];
-    t.hitIndices[idx * 6 + 5] = md.outerHitIndices[md3];
+    t.logicalLayers[idx * 3] = layer1;
+    t.logicalLayers[idx * 3 + 1] = layer2;
+    t.logicalLayers[idx * 3 + 2] = layer3;
+    for (int i = 0; i < 6; ++i)
+      t.hitIndices[idx * 6 + i] = hits[i];
     // The reference clears these flags for the whole store when it allocates it.
     t.partOfPT5[idx] = 0;
     t.partOfT5[idx] = 0;

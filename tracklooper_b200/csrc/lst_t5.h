@@ -1485,6 +1485,15 @@ namespace lst {
                       unsigned int idx) {
     short layer2_adjustment = (layer == 1) ? 1 : 0;
     unsigned int etaMD = s.mdIndices[2 * t.segmentIndices[2 * innerT3 + layer2_adjustment]];
+    // (loads before stores, as in storeMD)
+    unsigned int hits[10];
+    for (int i = 0; i < 6; ++i)
+      hits[i] = t.hitIndices[6 * innerT3 + i];
+    for (int i = 0; i < 4; ++i)
+      hits[6 + i] = t.hitIndices[6 * outerT3 + 2 + i];
+    const uint8_t layers[5] = {t.logicalLayers[3 * innerT3], t.logicalLayers[3 * innerT3 + 1],
+                               t.logicalLayers[3 * innerT3 + 2], t.logicalLayers[3 * outerT3 + 1],
+                               t.logicalLayers[3 * outerT3 + 2]};
     float phi = md.anchorPhi[etaMD];
     float eta = md.anchorEta[etaMD];
     float pt = (v.innerRadius + v.outerRadius) * 3.8f * 1.602f / (2 * 100 * 5.39f);
@@ -1506,15 +1515,10 @@ namespace lst {
     q.regressionRadius[idx] = v.regressionRadius;
     q.regressionG[idx] = v.regressionG;
     q.regressionF[idx] = v.regressionF;
-    q.logicalLayers[5 * idx] = t.logicalLayers[3 * innerT3];
-    q.logicalLayers[5 * idx + 1] = t.logicalLayers[3 * innerT3 + 1];
-    q.logicalLayers[5 * idx + 2] = t.logicalLayers[3 * innerT3 + 2];
-    q.logicalLayers[5 * idx + 3] = t.logicalLayers[3 * outerT3 + 1];
-    q.logicalLayers[5 * idx + 4] = t.logicalLayers[3 * outerT3 + 2];
-    for (int i = 0; i < 6; ++i)
-      q.hitIndices[10 * idx + i] = t.hitIndices[6 * innerT3 + i];
-    for (int i = 0; i < 4; ++i)
-      q.hitIndices[10 * idx + 6 + i] = t.hitIndices[6 * outerT3 + 2 + i];
+    for (int i = 0; i < 5; ++i)
+      q.logicalLayers[5 * idx + i] = layers[i];
+    for (int i = 0; i < 10; ++i)
+      q.hitIndices[10 * idx + i] = hits[i];
     q.bridgeRadius[idx] = v.bridgeRadius;
     q.rzChiSquared[idx] = v.rzChiSquared;
     q.chiSquared[idx] = v.chiSquared;
