@@ -30,6 +30,8 @@ namespace lst {
     unsigned int nTotalSegments;
     unsigned int maxTriplets;
     unsigned int maxQuintuplets;
+    const MDCut* mdCuts;  // per module: what the mini-doublet and segment cuts take from it
+    const LSCut* lsCuts;
     const unsigned int* detHashKey;
     const uint16_t* detHashVal;
     unsigned int detHashBits;

@@ -264,6 +264,9 @@ namespace {
     d.detHashKey = upload(c, h.detHashKey, copies, sizes);
     d.detHashVal = upload(c, h.detHashVal, copies, sizes);
     d.detHashBits = h.detHashBits;
+    // filled on the device by kModuleCuts
+    d.mdCuts = c.take<lst::MDCut>(h.nLowerModules);
+    d.lsCuts = c.take<lst::LSCut>(h.nLowerModules);
     // The positive- and negative-z pixel maps follow the inclusive one in
     // connectedPixels (SDL/Event.cc:1049-1052).
     const size_t last = lst::kSizeSuperbins - 1;
@@ -651,6 +654,7 @@ namespace {
   const std::vector<KernelEntry>& kernelTable() {
     static const std::vector<KernelEntry> t = {
         {"kResetEvent", (const void*)lst::kResetEvent},
+        {"kModuleCuts", (const void*)lst::kModuleCuts},
         {"kHitPrep", (const void*)lst::kHitPrep},
         {"kModuleRanges", (const void*)lst::kModuleRanges},
         {"kPixelIngest", (const void*)lst::kPixelIngest},
@@ -805,6 +809,16 @@ int lst_es_load_ex(const char* geometry_dir, const char* t5dnn_weights_path, int
   layoutES(fill, *es, copies, sizes);
   for (size_t i = 0; i < copies.size(); ++i)
     LST_CUDA(cudaMemcpy(copies[i].first, copies[i].second, sizes[i], cudaMemcpyHostToDevice));
+  cudaGetLastError();  // drop a stale non-sticky error
+  lst::kModuleCuts<<<ceilDiv(es->view.nLowerModules, 256), 256>>>(es->view.m, const_cast<lst::MDCut*>(es->view.mdCuts),
+                                                             const_cast<lst::LSCut*>(es->view.lsCuts));
+  cudaError_t ec = cudaGetLastError();
+  if (ec == cudaSuccess)
+    ec = cudaDeviceSynchronize();
+  if (ec != cudaSuccess) {
+    cudaFree(es->arena);
+    return cudaFail(ec, "kModuleCuts");
+  }
   if (t5dnn_weights_path) {
     int rc = uploadWeights(es.get());
     if (rc) {

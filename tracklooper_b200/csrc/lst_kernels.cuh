@@ -111,6 +111,15 @@ namespace lst {
     return excl;
   }
 
+  // The lower modules' cut constants, once per event setup.
+  __global__ void kModuleCuts(Modules m, MDCut* mdCuts, LSCut* lsCuts) {
+    const unsigned int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m.nLowerModules)
+      return;
+    mdCuts[i] = mdCut(m, static_cast<uint16_t>(i));
+    lsCuts[i] = lsCut(m, static_cast<uint16_t>(i));
+  }
+
   // =============================================================== reset
   // Hit -> pLS index of the pLS cleaning: chains of (pLS, hit slot) entries
   // e = 4 pLS + slot in a hash table keyed by the stored pixel hit
@@ -421,7 +430,7 @@ namespace lst {
         const int local = g - exj;
         lowerIdx = unsigned(loj + local / nUj);
         upperIdx = unsigned(upj + local % nUj);
-        ok = mdSelect(es.m, lm, h.xs[lowerIdx], h.ys[lowerIdx], h.zs[lowerIdx], h.rts[lowerIdx], h.xs[upperIdx],
+        ok = mdSelect(es.mdCuts[lm], h.xs[lowerIdx], h.ys[lowerIdx], h.zs[lowerIdx], h.rts[lowerIdx], h.xs[upperIdx],
                       h.ys[upperIdx], h.zs[upperIdx], h.rts[upperIdx], h.phis[lowerIdx], h.phis[upperIdx], pre,
                       lowerIdx, upperIdx, v);
       }
@@ -580,6 +589,7 @@ namespace lst {
     const int cap = es.lsCap[lm];
     const unsigned int base = es.lsOffset[lm];
     const unsigned int innerBase = es.mdOffset[lm];
+    const LSCut inner = es.lsCuts[lm];
     Segments ls = ev.ls;
     unsigned int count = 0;
     for (unsigned int start = 0; start < total; start += 32) {
@@ -595,7 +605,7 @@ namespace lst {
         unsigned int local = f - sc.pre[k];
         innerMD = innerBase + local / nOuterMDs;
         outerMD = sc.outerBase[k] + local % nOuterMDs;
-        ok = lsSelect(m, ev.md, lm, outerLM, innerMD, outerMD, v);
+        ok = lsSelect(inner, es.lsCuts[outerLM], m.ptCut, ev.md.rec[innerMD], ev.md.rec[outerMD], v);
       }
       unsigned int tot;
       unsigned int r = count + warpRank(ok, tot);

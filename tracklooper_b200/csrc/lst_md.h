@@ -73,37 +73,6 @@ namespace lst {
   // (computed once per hit by kHitPrep).
   LST_HD float mdMiniSlope(float rt, float ptCut) { return fasin(fmin_(rt * k2Rinv1GeVf / ptCut, kSinAlphaMax)); }
 
-  LST_HD float mdDPhiThresholdFromSlope(const Modules& m, float miniSlope, uint16_t mi, float dPhi = 0, float dz = 0) {
-    unsigned int iL = m.layers[mi] - 1;
-    const bool barrel = m.subdets[mi] == Barrel;
-    const float rLayNominal = barrel ? miniRminMeanBarrel(iL) : miniRminMeanEndcap(iL);
-    const float miniPVoff = 0.1f / rLayNominal;
-    const float miniMuls =
-        barrel ? miniMulsPtScaleBarrel(iL) * 3.f / m.ptCut : miniMulsPtScaleEndcap(iL) * 3.f / m.ptCut;
-    const bool isTilted = barrel and m.sides[mi] != Center;
-    float drdz;
-    if (isTilted) {
-      if (m.moduleType[mi] == PS and m.moduleLayerType[mi] == Strip)
-        drdz = m.drdzs[mi];
-      else
-        drdz = m.drdzs[m.partnerModuleIndices[mi]];
-    } else {
-      drdz = 0;
-    }
-    const float miniTilt =
-        isTilted ? 0.5f * kPixelPSZpitch * drdz / fsqrt(1.f + drdz * drdz) / moduleGap(m, mi) : 0;
-    const float miniLum = fabs_(dPhi * kDeltaZLum / dz);
-    if (barrel and m.sides[mi] == Center)
-      return miniSlope + fsqrt(miniMuls * miniMuls + miniPVoff * miniPVoff);
-    else if (barrel)
-      return miniSlope + fsqrt(miniMuls * miniMuls + miniPVoff * miniPVoff + miniTilt * miniTilt * miniSlope * miniSlope);
-    return miniSlope + fsqrt(miniMuls * miniMuls + miniPVoff * miniPVoff + miniLum * miniLum);
-  }
-
-  LST_HD float mdDPhiThreshold(const Modules& m, float rt, uint16_t mi, float dPhi = 0, float dz = 0) {
-    return mdDPhiThresholdFromSlope(m, mdMiniSlope(rt, m.ptCut), mi, dPhi, dz);
-  }
-
   // Moves the strip hit along the strip so that it lines up with the
   // interaction point and the pixel hit (SDL/MiniDoublet.h:404-568).
   // shiftStripHit (SDL/MiniDoublet.h:110-191) moves one hit of the pair (p)
@@ -152,20 +121,76 @@ namespace lst {
     zn = abszn * ((zp > 0) ? 1 : -1);
   }
 
-  // The projection next to the other hit (xo, yo) that completes shiftStripHit.
-  LST_HD void shiftStripFinish(const Modules& m, uint16_t lm, float xa, float ya, float xo, float yo, float& xn,
-                               float& yn) {
-    const float slope = m.dxdys[lm];
-    if (slope == kInf) {
-      xn = xa;
-      yn = yo;
-    } else if (slope == 0) {
-      xn = xo;
-      yn = ya;
+  // What the mini-doublet cuts take from a lower module, formed once per module
+  // when the event setup is loaded (kModuleCuts) instead of for every pair: the
+  // terms of the dPhi threshold (SDL/MiniDoublet.h:340-402) and of the strip
+  // shift's projection (:404-568).
+  struct alignas(16) MDCut {
+    float base, root;  // miniMuls^2 + miniPVoff^2, and its square root
+    float tilt2;       // miniTilt^2
+    float slope, slopeInv, slopeSum;  // the strip slope, 1 / slope, slope + 1 / slope
+    unsigned int flags;
+    unsigned int pad;
+  };
+  enum MDCutFlags : unsigned int {
+    kCutBarrel = 1,         // barrel module
+    kCutCenter = 2,         //   with sides == Center (not tilted)
+    kCutPS = 4,
+    kCutLowerIsPixel = 8,   // moduleLayerType == Pixel
+    kCutMovesLower = 16,    // shiftMovesLower
+    kCutEndcap = 32,
+    kCutEndcapTwoS = 64,
+    kCutInnerLayers = 128   // layers 1 and 2
+  };
+
+  LST_HD unsigned int cutFlags(const Modules& m, uint16_t mi) {
+    const bool barrel = m.subdets[mi] == Barrel, endcap = m.subdets[mi] == Endcap;
+    return (barrel ? kCutBarrel : 0u) | (barrel and m.sides[mi] == Center ? kCutCenter : 0u) |
+           (m.moduleType[mi] == PS ? kCutPS : 0u) | (m.moduleLayerType[mi] == Pixel ? kCutLowerIsPixel : 0u) |
+           (shiftMovesLower(m, mi) ? kCutMovesLower : 0u) | (endcap ? kCutEndcap : 0u) |
+           (endcap and m.moduleType[mi] == TwoS ? kCutEndcapTwoS : 0u) | (m.layers[mi] <= 2 ? kCutInnerLayers : 0u);
+  }
+
+  LST_HD MDCut mdCut(const Modules& m, uint16_t mi) {
+    unsigned int iL = m.layers[mi] - 1;
+    const bool barrel = m.subdets[mi] == Barrel;
+    const float rLayNominal = barrel ? miniRminMeanBarrel(iL) : miniRminMeanEndcap(iL);
+    const float miniPVoff = 0.1f / rLayNominal;
+    const float miniMuls =
+        barrel ? miniMulsPtScaleBarrel(iL) * 3.f / m.ptCut : miniMulsPtScaleEndcap(iL) * 3.f / m.ptCut;
+    const bool isTilted = barrel and m.sides[mi] != Center;
+    float drdz;
+    if (isTilted) {
+      if (m.moduleType[mi] == PS and m.moduleLayerType[mi] == Strip)
+        drdz = m.drdzs[mi];
+      else
+        drdz = m.drdzs[m.partnerModuleIndices[mi]];
     } else {
-      xn = (slope * xa + (1.f / slope) * xo - ya + yo) / (slope + (1.f / slope));
-      yn = (xn - xa) * slope + ya;
+      drdz = 0;
     }
+    const float miniTilt =
+        isTilted ? 0.5f * kPixelPSZpitch * drdz / fsqrt(1.f + drdz * drdz) / moduleGap(m, mi) : 0;
+    MDCut c;
+    c.base = miniMuls * miniMuls + miniPVoff * miniPVoff;
+    c.root = fsqrt(miniMuls * miniMuls + miniPVoff * miniPVoff);
+    c.tilt2 = miniTilt * miniTilt;
+    c.slope = m.dxdys[mi];
+    c.slopeInv = 1.f / c.slope;
+    c.slopeSum = c.slope + (1.f / c.slope);
+    c.flags = cutFlags(m, mi);
+    c.pad = 0;
+    return c;
+  }
+
+  // The dPhi threshold from the hit's slope term; dPhi and dz enter it for
+  // endcap modules only.
+  LST_HD float mdDPhiThreshold(const MDCut& c, float miniSlope, float dPhi, float dz) {
+    if (c.flags & kCutCenter)
+      return miniSlope + c.root;
+    if (c.flags & kCutBarrel)
+      return miniSlope + fsqrt(c.base + c.tilt2 * miniSlope * miniSlope);
+    const float miniLum = fabs_(dPhi * kDeltaZLum / dz);
+    return miniSlope + fsqrt(c.base + miniLum * miniLum);
   }
 
   // Per-hit values of the mini-doublet cuts computed once per hit: the slope
@@ -178,8 +203,21 @@ namespace lst {
     const float* shiftZn;
   };
 
-  LST_HD void shiftStripHit(const Modules& m,
-                            uint16_t lm,
+  // shiftStripHit's projection next to the other hit (xo, yo).
+  LST_HD void shiftStripFinish(const MDCut& c, float xa, float ya, float xo, float yo, float& xn, float& yn) {
+    if (c.slope == kInf) {
+      xn = xa;
+      yn = yo;
+    } else if (c.slope == 0) {
+      xn = xo;
+      yn = ya;
+    } else {
+      xn = (c.slope * xa + c.slopeInv * xo - ya + yo) / c.slopeSum;
+      yn = (xn - xa) * c.slope + ya;
+    }
+  }
+
+  LST_HD void shiftStripHit(const MDCut& c,
                             const MDHitPre& pre,
                             unsigned int lowerIdx,
                             unsigned int upperIdx,
@@ -190,11 +228,11 @@ namespace lst {
                             float& xn,
                             float& yn,
                             float& zn) {
-    const bool fromLower = shiftMovesLower(m, lm);
+    const bool fromLower = (c.flags & kCutMovesLower) != 0;
     const unsigned int p = fromLower ? lowerIdx : upperIdx;
     const float xo = fromLower ? xUpper : xLower, yo = fromLower ? yUpper : yLower;
     zn = pre.shiftZn[p];
-    shiftStripFinish(m, lm, pre.shiftXa[p], pre.shiftYa[p], xo, yo, xn, yn);
+    shiftStripFinish(c, pre.shiftXa[p], pre.shiftYa[p], xo, yo, xn, yn);
   }
 
   // The derived per-MD values of MiniDoublets (slope, tanSlope, slope3).
@@ -218,8 +256,7 @@ namespace lst {
   };
 
   // Barrel mini-doublet (SDL/MiniDoublet.h:645-777).
-  LST_HD_BIG bool mdBarrel(const Modules& m,
-                       uint16_t lm,
+  LST_HD_BIG bool mdBarrel(const MDCut& c,
                        float xLower,
                        float yLower,
                        float zLower,
@@ -235,20 +272,20 @@ namespace lst {
                        unsigned int upperIdx,
                        MDValues& v) {
     v.dz = zLower - zUpper;
-    const float dzCut = m.moduleType[lm] == PS ? 2.f : 10.f;
+    const float dzCut = (c.flags & kCutPS) ? 2.f : 10.f;
     const float sign = ((v.dz > 0) - (v.dz < 0)) * ((zLower > 0) - (zLower < 0));
     const float invertedcrossercut = (fabs_(v.dz) > 2) * sign;
     if (!((fabs_(v.dz) < dzCut) && (invertedcrossercut <= 0)))
       return false;
 
-    const bool lowerIsPixel = m.moduleLayerType[lm] == Pixel;
-    float miniCut = mdDPhiThresholdFromSlope(m, pre.miniSlope[lowerIsPixel ? lowerIdx : upperIdx], lm);
+    const bool lowerIsPixel = (c.flags & kCutLowerIsPixel) != 0;
+    float miniCut = mdDPhiThreshold(c, pre.miniSlope[lowerIsPixel ? lowerIdx : upperIdx], 0, 0);
 
     float shiftedRt = 0;
-    const bool tilted = m.sides[lm] != Center;
+    const bool tilted = !(c.flags & kCutCenter);
     if (tilted) {
       float xn, yn, zn;
-      shiftStripHit(m, lm, pre, lowerIdx, upperIdx, xLower, yLower, xUpper, yUpper, xn, yn, zn);
+      shiftStripHit(c, pre, lowerIdx, upperIdx, xLower, yLower, xUpper, yUpper, xn, yn, zn);
       v.shiftedX = xn;
       v.shiftedY = yn;
       shiftedRt = fsqrt(xn * xn + yn * yn);
@@ -290,8 +327,7 @@ namespace lst {
 
   // Endcap mini-doublet (SDL/MiniDoublet.h:779-892).  The stored "dz" of an
   // endcap mini-doublet is the transverse-radius difference.
-  LST_HD_BIG bool mdEndcap(const Modules& m,
-                       uint16_t lm,
+  LST_HD_BIG bool mdEndcap(const MDCut& c,
                        float xLower,
                        float yLower,
                        float zLower,
@@ -310,15 +346,15 @@ namespace lst {
     const float dzCut = 1.f;
     if (!(fabs_(dz) < dzCut))
       return false;
-    const float drtCut = m.moduleType[lm] == PS ? 2.f : 10.f;
+    const float drtCut = (c.flags & kCutPS) ? 2.f : 10.f;
     v.dz = rtLower - rtUpper;
     if (!(fabs_(v.dz) < drtCut))
       return false;
 
     float xn, yn, zn;
-    shiftStripHit(m, lm, pre, lowerIdx, upperIdx, xLower, yLower, xUpper, yUpper, xn, yn, zn);
-    const bool isPS = m.moduleType[lm] == PS;
-    const bool lowerIsPixel = m.moduleLayerType[lm] == Pixel;
+    shiftStripHit(c, pre, lowerIdx, upperIdx, xLower, yLower, xUpper, yUpper, xn, yn, zn);
+    const bool isPS = (c.flags & kCutPS) != 0;
+    const bool lowerIsPixel = (c.flags & kCutLowerIsPixel) != 0;
     v.shiftedX = xn;
     v.shiftedY = yn;
     if (isPS) {
@@ -338,7 +374,7 @@ namespace lst {
     if (isPS)
       dz = lowerIsPixel ? zLower - zn : zUpper - zn;
 
-    float miniCut = mdDPhiThresholdFromSlope(m, pre.miniSlope[lowerIsPixel ? lowerIdx : upperIdx], lm, v.dphi, dz);
+    float miniCut = mdDPhiThreshold(c, pre.miniSlope[lowerIsPixel ? lowerIdx : upperIdx], v.dphi, dz);
     if (!(fabs_(v.dphi) < miniCut))
       return false;
 
@@ -351,6 +387,27 @@ namespace lst {
 
   // phiLower / phiUpper are the hits' stored phi (hits.phis, phi() of the same
   // coordinates), used wherever the reference takes deltaPhi of a hit itself.
+  LST_HD bool mdSelect(const MDCut& c,
+                       float xLower,
+                       float yLower,
+                       float zLower,
+                       float rtLower,
+                       float xUpper,
+                       float yUpper,
+                       float zUpper,
+                       float rtUpper,
+                       float phiLower,
+                       float phiUpper,
+                       const MDHitPre& pre,
+                       unsigned int lowerIdx,
+                       unsigned int upperIdx,
+                       MDValues& v) {
+    if (c.flags & kCutBarrel)
+      return mdBarrel(c, xLower, yLower, zLower, rtLower, xUpper, yUpper, zUpper, rtUpper, phiLower, phiUpper, pre,
+                      lowerIdx, upperIdx, v);
+    return mdEndcap(c, xLower, yLower, zLower, rtLower, xUpper, yUpper, zUpper, rtUpper, phiLower, phiUpper, pre,
+                    lowerIdx, upperIdx, v);
+  }
   LST_HD bool mdSelect(const Modules& m,
                        uint16_t lm,
                        float xLower,
@@ -367,11 +424,8 @@ namespace lst {
                        unsigned int lowerIdx,
                        unsigned int upperIdx,
                        MDValues& v) {
-    if (m.subdets[lm] == Barrel)
-      return mdBarrel(m, lm, xLower, yLower, zLower, rtLower, xUpper, yUpper, zUpper, rtUpper, phiLower, phiUpper, pre,
-                      lowerIdx, upperIdx, v);
-    return mdEndcap(m, lm, xLower, yLower, zLower, rtLower, xUpper, yUpper, zUpper, rtUpper, phiLower, phiUpper, pre,
-                    lowerIdx, upperIdx, v);
+    return mdSelect(mdCut(m, lm), xLower, yLower, zLower, rtLower, xUpper, yUpper, zUpper, rtUpper, phiLower, phiUpper,
+                    pre, lowerIdx, upperIdx, v);
   }
 
   // Writes a mini-doublet record (SDL/MiniDoublet.h:193-266).  On PS modules
