@@ -28,6 +28,18 @@ def stores(s, slot):
                 continue
             a = s.field(slot, name)
             out[name] = a.reshape(room, -1)[:n].copy()
+    # the quintuplets of every module, and how many were found
+    counts = s.field(slot, "t5.nQuintuplets").astype(np.int64)
+    first = s.field(slot, "ranges.quintupletModuleIndices").astype(np.int64)
+    out["t5.nQuintuplets"], out["t5.totOccupancyQuintuplets"] = counts, s.field(slot, "t5.totOccupancyQuintuplets")
+    live = np.concatenate([np.arange(first[m], first[m] + counts[m]) for m in np.nonzero(counts)[0]]
+                          or [np.zeros(0, np.int64)])
+    room = s.es.info["maxQuintuplets"]
+    for name in lst.field_names():
+        if name.startswith("t5.") and name not in out:
+            a = s.field(slot, name)
+            if a.size % room == 0:
+                out[name] = a.reshape(room, -1)[live]
     return out
 
 

@@ -59,15 +59,17 @@ namespace lst {
     unsigned int nPT5Total;
     unsigned int nPT3Total;
     unsigned int nOutHits;  // output hit-list length of the event's track candidates
-    unsigned int t5CandTotal;     // quintuplet candidates of the event
-    unsigned int t5CandOverflow;  // more candidates than the flag buffer holds
-    unsigned int t5PassCount;     // passing candidates found by kT5Eval
+    unsigned int t5CandTotal;     // quintuplet candidates of the event (probe)
+    unsigned int t5Overflow;      // a quintuplet candidate's key does not fit: walk instead
+    unsigned int t5Tasks;         // tasks of kT5Eval's warps
+    unsigned int t5InnerPerTask;  //   inner triplets of a task, at most 32
+    unsigned int t5Next;          //   and the next one
+    unsigned int t5StagedCount;   // quintuplet candidates that pass the tracklet tests
+    unsigned int t5PassCount;     // passing quintuplet candidates
     unsigned int pixPassCount;    // passing candidates found by kPixEval
     unsigned int pixOverflow;     // a pLS has more candidates than a key can number
     unsigned int pixFallback;     // the pixel stage overflowed the staging: walk instead
     unsigned int pixQueueCount;   // pixel candidates passing the radius criterion and the first tracklet
-    unsigned int t5QueueCount;    // candidates passing the quintuplet pre-selection
-    unsigned int t5QueueBack;     // quintuplet candidates queued from the back (modules not all barrel)
     unsigned int t5SortCount;     // quintuplets binned by eta for the cross-module cleaning
     unsigned int mdNext;          // next task for kCreateMD's warps
     unsigned int lsNext;          // next lower module for kCreateLS's warps
@@ -115,11 +117,11 @@ namespace lst {
     unsigned int* t5CandPre;    // per inner triplet: its first candidate within the module
     unsigned int* t5ModCand;    // per eligible module: candidates
     unsigned int* t5ModOff;     // per eligible module: first candidate of the event
-    unsigned int* t5CandFlag;   // per candidate: 0 = fails, else 1 + slot of its values in t5PassValues
+    unsigned int* t5Task;       // tasks of kT5Eval's warps: module position and 32-triplet chunk
+    struct T5Staged* t5Staged;  // quintuplet candidates that pass the tracklet tests
     T5Values* t5PassValues;     // selection values of passing candidates
-    unsigned int* t5PassC;      //   and their candidate index
-    float* t5DnnFeat;           // candidates staged for the classifier (kT5Eval): 38 inputs each
-    struct T5DnnSlotG* t5DnnSlot;  //   and their selection state
+    unsigned int* t5PassC;      //   their key
+    uint2* t5PassT3;            //   and their triplets
     unsigned int* pixPassC;     // passing candidates: key
     unsigned int* pixPassObj;   //   the T5 / T3 index
     float* pixPassV;            //   the selection values (8 per candidate)
@@ -132,7 +134,6 @@ namespace lst {
     unsigned int* t5BinStart;   // start of each eta bin in t5Order (bins + 2 entries)
     unsigned int* candQueueObj; // and the object of a queued pixel candidate
     unsigned int* candQueue;    // candidates passing a pre-selection (T5, then pT5 / pT3), any order
-    unsigned int* t5ChunkMod;   // per 32 T5 candidates: the eligible module of the first one
     struct TCCleanInfo* tcCleanInfo;  // per track candidate: the pLS cross-cleaning record
     struct PLSRec* plsRec;      // pass-2 pLS records sorted by eta bin
     unsigned int* plsHitHead;   // hit -> pLS index of the pLS cleaning: chain head per bucket

@@ -302,6 +302,7 @@ namespace {
     std::memcpy(&w, es->dnn.data(), sizeof(w));
     LST_CUDA(cudaSetDevice(es->device));
     LST_CUDA(cudaMemcpyToSymbol(lst::c_t5dnn, &w, sizeof(w)));
+  LST_CUDA(cudaMemcpyToSymbol(lst::g_t5dnn, &w, sizeof(w)));
     LST_CUDA(cudaDeviceSynchronize());
     es->haveDnn = true;
     return 0;
@@ -531,15 +532,17 @@ namespace {
         if (ev->t5Method == LST_T5_DNN && !ev->es->haveDnn)
           return setError("the DNN T5 method needs weights (lst_es_load or lst_es_set_t5dnn_weights)");
         bool useDnn = ev->t5Method == LST_T5_DNN;
-        LST_LAUNCH(lst::kT5Eligible, one, 1024, d, v);
-        LST_LAUNCH(lst::kT5Prefix, warpGrid(ev->es->nEligibleMax, 8, count), 256, d, v);
-        LST_LAUNCH(lst::kT5ModScan, one, 1024, d, v);
-        LST_LAUNCH(lst::kT5Pre, dim3(blocksFor(size_t(1) << 20, count), count), kThreads, d, v);
-        LST_LAUNCH(lst::kT5Eval, tunedFlatGrid(ev, kTuT5Eval, count), tunedThreads(ev, kTuT5Eval), d, v, useDnn);
+
+        // 8 inner triplets per warp task: the candidates are very uneven, and with
+        // 32 the heaviest task set kT5Eval's length (8 PU200 events: 350 us, with 8
+        // 204, with 4 191; 64 events: 1057, 1019, 1065)
+        LST_LAUNCH(lst::kT5Eligible, one, 1024, d, v, 8u);
+        LST_LAUNCH(lst::kT5Eval, tunedFlatGrid(ev, kTuT5Eval, count), tunedThreads(ev, kTuT5Eval), d, v);
+        LST_LAUNCH(lst::kT5Classify, dim3(blocksFor(lst::kT5RankCap, count, lst::kT5ClassifyThreads), count),
+                   lst::kT5ClassifyThreads, d, v, useDnn);
         LST_LAUNCH(lst::kT5Walk, warpGrid(ev->es->nEligibleMax, lst::kT5Warps, count), 32 * lst::kT5Warps, d, v,
                    useDnn);
-        LST_LAUNCH_SMEM(lst::kT5RankEmit, dim3(1, count), 1024, lst::kT5RankSmem, d, v);
-        LST_LAUNCH(lst::kT5Emit, warpGrid(ev->es->nEligibleMax, 8, count), 256, d, v, useDnn);
+        LST_LAUNCH(lst::kT5RankEmit, rankGrid, lst::kT5RankThreads, d, v);
         // at most 64 blocks (512 warps) per event: a few hundred tile pairs
         LST_LAUNCH(lst::kT5DedupAfterBuild, dim3(std::min(64u, ceilDiv(kResidentBlocks, count)), count),
                    lst::kT5DedupThreads, d, v);
@@ -673,7 +676,7 @@ namespace {
         {"kT5Prefix", (const void*)lst::kT5Prefix},
         {"kT5ModScan", (const void*)lst::kT5ModScan},
         {"kT5Eval", (const void*)lst::kT5Eval},
-        {"kT5Emit", (const void*)lst::kT5Emit},
+        {"kT5Classify", (const void*)lst::kT5Classify},
         {"kT5RankEmit", (const void*)lst::kT5RankEmit},
         {"kT5Walk", (const void*)lst::kT5Walk},
         {"kT5Probe", (const void*)lst::kT5Probe},
@@ -685,7 +688,6 @@ namespace {
         {"kPLSCleanNear", (const void*)lst::kPLSCleanNear},
         {"kMergePLSFlag", (const void*)lst::kMergePLSFlag},
         {"kPixEval<5>", (const void*)lst::kPixEval<5>},
-        {"kT5Pre", (const void*)lst::kT5Pre},
         {"kPixMid<5>", (const void*)lst::kPixMid<5>},
         {"kPixMid<3>", (const void*)lst::kPixMid<3>},
         {"kPixEval<3>", (const void*)lst::kPixEval<3>},
@@ -984,8 +986,6 @@ int lst_event_create(lst_es* es, int n_slots, uint32_t max_hits, void* stream, l
   // Kernels whose shared memory exceeds the 48 KB default opt in (per device).
   LST_CUDA(cudaFuncSetAttribute(lst::kCrossCleanPLS, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(lst::kXCleanSmem)));
-  LST_CUDA(cudaFuncSetAttribute(lst::kT5RankEmit, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(lst::kT5RankSmem)));
   Carver measure;
   lst::EventView tmp{};
   carveEvent(measure, tmp, ev->sizes);

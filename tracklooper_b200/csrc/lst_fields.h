@@ -233,17 +233,16 @@
   X(t5CandPre, unsigned int, T3)                      \
   X(t5ModCand, unsigned int, L)                       \
   X(t5ModOff, unsigned int, L + 1)                    \
-  X(t5CandFlag, unsigned int, lst::kT5CandCap)        \
-  X(t5PassValues, lst::T5Values, lst::kT5PassCap)     \
-  X(t5PassC, unsigned int, lst::kT5PassCap)           \
-  X(t5DnnFeat, float, 38 * lst::kT5DnnCap)            \
-  X(t5DnnSlot, lst::T5DnnSlotG, lst::kT5DnnCap)      \
+  X(t5Task, unsigned int, T3 / 4 + L)                 \
+  X(t5Staged, lst::T5Staged, lst::kT5StagedCap)       \
+  X(t5PassValues, lst::T5Values, lst::kT5RankCap)     \
+  X(t5PassC, unsigned int, lst::kT5RankCap)           \
+  X(t5PassT3, uint2, lst::kT5RankCap)                 \
   X(pixPassC, unsigned int, lst::kPixPassCap)         \
   X(pixPassObj, unsigned int, lst::kPixPassCap)       \
   X(pixPassV, float, 8 * lst::kPixPassCap)            \
   X(candQueue, unsigned int, lst::kCandQueueCap)        \
   X(candQueueObj, unsigned int, lst::kCandQueueCap)     \
-  X(t5ChunkMod, unsigned int, lst::kT5CandCap / 32)     \
   X(hitMiniSlope, float, H)                           \
   X(t5Order, unsigned int, lst::kT5SortCap)           \
   X(t5OrderPos, uint16_t, lst::kT5SortCap)            \

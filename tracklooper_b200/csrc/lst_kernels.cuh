@@ -22,6 +22,8 @@ namespace lst {
   __constant__ T5DnnWeights c_t5dnn;
   __constant__ float c_t5dnnWP = kT5DnnWP;  // DNN working point of the loaded weights
 
+  __device__ T5DnnWeights g_t5dnn;         // the same weights in memory (kT5Classify stages them in shared memory)
+
   struct ConstDnn {
     __device__ __forceinline__ const T5DnnWeights& get() const { return c_t5dnn; }
   };
@@ -1019,36 +1021,67 @@ namespace lst {
   }
 
   // ========================================================= quintuplets
-  // Eligible T5 seed modules and their offsets (SDL/Quintuplet.h:3117-3213).
+  // A quintuplet candidate's key: its module's position in the eligible-module
+  // list (12 bits), its inner triplet's number in the module (10) and the outer
+  // triplet's position in the list of triplets that start at the shared
+  // mini-doublet (10), so that keys ascend in the order of the reference's loops.
+  // An event that does not fit (there are 2756 eligible modules in both shipped
+  // geometries, and a module holds at most 755 triplets) takes the walk.
+  constexpr unsigned int kT5KeyModuleShift = 20, kT5KeyInnerShift = 10;
+  constexpr unsigned int kT5KeyModules = 1u << (32 - kT5KeyModuleShift);
+  constexpr unsigned int kT5KeyLimit = 1u << kT5KeyInnerShift;  // inner triplets, outer triplets of one
+  constexpr unsigned int kT5StagedCap = 1u << 16;  // candidates per event that pass the tracklet tests
+  constexpr unsigned int kT5RankCap = 8192;        // passing candidates per event
+  // Eligible T5 seed modules and their offsets (SDL/Quintuplet.h:3117-3213),
+  // and the tasks of kT5Eval's warps: up to 32 inner triplets of one module.
   // Each thread takes a contiguous range of modules, so that one block scan
   // of the per-thread sums gives every eligible module its place.
-  __global__ void __launch_bounds__(1024) kT5Eligible(DeviceES es, const EventView* evs) {
+  __global__ void __launch_bounds__(1024) kT5Eligible(DeviceES es, const EventView* evs, unsigned int innerPerTask) {
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = es.nLowerModules;
     const unsigned int per = (n + blockDim.x - 1) / blockDim.x;
     const unsigned int i0 = min(threadIdx.x * per, n), i1 = min(i0 + per, n);
     auto eligible = [&](unsigned int i) { return ev.t3.nTriplets[i] != 0 && es.t5CapIfEligible[i] >= 0; };
-    unsigned int myN = 0, myQ = 0;
+    auto tasksOf = [&](unsigned int i) {
+      const int layer = es.m.layers[i];
+      return layer == 1 || layer == 2 ? (static_cast<unsigned int>(ev.t3.nTriplets[i]) + innerPerTask - 1u) / innerPerTask : 0u;
+    };
+    unsigned int myN = 0, myQ = 0, myT = 0;
     for (unsigned int i = i0; i < i1; ++i)
       if (eligible(i)) {
         ++myN;
         myQ += static_cast<unsigned int>(es.t5CapIfEligible[i]);
+        myT += tasksOf(i);
       }
-    unsigned int totN, totQ;
+    unsigned int totN, totQ, totT;
     unsigned int runN = blockExclusiveScan(myN, totN);
     unsigned int runQ = blockExclusiveScan(myQ, totQ);
+    unsigned int runT = blockExclusiveScan(myT, totT);
     for (unsigned int i = i0; i < i1; ++i) {
       if (!eligible(i))
         continue;
       const unsigned int occ = static_cast<unsigned int>(es.t5CapIfEligible[i]);
+      const unsigned int nTasks = tasksOf(i);
+      for (unsigned int k = 0; k < nTasks; ++k)
+        ev.t5Task[runT++] = (runN << kT5KeyModuleShift) | (k * innerPerTask);
       ev.rg.indicesOfEligibleT5Modules[runN++] = static_cast<uint16_t>(i);
       ev.rg.quintupletModuleIndices[i] = static_cast<int>(runQ);
       ev.rg.quintupletModuleOccupancy[i] = static_cast<int>(occ);
       runQ += occ;
+      // (the modules' counts are written by the kernels that store the T5s, for
+      // the modules that have any)
+      ev.t5.nQuintuplets[i] = 0;
+      ev.t5.totOccupancyQuintuplets[i] = 0;
     }
     if (threadIdx.x == 0) {
       *ev.rg.nEligibleT5Modules = static_cast<uint16_t>(totN);
       *ev.rg.device_nTotalQuints = totQ;
+      ev.sc->t5Tasks = totT;
+      ev.sc->t5InnerPerTask = innerPerTask;
+      ev.sc->t5Overflow = totN > kT5KeyModules ? 1u : 0u;
+      ev.sc->t5Next = 0;
+      ev.sc->t5StagedCount = 0;
+      ev.sc->t5PassCount = 0;
     }
   }
 
@@ -1115,19 +1148,20 @@ namespace lst {
 
   // ------------------------------------------ T5 as a candidate work list
   // The warp-per-module walk above leaves most lanes idle: a few modules own
-  // most candidates and the candidates diverge early.  The batched path
-  // instead (1) stores each module's candidate prefix over its inner
-  // triplets, (2) scans module totals, (3) evaluates every candidate on its
-  // own thread, and (4) walks each module's pass flags in candidate order,
-  // re-evaluating only the passing candidates to store them at their rank.
-  // Candidate c of module w is the c-th (inner, outer) pair of the walk, so
-  // ranks, caps and stored values are those of the walk.  Events with more
-  // candidates than the flag buffer holds take the walk instead.
-  constexpr unsigned int kT5CandCap = 1u << 21;  // candidates per event
-  constexpr unsigned int kCandQueueCap = 1u << 18;  // pre-selected candidates per event (T5, pT5, pT3)
+  // most candidates and the candidates diverge early.  Instead kT5Eval deals out
+  // the modules' inner triplets, 32 to a warp task, and runs the selection with
+  // full warps, kT5Classify the rest of it on what reaches the classifier, and
+  // kT5RankEmit stores the passing candidates in key order, so ranks, caps and
+  // stored values are those of the walk.  Events that overflow a list take the
+  // walk instead.
+  constexpr unsigned int kCandQueueCap = 1u << 18;  // pre-selected pT5 / pT3 candidates per event
   constexpr unsigned int kT5SortCap = 1u << 15;     // quintuplets per event sorted by eta for the TC cleaning
-  constexpr unsigned int kT5PassCap = 1u << 16;  // passing candidates per event whose values are kept
+  __device__ __forceinline__ bool t5NeedsWalk(const EventView& ev) {
+    return ev.forceWalk || ev.sc->t5Overflow || ev.sc->t5StagedCount > kT5StagedCap || ev.sc->t5PassCount > kT5RankCap;
+  }
 
+  // Candidate numbering over the event, for the probe: the prefix of the
+  // candidates over a module's inner triplets, and of the modules.
   __device__ __forceinline__ unsigned int t5CandidatesOf(const EventView& ev, unsigned int innerT3) {
     const Triplets& t3 = ev.t3;
     uint16_t lm3 = t3.lowerModuleIndices[3 * innerT3 + 2];
@@ -1203,200 +1237,336 @@ namespace lst {
     if (threadIdx.x == 0) {
       ev.t5ModOff[nE] = carry;
       ev.sc->t5CandTotal = carry;
-      ev.sc->t5CandOverflow = (carry > kT5CandCap || ev.forceWalk) ? 1u : 0u;
-      ev.sc->t5PassCount = 0;
-      ev.sc->t5QueueCount = 0;
-      ev.sc->t5QueueBack = 0;
-    }
-    // The chunk table: candidate 32 j lies in eligible module t5ChunkMod[j]
-    // (filled whenever the candidates are decoded, i.e. without overflow).
-    if (carry > kT5CandCap)
-      return;
-    __syncthreads();
-    for (unsigned int i = threadIdx.x; i < nE; i += blockDim.x) {
-      const unsigned int a = ev.t5ModOff[i], b = ev.t5ModOff[i + 1];
-      for (unsigned int j = (a + 31u) >> 5; j < ((b + 31u) >> 5); ++j)
-        ev.t5ChunkMod[j] = i;
     }
   }
 
-  // (inner T3, outer T3, lower modules) of quintuplet candidate c.
-  __device__ __forceinline__ void t5Decode(const EventView& ev, unsigned int c, unsigned int& innerT3,
-                                           unsigned int& outerT3, uint16_t* lm) {
-    // The largest w with off[w] <= c: from the chunk table and a short walk
-    // (eligible modules without candidates are stepped over).
-    const unsigned int* off = ev.t5ModOff;
-    int lo = static_cast<int>(ev.t5ChunkMod[c >> 5]);
-    while (off[lo + 1] <= c)
-      ++lo;
-    const uint16_t lm1 = ev.rg.indicesOfEligibleT5Modules[lo];
-    t5Candidate(ev, ev.rg.tripletModuleIndices[lm1], ev.t3.nTriplets[lm1], c - off[lo], innerT3, outerT3);
-    lm[0] = lm1;
-    lm[1] = ev.t3.lowerModuleIndices[3 * innerT3 + 1];
-    lm[2] = ev.t3.lowerModuleIndices[3 * innerT3 + 2];
-    lm[3] = ev.t3.lowerModuleIndices[3 * outerT3 + 1];
-    lm[4] = ev.t3.lowerModuleIndices[3 * outerT3 + 2];
+  // The T5 selection up to the classifier (SDL/Quintuplet.h:2508-2920).  A warp
+  // takes a task of up to 32 inner triplets of one module: its lanes fetch where
+  // their outer triplets are listed (those that start at the inner triplet's
+  // third mini-doublet), and the candidates are tested 32 at a time.  Each long
+  // test runs when the warp's own queue for it, in shared memory, holds a warp
+  // full of candidates: the radius tests leave about a quarter of the candidates
+  // of a PU200 event, the first tracklet test 70% of those, the second 45%; what
+  // passes goes to the event's list in any order.  The two tracklet tests share
+  // one copy of the code.  A candidate's outcome does not depend on which thread
+  // evaluates it.
+  //
+  // Bound by the latency of dependent gathers and of instruction fetches: with
+  // three inlined tracklet algorithms and the r-z fit's tables in this kernel it
+  // waited mostly for instructions (64 PU200 events: 1019 us, now 510).  Numbering
+  // the candidates over the event (a prefix kernel, a scan, a radius kernel that
+  // filled a queue in memory) and evaluating the classifier at the end of this
+  // kernel's blocks took, with the emission, 1.46 ms for 64 PU200 events and 360
+  // us for one; this, kT5Classify and kT5RankEmit take 0.82 ms and 120 us.
+  constexpr int kT5EvalWarps = 4;
+  struct T5Scratch {
+    unsigned int pre[33];
+    unsigned int listStart[32];  // per inner triplet: its first entry in t3ByMD
+    unsigned int outerBase[32];  //   and the first triplet of that list's module
+    unsigned int key[2][64], inner[2][64], outer[2][64];  // candidates waiting for the two tracklet tests
+  };
+  struct T5Staged {
+    unsigned int key, inner, outer;
+  };
+  struct T5Objects {  // a candidate's segments, mini-doublets and modules
+    unsigned int seg1, seg3, seg4;
+    unsigned int md[5];
+    uint16_t lm[5];
+  };
+  __device__ __forceinline__ void t5Objects(const EventView& ev, unsigned int inner, unsigned int outer, T5Objects& o) {
+    const Triplets& t = ev.t3;
+    const unsigned int* mdIdx = ev.ls.mdIndices;
+    const unsigned int seg2 = t.segmentIndices[2 * inner + 1];
+    o.seg1 = t.segmentIndices[2 * inner];
+    o.seg3 = t.segmentIndices[2 * outer];
+    o.seg4 = t.segmentIndices[2 * outer + 1];
+    o.lm[0] = t.lowerModuleIndices[3 * inner];
+    o.lm[1] = t.lowerModuleIndices[3 * inner + 1];
+    o.lm[2] = t.lowerModuleIndices[3 * inner + 2];
+    o.lm[3] = t.lowerModuleIndices[3 * outer + 1];
+    o.lm[4] = t.lowerModuleIndices[3 * outer + 2];
+    o.md[0] = mdIdx[2 * o.seg1];
+    o.md[1] = mdIdx[2 * seg2];
+    o.md[2] = mdIdx[2 * seg2 + 1];
+    o.md[3] = mdIdx[2 * o.seg3 + 1];
+    o.md[4] = mdIdx[2 * o.seg4 + 1];
   }
 
-  // Pre-selection of the quintuplet candidates: the shared-MD and radius tests
-  // that open the selection, which most candidates fail.  A failing candidate
-  // gets its flag here; the survivors are queued in any order for kT5Eval,
-  // which then runs the long tests with all lanes of a warp busy (a
-  // candidate's outcome does not depend on the thread that evaluates it).
-  // Candidates on all-barrel module patterns fill the queue from the front,
-  // the others from the back, so that a warp mostly runs one set of the
-  // tracklet algorithms.  A full queue makes kT5Eval evaluate every candidate.
-  __global__ void __launch_bounds__(256) kT5Pre(DeviceES es, const EventView* evs) {
+  __global__ void __launch_bounds__(LST_LB_T5EVAL) kT5Eval(DeviceES es, const EventView* evs) {
+    __shared__ T5Scratch sScratch[kT5EvalWarps];
     const EventView& ev = evs[blockIdx.y];
-    if (ev.sc->t5CandOverflow)
+    if (ev.forceWalk || ev.sc->t5Overflow)
       return;
-    const unsigned int total = ev.sc->t5CandTotal;
-    const unsigned int stride = gridDim.x * blockDim.x;
-    for (unsigned int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-      const unsigned int c = base + laneId();
-      bool pass = false, mixed = false;
-      if (c < total) {
-        unsigned int innerT3, outerT3;
-        uint16_t lm[5];
-        t5Decode(ev, c, innerT3, outerT3, lm);
-        T5Values v;
-        T5Stage st;
-        pass = t5RadiusStage(es.m, ev.md, ev.ls, ev.t3, lm, innerT3, outerT3, v, st);
-        if (!pass)
-          ev.t5CandFlag[c] = 0;
-        else
-          mixed = st.kind > 0;
+    T5Scratch& sc = sScratch[threadIdx.x >> 5];
+    const Triplets& t3 = ev.t3;
+    const unsigned int nTasks = ev.sc->t5Tasks, innerPerTask = ev.sc->t5InnerPerTask;
+    const unsigned int lane = laneId();
+    bool more = true;                // the event may have tasks left
+    unsigned int module = 0, inner0 = 0, t3Base = 0;  // the current task: module position, first inner triplet
+    unsigned int f0 = 0, total = 0;  //   and its candidates from f0 on
+    int nInner = 0;
+    unsigned int n0 = 0, n1 = 0;  // entries in the two queues
+    while (true) {
+      while (n0 < 32u) {
+        if (f0 < total) {
+          const unsigned int f = f0 + lane;
+          f0 += 32u;
+          bool pass = false;
+          unsigned int key = 0, inner = 0, outer = 0;
+          if (f < total) {
+            const int i = findSlot(sc.pre, nInner, f);
+            const unsigned int pos = f - sc.pre[i];
+            inner = t3Base + inner0 + unsigned(i);
+            outer = sc.outerBase[i] + ev.t3ByMD[sc.listStart[i] + pos];
+            key = (module << kT5KeyModuleShift) | ((inner0 + unsigned(i)) << kT5KeyInnerShift) | pos;
+            if (pos >= kT5KeyLimit || inner0 + unsigned(i) >= kT5KeyLimit) {
+              ev.sc->t5Overflow = 1;
+            } else {
+              const uint16_t lm[5] = {t3.lowerModuleIndices[3 * inner], t3.lowerModuleIndices[3 * inner + 1],
+                                      t3.lowerModuleIndices[3 * inner + 2], t3.lowerModuleIndices[3 * outer + 1],
+                                      t3.lowerModuleIndices[3 * outer + 2]};
+              T5Values v;
+              T5Stage st;
+              pass = t5RadiusStage(es.m, ev.md, ev.ls, t3, lm, inner, outer, v, st);
+            }
+          }
+          const unsigned int ok = __ballot_sync(kFullMask, pass);
+          if (pass) {
+            const unsigned int k = n0 + __popc(ok & lanesBelowMask());
+            sc.key[0][k] = key;
+            sc.inner[0][k] = inner;
+            sc.outer[0][k] = outer;
+          }
+          n0 += __popc(ok);
+        } else if (more) {
+          const unsigned int task = warpNextTask(&ev.sc->t5Next);
+          more = task < nTasks;
+          if (!more)
+            break;
+          __syncwarp();  // the previous task's scratch has been read
+          module = ev.t5Task[task] >> kT5KeyModuleShift;
+          inner0 = ev.t5Task[task] & ((1u << kT5KeyModuleShift) - 1u);
+          const uint16_t lm1 = ev.rg.indicesOfEligibleT5Modules[module];
+          t3Base = ev.rg.tripletModuleIndices[lm1];
+          nInner = int(min(innerPerTask, static_cast<unsigned int>(t3.nTriplets[lm1]) - inner0));
+          total = warpPrefix(sc.pre, nInner, [&](int i) {
+            const unsigned int in = t3Base + inner0 + unsigned(i);
+            const uint16_t lm3 = t3.lowerModuleIndices[3 * in + 2];
+            const unsigned int mdMid = ev.ls.mdIndices[2 * t3.segmentIndices[2 * in + 1] + 1];
+            if (t3.nTriplets[lm3] == 0)
+              return 0u;
+            const unsigned int base = ev.rg.tripletModuleIndices[lm3];
+            sc.outerBase[i] = base;
+            sc.listStart[i] = base + ev.mdT3Start[mdMid];
+            return static_cast<unsigned int>(ev.mdT3Count[mdMid]);
+          });
+          f0 = 0;
+        } else {
+          break;
+        }
       }
-      const unsigned int maskF = __ballot_sync(kFullMask, pass && !mixed);
-      const unsigned int maskB = __ballot_sync(kFullMask, pass && mixed);
-      if ((maskF | maskB) == 0u)
-        continue;
-      unsigned int startF = 0, startB = 0;
-      if (laneId() == 0) {
-        if (maskF)
-          startF = atomicAdd(&ev.sc->t5QueueCount, __popc(maskF));
-        if (maskB)
-          startB = atomicAdd(&ev.sc->t5QueueBack, __popc(maskB));
-      }
-      startF = __shfl_sync(kFullMask, startF, 0);
-      startB = __shfl_sync(kFullMask, startB, 0);
+      __syncwarp();
+      // the second queue if it holds a warp full, or, at the end of the candidates,
+      // the first that holds any
+      const bool second = n1 >= 32u || n0 == 0;
+      const unsigned int have = second ? n1 : n0;
+      if (have == 0)
+        break;
+      const unsigned int take = min(have, 32u), at = have - take;
+      bool pass = lane < take;
+      unsigned int key = 0, inner = 0, outer = 0;
       if (pass) {
-        const unsigned int k = mixed ? startB + __popc(maskB & lanesBelowMask())
-                                     : startF + __popc(maskF & lanesBelowMask());
-        if (k < kCandQueueCap)
-          ev.candQueue[mixed ? kCandQueueCap - 1 - k : k] = c;
+        key = sc.key[second][at + lane];
+        inner = sc.inner[second][at + lane];
+        outer = sc.outer[second][at + lane];
+      }
+      (second ? n1 : n0) = at;
+      __syncwarp();  // the entries have been read
+      if (pass) {
+        T5Objects o;
+        t5Objects(ev, inner, outer, o);
+        pass = t4Select(es.m, ev.md, ev.ls, t5Tracklet(o.lm, o.seg1, second ? o.seg4 : o.seg3, o.md, second ? 1 : 0));
+      }
+      const unsigned int ok = __ballot_sync(kFullMask, pass);
+      if (ok == 0u)
+        continue;
+      if (!second) {
+        if (pass) {
+          const unsigned int k = n1 + __popc(ok & lanesBelowMask());
+          sc.key[1][k] = key;
+          sc.inner[1][k] = inner;
+          sc.outer[1][k] = outer;
+        }
+        n1 += __popc(ok);
+        __syncwarp();
+        continue;
+      }
+      unsigned int start = 0;
+      if (lane == 0)
+        start = atomicAdd(&ev.sc->t5StagedCount, __popc(ok));
+      start = __shfl_sync(kFullMask, start, 0);
+      const unsigned int k = start + __popc(ok & lanesBelowMask());
+      if (pass && k < kT5StagedCap)
+        ev.t5Staged[k] = T5Staged{key, inner, outer};
+    }
+  }
+
+  // The forward pass of the classifier for a warp's candidates, accumulating in
+  // the reference's order (SDL/NeuralNetwork.h:116-164; t5DnnForward is the same
+  // sums one column at a time).  act: this thread's column of the block's
+  // activations in shared memory, row stride kT5ClassifyThreads.
+  constexpr int kT5ClassifyThreads = 64;
+  template <int kRows>
+  __device__ __forceinline__ void t5DnnLayer(const float* w, const float* b, float* act) {
+    float acc[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c)
+      acc[c] = 0;
+#pragma unroll 2
+    for (int in = 0; in < kRows; ++in) {
+      const float x = act[in * kT5ClassifyThreads];
+      const float4* row = reinterpret_cast<const float4*>(w + in * 32);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 q = row[c];
+        acc[4 * c] += x * q.x;
+        acc[4 * c + 1] += x * q.y;
+        acc[4 * c + 2] += x * q.z;
+        acc[4 * c + 3] += x * q.w;
       }
     }
-  }
-
-  // Records a candidate that passes the T5 selection: its values go to the
-  // pass buffer (flag = slot + 1), or, when the buffer is full, the flag asks
-  // for re-evaluation at emission (flag = kT5PassCap + 1).
-  __device__ __forceinline__ void t5Keep(const EventView& ev, unsigned int c, const T5Values& v) {
-    const unsigned int slot = atomicAdd(&ev.sc->t5PassCount, 1u);
-    if (slot < kT5PassCap) {
-      ev.t5PassValues[slot] = v;
-      ev.t5PassC[slot] = c;
-      ev.t5CandFlag[c] = slot + 1;
-    } else {
-      ev.t5CandFlag[c] = kT5PassCap + 1;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      const float v = acc[c] + b[c];
+      act[c * kT5ClassifyThreads] = v > 0.f ? v : 0.f;
     }
   }
 
-  // The T5 selection of the queued candidates with the DNN classifier in the
-  // same kernel (SDL/Quintuplet.h:2921-2941 evaluates it inline).  Each
-  // thread runs every test before the classifier on its candidates; a
-  // candidate that reaches the classifier leaves its 38 inputs and its
-  // selection state in the block's slice of the event's staging area (its
-  // own rows, in L2) instead of running the 38-32-32-1 forward pass there
-  // and then, on a few lanes of its warp.  When the block has evaluated all
-  // of its candidates, its threads classify the block's staged candidates,
-  // one per thread with the weights in shared memory, so that the forward
-  // passes run on full warps.  A candidate that finds its block's slice full
-  // is classified at once by its own thread; the arithmetic is the same
-  // either way.
-  __global__ void __launch_bounds__(LST_LB_T5EVAL) kT5Eval(DeviceES es, const EventView* evs, bool useDnn) {
-    __shared__ T5DnnWeights sW;
+  // The rest of the T5 selection (SDL/Quintuplet.h:2715-2984) on the candidates
+  // that pass the tracklet tests, a thread each: the r-z fit, and on those that
+  // pass it (about half, gathered in shared memory so that the threads are filled
+  // again) the circle regression, the DNN (or the cut-only method's chi-squared
+  // table) and the chi-squared of the non-anchor hits.  The weights come from
+  // memory (a copy beside the constant one, whose reads at 32 addresses a warp are
+  // served one by one), only in blocks that have a candidate.
+  __global__ void __launch_bounds__(kT5ClassifyThreads) kT5Classify(DeviceES es, const EventView* evs, bool useDnn) {
+    __shared__ __align__(16) float sW[kT5DnnParams + 3];
+    __shared__ float sAct[38 * kT5ClassifyThreads];
+    __shared__ T5Staged sFit[2 * kT5ClassifyThreads];  // candidates that pass the r-z fit
+    __shared__ float sRz[2 * kT5ClassifyThreads];
+    __shared__ bool sTight[2 * kT5ClassifyThreads];
     __shared__ unsigned int sCount;
     const EventView& ev = evs[blockIdx.y];
-    if (ev.sc->t5CandOverflow)
+    const unsigned int n = ev.sc->t5StagedCount;
+    if (ev.forceWalk || ev.sc->t5Overflow || n > kT5StagedCap || blockIdx.x * kT5ClassifyThreads >= n)
       return;
+    const T5DnnWeights& w = *reinterpret_cast<const T5DnnWeights*>(sW);
     if (useDnn) {
-      const float* src = reinterpret_cast<const float*>(&c_t5dnn);
-      float* dst = reinterpret_cast<float*>(&sW);
-      for (int i = threadIdx.x; i < kT5DnnParams; i += blockDim.x)
-        dst[i] = src[i];
+      const float* src = reinterpret_cast<const float*>(&g_t5dnn);
+      for (int i = threadIdx.x; i < kT5DnnParams; i += kT5ClassifyThreads)
+        sW[i] = src[i];
     }
     if (threadIdx.x == 0)
       sCount = 0;
     __syncthreads();
     const float wp = c_t5dnnWP;
-    const unsigned int slice = kT5DnnCap / gridDim.x;
-    const unsigned int base = blockIdx.x * slice;
-    const unsigned int total = ev.sc->t5CandTotal;
-    const unsigned int front = ev.sc->t5QueueCount, back = ev.sc->t5QueueBack;
-    const bool fromQueue = front <= kCandQueueCap && back <= kCandQueueCap - front;
-    const unsigned int n = fromQueue ? front + back : total;
-    for (unsigned int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-      const unsigned int c = fromQueue ? ev.candQueue[q < front ? q : kCandQueueCap - 1 - (q - front)] : q;
-      unsigned int innerT3, outerT3;
-      uint16_t lm[5];
-      t5Decode(ev, c, innerT3, outerT3, lm);
-      T5Values v;
-      T5Stage st;
-      if (!t5SelectPre(es.m, ev.md, ev.ls, ev.t3, lm, innerT3, outerT3, v, st)) {
-        ev.t5CandFlag[c] = 0;
-        continue;
-      }
-      const unsigned int k = useDnn ? atomicAdd(&sCount, 1u) : slice;
-      if (k < slice) {
-        float feat[38];
-        t5DnnFeatures(es.m, ev.md, ev.ls, ev.t3, st.xs, st.ys, st.mdIdx, lm, innerT3, v.innerRadius, v.outerRadius,
-                      v.bridgeRadius, feat);
-        for (int i = 0; i < 38; ++i)
-          ev.t5DnnFeat[size_t(base + k) * 38 + i] = feat[i];
-        T5DnnSlotG& sl = ev.t5DnnSlot[base + k];
-        sl.v = v;
-        for (int i = 0; i < 5; ++i) {
-          sl.mdIdx[i] = st.mdIdx[i];
-          sl.lm[i] = lm[i];
+    const MiniDoublets& md = ev.md;
+    for (unsigned int base = blockIdx.x * kT5ClassifyThreads;; base += gridDim.x * kT5ClassifyThreads) {
+      const bool more = base < n;
+      const unsigned int q = base + threadIdx.x;
+      if (more && q < n) {
+        const T5Staged st = ev.t5Staged[q];
+        T5Objects o;
+        t5Objects(ev, st.inner, st.outer, o);
+        const float radius = ev.t3.circleRadius[st.inner];
+        float rz = 0;
+        bool tight = false;
+        if (t5PassRZ(es.m, md, o.md, o.lm, rz, 2 * k2Rinv1GeVf * radius, radius, ev.t3.circleCenterX[st.inner],
+                     ev.t3.circleCenterY[st.inner], tight)) {
+          const unsigned int k = atomicAdd(&sCount, 1u);  // at most 63 left over and 64 new ones
+          sFit[k] = st;
+          sRz[k] = rz;
+          sTight[k] = tight;
         }
-        sl.cand = c;
-        sl.tight = st.tight ? 1 : 0;
-      } else if (t5Classify(es.m, ev.md, ev.ls, ev.t3, sW, useDnn, wp, lm, innerT3, v, st)) {
-        t5Keep(ev, c, v);
-      } else {
-        ev.t5CandFlag[c] = 0;
       }
-    }
-    __syncthreads();
-    const unsigned int m = sCount < slice ? sCount : slice;
-    for (unsigned int k = threadIdx.x; k < m; k += blockDim.x) {
-      float feat[38];
-      for (int i = 0; i < 38; ++i)
-        feat[i] = ev.t5DnnFeat[size_t(base + k) * 38 + i];
-      const float inference = t5DnnForward(sW, feat);
-      const T5DnnSlotG& sl = ev.t5DnnSlot[base + k];
-      if (!(inference > wp)) {
-        ev.t5CandFlag[sl.cand] = 0;
+      __syncthreads();
+      const unsigned int have = sCount;
+      __syncthreads();  // everyone has read the count before anyone adds to it again
+      if (have < kT5ClassifyThreads && more)
         continue;
+      const unsigned int take = min(have, unsigned(kT5ClassifyThreads)), at = have - take + threadIdx.x;
+      bool mine = threadIdx.x < take;
+      T5Staged st{};
+      T5Values v;
+      bool tight = false;
+      if (mine) {
+        st = sFit[at];
+        v.rzChiSquared = sRz[at];
+        tight = sTight[at];
       }
-      T5Values v = sl.v;
-      t5NonAnchor(es.m, ev.md, sl.lm, sl.mdIdx, v);
-      v.tightCutFlag = sl.tight != 0 and (inference > wp);
-      t5Keep(ev, sl.cand, v);
+      if (threadIdx.x == 0)
+        sCount = have - take;
+      __syncthreads();  // the entries have been read, the count is set
+      if (mine) {
+        T5Objects o;
+        t5Objects(ev, st.inner, st.outer, o);
+        v.innerRadius = ev.t3.circleRadius[st.inner];
+        v.outerRadius = ev.t3.circleRadius[st.outer];
+        float xs[5], ys[5];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          xs[i] = md.rec[o.md[i]].x;
+          ys[i] = md.rec[o.md[i]].y;
+        }
+        float g, f;
+        v.bridgeRadius = circleFrom3(xs[1], ys[1], xs[2], ys[2], xs[3], ys[3], g, f);
+        t5Regression(es.m, o.lm, xs, ys, v);
+        if (useDnn) {
+          float feat[38];
+          t5DnnFeatures(es.m, md, ev.ls, ev.t3, xs, ys, o.md, o.lm, st.inner, v.innerRadius, v.outerRadius,
+                        v.bridgeRadius, feat);
+          float* act = sAct + threadIdx.x;
+#pragma unroll
+          for (int i = 0; i < 38; ++i)
+            act[i * kT5ClassifyThreads] = feat[i];
+          t5DnnLayer<38>(w.w0, w.b0, act);
+          t5DnnLayer<32>(w.w2, w.b2, act);
+          float out = 0;
+#pragma unroll 8
+          for (int in = 0; in < 32; ++in)
+            out += act[in * kT5ClassifyThreads] * w.w4[in];
+          out += w.b4[0];
+          const float inference = fexp(out) / (fexp(out) + 1);
+          mine = inference > wp;
+          tight = tight and (inference > wp);
+        } else if (v.regressionRadius < 5.0f / (2.f * k2Rinv1GeVf)) {
+          mine = t5PassRPhiChi2(es.m, o.lm, v.chiSquared);
+        }
+        if (mine) {
+          t5NonAnchor(es.m, md, o.lm, o.md, v);
+          v.tightCutFlag = tight;
+          const unsigned int slot = atomicAdd(&ev.sc->t5PassCount, 1u);
+          if (slot < kT5RankCap) {
+            ev.t5PassValues[slot] = v;
+            ev.t5PassC[slot] = st.key;
+            ev.t5PassT3[slot] = make_uint2(st.inner, st.outer);
+          }
+        }
+      }
+      if (!more && have <= kT5ClassifyThreads)
+        break;
     }
   }
 
-  // The warp-per-module walk, for events whose candidates overflow the flag
-  // buffer (a no-op for the others).
+  // The warp-per-module walk, for events that overflow a list (a no-op for the
+  // others).
   // Register budget: this fallback does work only for events whose candidates
   // overflow the lists; for the others its blocks return at once, and the
   // budget lets more of them be resident, so the launch drains in fewer waves.
   __global__ void __launch_bounds__(128, 8) kT5Walk(DeviceES es, const EventView* evs, bool useDnn) {
     __shared__ unsigned int sPre[kT5Warps][kT5MaxInner + 1];
     const EventView& ev = evs[blockIdx.y];
-    if (!ev.sc->t5CandOverflow)
+    if (!t5NeedsWalk(ev))
       return;
     const int wib = threadIdx.x >> 5;
     const int nE = *ev.rg.nEligibleT5Modules;
@@ -1406,142 +1576,42 @@ namespace lst {
     }
   }
 
-  // The passing quintuplet candidates stored in candidate order, one block per
-  // event: their (candidate index, value slot) keys are bitonic-sorted in
-  // shared memory, so that a candidate's position among the passing ones of
-  // its module -- the reference's occupancy rank -- comes from two binary
-  // searches.  Events with more passing candidates than kT5RankCap leave the
-  // storing to kT5Emit's per-module walk.
-  constexpr unsigned int kT5RankCap = 8192;
-  constexpr size_t kT5RankSmem = kT5RankCap * sizeof(unsigned long long);
-  __global__ void __launch_bounds__(1024) kT5RankEmit(DeviceES es, const EventView* evs) {
-    extern __shared__ __align__(16) unsigned char rsm[];
-    unsigned long long* sKey = reinterpret_cast<unsigned long long*>(rsm);
+  // The passing quintuplet candidates stored in key order: a thread per candidate
+  // counts the candidates of its module with a smaller key -- the reference's
+  // occupancy rank -- and all of the module's, over the event's keys in shared
+  // memory; the one with the largest key writes the module's counts.  Bound by
+  // the scattered stores; one block per event with a bitonic sort of the keys took
+  // 76 us for 8 PU200 events, up to 16 blocks 29.
+  constexpr int kT5RankThreads = 128;
+  __global__ void __launch_bounds__(kT5RankThreads) kT5RankEmit(DeviceES es, const EventView* evs) {
+    __shared__ unsigned int sKey[kT5RankCap];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.sc->t5PassCount;
-    if (ev.sc->t5CandOverflow || n > kT5RankCap || ev.forceWalk)
+    if (t5NeedsWalk(ev) || blockIdx.x * kT5RankThreads >= n)
       return;
-    unsigned int N = 1;
-    while (N < n)
-      N <<= 1;
-    for (unsigned int t = threadIdx.x; t < N; t += blockDim.x)
-      sKey[t] = t < n ? (static_cast<unsigned long long>(ev.t5PassC[t]) << 32) | t : ~0ull;
+    for (unsigned int j = threadIdx.x; j < n; j += kT5RankThreads)
+      sKey[j] = ev.t5PassC[j];
     __syncthreads();
-    for (unsigned int k = 2; k <= N; k <<= 1) {
-      for (unsigned int j = k >> 1; j > 0; j >>= 1) {
-        for (unsigned int i = threadIdx.x; i < N; i += blockDim.x) {
-          const unsigned int l = i ^ j;
-          if (l > i) {
-            const unsigned long long a = sKey[i], b = sKey[l];
-            if (((i & k) == 0) == (a > b)) {
-              sKey[i] = b;
-              sKey[l] = a;
-            }
-          }
-        }
-        __syncthreads();
-      }
-    }
-    const int nE = *ev.rg.nEligibleT5Modules;
-    const unsigned int* off = ev.t5ModOff;
-    // first sorted position whose candidate index is at least c
-    auto lowerBound = [&](unsigned int c) {
-      unsigned int lo = 0, hi = n;
-      while (lo < hi) {
-        const unsigned int mid = (lo + hi) >> 1;
-        if (static_cast<unsigned int>(sKey[mid] >> 32) < c)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      return lo;
-    };
     Triplets t3 = ev.t3;
     Quintuplets t5 = ev.t5;
-    for (unsigned int p = threadIdx.x; p < n; p += blockDim.x) {
-      const unsigned int c = static_cast<unsigned int>(sKey[p] >> 32);
-      const unsigned int slot = static_cast<unsigned int>(sKey[p] & 0xffffffffu);
-      int lo = 0, hi = nE;  // module position w: largest with off[w] <= c
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (off[mid] <= c)
-          lo = mid;
-        else
-          hi = mid;
+    for (unsigned int q = blockIdx.x * kT5RankThreads + threadIdx.x; q < n; q += gridDim.x * kT5RankThreads) {
+      const unsigned int key = sKey[q], w = key >> kT5KeyModuleShift, base = w << kT5KeyModuleShift;
+      unsigned int r = 0, count = 0;
+      for (unsigned int j = 0; j < n; ++j) {
+        const unsigned int d = sKey[j] - base;  // wraps to a large value below the module's keys
+        r += d < key - base ? 1u : 0u;
+        count += d < (1u << kT5KeyModuleShift) ? 1u : 0u;
       }
-      const uint16_t lm1 = ev.rg.indicesOfEligibleT5Modules[lo];
-      const int layer = es.m.layers[lm1];
-      if (layer != 1 && layer != 2)
-        continue;
-      const unsigned int r = p - lowerBound(off[lo]);
-      if (int(r) >= ev.rg.quintupletModuleOccupancy[lm1])
-        continue;
-      unsigned int innerT3, outerT3;
-      t5Candidate(ev, ev.rg.tripletModuleIndices[lm1], t3.nTriplets[lm1], c - off[lo], innerT3, outerT3);
-      uint16_t lm[5] = {lm1, t3.lowerModuleIndices[3 * innerT3 + 1], t3.lowerModuleIndices[3 * innerT3 + 2],
-                        t3.lowerModuleIndices[3 * outerT3 + 1], t3.lowerModuleIndices[3 * outerT3 + 2]};
-      storeT5(ev.md, ev.ls, t3, t5, innerT3, outerT3, lm, layer, ev.t5PassValues[slot],
-              ev.rg.quintupletModuleIndices[lm1] + r);
-    }
-    for (int w = threadIdx.x; w < nE; w += blockDim.x) {
       const uint16_t lm1 = ev.rg.indicesOfEligibleT5Modules[w];
-      const int layer = es.m.layers[lm1];
-      if (layer != 1 && layer != 2)
-        continue;
-      const unsigned int count = lowerBound(off[w] + ev.t5ModCand[w]) - lowerBound(off[w]);
       const int cap = ev.rg.quintupletModuleOccupancy[lm1];
-      t5.nQuintuplets[lm1] = (int(count) < cap) ? count : (cap > 0 ? unsigned(cap) : 0u);
-      t5.totOccupancyQuintuplets[lm1] = count;
-      if (int(count) > cap)
-        atomicOr(&ev.sc->status, kStatusCapOverflow);
-    }
-  }
-
-  // Register budget: this fallback does work only for events whose candidates
-  // overflow the lists; for the others its blocks return at once, and the
-  // budget lets more of them be resident, so the launch drains in fewer waves.
-  __global__ void __launch_bounds__(256, 4) kT5Emit(DeviceES es, const EventView* evs, bool useDnn) {
-    const EventView& ev = evs[blockIdx.y];
-    if (ev.sc->t5CandOverflow || (ev.sc->t5PassCount <= kT5RankCap && !ev.forceWalk))
-      return;
-    const int wpb = blockDim.x >> 5;
-    const int nE = *ev.rg.nEligibleT5Modules;
-    ConstDnn dnn;
-    for (int w = blockIdx.x * wpb + (threadIdx.x >> 5); w < nE; w += gridDim.x * wpb) {
-      const uint16_t lm1 = ev.rg.indicesOfEligibleT5Modules[w];
-      const int layer = es.m.layers[lm1];
-      if (layer != 1 && layer != 2)
-        continue;
-      const unsigned int total = ev.t5ModCand[w];
-      const unsigned int off = ev.t5ModOff[w];
-      const unsigned int t3Base = ev.rg.tripletModuleIndices[lm1];
-      const unsigned int nInner = ev.t3.nTriplets[lm1];
-      const int cap = ev.rg.quintupletModuleOccupancy[lm1];
-      const unsigned int base = ev.rg.quintupletModuleIndices[lm1];
-      Triplets t3 = ev.t3;
-      Quintuplets t5 = ev.t5;
-      unsigned int count = 0;
-      for (unsigned int start = 0; start < total; start += 32) {
-        const unsigned int f = start + laneId();
-        const unsigned int flag = f < total ? ev.t5CandFlag[off + f] : 0u;
-        const bool ok = flag != 0;
-        unsigned int tot;
-        const unsigned int r = count + warpRank(ok, tot);
-        if (ok && int(r) < cap) {
-          unsigned int innerT3, outerT3;
-          t5Candidate(ev, t3Base, nInner, f, innerT3, outerT3);
-          uint16_t lm[5] = {lm1, t3.lowerModuleIndices[3 * innerT3 + 1], t3.lowerModuleIndices[3 * innerT3 + 2],
-                            t3.lowerModuleIndices[3 * outerT3 + 1], t3.lowerModuleIndices[3 * outerT3 + 2]};
-          T5Values v;
-          if (flag <= kT5PassCap)
-            v = ev.t5PassValues[flag - 1];
-          else
-            t5Select(es.m, ev.md, ev.ls, t3, dnn.get(), useDnn, c_t5dnnWP, lm, innerT3, outerT3, v);
-          storeT5(ev.md, ev.ls, t3, t5, innerT3, outerT3, lm, layer, v, base + r);
-        }
-        count += tot;
+      if (int(r) < cap) {
+        const uint2 t = ev.t5PassT3[q];
+        uint16_t lm[5] = {lm1, t3.lowerModuleIndices[3 * t.x + 1], t3.lowerModuleIndices[3 * t.x + 2],
+                          t3.lowerModuleIndices[3 * t.y + 1], t3.lowerModuleIndices[3 * t.y + 2]};
+        storeT5(ev.md, ev.ls, t3, t5, t.x, t.y, lm, es.m.layers[lm1], ev.t5PassValues[q],
+                ev.rg.quintupletModuleIndices[lm1] + r);
       }
-      if (laneId() == 0) {
+      if (r + 1 == count) {
         t5.nQuintuplets[lm1] = (int(count) < cap) ? count : (cap > 0 ? unsigned(cap) : 0u);
         t5.totOccupancyQuintuplets[lm1] = count;
         if (int(count) > cap)

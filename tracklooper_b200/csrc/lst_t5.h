@@ -83,99 +83,208 @@ namespace lst {
     unsigned int md1, md2, md3, md4;
   };
 
-  // Barrel-barrel-barrel-(barrel|endcap) (SDL/Quintuplet.h:1467-1746).
-  LST_HD_BIG bool t4BBBB(const Modules& m, const MiniDoublets& md, const Segments& s, const T4Input& q) {
-    bool isPS_InLo = (m.moduleType[q.lmII] == PS);
-    bool isPS_OutLo = (m.moduleType[q.lmOI] == PS);
-    float rt_InLo = md.anchorPos[q.md1].rt, rt_InOut = md.anchorPos[q.md2].rt, rt_OutLo = md.anchorPos[q.md3].rt;
-    float z_InLo = md.anchorPos[q.md1].z, z_InOut = md.anchorPos[q.md2].z, z_OutLo = md.anchorPos[q.md3].z;
-    float alpha1GeV_OutLo = md.slope[q.md3];
-    float rtRatio_OutLoInLo = rt_OutLo / rt_InLo;
-    float dzDrtScale = md.tanSlope[q.md3] / alpha1GeV_OutLo;
+  // dPhi between the midpoint of the two segments' inner mini-doublets and the
+  // vector that joins them.  Its cut is tested before the betas in the reference;
+  // it hardly ever rejects and takes two arctangents, so here it comes last (each
+  // test is a pure function of the pair and all must pass).
+  LST_HD float t4MidPointDPhi(const MiniDoublets& md, const T4Input& q) {
+    return deltaPhi(0.5f * (md.rec[q.md1].x + md.rec[q.md3].x), 0.5f * (md.rec[q.md1].y + md.rec[q.md3].y),
+                    md.rec[q.md3].x - md.rec[q.md1].x, md.rec[q.md3].y - md.rec[q.md1].y);
+  }
+
+  // The three algorithms by the subdetectors of the four modules
+  // (SDL/Quintuplet.h:2299-2506): barrel-barrel-barrel-any (:1467-1746),
+  // barrel-...-endcap-endcap (:1748-2029), all endcap (:2031-2297).  They differ
+  // in their opening windows and in where the betas' spreads come from; the rest
+  // is one copy (three inlined ones made kT5Eval wait for instructions).  Each
+  // test is a pure function of the pair and all must pass: the beta difference,
+  // which rejects most, comes before the betaOut and dPhi cuts.
+  enum T4Kind { kT4None, kT4BBBB, kT4BBEE, kT4EEEE };
+  LST_HD int t4Kind(const Modules& m, const T4Input& q) {
+    const bool a = m.subdets[q.lmII] == Barrel, b = m.subdets[q.lmIO] == Barrel, c = m.subdets[q.lmOI] == Barrel,
+               d = m.subdets[q.lmOO] == Barrel;
+    const bool ae = m.subdets[q.lmII] == Endcap, be = m.subdets[q.lmIO] == Endcap, ce = m.subdets[q.lmOI] == Endcap,
+               de = m.subdets[q.lmOO] == Endcap;
+    if (a and b and c and (d or de))
+      return kT4BBBB;
+    if (a and (b or be) and ce and de)
+      return kT4BBEE;
+    if (ae and be and ce and de)
+      return kT4EEEE;
+    return kT4None;
+  }
+
+  LST_HD_BIG bool t4Select(const Modules& m, const MiniDoublets& md, const Segments& s, const T4Input& q) {
+    const int kind = t4Kind(m, q);
+    if (kind == kT4None)
+      return false;
+    const MDRec& r1 = md.rec[q.md1];
+    const MDRec& r2 = md.rec[q.md2];
+    const MDRec& r3 = md.rec[q.md3];
+    const MDRec& r4 = md.rec[q.md4];
+    const bool isPS_InLo = (m.moduleType[q.lmII] == PS);
+    const bool isPS_OutLo = (m.moduleType[q.lmOI] == PS);
+    float rt_InLo = r1.rt, rt_InOut = r2.rt, rt_OutLo = r3.rt;
+    float z_InLo = r1.z, z_InOut = r2.z, z_OutLo = r3.z;
+    float alpha1GeV_OutLo = r3.slope;
+    float dzDrtScale = r3.tanSlope / alpha1GeV_OutLo;
     float zpitch_InLo = (isPS_InLo ? kPixelPSZpitch : kStrip2SZpitch);
     float zpitch_OutLo = (isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch);
-    float zHi = z_InLo + (z_InLo + kDeltaZLum) * (rtRatio_OutLoInLo - 1.f) * (z_InLo < 0.f ? 1.f : dzDrtScale) +
-                (zpitch_InLo + zpitch_OutLo);
-    float zLo = z_InLo + (z_InLo - kDeltaZLum) * (rtRatio_OutLoInLo - 1.f) * (z_InLo > 0.f ? 1.f : dzDrtScale) -
-                (zpitch_InLo + zpitch_OutLo);
-    if (!((z_OutLo >= zLo) && (z_OutLo <= zHi)))
-      return false;
-
-    float drt_OutLo_InLo = (rt_OutLo - rt_InLo);
-    float r3_InLo = fsqrt(z_InLo * z_InLo + rt_InLo * rt_InLo);
-    float drt_InSeg = rt_InOut - rt_InLo;
-    float dz_InSeg = z_InOut - z_InLo;
-    float dr3_InSeg = fsqrt(rt_InOut * rt_InOut + z_InOut * z_InOut) - fsqrt(rt_InLo * rt_InLo + z_InLo * z_InLo);
-    float coshEta = dr3_InSeg / drt_InSeg;
-    float dzErr = (zpitch_InLo + zpitch_OutLo) * (zpitch_InLo + zpitch_OutLo) * 2.f;
-    float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rt_OutLo - rt_InLo) / 50.f) * fsqrt(r3_InLo / rt_InLo);
-    float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    dzErr += sdlMuls * sdlMuls * drt_OutLo_InLo * drt_OutLo_InLo / 3.f * coshEta * coshEta;
-    dzErr = fsqrt(dzErr);
-    const float dzMean = dz_InSeg / drt_InSeg * drt_OutLo_InLo;
-    const float zWindow = dzErr / drt_InSeg * drt_OutLo_InLo + (zpitch_InLo + zpitch_OutLo);
-    float zLoPointed = z_InLo + dzMean * (z_InLo > 0.f ? 1.f : dzDrtScale) - zWindow;
-    float zHiPointed = z_InLo + dzMean * (z_InLo < 0.f ? 1.f : dzDrtScale) + zWindow;
-    if (!((z_OutLo >= zLoPointed) && (z_OutLo <= zHiPointed)))
-      return false;
-
-    float sdlPVoff = 0.1f / rt_OutLo;
-    float sdlCut = alpha1GeV_OutLo + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
-    float deltaPhiPos = phiMpiPi(md.anchorPhi[q.md4] - md.anchorPhi[q.md2]);
-    if (!(fabs_(deltaPhiPos) <= sdlCut))
-      return false;
-    float midPointX = 0.5f * (md.anchorPos[q.md1].x + md.anchorPos[q.md3].x);
-    float midPointY = 0.5f * (md.anchorPos[q.md1].y + md.anchorPos[q.md3].y);
-    float diffX = md.anchorPos[q.md3].x - md.anchorPos[q.md1].x;
-    float diffY = md.anchorPos[q.md3].y - md.anchorPos[q.md1].y;
-    float dPhi = deltaPhi(midPointX, midPointY, diffX, diffY);
-    if (!(fabs_(dPhi) <= sdlCut))
-      return false;
-
-    float alpha_InLo = s.dPhiChanges[q.innerSeg];
-    float alpha_OutLo = s.dPhiChanges[q.outerSeg];
-    bool isEC_lastLayer = m.subdets[q.lmOO] == Endcap and m.moduleType[q.lmOO] == TwoS;
-    float alpha_OutUp = phiMpiPi(phiOf(md.anchorPos[q.md4].x - md.anchorPos[q.md3].x, md.anchorPos[q.md4].y - md.anchorPos[q.md3].y) -
-                                 md.anchorPhi[q.md4]);
-    float tl_axis_x = md.anchorPos[q.md4].x - md.anchorPos[q.md1].x;
-    float tl_axis_y = md.anchorPos[q.md4].y - md.anchorPos[q.md1].y;
-    float betaIn = alpha_InLo - phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.anchorPhi[q.md1]);
-    float betaInRHmin = betaIn;
-    float betaInRHmax = betaIn;
-    float betaOut = -alpha_OutUp + phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.anchorPhi[q.md4]);
-    float betaOutRHmin = betaOut;
-    float betaOutRHmax = betaOut;
-    if (isEC_lastLayer) {
-      float alpha_OutUp_highEdge =
-          phiMpiPi(phiOf(md.anchorHighEdgeX[q.md4] - md.anchorPos[q.md3].x, md.anchorHighEdgeY[q.md4] - md.anchorPos[q.md3].y) -
-                   md.anchorHighEdgePhi[q.md4]);
-      float alpha_OutUp_lowEdge =
-          phiMpiPi(phiOf(md.anchorLowEdgeX[q.md4] - md.anchorPos[q.md3].x, md.anchorLowEdgeY[q.md4] - md.anchorPos[q.md3].y) -
-                   md.anchorLowEdgePhi[q.md4]);
-      float tl_axis_highEdge_x = md.anchorHighEdgeX[q.md4] - md.anchorPos[q.md1].x;
-      float tl_axis_highEdge_y = md.anchorHighEdgeY[q.md4] - md.anchorPos[q.md1].y;
-      float tl_axis_lowEdge_x = md.anchorLowEdgeX[q.md4] - md.anchorPos[q.md1].x;
-      float tl_axis_lowEdge_y = md.anchorLowEdgeY[q.md4] - md.anchorPos[q.md1].y;
-      betaOutRHmin = -alpha_OutUp_highEdge +
-                     phiMpiPi(phiOf(tl_axis_highEdge_x, tl_axis_highEdge_y) - md.anchorHighEdgePhi[q.md4]);
-      betaOutRHmax =
-          -alpha_OutUp_lowEdge + phiMpiPi(phiOf(tl_axis_lowEdge_x, tl_axis_lowEdge_y) - md.anchorLowEdgePhi[q.md4]);
+    const float drt_InSeg = rt_InOut - rt_InLo;
+    const float dz_InSeg = z_InOut - z_InLo;
+    // (the first window, then the terms the second one and the cuts share)
+    float rtLo = 0, rtHi = 0, rtGeom = 0;
+    if (kind == kT4BBBB) {
+      float rtRatio_OutLoInLo = rt_OutLo / rt_InLo;
+      float zHi = z_InLo + (z_InLo + kDeltaZLum) * (rtRatio_OutLoInLo - 1.f) * (z_InLo < 0.f ? 1.f : dzDrtScale) +
+                  (zpitch_InLo + zpitch_OutLo);
+      float zLo = z_InLo + (z_InLo - kDeltaZLum) * (rtRatio_OutLoInLo - 1.f) * (z_InLo > 0.f ? 1.f : dzDrtScale) -
+                  (zpitch_InLo + zpitch_OutLo);
+      if (!((z_OutLo >= zLo) && (z_OutLo <= zHi)))
+        return false;
+    } else {
+      if (!(z_InLo * z_OutLo > 0))
+        return false;
+      const float dLum = signTransfer(kDeltaZLum, z_InLo);
+      if (kind == kT4BBEE) {
+        float zGeom = zpitch_InLo + zpitch_OutLo;
+        rtGeom = isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch;
+        float zGeom1 = signTransfer(zGeom, z_InLo);
+        rtLo = rt_InLo * (1.f + (z_OutLo - z_InLo - zGeom1) / (z_InLo + zGeom1 + dLum) / dzDrtScale) - rtGeom;
+        float zInForHi = z_InLo - zGeom1 - dLum;
+        if (zInForHi * z_InLo < 0) {
+          zInForHi = signTransfer(0.1f, z_InLo);
+        }
+        rtHi = rt_InLo * (1.f + (z_OutLo - z_InLo + zGeom1) / zInForHi) + rtGeom;
+      } else {
+        rtGeom = (isPS_InLo and isPS_OutLo)  ? 2.f * kPixelPSZpitch
+                 : (isPS_InLo or isPS_OutLo) ? kPixelPSZpitch + kStrip2SZpitch
+                                             : 2.f * kStrip2SZpitch;
+        float dz = z_OutLo - z_InLo;
+        rtLo = rt_InLo * (1.f + dz / (z_InLo + dLum) / dzDrtScale) - rtGeom;
+        rtHi = rt_InLo * (1.f + dz / (z_InLo - dLum)) + rtGeom;
+      }
+      if (!((rt_OutLo >= rtLo) && (rt_OutLo <= rtHi)))
+        return false;
     }
 
-    float drt_tl_axis = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    float corrF = 1.f;
+    const float r3_InLo = fsqrt(z_InLo * z_InLo + rt_InLo * rt_InLo);
+    const float dr3_InSeg = fsqrt(rt_InOut * rt_InOut + z_InOut * z_InOut) - fsqrt(rt_InLo * rt_InLo + z_InLo * z_InLo);
+    const float coshEta = dr3_InSeg / drt_InSeg;
+    float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rt_OutLo - rt_InLo) / 50.f);
+    if (kind != kT4EEEE)
+      sdlThetaMulsF = sdlThetaMulsF * fsqrt(r3_InLo / rt_InLo);
+    const float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
+    if (kind == kT4BBBB) {
+      const float drt_OutLo_InLo = (rt_OutLo - rt_InLo);
+      float dzErr = (zpitch_InLo + zpitch_OutLo) * (zpitch_InLo + zpitch_OutLo) * 2.f;
+      dzErr += sdlMuls * sdlMuls * drt_OutLo_InLo * drt_OutLo_InLo / 3.f * coshEta * coshEta;
+      dzErr = fsqrt(dzErr);
+      const float dzMean = dz_InSeg / drt_InSeg * drt_OutLo_InLo;
+      const float zWindow = dzErr / drt_InSeg * drt_OutLo_InLo + (zpitch_InLo + zpitch_OutLo);
+      float zLoPointed = z_InLo + dzMean * (z_InLo > 0.f ? 1.f : dzDrtScale) - zWindow;
+      float zHiPointed = z_InLo + dzMean * (z_InLo < 0.f ? 1.f : dzDrtScale) + zWindow;
+      if (!((z_OutLo >= zLoPointed) && (z_OutLo <= zHiPointed)))
+        return false;
+    } else {
+      const float kZ = (z_OutLo - z_InLo) / dz_InSeg;
+      if (kind == kT4BBEE) {
+        // (the reference also forms an r error here that no cut reads)
+        if (!(kZ >= 0))
+          return false;
+      } else if (isPS_InLo and m.moduleType[q.lmIO] == PS) {
+        const float dzOutInAbs = fabs_(z_OutLo - z_InLo);
+        const float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
+        float drtErr = fsqrt(kPixelPSZpitch * kPixelPSZpitch * 2.f / (dz_InSeg * dz_InSeg) * (dzOutInAbs * dzOutInAbs) +
+                             sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta);
+        float drtMean = drt_InSeg * dzOutInAbs / fabs_(dz_InSeg);
+        float rtWindow = drtErr + rtGeom;
+        float rtLo_point = rt_InLo + drtMean / dzDrtScale - rtWindow;
+        float rtHi_point = rt_InLo + drtMean + rtWindow;
+        if (!(kZ >= 0 and rt_OutLo >= rtLo_point and rt_OutLo <= rtHi_point))
+          return false;
+      }
+    }
+
+    const float sdlPVoff = 0.1f / rt_OutLo;
+    const float sdlCut = alpha1GeV_OutLo + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
+    const float deltaPhiPos = phiMpiPi(r4.phi - r2.phi);
+    if (!(fabs_(deltaPhiPos) <= sdlCut))
+      return false;
+
+    const float alpha_InLo = s.dPhiChanges[q.innerSeg];
+    const bool isTwoS_OutUp = m.moduleType[q.lmOO] == TwoS;
+    const bool isEC_lastLayer = kind == kT4BBBB and m.subdets[q.lmOO] == Endcap and isTwoS_OutUp;
+    const float tl_axis_x = r4.x - r1.x;
+    const float tl_axis_y = r4.y - r1.y;
+    const float phiTlAxis = phiOf(tl_axis_x, tl_axis_y);
+    float betaIn = alpha_InLo - phiMpiPi(phiTlAxis - r1.phi);
+    float betaInRHmin = betaIn;
+    float betaInRHmax = betaIn;
+    float alpha_OutLo, alpha_OutUp;
+    if (kind == kT4EEEE)
+      alpha_OutUp = phiMpiPi(s.dPhiChanges[q.outerSeg] - phiMpiPi(r4.phi - r3.phi));
+    else
+      alpha_OutUp = phiMpiPi(phiOf(r4.x - r3.x, r4.y - r3.y) - r4.phi);
+    float betaOut = -alpha_OutUp + phiMpiPi(phiTlAxis - r4.phi);
+    float betaOutRHmin = betaOut;
+    float betaOutRHmax = betaOut;
+    if (kind == kT4BBBB) {
+      alpha_OutLo = s.dPhiChanges[q.outerSeg];
+      if (isEC_lastLayer) {
+        const float hx = md.anchorHighEdgeX[q.md4], hy = md.anchorHighEdgeY[q.md4];
+        const float lx = md.anchorLowEdgeX[q.md4], ly = md.anchorLowEdgeY[q.md4];
+        const float alpha_OutUp_highEdge = phiMpiPi(phiOf(hx - r3.x, hy - r3.y) - r4.highEdgePhi);
+        const float alpha_OutUp_lowEdge = phiMpiPi(phiOf(lx - r3.x, ly - r3.y) - r4.lowEdgePhi);
+        betaOutRHmin = -alpha_OutUp_highEdge + phiMpiPi(phiOf(hx - r1.x, hy - r1.y) - r4.highEdgePhi);
+        betaOutRHmax = -alpha_OutUp_lowEdge + phiMpiPi(phiOf(lx - r1.x, ly - r1.y) - r4.lowEdgePhi);
+      }
+    } else {
+      alpha_OutLo = alpha_InLo;
+      if (kind == kT4BBEE) {
+        const float alphaOut_min = phiMpiPi(s.dPhiChangeMins[q.outerSeg] - s.dPhiMins[q.outerSeg]);
+        const float alphaOut_max = phiMpiPi(s.dPhiChangeMaxs[q.outerSeg] - s.dPhiMaxs[q.outerSeg]);
+        if ((m.subdets[q.lmIO] == Endcap) and (m.moduleType[q.lmIO] == TwoS)) {
+          betaInRHmin = betaIn - s.dPhiChangeMins[q.innerSeg] + alpha_InLo;
+          betaInRHmax = betaIn - s.dPhiChangeMaxs[q.innerSeg] + alpha_InLo;
+        }
+        betaOutRHmin = betaOut - alphaOut_min + alpha_OutUp;
+        betaOutRHmax = betaOut - alphaOut_max + alpha_OutUp;
+      } else {
+        const float dPhiPos = phiMpiPi(r4.phi - r3.phi);
+        const float alphaOutRHmin = phiMpiPi(s.dPhiChangeMins[q.outerSeg] - dPhiPos);
+        const float alphaOutRHmax = phiMpiPi(s.dPhiChangeMaxs[q.outerSeg] - dPhiPos);
+        betaInRHmin = betaIn + s.dPhiChangeMins[q.innerSeg] - alpha_InLo;
+        betaInRHmax = betaIn + s.dPhiChangeMaxs[q.innerSeg] - alpha_InLo;
+        betaOutRHmin = betaOut - alphaOutRHmin + alpha_OutUp;
+        betaOutRHmax = betaOut - alphaOutRHmax + alpha_OutUp;
+      }
+      float swapTemp;
+      if (fabs_(betaOutRHmin) > fabs_(betaOutRHmax)) {
+        swapTemp = betaOutRHmin;
+        betaOutRHmin = betaOutRHmax;
+        betaOutRHmax = swapTemp;
+      }
+      if (fabs_(betaInRHmin) > fabs_(betaInRHmax)) {
+        swapTemp = betaInRHmin;
+        betaInRHmin = betaInRHmax;
+        betaInRHmax = swapTemp;
+      }
+    }
+
+    const float drt_tl_axis = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
     const float rt_InSeg = segmentDr(md, q.md1, q.md2);
-    float betaInCut = fasin(fmin_((-rt_InSeg * corrF + drt_tl_axis) * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) +
-                      (0.02f / drt_InSeg);
+    const float betaInCut =
+        fasin(fmin_((-rt_InSeg + drt_tl_axis) * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / drt_InSeg);
     if (!(fabs_(betaInRHmin) < betaInCut))
       return false;
 
     float betaAv = 0.5f * (betaIn + betaOut);
     float pt_beta = drt_tl_axis * k2Rinv1GeVf / fsin(betaAv);
-    int lIn = 5;
-    int lOut = isEC_lastLayer ? 11 : 5;
-    float sdOut_dr = segmentDr(md, q.md3, q.md4);
-    float sdOut_d = md.anchorPos[q.md4].rt - md.anchorPos[q.md3].rt;
+    const float lIn = kind == kT4EEEE ? 11 : 5;
+    const int lOut = kind == kT4BBBB ? (isEC_lastLayer ? 11 : 5) : (kind == kT4BBEE ? 11 : 13);
+    const float sdOut_dr = segmentDr(md, q.md3, q.md4);
+    const float sdOut_d = r4.rt - r3.rt;
     deltaBetaIterations(betaIn, betaOut, betaAv, pt_beta, rt_InSeg, sdOut_dr, drt_tl_axis, lIn);
 
     const float betaInMMSF =
@@ -193,10 +302,13 @@ namespace lst {
     const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InLo);
     const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
     const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);
-    const float sinDPhi = fsin(dPhi);
     const float dBetaRIn2 = 0;
     float dBetaROut = 0;
-    if (isEC_lastLayer) {
+    float dPhi = 0;
+    const bool spreadOut = isEC_lastLayer or (kind == kT4BBEE and isTwoS_OutUp);
+    if (spreadOut) {
+      dPhi = t4MidPointDPhi(md, q);
+      const float sinDPhi = fsin(dPhi);
       dBetaROut = (fsqrt(md.anchorHighEdgeX[q.md4] * md.anchorHighEdgeX[q.md4] +
                          md.anchorHighEdgeY[q.md4] * md.anchorHighEdgeY[q.md4]) -
                    fsqrt(md.anchorLowEdgeX[q.md4] * md.anchorLowEdgeX[q.md4] +
@@ -204,304 +316,17 @@ namespace lst {
                   sinDPhi / drt_tl_axis;
     }
     const float dBetaROut2 = dBetaROut * dBetaROut;
-    float betaOutCut = fasin(fmin_(drt_tl_axis * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdOut_d) +
-                       fsqrt(dBetaLum2 + dBetaMuls * dBetaMuls);
+    const float dBetaRes = 0.02f / fmin_(sdOut_d, drt_InSeg);
+    if (!betaDifferenceCut(betaIn, betaOut, betaInRHmin, betaInRHmax, betaOutRHmin, betaOutRHmax, dBetaRes, dBetaMuls,
+                           dBetaLum2, dBetaRIn2, dBetaROut2))
+      return false;
+    const float betaOutCut = fasin(fmin_(drt_tl_axis * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdOut_d) +
+                             fsqrt(dBetaLum2 + dBetaMuls * dBetaMuls);
     if (!(fabs_(betaOut) < betaOutCut))
       return false;
-    float dBetaRes = 0.02f / fmin_(sdOut_d, drt_InSeg);
-    return betaDifferenceCut(betaIn, betaOut, betaInRHmin, betaInRHmax, betaOutRHmin, betaOutRHmax, dBetaRes, dBetaMuls,
-                             dBetaLum2, dBetaRIn2, dBetaROut2);
-  }
-
-  // Barrel-barrel-endcap-endcap and barrel-endcap-endcap-endcap
-  // (SDL/Quintuplet.h:1748-2029).
-  LST_HD_BIG bool t4BBEE(const Modules& m, const MiniDoublets& md, const Segments& s, const T4Input& q) {
-    bool isPS_InLo = (m.moduleType[q.lmII] == PS);
-    bool isPS_OutLo = (m.moduleType[q.lmOI] == PS);
-    float rt_InLo = md.anchorPos[q.md1].rt, rt_InOut = md.anchorPos[q.md2].rt, rt_OutLo = md.anchorPos[q.md3].rt;
-    float z_InLo = md.anchorPos[q.md1].z, z_InOut = md.anchorPos[q.md2].z, z_OutLo = md.anchorPos[q.md3].z;
-    float alpha1GeV_OutLo = md.slope[q.md3];
-    float dzDrtScale = md.tanSlope[q.md3] / alpha1GeV_OutLo;
-    float zpitch_InLo = (isPS_InLo ? kPixelPSZpitch : kStrip2SZpitch);
-    float zpitch_OutLo = (isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch);
-    float zGeom = zpitch_InLo + zpitch_OutLo;
-    if (!(z_InLo * z_OutLo > 0))
-      return false;
-    float dLum = signTransfer(kDeltaZLum, z_InLo);
-    bool isOutSgInnerMDPS = m.moduleType[q.lmOI] == PS;
-    float rtGeom1 = isOutSgInnerMDPS ? kPixelPSZpitch : kStrip2SZpitch;
-    float zGeom1 = signTransfer(zGeom, z_InLo);
-    float rtLo = rt_InLo * (1.f + (z_OutLo - z_InLo - zGeom1) / (z_InLo + zGeom1 + dLum) / dzDrtScale) - rtGeom1;
-    float rtOut = rt_OutLo;
-    if (!(rtOut >= rtLo))
-      return false;
-    float zInForHi = z_InLo - zGeom1 - dLum;
-    if (zInForHi * z_InLo < 0) {
-      zInForHi = signTransfer(0.1f, z_InLo);
-    }
-    float rtHi = rt_InLo * (1.f + (z_OutLo - z_InLo + zGeom1) / zInForHi) + rtGeom1;
-    if (!((rt_OutLo >= rtLo) && (rt_OutLo <= rtHi)))
-      return false;
-
-    float rIn = fsqrt(z_InLo * z_InLo + rt_InLo * rt_InLo);
-    const float drtSDIn = rt_InOut - rt_InLo;
-    const float dzSDIn = z_InOut - z_InLo;
-    const float dr3SDIn = fsqrt(rt_InOut * rt_InOut + z_InOut * z_InOut) - fsqrt(rt_InLo * rt_InLo + z_InLo * z_InLo);
-    const float coshEta = dr3SDIn / drtSDIn;
-    const float dzOutInAbs = fabs_(z_OutLo - z_InLo);
-    const float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
-    const float zGeom1_another = kPixelPSZpitch;
-    float kZ = (z_OutLo - z_InLo) / dzSDIn;
-    float drtErr =
-        zGeom1_another * zGeom1_another * drtSDIn * drtSDIn / dzSDIn / dzSDIn * (1.f - 2.f * kZ + 2.f * kZ * kZ);
-    const float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rt_OutLo - rt_InLo) / 50.f) * fsqrt(rIn / rt_InLo);
-    const float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    drtErr += sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta;
-    drtErr = fsqrt(drtErr);
-    if (!((kZ >= 0) && (rtOut >= rtLo) && (rtOut <= rtHi)))
-      return false;
-
-    const float sdlPVoff = 0.1f / rt_OutLo;
-    float sdlCut = alpha1GeV_OutLo + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
-    float deltaPhiPos = phiMpiPi(md.anchorPhi[q.md4] - md.anchorPhi[q.md2]);
-    if (!(fabs_(deltaPhiPos) <= sdlCut))
-      return false;
-    float midPointX = 0.5f * (md.anchorPos[q.md1].x + md.anchorPos[q.md3].x);
-    float midPointY = 0.5f * (md.anchorPos[q.md1].y + md.anchorPos[q.md3].y);
-    float diffX = md.anchorPos[q.md3].x - md.anchorPos[q.md1].x;
-    float diffY = md.anchorPos[q.md3].y - md.anchorPos[q.md1].y;
-    float dPhi = deltaPhi(midPointX, midPointY, diffX, diffY);
-    if (!(fabs_(dPhi) <= sdlCut))
-      return false;
-
-    float sdIn_alpha = s.dPhiChanges[q.innerSeg];
-    float sdIn_alpha_min = s.dPhiChangeMins[q.innerSeg];
-    float sdIn_alpha_max = s.dPhiChangeMaxs[q.innerSeg];
-    float sdOut_alpha = sdIn_alpha;
-    float sdOut_alphaOut = phiMpiPi(phiOf(md.anchorPos[q.md4].x - md.anchorPos[q.md3].x, md.anchorPos[q.md4].y - md.anchorPos[q.md3].y) -
-                                    md.anchorPhi[q.md4]);
-    float sdOut_alphaOut_min = phiMpiPi(s.dPhiChangeMins[q.outerSeg] - s.dPhiMins[q.outerSeg]);
-    float sdOut_alphaOut_max = phiMpiPi(s.dPhiChangeMaxs[q.outerSeg] - s.dPhiMaxs[q.outerSeg]);
-    float tl_axis_x = md.anchorPos[q.md4].x - md.anchorPos[q.md1].x;
-    float tl_axis_y = md.anchorPos[q.md4].y - md.anchorPos[q.md1].y;
-    float betaIn = sdIn_alpha - phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.anchorPhi[q.md1]);
-    float betaInRHmin = betaIn;
-    float betaInRHmax = betaIn;
-    float betaOut = -sdOut_alphaOut + phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.anchorPhi[q.md4]);
-    float betaOutRHmin = betaOut;
-    float betaOutRHmax = betaOut;
-    bool isEC_secondLayer = (m.subdets[q.lmIO] == Endcap) and (m.moduleType[q.lmIO] == TwoS);
-    if (isEC_secondLayer) {
-      betaInRHmin = betaIn - sdIn_alpha_min + sdIn_alpha;
-      betaInRHmax = betaIn - sdIn_alpha_max + sdIn_alpha;
-    }
-    betaOutRHmin = betaOut - sdOut_alphaOut_min + sdOut_alphaOut;
-    betaOutRHmax = betaOut - sdOut_alphaOut_max + sdOut_alphaOut;
-    float swapTemp;
-    if (fabs_(betaOutRHmin) > fabs_(betaOutRHmax)) {
-      swapTemp = betaOutRHmin;
-      betaOutRHmin = betaOutRHmax;
-      betaOutRHmax = swapTemp;
-    }
-    if (fabs_(betaInRHmin) > fabs_(betaInRHmax)) {
-      swapTemp = betaInRHmin;
-      betaInRHmin = betaInRHmax;
-      betaInRHmax = swapTemp;
-    }
-    float sdIn_dr = segmentDr(md, q.md1, q.md2);
-    float sdIn_d = rt_InOut - rt_InLo;
-    float dr = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    const float corrF = 1.f;
-    float betaInCut =
-        fasin(fmin_((-sdIn_dr * corrF + dr) * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdIn_d);
-    if (!(fabs_(betaInRHmin) < betaInCut))
-      return false;
-
-    float betaAv = 0.5f * (betaIn + betaOut);
-    float pt_beta = dr * k2Rinv1GeVf / fsin(betaAv);
-    float lIn = 5;
-    float lOut = 11;
-    float sdOut_dr = segmentDr(md, q.md3, q.md4);
-    float sdOut_d = md.anchorPos[q.md4].rt - md.anchorPos[q.md3].rt;
-    deltaBetaIterations(betaIn, betaOut, betaAv, pt_beta, sdIn_dr, sdOut_dr, dr, lIn);
-
-    const float betaInMMSF =
-        (fabs_(betaInRHmin + betaInRHmax) > 0) ? (2.f * betaIn / fabs_(betaInRHmin + betaInRHmax)) : 0.f;
-    const float betaOutMMSF =
-        (fabs_(betaOutRHmin + betaOutRHmax) > 0) ? (2.f * betaOut / fabs_(betaOutRHmin + betaOutRHmax)) : 0.f;
-    betaInRHmin *= betaInMMSF;
-    betaInRHmax *= betaInMMSF;
-    betaOutRHmin *= betaOutMMSF;
-    betaOutRHmax *= betaOutMMSF;
-
-    const float dBetaMuls = sdlThetaMulsF * 4.f / fmin_(fabs_(pt_beta), kPtBetaMax);
-    const float alphaInAbsReg = fmax_(fabs_(sdIn_alpha), md.slope3[q.md1]);
-    const float alphaOutAbsReg = fmax_(fabs_(sdOut_alpha), md.slope3[q.md3]);
-    const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InLo);
-    const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
-    const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);
-    const float sinDPhi = fsin(dPhi);
-    const float dBetaRIn2 = 0;
-    float dBetaROut = 0;
-    if (m.moduleType[q.lmOO] == TwoS) {
-      dBetaROut = (fsqrt(md.anchorHighEdgeX[q.md4] * md.anchorHighEdgeX[q.md4] +
-                         md.anchorHighEdgeY[q.md4] * md.anchorHighEdgeY[q.md4]) -
-                   fsqrt(md.anchorLowEdgeX[q.md4] * md.anchorLowEdgeX[q.md4] +
-                         md.anchorLowEdgeY[q.md4] * md.anchorLowEdgeY[q.md4])) *
-                  sinDPhi / dr;
-    }
-    const float dBetaROut2 = dBetaROut * dBetaROut;
-    float betaOutCut = fasin(fmin_(dr * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdOut_d) +
-                       fsqrt(dBetaLum2 + dBetaMuls * dBetaMuls);
-    if (!(fabs_(betaOut) < betaOutCut))
-      return false;
-    float dBetaRes = 0.02f / fmin_(sdOut_d, sdIn_d);
-    return betaDifferenceCut(betaIn, betaOut, betaInRHmin, betaInRHmax, betaOutRHmin, betaOutRHmax, dBetaRes, dBetaMuls,
-                             dBetaLum2, dBetaRIn2, dBetaROut2);
-  }
-
-  // Endcap-endcap-endcap-endcap (SDL/Quintuplet.h:2031-2297).
-  LST_HD_BIG bool t4EEEE(const Modules& m, const MiniDoublets& md, const Segments& s, const T4Input& q) {
-    float rt_InLo = md.anchorPos[q.md1].rt, rt_InOut = md.anchorPos[q.md2].rt, rt_OutLo = md.anchorPos[q.md3].rt;
-    float z_InLo = md.anchorPos[q.md1].z, z_InOut = md.anchorPos[q.md2].z, z_OutLo = md.anchorPos[q.md3].z;
-    float alpha1GeV_OutLo = md.slope[q.md3];
-    float dzDrtScale = md.tanSlope[q.md3] / alpha1GeV_OutLo;
-    if (!((z_InLo * z_OutLo) > 0))
-      return false;
-    float dLum = signTransfer(kDeltaZLum, z_InLo);
-    bool isOutSgInnerMDPS = m.moduleType[q.lmOI] == PS;
-    bool isInSgInnerMDPS = m.moduleType[q.lmII] == PS;
-    float rtGeom = (isInSgInnerMDPS and isOutSgInnerMDPS)  ? 2.f * kPixelPSZpitch
-                   : (isInSgInnerMDPS or isOutSgInnerMDPS) ? kPixelPSZpitch + kStrip2SZpitch
-                                                           : 2.f * kStrip2SZpitch;
-    float dz = z_OutLo - z_InLo;
-    float rtLo = rt_InLo * (1.f + dz / (z_InLo + dLum) / dzDrtScale) - rtGeom;
-    float rtOut = rt_OutLo;
-    float rtHi = rt_InLo * (1.f + dz / (z_InLo - dLum)) + rtGeom;
-    if (!((rtOut >= rtLo) && (rtOut <= rtHi)))
-      return false;
-
-    bool isInSgOuterMDPS = m.moduleType[q.lmIO] == PS;
-    const float drtSDIn = rt_InOut - rt_InLo;
-    const float dzSDIn = z_InOut - z_InLo;
-    const float dr3SDIn = fsqrt(rt_InOut * rt_InOut + z_InOut * z_InOut) - fsqrt(rt_InLo * rt_InLo + z_InLo * z_InLo);
-    float coshEta = dr3SDIn / drtSDIn;
-    float dzOutInAbs = fabs_(z_OutLo - z_InLo);
-    float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
-    float kZ = (z_OutLo - z_InLo) / dzSDIn;
-    float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rt_OutLo - rt_InLo) / 50.f);
-    float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    float drtErr = fsqrt(kPixelPSZpitch * kPixelPSZpitch * 2.f / (dzSDIn * dzSDIn) * (dzOutInAbs * dzOutInAbs) +
-                         sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta);
-    float drtMean = drtSDIn * dzOutInAbs / fabs_(dzSDIn);
-    float rtWindow = drtErr + rtGeom;
-    float rtLo_point = rt_InLo + drtMean / dzDrtScale - rtWindow;
-    float rtHi_point = rt_InLo + drtMean + rtWindow;
-    if (isInSgInnerMDPS and isInSgOuterMDPS) {
-      if (!(kZ >= 0 and rtOut >= rtLo_point and rtOut <= rtHi_point))
-        return false;
-    }
-
-    float sdlPVoff = 0.1f / rtOut;
-    float sdlCut = alpha1GeV_OutLo + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
-    float deltaPhiPos = phiMpiPi(md.anchorPhi[q.md4] - md.anchorPhi[q.md2]);
-    if (!(fabs_(deltaPhiPos) <= sdlCut))
-      return false;
-    float midPointX = 0.5f * (md.anchorPos[q.md1].x + md.anchorPos[q.md3].x);
-    float midPointY = 0.5f * (md.anchorPos[q.md1].y + md.anchorPos[q.md3].y);
-    float diffX = md.anchorPos[q.md3].x - md.anchorPos[q.md1].x;
-    float diffY = md.anchorPos[q.md3].y - md.anchorPos[q.md1].y;
-    float dPhi = deltaPhi(midPointX, midPointY, diffX, diffY);
-    if (!((fabs_(dPhi) <= sdlCut)))
-      return false;
-
-    float sdIn_alpha = s.dPhiChanges[q.innerSeg];
-    float sdOut_alpha = sdIn_alpha;
-    float sdOut_dPhiPos = phiMpiPi(md.anchorPhi[q.md4] - md.anchorPhi[q.md3]);
-    float sdOut_dPhiChange = s.dPhiChanges[q.outerSeg];
-    float sdOut_dPhiChange_min = s.dPhiChangeMins[q.outerSeg];
-    float sdOut_dPhiChange_max = s.dPhiChangeMaxs[q.outerSeg];
-    float sdOut_alphaOutRHmin = phiMpiPi(sdOut_dPhiChange_min - sdOut_dPhiPos);
-    float sdOut_alphaOutRHmax = phiMpiPi(sdOut_dPhiChange_max - sdOut_dPhiPos);
-    float sdOut_alphaOut = phiMpiPi(sdOut_dPhiChange - sdOut_dPhiPos);
-    float tl_axis_x = md.anchorPos[q.md4].x - md.anchorPos[q.md1].x;
-    float tl_axis_y = md.anchorPos[q.md4].y - md.anchorPos[q.md1].y;
-    float betaIn = sdIn_alpha - phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.anchorPhi[q.md1]);
-    float sdIn_alphaRHmin = s.dPhiChangeMins[q.innerSeg];
-    float sdIn_alphaRHmax = s.dPhiChangeMaxs[q.innerSeg];
-    float betaInRHmin = betaIn + sdIn_alphaRHmin - sdIn_alpha;
-    float betaInRHmax = betaIn + sdIn_alphaRHmax - sdIn_alpha;
-    float betaOut = -sdOut_alphaOut + phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.anchorPhi[q.md4]);
-    float betaOutRHmin = betaOut - sdOut_alphaOutRHmin + sdOut_alphaOut;
-    float betaOutRHmax = betaOut - sdOut_alphaOutRHmax + sdOut_alphaOut;
-    float swapTemp;
-    if (fabs_(betaOutRHmin) > fabs_(betaOutRHmax)) {
-      swapTemp = betaOutRHmin;
-      betaOutRHmin = betaOutRHmax;
-      betaOutRHmax = swapTemp;
-    }
-    if (fabs_(betaInRHmin) > fabs_(betaInRHmax)) {
-      swapTemp = betaInRHmin;
-      betaInRHmin = betaInRHmax;
-      betaInRHmax = swapTemp;
-    }
-    float sdIn_dr = segmentDr(md, q.md1, q.md2);
-    float sdIn_d = rt_InOut - rt_InLo;
-    float dr = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    const float corrF = 1.f;
-    float betaInCut =
-        fasin(fmin_((-sdIn_dr * corrF + dr) * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdIn_d);
-    if (!(fabs_(betaInRHmin) < betaInCut))
-      return false;
-
-    float betaAv = 0.5f * (betaIn + betaOut);
-    float pt_beta = dr * k2Rinv1GeVf / fsin(betaAv);
-    int lIn = 11;
-    int lOut = 13;
-    float sdOut_dr = segmentDr(md, q.md3, q.md4);
-    float sdOut_d = md.anchorPos[q.md4].rt - md.anchorPos[q.md3].rt;
-    deltaBetaIterations(betaIn, betaOut, betaAv, pt_beta, sdIn_dr, sdOut_dr, dr, lIn);
-
-    const float betaInMMSF =
-        (fabs_(betaInRHmin + betaInRHmax) > 0) ? (2.f * betaIn / fabs_(betaInRHmin + betaInRHmax)) : 0.f;
-    const float betaOutMMSF =
-        (fabs_(betaOutRHmin + betaOutRHmax) > 0) ? (2.f * betaOut / fabs_(betaOutRHmin + betaOutRHmax)) : 0.f;
-    betaInRHmin *= betaInMMSF;
-    betaInRHmax *= betaInMMSF;
-    betaOutRHmin *= betaOutMMSF;
-    betaOutRHmax *= betaOutMMSF;
-
-    const float dBetaMuls = sdlThetaMulsF * 4.f / fmin_(fabs_(pt_beta), kPtBetaMax);
-    const float alphaInAbsReg = fmax_(fabs_(sdIn_alpha), md.slope3[q.md1]);
-    const float alphaOutAbsReg = fmax_(fabs_(sdOut_alpha), md.slope3[q.md3]);
-    const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InLo);
-    const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
-    const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);
-    const float dBetaRIn2 = 0;
-    float dBetaROut2 = 0;
-    float betaOutCut = fasin(fmin_(dr * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdOut_d) +
-                       fsqrt(dBetaLum2 + dBetaMuls * dBetaMuls);
-    if (!(fabs_(betaOut) < betaOutCut))
-      return false;
-    float dBetaRes = 0.02f / fmin_(sdOut_d, sdIn_d);
-    return betaDifferenceCut(betaIn, betaOut, betaInRHmin, betaInRHmax, betaOutRHmin, betaOutRHmax, dBetaRes, dBetaMuls,
-                             dBetaLum2, dBetaRIn2, dBetaROut2);
-  }
-
-  // Dispatch on the subdetectors of the four modules (SDL/Quintuplet.h:2299-2506).
-  LST_HD bool t4Select(const Modules& m, const MiniDoublets& md, const Segments& s, const T4Input& q) {
-    short a = m.subdets[q.lmII], b = m.subdets[q.lmIO], c = m.subdets[q.lmOI], d = m.subdets[q.lmOO];
-    if (a == Barrel and b == Barrel and c == Barrel and d == Barrel)
-      return t4BBBB(m, md, s, q);
-    if (a == Barrel and b == Barrel and c == Endcap and d == Endcap)
-      return t4BBEE(m, md, s, q);
-    if (a == Barrel and b == Barrel and c == Barrel and d == Endcap)
-      return t4BBBB(m, md, s, q);
-    if (a == Barrel and b == Endcap and c == Endcap and d == Endcap)
-      return t4BBEE(m, md, s, q);
-    if (a == Endcap and b == Endcap and c == Endcap and d == Endcap)
-      return t4EEEE(m, md, s, q);
-    return false;
+    if (!spreadOut)
+      dPhi = t4MidPointDPhi(md, q);
+    return fabs_(dPhi) <= sdlCut;
   }
 
   // ------------------------------------------------------- radius checks
@@ -1228,17 +1053,6 @@ namespace lst {
     bool tightCutFlag;
   };
 
-  // A candidate staged for the classifier pass at the end of kT5Eval's
-  // block (the event's kT5DnnCap slots are split among the blocks).
-  constexpr unsigned int kT5DnnCap = 1u << 14;
-  struct T5DnnSlotG {
-    T5Values v;
-    unsigned int mdIdx[5];
-    unsigned int cand;
-    uint16_t lm[5];
-    uint8_t tight;
-  };
-
   // T5 selection for one (inner T3, outer T3) pair
   // (SDL/Quintuplet.h:2508-2984).  useDnn selects the DNN method
   // (USE_RZCHI2 + USE_T5_DNN) with working point dnnWP (the reference's is
@@ -1340,6 +1154,23 @@ namespace lst {
         kind, v.innerRadius, v.bridgeRadius, innerRadiusMin2S, innerRadiusMax2S, bridgeRadiusMin2S, bridgeRadiusMax2S);
   }
 
+  // The pair of segments of tracklet test k: the inner triplet's first segment
+  // with the outer triplet's first (k = 0) or second one.
+  LST_HD T4Input t5Tracklet(const uint16_t* lm, unsigned int innerSeg, unsigned int outerSeg, const unsigned int* mdIdx,
+                            int k) {
+    return T4Input{lm[0], lm[1], lm[2 + k], lm[3 + k], innerSeg, outerSeg, mdIdx[0], mdIdx[1], mdIdx[2 + k], mdIdx[3 + k]};
+  }
+
+  // The circle regression of a candidate that passes every test before the
+  // classifier; no test before it reads its results.
+  LST_HD void t5Regression(const Modules& m, const uint16_t* lm, const float* xs, const float* ys, T5Values& v) {
+    float sigmas[5], delta1[5], delta2[5], slopes[5];
+    bool isFlat[5];
+    regressionSigmas(m, lm, delta1, delta2, slopes, isFlat, 5, true);
+    v.regressionRadius =
+        circleRegression(5, xs, ys, delta1, delta2, slopes, isFlat, v.regressionG, v.regressionF, sigmas, v.chiSquared);
+  }
+
   LST_HD bool t5SelectPre(const Modules& m,
                           const MiniDoublets& md,
                           const Segments& s,
@@ -1358,12 +1189,13 @@ namespace lst {
     const unsigned int seg3 = t.segmentIndices[2 * outerT3];
     const unsigned int seg4 = t.segmentIndices[2 * outerT3 + 1];
     float g, f;
-    T4Input q1{lm[0], lm[1], lm[2], lm[3], seg1, seg3, mdIdx[0], mdIdx[1], mdIdx[2], mdIdx[3]};
-    if (!t4Select(m, md, s, q1))
-      return false;
-    T4Input q2{lm[0], lm[1], lm[3], lm[4], seg1, seg4, mdIdx[0], mdIdx[1], mdIdx[3], mdIdx[4]};
-    if (!t4Select(m, md, s, q2))
-      return false;
+    // (one copy of the tracklet algorithms for the two tests)
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int k = 0; k < 2; ++k)
+      if (!t4Select(m, md, s, t5Tracklet(lm, seg1, k == 0 ? seg3 : seg4, mdIdx, k)))
+        return false;
 
     g = t.circleCenterX[innerT3];
     f = t.circleCenterY[innerT3];
@@ -1372,11 +1204,7 @@ namespace lst {
     if (!t5PassRZ(m, md, mdIdx, lm, v.rzChiSquared, inner_pt, v.innerRadius, g, f, tight))
       return false;
 
-    float sigmas[5], delta1[5], delta2[5], slopes[5];
-    bool isFlat[5];
-    regressionSigmas(m, lm, delta1, delta2, slopes, isFlat, 5, true);
-    v.regressionRadius =
-        circleRegression(5, xs, ys, delta1, delta2, slopes, isFlat, v.regressionG, v.regressionF, sigmas, v.chiSquared);
+    t5Regression(m, lm, xs, ys, v);
     st.tight = tight;
     return true;
   }
