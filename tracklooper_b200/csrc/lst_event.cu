@@ -84,6 +84,24 @@ namespace {
       return cudaFail(e_, #call);      \
   } while (0)
 
+  // A launch whose blocks may become resident before the stream's previous kernel
+  // has completed; they wait for it in kernelEntry(), which every kernel launched
+  // here begins with.
+  template <typename... P, typename... A>
+  cudaError_t launchKernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = s;
+    config.attrs = &early;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+  }
+
   // Launches a kernel on stream `s` and returns an error naming it if the
   // launch is rejected.
   // With profiling on, each launch is bracketed by two CUDA events on the
@@ -95,8 +113,7 @@ namespace {
     cudaEvent_t p0_ = nullptr;                                 \
     if (ev->profiling && (p0_ = profEvent(ev)))                \
       cudaEventRecord(p0_, s);                                 \
-    kernel<<<(grid), (block), (smem), s>>>(__VA_ARGS__);       \
-    cudaError_t e_ = cudaGetLastError();                       \
+    cudaError_t e_ = launchKernel(kernel, grid, block, smem, s, __VA_ARGS__); \
     if (e_ != cudaSuccess)                                     \
       return cudaFail(e_, #kernel);                            \
     ++ev->launches;                                            \

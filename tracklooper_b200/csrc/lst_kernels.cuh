@@ -28,6 +28,20 @@ namespace lst {
     __device__ __forceinline__ const T5DnnWeights& get() const { return c_t5dnn; }
   };
 
+  // First statement of every kernel that LST_LAUNCH launches.  Those launches let
+  // a kernel's blocks in as soon as the last block of the stream's previous kernel
+  // has exited (programmatic dependent launch), so that the launch overlaps the
+  // previous kernel's completion: a step is some 65 kernels, most of them a few
+  // microseconds long.  The wait returns when the previous kernel has completed
+  // and its writes are visible; since every block of every kernel waits here
+  // before it does anything (or exits), that holds for all kernels before it as
+  // well.  One muon's lst_run 437 -> 289 us, five PU30 events 865 -> 750, one
+  // PU200 event 1734 -> 1582, 64 PU200 events unchanged.  Letting the next kernel
+  // in at the start of the previous one brought no more, and blocks waiting
+  // behind a one-block kernel kept other streams' kernels off the SMs (two event
+  // sets in turn 9.36 -> 11.0 ms).
+  __device__ __forceinline__ void kernelEntry() { cudaGridDependencySynchronize(); }
+
   __device__ __forceinline__ unsigned int laneId() { return threadIdx.x & 31u; }
   __device__ __forceinline__ unsigned int lanesBelowMask() { return (1u << laneId()) - 1u; }
 
@@ -133,12 +147,14 @@ namespace lst {
   LST_DEV unsigned int plsHitBucket(unsigned int h) { return (h * 2654435761u) >> (32 - kPLSHitBucketBits); }
 
   __global__ void kPLSHitReset(const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < kPLSHitBuckets; i += gridDim.x * blockDim.x)
       ev.plsHitHead[i] = kPLSHitNone;
   }
 
   __global__ void kResetEvent(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nMod = es.nModules, nLower = es.nLowerModules;
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2u * nMod; i += gridDim.x * blockDim.x) {
@@ -198,6 +214,7 @@ namespace lst {
   // ================================================================ hits
   // SDL/Hit.h:217-269
   __global__ void __launch_bounds__(256, 4) kHitPrep(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nHits = ev.sc->nHits;
     const Modules& m = es.m;
@@ -285,6 +302,7 @@ namespace lst {
 
   // SDL/Hit.h:194-215
   __global__ void kModuleRanges(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     Hits h = ev.hits;
     for (unsigned int lower = blockIdx.x * blockDim.x + threadIdx.x; lower < es.nLowerModules;
@@ -304,6 +322,7 @@ namespace lst {
   // Register budget: four 256-thread blocks per SM (at 154 registers a thread
   // only one fitted, and the kernel waits on gathers).
   __global__ void __launch_bounds__(256, 4) kPixelIngest(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nPLS = ev.sc->nPLS;
     const uint16_t pix = es.pixelModule;
@@ -344,6 +363,7 @@ namespace lst {
   // drew light tasks takes more: the work per module is very uneven; and the
   // list lengths of the pixel stages.  Zeroed before each of those kernels runs.
   __global__ void kTaskCountersReset(const EventView* evs) {
+    kernelEntry();
     if (threadIdx.x == 0) {
       EventScalars* sc = evs[blockIdx.y].sc;
       sc->mdNext = 0;
@@ -490,6 +510,7 @@ namespace lst {
   // modulesPerTask (1..32): 8 for batches; fewer for a single event, whose
   // 13 000 lower modules would otherwise make only ~400 warp tasks.
   __global__ void __launch_bounds__(LST_LB_MD) kCreateMD(DeviceES es, const EventView* evs, unsigned int modulesPerTask) {
+    kernelEntry();
     __shared__ unsigned int sCount[kMDMaxWarps][32];
     const EventView& ev = evs[blockIdx.y];
     const int w = threadIdx.x >> 5;
@@ -506,6 +527,7 @@ namespace lst {
   // The pixel module's mini-doublets (two per pLS, thousands per event) are
   // shared out over all of the event's threads.
   __global__ void kMDDerived(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nWarps = gridDim.x * (blockDim.x >> 5);
     const unsigned int lane = laneId();
@@ -548,6 +570,7 @@ namespace lst {
 
   // SDL/MiniDoublet.h:1084-1104
   __global__ void kMDRanges(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
       if (ev.md.nMDs[i] == 0 or ev.hits.hitRanges[i * 2] == -1) {
@@ -624,6 +647,7 @@ namespace lst {
   }
 
   __global__ void __launch_bounds__(LST_LB_LS) kCreateLS(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ LSScratch sScratch[kLSWarps];
     const EventView& ev = evs[blockIdx.y];
     const int wib = threadIdx.x >> 5;
@@ -636,6 +660,7 @@ namespace lst {
 
   // SDL/Segment.h:1010-1029
   __global__ void kLSRanges(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
       if (ev.ls.nSegments[i] == 0) {
@@ -832,6 +857,7 @@ namespace lst {
   // not fit (or the fallback paths are forced).
   constexpr int kIdxWarps = 4;
   __global__ void kLSByMD(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sBins[kIdxWarps][kByMDGroupBins];
     __shared__ unsigned int sCursor[kIdxWarps][kByMDGroupBins];
     const EventView& ev = evs[blockIdx.y];
@@ -865,6 +891,7 @@ namespace lst {
   // Triplets of each lower module grouped by first MD (after kCreateT3), in
   // the same way.
   __global__ void kT3ByMD(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sBins[kIdxWarps][kByMDGroupBins];
     __shared__ unsigned int sCursor[kIdxWarps][kByMDGroupBins];
     const EventView& ev = evs[blockIdx.y];
@@ -901,6 +928,7 @@ namespace lst {
   // ============================================================ triplets
   // Per-module triplet offsets (SDL/Triplet.h:1007-1102); one block per event.
   __global__ void __launch_bounds__(1024) kT3Offsets(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     unsigned int carry = 0;
     for (unsigned int base = 0; base < es.nLowerModules; base += blockDim.x) {
@@ -996,6 +1024,7 @@ namespace lst {
   }
 
   __global__ void __launch_bounds__(LST_LB_T3) kCreateT3(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ T3Scratch sScratch[kT3Warps];
     const EventView& ev = evs[blockIdx.y];
     const int wib = threadIdx.x >> 5;
@@ -1008,6 +1037,7 @@ namespace lst {
 
   // SDL/Triplet.h:1104-1122
   __global__ void kT3Ranges(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
       if (ev.t3.nTriplets[i] == 0) {
@@ -1037,6 +1067,7 @@ namespace lst {
   // Each thread takes a contiguous range of modules, so that one block scan
   // of the per-thread sums gives every eligible module its place.
   __global__ void __launch_bounds__(1024) kT5Eligible(DeviceES es, const EventView* evs, unsigned int innerPerTask) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = es.nLowerModules;
     const unsigned int per = (n + blockDim.x - 1) / blockDim.x;
@@ -1191,6 +1222,7 @@ namespace lst {
   }
 
   __global__ void kT5Prefix(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const int wpb = blockDim.x >> 5;
     const int nE = *ev.rg.nEligibleT5Modules;
@@ -1222,6 +1254,7 @@ namespace lst {
   }
 
   __global__ void __launch_bounds__(1024) kT5ModScan(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nE = *ev.rg.nEligibleT5Modules;
     unsigned int carry = 0;
@@ -1293,6 +1326,7 @@ namespace lst {
   }
 
   __global__ void __launch_bounds__(LST_LB_T5EVAL) kT5Eval(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ T5Scratch sScratch[kT5EvalWarps];
     const EventView& ev = evs[blockIdx.y];
     if (ev.forceWalk || ev.sc->t5Overflow)
@@ -1450,6 +1484,7 @@ namespace lst {
   // memory (a copy beside the constant one, whose reads at 32 addresses a warp are
   // served one by one), only in blocks that have a candidate.
   __global__ void __launch_bounds__(kT5ClassifyThreads) kT5Classify(DeviceES es, const EventView* evs, bool useDnn) {
+    kernelEntry();
     __shared__ __align__(16) float sW[kT5DnnParams + 3];
     __shared__ float sAct[38 * kT5ClassifyThreads];
     __shared__ T5Staged sFit[2 * kT5ClassifyThreads];  // candidates that pass the r-z fit
@@ -1564,6 +1599,7 @@ namespace lst {
   // overflow the lists; for the others its blocks return at once, and the
   // budget lets more of them be resident, so the launch drains in fewer waves.
   __global__ void __launch_bounds__(128, 8) kT5Walk(DeviceES es, const EventView* evs, bool useDnn) {
+    kernelEntry();
     __shared__ unsigned int sPre[kT5Warps][kT5MaxInner + 1];
     const EventView& ev = evs[blockIdx.y];
     if (!t5NeedsWalk(ev))
@@ -1584,6 +1620,7 @@ namespace lst {
   // 76 us for 8 PU200 events, up to 16 blocks 29.
   constexpr int kT5RankThreads = 128;
   __global__ void __launch_bounds__(kT5RankThreads) kT5RankEmit(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sKey[kT5RankCap];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.sc->t5PassCount;
@@ -1635,6 +1672,7 @@ namespace lst {
   };
 
   __global__ void kT5Probe(DeviceES es, const EventView* evs, int firstSlot, T5ProbeOut out) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int total = ev.sc->t5CandTotal;
     const int nE = *ev.rg.nEligibleT5Modules;
@@ -1710,6 +1748,7 @@ namespace lst {
   constexpr unsigned int kT5DedupPerThread = 8;
   constexpr unsigned int kT5DedupChunk = kT5DedupThreads * kT5DedupPerThread;  // eligible modules scanned at a time
   __global__ void __launch_bounds__(kT5DedupThreads) kT5DedupAfterBuild(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sPre[kT5DedupChunk + 1];  // first tile pair of each listed module
     __shared__ uint16_t sMods[kT5DedupChunk];
     const EventView& ev = evs[blockIdx.y];
@@ -1808,6 +1847,7 @@ namespace lst {
 
   // SDL/Quintuplet.h:3215-3235
   __global__ void kT5Ranges(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
       if (ev.t5.nQuintuplets[i] == 0 or ev.rg.quintupletModuleIndices[i] == -1) {
@@ -1886,6 +1926,7 @@ namespace lst {
   // higher-index pLS jx found there.  A pair met through several hits is
   // tested again, which changes nothing.
   __global__ void kPLSCleanHits(DeviceES es, const EventView* evs, bool secondpass) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const Segments& s = ev.ls;
     unsigned int nPix = s.nSegments[es.pixelModule];
@@ -1942,6 +1983,7 @@ namespace lst {
   // without a pass-1 mark), one block per event; writes the bin starts (the
   // last entry being the number of records) and the sorted records.
   __global__ void __launch_bounds__(1024) kPLSBin(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sCount[kPLSBins + 1];
     __shared__ unsigned int sCursor[kPLSBins + 1];
     const EventView& ev = evs[blockIdx.y];
@@ -1990,6 +2032,7 @@ namespace lst {
   constexpr int kPLSCleanTile = 128;
 
   __global__ void __launch_bounds__(kPLSCleanTile) kPLSCleanNear(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ PLSRec sT[kPLSCleanTile];
     const EventView& ev = evs[blockIdx.y];
     const PLSRec* rec = ev.plsRec;
@@ -2040,6 +2083,7 @@ namespace lst {
   }
 
   __global__ void kMergePLSFlag(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     unsigned int nPix = ev.ls.nSegments[es.pixelModule];
     if (nPix > kMaxPixelSegments)
@@ -2131,6 +2175,7 @@ namespace lst {
   // overflow the lists; for the others its blocks return at once, and the
   // budget lets more of them be resident, so the launch drains in fewer waves.
   __global__ void __launch_bounds__(128, 8) kPT5Count(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sPre[kPixWarps][kMaxConnectedModules + 1];
     __shared__ uint16_t sMods[kPixWarps][kMaxConnectedModules];
     const EventView& ev = evs[blockIdx.y];
@@ -2150,6 +2195,7 @@ namespace lst {
   // overflow the lists; for the others its blocks return at once, and the
   // budget lets more of them be resident, so the launch drains in fewer waves.
   __global__ void __launch_bounds__(128, 8) kPT5Emit(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sPre[kPixWarps][kMaxConnectedModules + 1];
     __shared__ uint16_t sMods[kPixWarps][kMaxConnectedModules];
     const EventView& ev = evs[blockIdx.y];
@@ -2168,6 +2214,7 @@ namespace lst {
   // Exclusive scan of the per-pLS pass counts; one block per event.
   // which = 0: pT5 (cap 15000), 1: pT3 (cap 5000).
   __global__ void __launch_bounds__(1024) kPLSScan(DeviceES es, const EventView* evs, int which) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     if (!ev.sc->pixFallback)
       return;
@@ -2217,6 +2264,7 @@ namespace lst {
   LST_DEV unsigned int pt5HitBucket(unsigned int h) { return (h * 2654435761u) >> (32 - kPT5HitBucketBits); }
 
   __global__ void kPT5DedupHits(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.pt5.nPixelQuintuplets;
     if (ev.sc->pixFallback)
@@ -2263,6 +2311,7 @@ namespace lst {
 
   constexpr int kDedupTile = 128;
   __global__ void __launch_bounds__(kDedupTile) kPT5Dedup(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sHits[kDedupTile * 14];
     __shared__ float sScore[kDedupTile];
     const EventView& ev = evs[blockIdx.y];
@@ -2354,6 +2403,7 @@ namespace lst {
 
   // pT5 -> TC (SDL/TrackCandidate.h:531-581); one block per event.
   __global__ void __launch_bounds__(1024) kAddPT5TC(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.pt5.nPixelQuintuplets;
     const unsigned int pLS_offset = es.lsOffset[es.nLowerModules];
@@ -2444,6 +2494,7 @@ namespace lst {
   // overflow the lists; for the others its blocks return at once, and the
   // budget lets more of them be resident, so the launch drains in fewer waves.
   __global__ void __launch_bounds__(128, 8) kPT3Count(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sPre[kPixWarps][kMaxConnectedModules + 1];
     __shared__ uint16_t sMods[kPixWarps][kMaxConnectedModules];
     const EventView& ev = evs[blockIdx.y];
@@ -2463,6 +2514,7 @@ namespace lst {
   // overflow the lists; for the others its blocks return at once, and the
   // budget lets more of them be resident, so the launch drains in fewer waves.
   __global__ void __launch_bounds__(128, 8) kPT3Emit(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sPre[kPixWarps][kMaxConnectedModules + 1];
     __shared__ uint16_t sMods[kPixWarps][kMaxConnectedModules];
     const EventView& ev = evs[blockIdx.y];
@@ -2543,6 +2595,7 @@ namespace lst {
   };
   template <int K>
   __global__ void __launch_bounds__(LST_LB_PIXMID) kPixMid(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ PixScratch sScratch[kPixMidWarps];
     const EventView& ev = evs[blockIdx.y];
     PixScratch& sc = sScratch[threadIdx.x >> 5];
@@ -2687,6 +2740,7 @@ namespace lst {
   // The rest of the selection for the queued candidates.
   template <int K>
   __global__ void __launch_bounds__(LST_LB_EVAL) kPixEval(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     if (K == 5)
       for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < kPT5HitBuckets; i += gridDim.x * blockDim.x)
@@ -2742,6 +2796,7 @@ namespace lst {
   constexpr int kPixRankThreads = 128;
   template <int K>
   __global__ void __launch_bounds__(kPixRankThreads) kPixRankEmit(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sKey[kPixPassCap];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.sc->pixPassCount;
@@ -2830,6 +2885,7 @@ namespace lst {
   // condition (the reference's loop breaks there), so the outcome is the OR of
   // the condition over jx: one warp per ix, its lanes over jx.
   __global__ void kPT3Dedup(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.pt3.nPixelTriplets;
     PixelTriplets p = ev.pt3;
@@ -2884,6 +2940,7 @@ namespace lst {
   // pT3 vs pT5 pixel eta/phi (SDL/TrackCandidate.h:204-243).  One warp per
   // pT3, its lanes splitting the pT5 loop; the outcome is an "any" over it.
   __global__ void kCrossCleanPT3(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nPT3 = *ev.pt3.nPixelTriplets;
     const unsigned int nPT5 = *ev.pt5.nPixelQuintuplets;
@@ -2911,6 +2968,7 @@ namespace lst {
 
   // pT3 -> TC (SDL/TrackCandidate.h:383-433); one block per event.
   __global__ void __launch_bounds__(1024) kAddPT3TC(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.pt3.nPixelTriplets;
     const unsigned int pLS_offset = es.lsOffset[es.nLowerModules];
@@ -2954,6 +3012,7 @@ namespace lst {
   // every quintuplet, as does a quintuplet of non-finite eta).  Events with
   // more quintuplets than kT5SortCap keep the module-pair walk.
   __global__ void __launch_bounds__(1024) kT5Bin(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sCount[kPLSBins + 1];
     const EventView& ev = evs[blockIdx.y];
     const int nE = *ev.rg.nEligibleT5Modules;
@@ -3022,6 +3081,7 @@ namespace lst {
   }
 
   __global__ void kT5DedupBinned(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.sc->t5SortCount;
     if (n > kT5SortCap || ev.forceWalk)
@@ -3056,6 +3116,7 @@ namespace lst {
   }
 
   __global__ void kT5DedupBeforeTC(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     if (ev.sc->t5SortCount <= kT5SortCap && !ev.forceWalk)
       return;  // kT5DedupBinned has done this event
@@ -3107,6 +3168,7 @@ namespace lst {
   }
 
   __global__ void kMergeT5Flag(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (warp >= int(*ev.rg.nEligibleT5Modules))
@@ -3126,6 +3188,7 @@ namespace lst {
   // eligible module, taking its T5s one after the other with the lanes
   // splitting the pT5 / pT3 loop (the outcome is an "any" over it).
   __global__ void kCrossCleanT5(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (warp >= int(*ev.rg.nEligibleT5Modules))
@@ -3164,6 +3227,7 @@ namespace lst {
   // T5 -> TC (SDL/TrackCandidate.h:435-487): count per eligible module, scan,
   // then emit in (module, T5) order.
   __global__ void kT5TCCount(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (warp >= int(*ev.rg.nEligibleT5Modules))
@@ -3186,6 +3250,7 @@ namespace lst {
   }
 
   __global__ void __launch_bounds__(1024) kT5TCScan(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.rg.nEligibleT5Modules;
     unsigned int carry = 0;
@@ -3207,6 +3272,7 @@ namespace lst {
   }
 
   __global__ void kT5TCEmit(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nE = *ev.rg.nEligibleT5Modules;
@@ -3235,6 +3301,7 @@ namespace lst {
   }
 
   __global__ void kT5TCFinish(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     if (threadIdx.x == 0 && blockIdx.x == 0) {
       unsigned int accepted = ev.moduleOffset[*ev.rg.nEligibleT5Modules];
@@ -3281,6 +3348,7 @@ namespace lst {
   }
 
   __global__ void kTCCleanInfo(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nTC = *ev.tc.nTrackCandidates;
     const unsigned int prefix = es.lsOffset[es.nLowerModules];
@@ -3346,6 +3414,7 @@ namespace lst {
   }
 
   __global__ void __launch_bounds__(1024) kCrossCleanPLS(DeviceES es, const EventView* evs) {
+    kernelEntry();
     extern __shared__ __align__(16) unsigned char xsm[];
     unsigned int* sHash = reinterpret_cast<unsigned int*>(xsm);
     unsigned int* sBinStart = sHash + kXCleanHashSlots;
@@ -3464,6 +3533,7 @@ namespace lst {
   }
 
   __global__ void __launch_bounds__(1024) kAddPLSTC(DeviceES es, const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.ls.nSegments[es.pixelModule];
     const unsigned int start = *ev.tc.nTrackCandidates;
@@ -3515,6 +3585,7 @@ namespace lst {
   // (SDL/Event.cc:1148-1487): per-layer sums over lower modules with the
   // same inclusion rules as add*ToEventExplicit.  One block per event.
   __global__ void kCounts(DeviceES es, const EventView* evs) {
+    kernelEntry();
     __shared__ unsigned int sBins[4][11];
     const EventView& ev = evs[blockIdx.y];
     for (int i = threadIdx.x; i < 44; i += blockDim.x)
@@ -3582,6 +3653,7 @@ namespace lst {
   // Sets the hit and pLS counts of one event (per-event input path).
   __global__ void kSetInputCounts(const EventView* evs, int slot, int setHits, unsigned int nHits, int setPLS,
                                   unsigned int nPLS, unsigned int statusBits) {
+    kernelEntry();
     const EventView& ev = evs[slot];
     if (setHits)
       ev.sc->nHits = nHits;
@@ -3631,6 +3703,7 @@ namespace lst {
   // (addPixelSegmentToEvent's copies).  blockIdx.y = event within the batch.
   __global__ void kUnpack(const EventView* evs, const unsigned char* blobs, const unsigned long long* offsets,
                           unsigned long long totalBytes) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned char* b = blobs + offsets[blockIdx.y];
     const unsigned int* hdr = reinterpret_cast<const unsigned int*>(b);
@@ -3746,6 +3819,7 @@ namespace lst {
   // Per event: output length of every candidate and their offsets; one block
   // per event.
   __global__ void __launch_bounds__(1024) kOutputSizes(const EventView* evs) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.tc.nTrackCandidates;
     unsigned int carry = 0;
@@ -3768,6 +3842,7 @@ namespace lst {
   // (exclusive scans over the events); one block.
   __global__ void __launch_bounds__(1024) kOutputEventOffsets(const EventView* evs, int count,
                                                               unsigned long long* offsets) {
+    kernelEntry();
     unsigned long long carryTC = 0, carryHits = 0;
     for (int base = 0; base < count; base += blockDim.x) {
       int i = base + threadIdx.x;
@@ -3792,6 +3867,7 @@ namespace lst {
   // Writes the batch output: hits, len, seedIdx and type, contiguous.
   __global__ void kOutputGather(const EventView* evs, int count, const unsigned long long* offsets,
                                 unsigned int* outHits, unsigned int* outLen, int* outSeed, short* outType) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.tc.nTrackCandidates;
     const unsigned long long tc0 = offsets[blockIdx.y];

@@ -120,6 +120,7 @@ namespace lst {
   __global__ void __launch_bounds__(1024) kPrepareInput(const EventView* evs, const unsigned char* blobs,
                                                         const unsigned long long* offsets,
                                                         unsigned long long totalBytes) {
+    kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned char* b = blobs + offsets[blockIdx.y];
     const unsigned int* hdr = reinterpret_cast<const unsigned int*>(b);
