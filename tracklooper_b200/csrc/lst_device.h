@@ -136,6 +136,7 @@ namespace lst {
     unsigned int* candQueue;    // candidates passing a pre-selection (T5, then pT5 / pT3), any order
     struct TCCleanInfo* tcCleanInfo;  // per track candidate: the pLS cross-cleaning record
     struct PLSRec* plsRec;      // pass-2 pLS records sorted by eta bin
+    uint2* seedChunk;           // per chunk of seeds: kept seeds and their pseudo-hits
     unsigned int* plsHitHead;   // hit -> pLS index of the pLS cleaning: chain head per bucket
     unsigned int* plsHitNext;   //   and the next entry (4 pLS + hit slot) per entry
     unsigned int* pt5HitHead;   // hit -> (pT5, slot) chains of the pT5 duplicate removal

@@ -637,10 +637,14 @@ namespace {
       return rc;
     cudaStream_t s = ev->stream;
     const unsigned long long total = ev->inboxUsed;
-    if (ev->inboxKind == 1)
-      LST_LAUNCH(lst::kPrepareInput, dim3(1 + blocksFor(ev->maxHits, count, 1024), count), 1024, ev->dv + first,
-                 ev->inbox, ev->dOffsets + first, total);
-    else
+    if (ev->inboxKind == 1) {
+      // chunks of 256 seeds: 80 in a PU200 event
+      const unsigned int seedBlocks = std::min(128u, std::max(8u, ceilDiv(kResidentBlocks, count)));
+      LST_LAUNCH(lst::kSeedCount, dim3(seedBlocks, count), lst::kSeedThreads, ev->dv + first, ev->inbox,
+                 ev->dOffsets + first, total);
+      LST_LAUNCH(lst::kPrepareInput, dim3(seedBlocks + blocksFor(ev->maxHits, count, lst::kSeedThreads), count),
+                 lst::kSeedThreads, ev->dv + first, ev->inbox, ev->dOffsets + first, total, seedBlocks);
+    } else
       LST_LAUNCH(lst::kUnpack, dim3(blocksFor(ev->maxHits, count), count), kThreads, ev->dv + first, ev->inbox,
                  ev->dOffsets + first, total);
     rc = runHitKernels(ev, first, count);

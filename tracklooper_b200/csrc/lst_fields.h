@@ -254,6 +254,7 @@
   X(plsRec, lst::PLSRec, P)                           \
   X(plsHitHead, unsigned int, lst::kPLSHitBuckets)      \
   X(plsHitNext, unsigned int, 4 * P)                   \
+  X(seedChunk, uint2, lst::kSeedChunks)                 \
   X(pt5HitHead, unsigned int, lst::kPT5HitBuckets)      \
   X(pt5HitNext, unsigned int, 14 * P5)                 \
   X(plsBinStart, unsigned int, lst::kPLSBins + 2)
