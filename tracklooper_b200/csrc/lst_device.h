@@ -70,7 +70,10 @@ namespace lst {
     unsigned int pixOverflow;     // a pLS has more candidates than a key can number
     unsigned int pixFallback;     // the pixel stage overflowed the staging: walk instead
     unsigned int pixQueueCount;   // pixel candidates passing the radius criterion and the first tracklet
-    unsigned int t5SortCount;     // quintuplets binned by eta for the cross-module cleaning
+    unsigned int t5ListCount;     // stored quintuplets (listed in t5List)
+    unsigned int t5TCStart;       // first track candidate that is a quintuplet
+    unsigned int plsTCTotal;      // pLS that become track candidates, before the cap
+    unsigned int plsTCDone;       // blocks of kAddPLSTC that have finished
     unsigned int mdNext;          // next task for kCreateMD's warps
     unsigned int lsNext;          // next lower module for kCreateLS's warps
     unsigned int pixNext; // next task (a few pLS) for kPixMid's warps
@@ -129,6 +132,7 @@ namespace lst {
     float* hitShiftXa;          // per hit moved by the strip shift: its moved point and z
     float* hitShiftYa;
     float* hitShiftZn;
+    uint2* t5List;              // stored quintuplets: index and module position, any order
     unsigned int* t5Order;      // quintuplets sorted by eta bin (their index)
     uint16_t* t5OrderPos;       //   and their module's position in the eligible-module list
     unsigned int* t5BinStart;   // start of each eta bin in t5Order (bins + 2 entries)

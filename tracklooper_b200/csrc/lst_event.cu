@@ -598,22 +598,18 @@ namespace {
         LST_LAUNCH(lst::kCrossCleanPT3, dim3(blocksFor(lst::kMaxPixelTriplets, count), count), kThreads, d, v);
         LST_LAUNCH(lst::kAddPT3TC, one, 1024, d, v);
         LST_LAUNCH(lst::kT5Bin, one, 1024, d, v);
-        LST_LAUNCH(lst::kT5DedupBinned, dim3(blocksFor(4096, count), count), kThreads, d, v);
-        LST_LAUNCH(lst::kT5DedupBeforeTC, dim3(blocksFor(nE * 32, count), count), 256, d, v);
-        LST_LAUNCH(lst::kMergeT5Flag, eligGrid, 256, d, v);
-        LST_LAUNCH(lst::kCrossCleanT5, eligGrid, 256, d, v);
-        LST_LAUNCH(lst::kT5TCCount, eligGrid, 256, d, v);
+        LST_LAUNCH(lst::kT5DedupBinned, warpGrid(4096, 4, count), 128, d, v);
+        LST_LAUNCH(lst::kCrossCleanT5, warpGrid(4096, 4, count), 128, d, v);
         LST_LAUNCH(lst::kT5TCScan, one, 1024, d, v);
         LST_LAUNCH(lst::kT5TCEmit, eligGrid, 256, d, v);
-        LST_LAUNCH(lst::kT5TCFinish, one, 32, d, v);
         LST_LAUNCH(lst::kPLSBin, one, 1024, d, v);
         LST_LAUNCH(lst::kPLSCleanHits, dim3(blocksFor(P, count), count), kThreads, d, v, true);
         LST_LAUNCH(lst::kPLSCleanNear, dim3(blocksFor(P, count, lst::kPLSCleanTile), count), lst::kPLSCleanTile, d,
                    v);
-        LST_LAUNCH(lst::kMergePLSFlag, dim3(blocksFor(P, count), count), kThreads, d, v);
         LST_LAUNCH(lst::kTCCleanInfo, dim3(blocksFor(lst::kMaxTrackCandidates, count), count), kThreads, d, v);
         LST_LAUNCH_SMEM(lst::kCrossCleanPLS, dim3(lst::kXCleanBlocksPerEvent, count), 1024, lst::kXCleanSmem, d, v);
-        LST_LAUNCH(lst::kAddPLSTC, one, 1024, d, v);
+        LST_LAUNCH(lst::kAddPLSTC, dim3(blocksFor(size_t(64) * lst::kAddPLSThreads, count), count), lst::kAddPLSThreads, d,
+                   v);
         break;
       }
       default:
@@ -707,7 +703,6 @@ namespace {
         {"kPLSHitReset", (const void*)lst::kPLSHitReset},
         {"kPLSCleanHits", (const void*)lst::kPLSCleanHits},
         {"kPLSCleanNear", (const void*)lst::kPLSCleanNear},
-        {"kMergePLSFlag", (const void*)lst::kMergePLSFlag},
         {"kPixEval<5>", (const void*)lst::kPixEval<5>},
         {"kPixMid<5>", (const void*)lst::kPixMid<5>},
         {"kPixMid<3>", (const void*)lst::kPixMid<3>},
@@ -725,15 +720,11 @@ namespace {
         {"kPT3Dedup", (const void*)lst::kPT3Dedup},
         {"kCrossCleanPT3", (const void*)lst::kCrossCleanPT3},
         {"kAddPT3TC", (const void*)lst::kAddPT3TC},
-        {"kT5DedupBeforeTC", (const void*)lst::kT5DedupBeforeTC},
         {"kT5Bin", (const void*)lst::kT5Bin},
         {"kT5DedupBinned", (const void*)lst::kT5DedupBinned},
-        {"kMergeT5Flag", (const void*)lst::kMergeT5Flag},
         {"kCrossCleanT5", (const void*)lst::kCrossCleanT5},
-        {"kT5TCCount", (const void*)lst::kT5TCCount},
         {"kT5TCScan", (const void*)lst::kT5TCScan},
         {"kT5TCEmit", (const void*)lst::kT5TCEmit},
-        {"kT5TCFinish", (const void*)lst::kT5TCFinish},
         {"kTCCleanInfo", (const void*)lst::kTCCleanInfo},
         {"kCrossCleanPLS", (const void*)lst::kCrossCleanPLS},
         {"kAddPLSTC", (const void*)lst::kAddPLSTC},

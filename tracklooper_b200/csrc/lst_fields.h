@@ -244,6 +244,7 @@
   X(candQueue, unsigned int, lst::kCandQueueCap)        \
   X(candQueueObj, unsigned int, lst::kCandQueueCap)     \
   X(hitMiniSlope, float, H)                           \
+  X(t5List, uint2, lst::kT5SortCap)                   \
   X(t5Order, unsigned int, lst::kT5SortCap)           \
   X(t5OrderPos, uint16_t, lst::kT5SortCap)            \
   X(t5BinStart, unsigned int, lst::kPLSBins + 2)      \

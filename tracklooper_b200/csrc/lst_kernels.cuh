@@ -191,6 +191,7 @@ namespace lst {
       }
       if (i == 0) {
         ev.sc->status = 0;
+        ev.sc->plsTCDone = 0;
         ev.sc->nPT5Total = 0;
         ev.sc->nPT3Total = 0;
         *ev.pt3.nPixelTriplets = 0;
@@ -345,6 +346,7 @@ namespace lst {
           es.m, ev.hits, md, ls, pix, mdBase, lsBase, tid, hit[0], hit[1], hit[2], hit[3], ev.plsDPhiChange[tid]);
       ls.partOfPT5[tid] = 0;
       ev.plsPhiP[tid] = phiOf(ls.px[tid], ls.py[tid]);
+      ev.plsFlag[tid] = 0;
       for (unsigned int slot = 0; slot < 4; ++slot) {
         const unsigned int e = 4 * tid + slot;
         ev.plsHitNext[e] = atomicExch(&ev.plsHitHead[plsHitBucket(ls.pLSHitsIdxs[e])], e);
@@ -1062,6 +1064,7 @@ namespace lst {
   constexpr unsigned int kT5KeyLimit = 1u << kT5KeyInnerShift;  // inner triplets, outer triplets of one
   constexpr unsigned int kT5StagedCap = 1u << 16;  // candidates per event that pass the tracklet tests
   constexpr unsigned int kT5RankCap = 8192;        // passing candidates per event
+  constexpr unsigned int kT5SortCap = 1u << 15;    // quintuplets per event listed for the track-candidate stage
   // Eligible T5 seed modules and their offsets (SDL/Quintuplet.h:3117-3213),
   // and the tasks of kT5Eval's warps: up to 32 inner triplets of one module.
   // Each thread takes a contiguous range of modules, so that one block scan
@@ -1113,7 +1116,16 @@ namespace lst {
       ev.sc->t5Next = 0;
       ev.sc->t5StagedCount = 0;
       ev.sc->t5PassCount = 0;
+      ev.sc->t5ListCount = 0;
     }
+  }
+
+  // Appends a stored quintuplet to the event's list (any order), which the
+  // kernels of the track-candidate stage share out over their warps.
+  __device__ __forceinline__ void t5ListAdd(const EventView& ev, unsigned int q, unsigned int module) {
+    const unsigned int k = atomicAdd(&ev.sc->t5ListCount, 1u);
+    if (k < kT5SortCap)
+      ev.t5List[k] = make_uint2(q, module);
   }
 
   // One warp per eligible module walking (inner T3, outer T3) in order
@@ -1121,7 +1133,8 @@ namespace lst {
   constexpr int kT5Warps = 4;
   constexpr int kT5MaxInner = 1024;
   __device__ __forceinline__ void t5Module(
-      DeviceES const& es, const EventView& ev, uint16_t lm1, unsigned int* pre, bool useDnn) {
+      DeviceES const& es, const EventView& ev, unsigned int module, unsigned int* pre, bool useDnn) {
+    const uint16_t lm1 = ev.rg.indicesOfEligibleT5Modules[module];
     const Modules& m = es.m;
     const int layer = m.layers[lm1];
     if (layer != 1 && layer != 2)
@@ -1165,8 +1178,10 @@ namespace lst {
       }
       unsigned int tot;
       unsigned int r = count + warpRank(ok, tot);
-      if (ok && int(r) < cap)
+      if (ok && int(r) < cap) {
         storeT5(ev.md, ev.ls, t3, t5, innerT3, outerT3, lm, layer, v, base + r);
+        t5ListAdd(ev, base + r, module);
+      }
       count += tot;
     }
     if (laneId() == 0) {
@@ -1186,7 +1201,6 @@ namespace lst {
   // stored values are those of the walk.  Events that overflow a list take the
   // walk instead.
   constexpr unsigned int kCandQueueCap = 1u << 18;  // pre-selected pT5 / pT3 candidates per event
-  constexpr unsigned int kT5SortCap = 1u << 15;     // quintuplets per event sorted by eta for the TC cleaning
   __device__ __forceinline__ bool t5NeedsWalk(const EventView& ev) {
     return ev.forceWalk || ev.sc->t5Overflow || ev.sc->t5StagedCount > kT5StagedCap || ev.sc->t5PassCount > kT5RankCap;
   }
@@ -1608,7 +1622,7 @@ namespace lst {
     const int nE = *ev.rg.nEligibleT5Modules;
     for (int w = blockIdx.x * kT5Warps + wib; w < nE; w += gridDim.x * kT5Warps) {
       __syncwarp();
-      t5Module(es, ev, ev.rg.indicesOfEligibleT5Modules[w], sPre[wib], useDnn);
+      t5Module(es, ev, unsigned(w), sPre[wib], useDnn);
     }
   }
 
@@ -1647,6 +1661,7 @@ namespace lst {
                           t3.lowerModuleIndices[3 * t.y + 1], t3.lowerModuleIndices[3 * t.y + 2]};
         storeT5(ev.md, ev.ls, t3, t5, t.x, t.y, lm, es.m.layers[lm1], ev.t5PassValues[q],
                 ev.rg.quintupletModuleIndices[lm1] + r);
+        t5ListAdd(ev, ev.rg.quintupletModuleIndices[lm1] + r, w);
       }
       if (r + 1 == count) {
         t5.nQuintuplets[lm1] = (int(count) < cap) ? count : (cap > 0 ? unsigned(cap) : 0u);
@@ -1862,7 +1877,7 @@ namespace lst {
 
   // ==================================================== pLS cleaning
   // SDL/Kernels.h:384-473.  Pass 1 sets bit 1 of isDup directly; pass 2 marks
-  // plsFlag and kMergePLSFlag folds it into bit 2 afterwards, so that pass 2
+  // plsFlag and kCrossCleanPLS folds it into bit 2 afterwards, so that pass 2
   // reads the pass-1 bit while other threads mark removals.
   // pLS binned by eta: bins of width 0.02 over [-6, 6) (clamped at both ends)
   // plus a last bin for non-finite eta, which must meet every pLS because a
@@ -1910,7 +1925,7 @@ namespace lst {
   }
 
   // pLS duplicate removal (SDL/Kernels.h:384-473).  Pass 1 sets bit 1 of
-  // isDup directly; pass 2 marks plsFlag and kMergePLSFlag folds it into bit 2
+  // isDup directly; pass 2 marks plsFlag and kCrossCleanPLS folds it into bit 2
   // afterwards, so that pass 2 reads the pass-1 bit while other threads mark
   // removals.  The outcome of a pair (ix < jx) depends only on the two pLS, and
   // marks are only ever set, so any visiting order and any repeat visit give
@@ -2078,20 +2093,6 @@ namespace lst {
           if (dR2 < 1e-5f)
             plsRemoveOf(ev, meLow ? me.index : o.index, meLow ? o.index : me.index, true);
         }
-      }
-    }
-  }
-
-  __global__ void kMergePLSFlag(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    unsigned int nPix = ev.ls.nSegments[es.pixelModule];
-    if (nPix > kMaxPixelSegments)
-      nPix = kMaxPixelSegments;
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < nPix; i += gridDim.x * blockDim.x) {
-      if (ev.plsFlag[i]) {
-        ev.ls.isDup[i] |= 2;
-        ev.plsFlag[i] = 0;
       }
     }
   }
@@ -2384,18 +2385,32 @@ namespace lst {
                        float radius,
                        unsigned int idx,
                        unsigned int directIdx) {
+    // (loads before stores, as in storeMD)
+    const bool seven = type == 7;
+    uint8_t layers[7];
+    uint16_t modules[7];
+    unsigned int hits[14];
+#pragma unroll
+    for (int i = 0; i < 7; i++) {
+      const bool has = i < 5 || seven;
+      layers[i] = has ? logicalLayers[i] : 0;
+      modules[i] = has ? lowerModules[i] : 0;
+      hits[2 * i] = has ? hitIndices[2 * i] : 0;
+      hits[2 * i + 1] = has ? hitIndices[2 * i + 1] : 0;
+    }
     tc.trackCandidateType[idx] = type;
     tc.directObjectIndices[idx] = directIdx;
     tc.pixelSeedIndex[idx] = pixelSeedIndex;
     tc.objectIndices[2 * idx] = innerIdx;
     tc.objectIndices[2 * idx + 1] = outerIdx;
-    const int limits = type == 7 ? 7 : 5;
+#pragma unroll
     for (int i = 0; i < 7; i++) {
-      tc.logicalLayers[7 * idx + i] = i < limits ? logicalLayers[i] : 0;
-      tc.lowerModuleIndices[7 * idx + i] = i < limits ? lowerModules[i] : 0;
+      tc.logicalLayers[7 * idx + i] = layers[i];
+      tc.lowerModuleIndices[7 * idx + i] = modules[i];
     }
+#pragma unroll
     for (int i = 0; i < 14; i++)
-      tc.hitIndices[14 * idx + i] = i < 2 * limits ? hitIndices[i] : 0;
+      tc.hitIndices[14 * idx + i] = hits[i];
     tc.centerX[idx] = centerX;
     tc.centerY[idx] = centerY;
     tc.radius[idx] = radius;
@@ -3015,21 +3030,30 @@ namespace lst {
     kernelEntry();
     __shared__ unsigned int sCount[kPLSBins + 1];
     const EventView& ev = evs[blockIdx.y];
-    const int nE = *ev.rg.nEligibleT5Modules;
+    const unsigned int nE = *ev.rg.nEligibleT5Modules;
+    const unsigned int total = ev.sc->t5ListCount;
     const Quintuplets& q = ev.t5;
+    // (the counts that kCrossCleanT5 adds to, and the marks of the cleaning)
+    for (unsigned int e = threadIdx.x; e < nE; e += blockDim.x)
+      ev.moduleCount[e] = 0;
+    if (total > kT5SortCap || ev.forceWalk) {
+      for (unsigned int e = threadIdx.x; e < nE; e += blockDim.x) {
+        const uint16_t lm = ev.rg.indicesOfEligibleT5Modules[e];
+        const unsigned int n = q.nQuintuplets[lm], base = ev.rg.quintupletModuleIndices[lm];
+        for (unsigned int j = 0; j < n; ++j)
+          ev.t5Flag[base + j] = 0;
+      }
+      return;
+    }
     for (int b = threadIdx.x; b <= kPLSBins; b += blockDim.x)
       sCount[b] = 0;
     __syncthreads();
-    unsigned int mine = 0;
-    for (int e = threadIdx.x; e < nE; e += blockDim.x) {
-      const uint16_t lm = ev.rg.indicesOfEligibleT5Modules[e];
-      const unsigned int n = q.nQuintuplets[lm], base = ev.rg.quintupletModuleIndices[lm];
-      for (unsigned int j = 0; j < n; ++j)
-        atomicAdd(&sCount[plsEtaBin(q.eta[base + j])], 1u);
-      mine += n;
+    for (unsigned int k = threadIdx.x; k < total; k += blockDim.x) {
+      const unsigned int ix = ev.t5List[k].x;
+      ev.t5Flag[ix] = 0;
+      atomicAdd(&sCount[plsEtaBin(q.eta[ix])], 1u);
     }
-    unsigned int total;
-    blockExclusiveScan(mine, total);
+    __syncthreads();
     const unsigned int c = threadIdx.x <= kPLSBins ? sCount[threadIdx.x] : 0u;
     unsigned int tot;
     const unsigned int ex = blockExclusiveScan(c, tot);
@@ -3037,21 +3061,14 @@ namespace lst {
       sCount[threadIdx.x] = ex;
       ev.t5BinStart[threadIdx.x] = ex;
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0)
       ev.t5BinStart[kPLSBins + 1] = tot;
-      ev.sc->t5SortCount = total;
-    }
     __syncthreads();
-    if (total > kT5SortCap)
-      return;
-    for (int e = threadIdx.x; e < nE; e += blockDim.x) {
-      const uint16_t lm = ev.rg.indicesOfEligibleT5Modules[e];
-      const unsigned int n = q.nQuintuplets[lm], base = ev.rg.quintupletModuleIndices[lm];
-      for (unsigned int j = 0; j < n; ++j) {
-        const unsigned int pos = atomicAdd(&sCount[plsEtaBin(q.eta[base + j])], 1u);
-        ev.t5Order[pos] = base + j;
-        ev.t5OrderPos[pos] = static_cast<uint16_t>(e);
-      }
+    for (unsigned int k = threadIdx.x; k < total; k += blockDim.x) {
+      const uint2 t = ev.t5List[k];
+      const unsigned int pos = atomicAdd(&sCount[plsEtaBin(q.eta[t.x])], 1u);
+      ev.t5Order[pos] = t.x;
+      ev.t5OrderPos[pos] = static_cast<uint16_t>(t.y);
     }
   }
 
@@ -3080,16 +3097,64 @@ namespace lst {
     }
   }
 
+  // A warp per quintuplet, its lanes over the partners within reach (one thread
+  // per quintuplet walked some 65 partners one after the other: 97 us for one
+  // PU200 event, now 25).  Events with more quintuplets than the list holds
+  // visit the module pairs, a warp per module.
   __global__ void kT5DedupBinned(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
-    const unsigned int n = ev.sc->t5SortCount;
-    if (n > kT5SortCap || ev.forceWalk)
-      return;
+    const unsigned int n = ev.sc->t5ListCount;
     const Quintuplets& q = ev.t5;
+    if (n > kT5SortCap || ev.forceWalk) {
+      const int nE = *ev.rg.nEligibleT5Modules;
+      const int nWarps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
+      for (int warp = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); warp < nE; warp += nWarps) {
+        uint16_t lowmod1 = ev.rg.indicesOfEligibleT5Modules[warp];
+        unsigned int n1 = q.nQuintuplets[lowmod1];
+        unsigned int base1 = ev.rg.quintupletModuleIndices[lowmod1];
+        for (unsigned int ix1 = laneId(); ix1 < n1; ix1 += 32) {
+          unsigned int ix = base1 + ix1;
+          if (q.partOfPT5[ix] || (q.isDup[ix] & 1))
+            continue;
+          float eta1 = q.eta[ix], phi1 = q.phi[ix], score1 = q.score_rphisum[ix];
+          for (int idx2 = warp; idx2 < nE; idx2++) {
+            uint16_t lowmod2 = ev.rg.indicesOfEligibleT5Modules[idx2];
+            unsigned int n2 = q.nQuintuplets[lowmod2];
+            unsigned int base2 = ev.rg.quintupletModuleIndices[lowmod2];
+            for (unsigned int jx1 = 0; jx1 < n2; jx1++) {
+              unsigned int jx = base2 + jx1;
+              if (ix == jx)
+                continue;
+              if (q.partOfPT5[jx] || (q.isDup[jx] & 1))
+                continue;
+              float eta2 = q.eta[jx], phi2 = q.phi[jx], score2 = q.score_rphisum[jx];
+              float dEta = fabs_(eta1 - eta2);
+              float dPhi = wrapDPhi(phi1, phi2);
+              if (dEta > 0.1f)
+                continue;
+              if (fabs_(dPhi) > 0.1f)
+                continue;
+              float dR2 = dEta * dEta + dPhi * dPhi;
+              int nMatched = sharedHitsT5(q, ix, jx);
+              if (dR2 < 0.001f || nMatched >= 5) {
+                if (score1 > score2)
+                  ev.t5Flag[ix] = 1;
+                else if (score1 < score2)
+                  ev.t5Flag[jx] = 1;
+                else
+                  ev.t5Flag[ix < jx ? ix : jx] = 1;
+              }
+            }
+          }
+        }
+      }
+      return;
+    }
     const unsigned int* binStart = ev.t5BinStart;
     const unsigned int nFinite = binStart[kPLSBins];
-    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const unsigned int wpb = blockDim.x >> 5;
+    for (unsigned int k = blockIdx.x * wpb + (threadIdx.x >> 5); k < n; k += gridDim.x * wpb) {
       const unsigned int ix = ev.t5Order[k];
       if (q.partOfPT5[ix] || (q.isDup[ix] & 1))
         continue;
@@ -3104,7 +3169,7 @@ namespace lst {
       }
       for (int part = 0; part < 2; ++part) {
         const unsigned int p0 = part == 0 ? lo : lo2, p1 = part == 0 ? hi : n;
-        for (unsigned int p = p0; p < p1; ++p) {
+        for (unsigned int p = p0 + laneId(); p < p1; p += 32) {
           const unsigned int jx = ev.t5Order[p];
           const unsigned int posJ = ev.t5OrderPos[p];
           if (jx == ix || posJ < posI)
@@ -3115,140 +3180,62 @@ namespace lst {
     }
   }
 
-  __global__ void kT5DedupBeforeTC(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    if (ev.sc->t5SortCount <= kT5SortCap && !ev.forceWalk)
-      return;  // kT5DedupBinned has done this event
-    // A warp per eligible module, grid-stride (the grid is kept small: most
-    // events return above).
-    const int nE = *ev.rg.nEligibleT5Modules;
-    const int nWarps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
-    const Quintuplets& q = ev.t5;
-    for (int warp = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); warp < nE; warp += nWarps) {
-      uint16_t lowmod1 = ev.rg.indicesOfEligibleT5Modules[warp];
-      unsigned int n1 = q.nQuintuplets[lowmod1];
-      unsigned int base1 = ev.rg.quintupletModuleIndices[lowmod1];
-      for (unsigned int ix1 = laneId(); ix1 < n1; ix1 += 32) {
-        unsigned int ix = base1 + ix1;
-        if (q.partOfPT5[ix] || (q.isDup[ix] & 1))
-          continue;
-        float eta1 = q.eta[ix], phi1 = q.phi[ix], score1 = q.score_rphisum[ix];
-        for (int idx2 = warp; idx2 < nE; idx2++) {
-          uint16_t lowmod2 = ev.rg.indicesOfEligibleT5Modules[idx2];
-          unsigned int n2 = q.nQuintuplets[lowmod2];
-          unsigned int base2 = ev.rg.quintupletModuleIndices[lowmod2];
-          for (unsigned int jx1 = 0; jx1 < n2; jx1++) {
-            unsigned int jx = base2 + jx1;
-            if (ix == jx)
-              continue;
-            if (q.partOfPT5[jx] || (q.isDup[jx] & 1))
-              continue;
-            float eta2 = q.eta[jx], phi2 = q.phi[jx], score2 = q.score_rphisum[jx];
-            float dEta = fabs_(eta1 - eta2);
-            float dPhi = wrapDPhi(phi1, phi2);
-            if (dEta > 0.1f)
-              continue;
-            if (fabs_(dPhi) > 0.1f)
-              continue;
-            float dR2 = dEta * dEta + dPhi * dPhi;
-            int nMatched = sharedHitsT5(q, ix, jx);
-            if (dR2 < 0.001f || nMatched >= 5) {
-              if (score1 > score2)
-                ev.t5Flag[ix] = 1;
-              else if (score1 < score2)
-                ev.t5Flag[jx] = 1;
-              else
-                ev.t5Flag[ix < jx ? ix : jx] = 1;
-            }
-          }
-        }
-      }
-    }
-  }
-
-  __global__ void kMergeT5Flag(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= int(*ev.rg.nEligibleT5Modules))
-      return;
-    uint16_t lm = ev.rg.indicesOfEligibleT5Modules[warp];
-    unsigned int n = ev.t5.nQuintuplets[lm];
-    unsigned int base = ev.rg.quintupletModuleIndices[lm];
-    for (unsigned int j = laneId(); j < n; j += 32) {
-      if (ev.t5Flag[base + j]) {
-        ev.t5.isDup[base + j] |= 2;
-        ev.t5Flag[base + j] = 0;
-      }
-    }
-  }
-
-  // T5 vs pT5/pT3 eta/phi (SDL/TrackCandidate.h:245-300); one warp per
-  // eligible module, taking its T5s one after the other with the lanes
-  // splitting the pT5 / pT3 loop (the outcome is an "any" over it).
-  __global__ void kCrossCleanT5(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= int(*ev.rg.nEligibleT5Modules))
-      return;
-    uint16_t lm = ev.rg.indicesOfEligibleT5Modules[warp];
-    unsigned int n = ev.t5.nQuintuplets[lm];
-    unsigned int base = ev.rg.quintupletModuleIndices[lm];
+  // T5 vs pT5/pT3 eta/phi (SDL/TrackCandidate.h:245-300), after folding the mark
+  // of the cross-module cleaning into isDup; and the count, per eligible module,
+  // of the T5s that become track candidates (SDL/TrackCandidate.h:435-487).  A
+  // warp per T5, its lanes over the pT5s and pT3s (the outcome is an "any").
+  __device__ __forceinline__ void t5CrossClean(const EventView& ev, unsigned int q, unsigned int module) {
+    const Quintuplets& t5 = ev.t5;
     const unsigned int nPT5 = *ev.pt5.nPixelQuintuplets;
     const unsigned int loop_bound = nPT5 + *ev.pt3.nPixelTriplets;
-    for (unsigned int j = 0; j < n; ++j) {
-      const unsigned int q = base + j;
-      if (ev.t5.isDup[q] or ev.t5.partOfPT5[q])
-        continue;
-      const float eta1 = ev.t5.eta[q], phi1 = ev.t5.phi[q];
-      bool dup = false;
+    const float eta1 = t5.eta[q], phi1 = t5.phi[q];
+    const bool marked = ev.t5Flag[q] != 0;
+    const bool kept = t5.isDup[q] == 0 && !marked && !t5.partOfPT5[q];
+    bool dup = false;
+    if (kept)
       for (unsigned int jx = laneId(); jx < loop_bound; jx += 32) {
-        float eta2, phi2;
-        if (jx < nPT5) {
-          eta2 = ev.pt5.eta[jx];
-          phi2 = ev.pt5.phi[jx];
-        } else {
-          eta2 = ev.pt3.eta[jx - nPT5];
-          phi2 = ev.pt3.phi[jx - nPT5];
-        }
+        const float eta2 = jx < nPT5 ? ev.pt5.eta[jx] : ev.pt3.eta[jx - nPT5];
+        const float phi2 = jx < nPT5 ? ev.pt5.phi[jx] : ev.pt3.phi[jx - nPT5];
         float dEta = fabs_(eta1 - eta2);
         float dPhi = wrapDPhi(phi1, phi2);
         float dR2 = dEta * dEta + dPhi * dPhi;
         if (dR2 < 1e-3f)
           dup = true;
       }
-      if (__any_sync(kFullMask, dup) && laneId() == 0)
-        ev.t5.isDup[q] = 1;
+    dup = __any_sync(kFullMask, dup);
+    if (laneId() == 0) {
+      if (marked)
+        t5.isDup[q] |= 2;
+      else if (dup)
+        t5.isDup[q] = 1;
+      else if (kept && t5.TightCutFlag[q])
+        atomicAdd(&ev.moduleCount[module], 1u);
     }
   }
-
-  // T5 -> TC (SDL/TrackCandidate.h:435-487): count per eligible module, scan,
-  // then emit in (module, T5) order.
-  __global__ void kT5TCCount(DeviceES es, const EventView* evs) {
+  __global__ void kCrossCleanT5(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= int(*ev.rg.nEligibleT5Modules))
-      return;
-    uint16_t lm = ev.rg.indicesOfEligibleT5Modules[warp];
-    unsigned int n = ev.t5.nQuintuplets[lm];
-    unsigned int base = ev.rg.quintupletModuleIndices[lm];
-    unsigned int count = 0;
-    for (unsigned int start = 0; start < n; start += 32) {
-      unsigned int j = start + laneId();
-      bool f = false;
-      if (j < n) {
-        unsigned int q = base + j;
-        f = !(ev.t5.isDup[q] or ev.t5.partOfPT5[q]) && ev.t5.TightCutFlag[q];
+    const unsigned int wpb = blockDim.x >> 5;
+    const unsigned int warp = blockIdx.x * wpb + (threadIdx.x >> 5), nWarps = gridDim.x * wpb;
+    const unsigned int n = ev.sc->t5ListCount;
+    if (n <= kT5SortCap) {
+      for (unsigned int k = warp; k < n; k += nWarps) {
+        const uint2 t = ev.t5List[k];
+        t5CrossClean(ev, t.x, t.y);
       }
-      count += __popc(__ballot_sync(kFullMask, f));
+      return;
     }
-    if (laneId() == 0)
-      ev.moduleCount[warp] = count;
+    const unsigned int nE = *ev.rg.nEligibleT5Modules;
+    for (unsigned int e = warp; e < nE; e += nWarps) {
+      const uint16_t lm = ev.rg.indicesOfEligibleT5Modules[e];
+      const unsigned int nT5 = ev.t5.nQuintuplets[lm], base = ev.rg.quintupletModuleIndices[lm];
+      for (unsigned int j = 0; j < nT5; ++j)
+        t5CrossClean(ev, base + j, e);
+    }
   }
 
+  // T5 -> TC (SDL/TrackCandidate.h:435-487): scan of the modules' counts, then
+  // emit in (module, T5) order.
   __global__ void __launch_bounds__(1024) kT5TCScan(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
@@ -3267,7 +3254,9 @@ namespace lst {
       unsigned int accepted = carry < kMaxNonPixelTrackCandidates ? carry : kMaxNonPixelTrackCandidates;
       if (accepted < carry)
         atomicOr(&ev.sc->status, kStatusTCTruncated);
-      ev.moduleOffset[n] = accepted;
+      ev.sc->t5TCStart = *ev.tc.nTrackCandidates;
+      *ev.tc.nTrackCandidates += accepted;
+      *ev.tc.nTrackCandidatesT5 += accepted;
     }
   }
 
@@ -3278,7 +3267,7 @@ namespace lst {
     const int nE = *ev.rg.nEligibleT5Modules;
     if (warp >= nE)
       return;
-    const unsigned int start = *ev.tc.nTrackCandidates;
+    const unsigned int start = ev.sc->t5TCStart;
     uint16_t lm = ev.rg.indicesOfEligibleT5Modules[warp];
     unsigned int n = ev.t5.nQuintuplets[lm];
     unsigned int base = ev.rg.quintupletModuleIndices[lm];
@@ -3297,16 +3286,6 @@ namespace lst {
         storeTC(tc, 4, qi, qi, &q.logicalLayers[5 * qi], &q.lowerModuleIndices[5 * qi], &q.hitIndices[10 * qi], -1,
                 q.regressionG[qi], q.regressionF[qi], q.regressionRadius[qi], start + r, qi);
       rank += tot;
-    }
-  }
-
-  __global__ void kT5TCFinish(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-      unsigned int accepted = ev.moduleOffset[*ev.rg.nEligibleT5Modules];
-      *ev.tc.nTrackCandidates += accepted;
-      *ev.tc.nTrackCandidatesT5 += accepted;
     }
   }
 
@@ -3489,6 +3468,13 @@ namespace lst {
     }
 
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < nPix; i += gridDim.x * blockDim.x) {
+      // the mark of the second cleaning pass (SDL/Kernels.h:384-473), set between
+      // quads without a pass-1 mark only
+      if (i < kMaxPixelSegments && ev.plsFlag[i]) {
+        s.isDup[i] |= 2;
+        ev.plsFlag[i] = 0;
+        continue;
+      }
       if (!s.isQuad[i] || s.isDup[i])
         continue;
       int phits1[4];
@@ -3532,51 +3518,93 @@ namespace lst {
     }
   }
 
-  __global__ void __launch_bounds__(1024) kAddPLSTC(DeviceES es, const EventView* evs) {
+  // pLS -> TC (SDL/TrackCandidate.h:489-529): the quads without a duplicate mark,
+  // in order.  Each block takes chunks of 256 pLS, counts the candidates before
+  // its chunk itself (their flags are two bytes a pLS), lists its own in shared
+  // memory and writes their rows, which lie side by side, as whole lines.  The
+  // last block to finish sets the counts, which all blocks have read by then.
+  // Bound by the row stores; one block per event with a store per word took 78 us
+  // for one PU200 event, now under 19 (64 events: 93, now 56).
+  constexpr int kAddPLSThreads = 256;
+  __global__ void __launch_bounds__(kAddPLSThreads) kAddPLSTC(DeviceES es, const EventView* evs) {
     kernelEntry();
+    __shared__ unsigned int sList[kAddPLSThreads];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.ls.nSegments[es.pixelModule];
     const unsigned int start = *ev.tc.nTrackCandidates;
     const unsigned int nT5TC = *ev.tc.nTrackCandidatesT5;
+    const unsigned int nChunks = (n + kAddPLSThreads - 1) / kAddPLSThreads;
     TrackCandidates tc = ev.tc;
     const Segments& s = ev.ls;
-    unsigned int carry = 0;
-    for (unsigned int base = 0; base < n; base += blockDim.x) {
-      unsigned int i = base + threadIdx.x;
-      bool f = i < n && s.isQuad[i] && !s.isDup[i];
+    // candidates with idx - nT5TC < kMaxPixelTrackCandidates are stored: `room` of them
+    const unsigned int room =
+        (start - nT5TC < kMaxPixelTrackCandidates) ? kMaxPixelTrackCandidates - (start - nT5TC) : 0u;
+    auto chosen = [&](unsigned int i) { return i < n && s.isQuad[i] && !s.isDup[i]; };
+    unsigned int before = 0, counted = 0;  // candidates in the pLS [0, counted)
+    for (unsigned int c = blockIdx.x; c < nChunks; c += gridDim.x) {
+      const unsigned int base = c * kAddPLSThreads;
+      // four pLS a word (the flag arrays start 256-byte aligned, the chunks are
+      // multiples of 256)
+      unsigned int mine = 0;
+      const unsigned int* quads = reinterpret_cast<const unsigned int*>(s.isQuad);
+      const unsigned int* dups = reinterpret_cast<const unsigned int*>(s.isDup);
+#pragma unroll 4
+      for (unsigned int w = counted / 4 + threadIdx.x; w < base / 4; w += kAddPLSThreads)
+        mine += __popc(__vcmpne4(quads[w], 0u) & __vcmpeq4(dups[w], 0u) & 0x01010101u);
+      unsigned int add;
+      blockExclusiveScan(mine, add);
+      before += add;
+      const unsigned int i = base + threadIdx.x;
+      const bool f = chosen(i);
       unsigned int tot;
-      unsigned int ex = blockExclusiveScan(f ? 1u : 0u, tot);
-      unsigned int idx = start + carry + ex;
-      if (f && idx - nT5TC < kMaxPixelTrackCandidates) {
-        tc.trackCandidateType[idx] = 8;
-        tc.directObjectIndices[idx] = i;
-        tc.pixelSeedIndex[idx] = static_cast<int>(s.seedIdx[i]);
-        tc.objectIndices[2 * idx] = i;
-        tc.objectIndices[2 * idx + 1] = i;
-        tc.hitIndices[14 * idx + 0] = s.pLSHitsIdxs[4 * i + 0];
-        tc.hitIndices[14 * idx + 1] = s.pLSHitsIdxs[4 * i + 2];
-        tc.hitIndices[14 * idx + 2] = s.pLSHitsIdxs[4 * i + 1];
-        tc.hitIndices[14 * idx + 3] = s.pLSHitsIdxs[4 * i + 3];
-        for (int k = 4; k < 14; ++k)
-          tc.hitIndices[14 * idx + k] = 0;
-        for (int k = 0; k < 7; ++k) {
-          tc.logicalLayers[7 * idx + k] = 0;
-          tc.lowerModuleIndices[7 * idx + k] = 0;
-        }
-        tc.centerX[idx] = 0;
-        tc.centerY[idx] = 0;
-        tc.radius[idx] = 0;
+      const unsigned int ex = blockExclusiveScan(f ? 1u : 0u, tot);
+      if (f)
+        sList[ex] = i;
+      __syncthreads();
+      const unsigned int rows = before < room ? min(tot, room - before) : 0u;
+      const unsigned int idx0 = start + before;
+      for (unsigned int r = threadIdx.x; r < rows; r += kAddPLSThreads) {
+        const unsigned int pls = sList[r];
+        const int seed = static_cast<int>(s.seedIdx[pls]);
+        tc.trackCandidateType[idx0 + r] = 8;
+        tc.directObjectIndices[idx0 + r] = pls;
+        tc.pixelSeedIndex[idx0 + r] = seed;
+        tc.objectIndices[2 * (idx0 + r)] = pls;
+        tc.objectIndices[2 * (idx0 + r) + 1] = pls;
+        tc.centerX[idx0 + r] = 0;
+        tc.centerY[idx0 + r] = 0;
+        tc.radius[idx0 + r] = 0;
       }
-      carry += tot;
+      for (unsigned int w = threadIdx.x; w < 14 * rows; w += kAddPLSThreads) {
+        const unsigned int r = w / 14, k = w % 14;
+        // hits 0, 2, 1, 3 of the pLS, then zeros
+        tc.hitIndices[14 * idx0 + w] =
+            k < 4 ? s.pLSHitsIdxs[4 * sList[r] + (k == 1 ? 2u : k == 2 ? 1u : k)] : 0u;
+      }
+      for (unsigned int w = threadIdx.x; w < 7 * rows; w += kAddPLSThreads) {
+        tc.logicalLayers[7 * idx0 + w] = 0;
+        tc.lowerModuleIndices[7 * idx0 + w] = 0;
+      }
+      before += tot;
+      counted = base + kAddPLSThreads;
+      __syncthreads();  // sList is rewritten for the next chunk
     }
-    if (threadIdx.x == 0) {
-      unsigned int room = (start - nT5TC < kMaxPixelTrackCandidates) ? kMaxPixelTrackCandidates - (start - nT5TC) : 0u;
-      unsigned int accepted = carry < room ? carry : room;
-      if (accepted < carry)
-        atomicOr(&ev.sc->status, kStatusTCTruncated);
-      *tc.nTrackCandidates = start + accepted;
-      *tc.nTrackCandidatespLS += accepted;
-    }
+    // (the block with the last chunk knows the event's total)
+    if (threadIdx.x != 0)
+      return;
+    if (nChunks == 0 ? blockIdx.x == 0 : (nChunks - 1) % gridDim.x == blockIdx.x)
+      ev.sc->plsTCTotal = before;
+    __threadfence();
+    if (atomicAdd(&ev.sc->plsTCDone, 1u) + 1u != gridDim.x)
+      return;
+    __threadfence();
+    ev.sc->plsTCDone = 0;
+    const unsigned int total = *static_cast<volatile unsigned int*>(&ev.sc->plsTCTotal);
+    const unsigned int accepted = total < room ? total : room;
+    if (accepted < total)
+      atomicOr(&ev.sc->status, kStatusTCTruncated);
+    *tc.nTrackCandidates = start + accepted;
+    *tc.nTrackCandidatespLS += accepted;
   }
 
 
