@@ -73,6 +73,7 @@ namespace lst {
     unsigned int t5ListCount;     // stored quintuplets (listed in t5List)
     unsigned int t5TCStart;       // first track candidate that is a quintuplet
     unsigned int plsTCTotal;      // pLS that become track candidates, before the cap
+    unsigned int walkDone;        // blocks of a fallback count kernel that have finished
     unsigned int plsTCDone;       // blocks of kAddPLSTC that have finished
     unsigned int mdNext;          // next task for kCreateMD's warps
     unsigned int lsNext;          // next lower module for kCreateLS's warps

@@ -469,19 +469,31 @@ namespace {
     return 0;
   }
 
-  int runHitKernels(lst_event* ev, int first, int count) {
+  int runHitPrep(lst_event* ev, int first, int count) {
     const lst::DeviceES& d = ev->es->view;
     cudaStream_t s = ev->stream;
     LST_LAUNCH(lst::kHitPrep, dim3(blocksFor(ev->maxHits, count), count), kThreads, d, ev->dv + first);
+    return 0;
+  }
+
+  int runModuleRanges(lst_event* ev, int first, int count) {
+    const lst::DeviceES& d = ev->es->view;
+    cudaStream_t s = ev->stream;
     LST_LAUNCH(lst::kModuleRanges, dim3(blocksFor(d.nLowerModules, count), count), kThreads, d, ev->dv + first);
     return 0;
   }
 
-  int runPixelIngest(lst_event* ev, int first, int count) {
-    const lst::DeviceES& d = ev->es->view;
+  int runPLSHitReset(lst_event* ev, int first, int count) {
     cudaStream_t s = ev->stream;
     LST_LAUNCH(lst::kPLSHitReset, dim3(blocksFor(lst::kPLSHitBuckets, count), count), kThreads, ev->dv + first);
-    LST_LAUNCH(lst::kPixelIngest, dim3(blocksFor(lst::kMaxPixelSegments, count), count), kThreads, d, ev->dv + first);
+    return 0;
+  }
+
+  int runPixelIngest(lst_event* ev, int first, int count, bool withRanges) {
+    const lst::DeviceES& d = ev->es->view;
+    cudaStream_t s = ev->stream;
+    LST_LAUNCH(lst::kPixelIngest, dim3(blocksFor(lst::kMaxPixelSegments, count), count), kThreads, d, ev->dv + first,
+               withRanges);
     return 0;
   }
 
@@ -524,25 +536,19 @@ namespace {
 #define LST_MD_MPT 8u
 #endif
         const unsigned int mpt = count >= 4 ? LST_MD_MPT : 4u;
-        LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kCreateMD, tunedWarpGrid(ev, kTuMD, ceilDiv(nLower, mpt), count), tunedThreads(ev, kTuMD), d, v,
                    mpt);
-        LST_LAUNCH(lst::kMDRanges, dim3(blocksFor(nLower, count), count), kThreads, d, v);
         LST_LAUNCH(lst::kMDDerived, tunedWarpGrid(ev, kTuMDDerived, nLower + 1, count), tunedThreads(ev, kTuMDDerived),
                    d, v);
         break;
       }
       case LST_STAGE_SEGMENTS:
-        LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kCreateLS, tunedWarpGrid(ev, kTuLS, nLower, count), tunedThreads(ev, kTuLS), d, v);
-        LST_LAUNCH(lst::kLSRanges, dim3(blocksFor(nLower, count), count), kThreads, d, v);
         LST_LAUNCH(lst::kLSByMD, warpGrid(ceilDiv(nLower, 32), lst::kIdxWarps, count), 32 * lst::kIdxWarps, d, v);
         break;
       case LST_STAGE_TRIPLETS:
         LST_LAUNCH(lst::kT3Offsets, one, 1024, d, v);
-        LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kCreateT3, tunedWarpGrid(ev, kTuT3, nLower, count), tunedThreads(ev, kTuT3), d, v);
-        LST_LAUNCH(lst::kT3Ranges, dim3(blocksFor(nLower, count), count), kThreads, d, v);
         LST_LAUNCH(lst::kT3ByMD, warpGrid(ceilDiv(nLower, 32), lst::kIdxWarps, count), 32 * lst::kIdxWarps, d, v);
         break;
       case LST_STAGE_QUINTUPLETS: {
@@ -563,32 +569,26 @@ namespace {
         // at most 64 blocks (512 warps) per event: a few hundred tile pairs
         LST_LAUNCH(lst::kT5DedupAfterBuild, dim3(std::min(64u, ceilDiv(kResidentBlocks, count)), count),
                    lst::kT5DedupThreads, d, v);
-        LST_LAUNCH(lst::kT5Ranges, dim3(blocksFor(nLower, count), count), kThreads, d, v);
         break;
       }
       case LST_STAGE_PLS_CLEANING:
         LST_LAUNCH(lst::kPLSCleanHits, dim3(blocksFor(P, count), count), kThreads, d, v, false);
         break;
       case LST_STAGE_PIXEL_QUINTUPLETS:
-        LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kPixMid<5>, tunedFlatGrid(ev, kTuMid5, count), tunedThreads(ev, kTuMid5), d, v);
         LST_LAUNCH(lst::kPixEval<5>, tunedFlatGrid(ev, kTuPix5, count), tunedThreads(ev, kTuPix5), d, v);
         LST_LAUNCH(lst::kPixRankEmit<5>, rankGrid, lst::kPixRankThreads, d, v);
         LST_LAUNCH(lst::kPT5Count, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
-        LST_LAUNCH(lst::kPLSScan, one, 1024, d, v, 0);
         LST_LAUNCH(lst::kPT5Emit, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
-        LST_LAUNCH(lst::kPT5DedupHits, dim3(blocksFor(lst::kPT5DedupSlots * 2048, count, 64), count), 64, d, v);
-        LST_LAUNCH(lst::kPT5Dedup, dim3(blocksFor(lst::kMaxPixelQuintuplets, count, lst::kDedupTile), count),
+        LST_LAUNCH(lst::kPT5DedupHits, dim3(blocksFor(lst::kPT5DedupSlots * 2048, count, lst::kDedupTile), count),
                    lst::kDedupTile, d, v);
         LST_LAUNCH(lst::kAddPT5TC, one, 1024, d, v);
         break;
       case LST_STAGE_PIXEL_TRIPLETS:
-        LST_LAUNCH(lst::kTaskCountersReset, dim3(1, count), 32, v);
         LST_LAUNCH(lst::kPixMid<3>, tunedFlatGrid(ev, kTuMid3, count), tunedThreads(ev, kTuMid3), d, v);
         LST_LAUNCH(lst::kPixEval<3>, tunedFlatGrid(ev, kTuPix3, count), tunedThreads(ev, kTuPix3), d, v);
         LST_LAUNCH(lst::kPixRankEmit<3>, rankGrid, lst::kPixRankThreads, d, v);
         LST_LAUNCH(lst::kPT3Count, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
-        LST_LAUNCH(lst::kPLSScan, one, 1024, d, v, 1);
         LST_LAUNCH(lst::kPT3Emit, warpGrid(P, lst::kPixWarps, count), 32 * lst::kPixWarps, d, v);
         LST_LAUNCH(lst::kPT3Dedup, warpGrid(lst::kMaxPixelTriplets, 8, count), 256, d, v);
         break;
@@ -643,10 +643,10 @@ namespace {
     } else
       LST_LAUNCH(lst::kUnpack, dim3(blocksFor(ev->maxHits, count), count), kThreads, ev->dv + first, ev->inbox,
                  ev->dOffsets + first, total);
-    rc = runHitKernels(ev, first, count);
+    rc = runHitPrep(ev, first, count);
     if (rc)
       return rc;
-    return runPixelIngest(ev, first, count);
+    return runPixelIngest(ev, first, count, true);
   }
 
   int readCounts(lst_event* ev, int first, int count, lst_counts* out) {
@@ -679,16 +679,12 @@ namespace {
         {"kModuleRanges", (const void*)lst::kModuleRanges},
         {"kPixelIngest", (const void*)lst::kPixelIngest},
         {"kCreateMD", (const void*)lst::kCreateMD},
-        {"kMDRanges", (const void*)lst::kMDRanges},
         {"kMDDerived", (const void*)lst::kMDDerived},
-        {"kTaskCountersReset", (const void*)lst::kTaskCountersReset},
         {"kCreateLS", (const void*)lst::kCreateLS},
-        {"kLSRanges", (const void*)lst::kLSRanges},
         {"kT3Offsets", (const void*)lst::kT3Offsets},
         {"kCreateT3", (const void*)lst::kCreateT3},
         {"kLSByMD", (const void*)lst::kLSByMD},
         {"kT3ByMD", (const void*)lst::kT3ByMD},
-        {"kT3Ranges", (const void*)lst::kT3Ranges},
         {"kT5Eligible", (const void*)lst::kT5Eligible},
         {"kT5Prefix", (const void*)lst::kT5Prefix},
         {"kT5ModScan", (const void*)lst::kT5ModScan},
@@ -698,7 +694,6 @@ namespace {
         {"kT5Walk", (const void*)lst::kT5Walk},
         {"kT5Probe", (const void*)lst::kT5Probe},
         {"kT5DedupAfterBuild", (const void*)lst::kT5DedupAfterBuild},
-        {"kT5Ranges", (const void*)lst::kT5Ranges},
         {"kPLSBin", (const void*)lst::kPLSBin},
         {"kPLSHitReset", (const void*)lst::kPLSHitReset},
         {"kPLSCleanHits", (const void*)lst::kPLSCleanHits},
@@ -711,8 +706,6 @@ namespace {
         {"kPixRankEmit<3>", (const void*)lst::kPixRankEmit<3>},
         {"kPT5Count", (const void*)lst::kPT5Count},
         {"kPT5Emit", (const void*)lst::kPT5Emit},
-        {"kPLSScan", (const void*)lst::kPLSScan},
-        {"kPT5Dedup", (const void*)lst::kPT5Dedup},
         {"kPT5DedupHits", (const void*)lst::kPT5DedupHits},
         {"kAddPT5TC", (const void*)lst::kAddPT5TC},
         {"kPT3Count", (const void*)lst::kPT3Count},
@@ -1159,7 +1152,10 @@ int lst_event_add_hits(lst_event* ev, int slot, uint32_t n, const float* x, cons
     LST_CUDA(cudaMemcpyAsync(v.hits.idxs, idxInNtuple, n * sizeof(uint32_t), cudaMemcpyDefault, s));
   }
   LST_LAUNCH(lst::kSetInputCounts, 1, 1, ev->dv, slot, 1, n, 1, 0u, 0u);
-  return runHitKernels(ev, slot, 1);
+  rc = runHitPrep(ev, slot, 1);
+  if (rc)
+    return rc;
+  return runModuleRanges(ev, slot, 1);
   LST_ABI_CATCH_INT
 }
 
@@ -1207,7 +1203,10 @@ int lst_event_add_pixel_segments(lst_event* ev, int slot, uint32_t n, const uint
     LST_CUDA(cudaMemcpyAsync(v.ls.pixelType, pixelType, size, cudaMemcpyDefault, s));
   }
   LST_LAUNCH(lst::kSetInputCounts, 1, 1, ev->dv, slot, 0, 0u, 1, size, status);
-  return runPixelIngest(ev, slot, 1);
+  rc = runPLSHitReset(ev, slot, 1);
+  if (rc)
+    return rc;
+  return runPixelIngest(ev, slot, 1, false);
   LST_ABI_CATCH_INT
 }
 

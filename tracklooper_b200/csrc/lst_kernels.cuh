@@ -139,8 +139,9 @@ namespace lst {
   // =============================================================== reset
   // Hit -> pLS index of the pLS cleaning: chains of (pLS, hit slot) entries
   // e = 4 pLS + slot in a hash table keyed by the stored pixel hit
-  // (pLSHitsIdxs[e]): a head per bucket, a next entry per entry.  kPLSHitReset
-  // empties the heads right before kPixelIngest inserts every entry once.
+  // (pLSHitsIdxs[e]): a head per bucket, a next entry per entry.  The heads are
+  // empty when kPixelIngest inserts every entry once: kResetEvent empties them,
+  // and for pixel segments added to an event on their own kPLSHitReset does.
   constexpr unsigned int kPLSHitBucketBits = 15;
   constexpr unsigned int kPLSHitBuckets = 1u << kPLSHitBucketBits;
   constexpr unsigned int kPLSHitNone = 0xffffffffu;
@@ -153,9 +154,18 @@ namespace lst {
       ev.plsHitHead[i] = kPLSHitNone;
   }
 
+  LST_DEV void pixCountersClear(const EventView& ev) {
+    ev.sc->pixNext = 0;
+    ev.sc->pixQueueCount = 0;
+    ev.sc->pixPassCount = 0;
+    ev.sc->pixOverflow = 0;
+  }
+
   __global__ void kResetEvent(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
+    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < kPLSHitBuckets; i += gridDim.x * blockDim.x)
+      ev.plsHitHead[i] = kPLSHitNone;
     const unsigned int nMod = es.nModules, nLower = es.nLowerModules;
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2u * nMod; i += gridDim.x * blockDim.x) {
       ev.hits.hitRanges[i] = -1;
@@ -191,6 +201,11 @@ namespace lst {
       }
       if (i == 0) {
         ev.sc->status = 0;
+        ev.sc->mdNext = 0;
+        ev.sc->lsNext = 0;
+        ev.sc->t3Next = 0;
+        pixCountersClear(ev);
+        ev.sc->walkDone = 0;
         ev.sc->plsTCDone = 0;
         ev.sc->nPT5Total = 0;
         ev.sc->nPT3Total = 0;
@@ -302,9 +317,7 @@ namespace lst {
   }
 
   // SDL/Hit.h:194-215
-  __global__ void kModuleRanges(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
+  __device__ __forceinline__ void moduleRanges(DeviceES const& es, const EventView& ev) {
     Hits h = ev.hits;
     for (unsigned int lower = blockIdx.x * blockDim.x + threadIdx.x; lower < es.nLowerModules;
          lower += gridDim.x * blockDim.x) {
@@ -318,13 +331,21 @@ namespace lst {
     }
   }
 
+  __global__ void kModuleRanges(DeviceES es, const EventView* evs) {
+    kernelEntry();
+    moduleRanges(es, evs[blockIdx.y]);
+  }
+
   // ========================================================= pixel segments
   // SDL/Segment.h:1031-1117
   // Register budget: four 256-thread blocks per SM (at 154 registers a thread
   // only one fitted, and the kernel waits on gathers).
-  __global__ void __launch_bounds__(256, 4) kPixelIngest(DeviceES es, const EventView* evs) {
+  // withRanges: sets the modules' hit ranges as well (batched ingest).
+  __global__ void __launch_bounds__(256, 4) kPixelIngest(DeviceES es, const EventView* evs, bool withRanges) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
+    if (withRanges)
+      moduleRanges(es, ev);
     const unsigned int nPLS = ev.sc->nPLS;
     const uint16_t pix = es.pixelModule;
     MiniDoublets md = ev.md;
@@ -361,22 +382,10 @@ namespace lst {
   }
 
   // Work counters of the kernels whose warps take their next task from the
-  // event's counter (kCreateMD, kCreateLS, kCreateT3), so that a warp that
-  // drew light tasks takes more: the work per module is very uneven; and the
-  // list lengths of the pixel stages.  Zeroed before each of those kernels runs.
-  __global__ void kTaskCountersReset(const EventView* evs) {
-    kernelEntry();
-    if (threadIdx.x == 0) {
-      EventScalars* sc = evs[blockIdx.y].sc;
-      sc->mdNext = 0;
-      sc->lsNext = 0;
-      sc->t3Next = 0;
-      sc->pixNext = 0;
-      sc->pixQueueCount = 0;
-      sc->pixPassCount = 0;
-      sc->pixOverflow = 0;
-    }
-  }
+  // event's counter, so that a warp that drew light tasks takes more: the work per
+  // module or pLS is very uneven.  A counter is zero before its kernel runs:
+  // kResetEvent clears them all, and the kernel after the one that counts clears
+  // its counter again, in case the stage is run again.
   // The next task of the calling warp from counter *next (the same value on
   // every lane).
   __device__ __forceinline__ unsigned int warpNextTask(unsigned int* next) {
@@ -517,9 +526,22 @@ namespace lst {
     const EventView& ev = evs[blockIdx.y];
     const int w = threadIdx.x >> 5;
     const unsigned int nTasks = (es.nLowerModules + modulesPerTask - 1u) / modulesPerTask;
-    // tasks from the event's counter (kTaskCountersReset zeroes it before)
+    // tasks from the event's counter (zero before the kernel)
     for (unsigned int task = warpNextTask(&ev.sc->mdNext); task < nTasks; task = warpNextTask(&ev.sc->mdNext))
       mdTask(es, ev, task, modulesPerTask, sCount[w]);
+  }
+
+  // SDL/MiniDoublet.h:1084-1104
+  __device__ __forceinline__ void mdRanges(DeviceES const& es, const EventView& ev) {
+    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
+      if (ev.md.nMDs[i] == 0 or ev.hits.hitRanges[i * 2] == -1) {
+        ev.rg.mdRanges[i * 2] = -1;
+        ev.rg.mdRanges[i * 2 + 1] = -1;
+      } else {
+        ev.rg.mdRanges[i * 2] = es.mdOffset[i];
+        ev.rg.mdRanges[i * 2 + 1] = es.mdOffset[i] + ev.md.nMDs[i] - 1;
+      }
+    }
   }
 
   // Derived per-MD values for every stored MD (lower modules and the pixel
@@ -528,9 +550,13 @@ namespace lst {
   // modules' counts, and per MD the owning lane by a search over it.
   // The pixel module's mini-doublets (two per pLS, thousands per event) are
   // shared out over all of the event's threads.
+  // Also sets the modules' mini-doublet ranges and clears kCreateMD's counter.
   __global__ void kMDDerived(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
+    mdRanges(es, ev);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      ev.sc->mdNext = 0;
     const unsigned int nWarps = gridDim.x * (blockDim.x >> 5);
     const unsigned int lane = laneId();
     MiniDoublets md = ev.md;
@@ -568,21 +594,6 @@ namespace lst {
     const unsigned int pixBase = es.mdOffset[es.nLowerModules];
     for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < nPix; k += gridDim.x * blockDim.x)
       storeMDDerived(md, pixBase + k, es.m.ptCut);
-  }
-
-  // SDL/MiniDoublet.h:1084-1104
-  __global__ void kMDRanges(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
-      if (ev.md.nMDs[i] == 0 or ev.hits.hitRanges[i * 2] == -1) {
-        ev.rg.mdRanges[i * 2] = -1;
-        ev.rg.mdRanges[i * 2 + 1] = -1;
-      } else {
-        ev.rg.mdRanges[i * 2] = es.mdOffset[i];
-        ev.rg.mdRanges[i * 2 + 1] = es.mdOffset[i] + ev.md.nMDs[i] - 1;
-      }
-    }
   }
 
   // ======================================================== line segments
@@ -653,7 +664,7 @@ namespace lst {
     __shared__ LSScratch sScratch[kLSWarps];
     const EventView& ev = evs[blockIdx.y];
     const int wib = threadIdx.x >> 5;
-    // modules from the event's counter (kTaskCountersReset zeroes it before)
+    // modules from the event's counter (zero before the kernel)
     for (unsigned int w = warpNextTask(&ev.sc->lsNext); w < es.nLowerModules; w = warpNextTask(&ev.sc->lsNext)) {
       __syncwarp();
       lsModule(es, ev, static_cast<uint16_t>(w), sScratch[wib]);
@@ -661,9 +672,7 @@ namespace lst {
   }
 
   // SDL/Segment.h:1010-1029
-  __global__ void kLSRanges(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
+  __device__ __forceinline__ void lsRanges(DeviceES const& es, const EventView& ev) {
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
       if (ev.ls.nSegments[i] == 0) {
         ev.rg.segmentRanges[i * 2] = -1;
@@ -856,13 +865,17 @@ namespace lst {
 
   // Segments of each lower module grouped by inner MD (after kCreateLS): a
   // warp takes 32 modules at a time, module by module where their bins do
-  // not fit (or the fallback paths are forced).
+  // not fit (or the fallback paths are forced).  Also sets the modules' segment
+  // ranges and clears kCreateLS's counter.
   constexpr int kIdxWarps = 4;
   __global__ void kLSByMD(DeviceES es, const EventView* evs) {
     kernelEntry();
     __shared__ unsigned int sBins[kIdxWarps][kByMDGroupBins];
     __shared__ unsigned int sCursor[kIdxWarps][kByMDGroupBins];
     const EventView& ev = evs[blockIdx.y];
+    lsRanges(es, ev);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      ev.sc->lsNext = 0;
     const int wib = threadIdx.x >> 5;
     const unsigned int* mdIdx = ev.ls.mdIndices;
     const unsigned int nWarps = gridDim.x * kIdxWarps;
@@ -890,13 +903,29 @@ namespace lst {
     }
   }
 
+  // SDL/Triplet.h:1104-1122
+  __device__ __forceinline__ void t3Ranges(DeviceES const& es, const EventView& ev) {
+    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
+      if (ev.t3.nTriplets[i] == 0) {
+        ev.rg.tripletRanges[i * 2] = -1;
+        ev.rg.tripletRanges[i * 2 + 1] = -1;
+      } else {
+        ev.rg.tripletRanges[i * 2] = ev.rg.tripletModuleIndices[i];
+        ev.rg.tripletRanges[i * 2 + 1] = ev.rg.tripletModuleIndices[i] + ev.t3.nTriplets[i] - 1;
+      }
+    }
+  }
+
   // Triplets of each lower module grouped by first MD (after kCreateT3), in
-  // the same way.
+  // the same way, with the modules' triplet ranges and kCreateT3's counter.
   __global__ void kT3ByMD(DeviceES es, const EventView* evs) {
     kernelEntry();
     __shared__ unsigned int sBins[kIdxWarps][kByMDGroupBins];
     __shared__ unsigned int sCursor[kIdxWarps][kByMDGroupBins];
     const EventView& ev = evs[blockIdx.y];
+    t3Ranges(es, ev);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      ev.sc->t3Next = 0;
     const int wib = threadIdx.x >> 5;
     const unsigned int* segIdx = ev.t3.segmentIndices;
     const unsigned int* mdIdx = ev.ls.mdIndices;
@@ -1030,25 +1059,10 @@ namespace lst {
     __shared__ T3Scratch sScratch[kT3Warps];
     const EventView& ev = evs[blockIdx.y];
     const int wib = threadIdx.x >> 5;
-    // modules from the event's counter (kTaskCountersReset zeroes it before)
+    // modules from the event's counter (zero before the kernel)
     for (unsigned int w = warpNextTask(&ev.sc->t3Next); w < es.nLowerModules; w = warpNextTask(&ev.sc->t3Next)) {
       __syncwarp();
       t3Module(es, ev, static_cast<uint16_t>(w), sScratch[wib]);
-    }
-  }
-
-  // SDL/Triplet.h:1104-1122
-  __global__ void kT3Ranges(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
-      if (ev.t3.nTriplets[i] == 0) {
-        ev.rg.tripletRanges[i * 2] = -1;
-        ev.rg.tripletRanges[i * 2 + 1] = -1;
-      } else {
-        ev.rg.tripletRanges[i * 2] = ev.rg.tripletModuleIndices[i];
-        ev.rg.tripletRanges[i * 2 + 1] = ev.rg.tripletModuleIndices[i] + ev.t3.nTriplets[i] - 1;
-      }
     }
   }
 
@@ -1747,6 +1761,19 @@ namespace lst {
     return nMatched;
   }
 
+  // SDL/Quintuplet.h:3215-3235
+  __device__ __forceinline__ void t5Ranges(DeviceES const& es, const EventView& ev) {
+    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
+      if (ev.t5.nQuintuplets[i] == 0 or ev.rg.quintupletModuleIndices[i] == -1) {
+        ev.rg.quintupletRanges[i * 2] = -1;
+        ev.rg.quintupletRanges[i * 2 + 1] = -1;
+      } else {
+        ev.rg.quintupletRanges[i * 2] = ev.rg.quintupletModuleIndices[i];
+        ev.rg.quintupletRanges[i * 2 + 1] = ev.rg.quintupletModuleIndices[i] + ev.t5.nQuintuplets[i] - 1;
+      }
+    }
+  }
+
   // Duplicate removal among the T5s of one module (SDL/Kernels.h:202-249).
   // Every pair (i < j) of a module is independent and only ever sets isDup
   // bit 1, so the pairs are dealt out in tiles of 32 x 32 to all warps of the
@@ -1767,6 +1794,7 @@ namespace lst {
     __shared__ unsigned int sPre[kT5DedupChunk + 1];  // first tile pair of each listed module
     __shared__ uint16_t sMods[kT5DedupChunk];
     const EventView& ev = evs[blockIdx.y];
+    t5Ranges(es, ev);
     const unsigned int nElig = *ev.rg.nEligibleT5Modules;
     const unsigned int lane = laneId();
     Quintuplets q = ev.t5;
@@ -1857,21 +1885,6 @@ namespace lst {
         }
       }
       __syncthreads();  // sMods / sPre are rewritten for the next chunk
-    }
-  }
-
-  // SDL/Quintuplet.h:3215-3235
-  __global__ void kT5Ranges(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < es.nLowerModules; i += gridDim.x * blockDim.x) {
-      if (ev.t5.nQuintuplets[i] == 0 or ev.rg.quintupletModuleIndices[i] == -1) {
-        ev.rg.quintupletRanges[i * 2] = -1;
-        ev.rg.quintupletRanges[i * 2 + 1] = -1;
-      } else {
-        ev.rg.quintupletRanges[i * 2] = ev.rg.quintupletModuleIndices[i];
-        ev.rg.quintupletRanges[i * 2 + 1] = ev.rg.quintupletModuleIndices[i] + ev.t5.nQuintuplets[i] - 1;
-      }
     }
   }
 
@@ -2130,6 +2143,48 @@ namespace lst {
     return ev.t5.nQuintuplets[mod];
   }
 
+  // Ends a count kernel of the fallback walk: the last block of the event to get
+  // here scans the per-pLS pass counts (the others' writes are visible: each block
+  // fences its own before it is counted).
+  // which = 0: pT5 (cap 15000), 1: pT3 (cap 5000).
+  __device__ __forceinline__ void plsScanByLast(DeviceES const& es, const EventView& ev, int which) {
+    __shared__ bool sLast;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+      sLast = atomicAdd(&ev.sc->walkDone, 1u) + 1u == gridDim.x;
+    __syncthreads();
+    if (!sLast)
+      return;
+    __threadfence();
+    const unsigned int n = ev.ls.nSegments[es.pixelModule];
+    const volatile unsigned int* counts = ev.plsCount;
+    unsigned int carry = 0;
+    for (unsigned int base = 0; base < n; base += blockDim.x) {
+      unsigned int i = base + threadIdx.x;
+      unsigned int c = (i < n) ? counts[i] : 0u;
+      unsigned int tot;
+      unsigned int ex = blockExclusiveScan(c, tot);
+      if (i < n)
+        ev.plsOffset[i] = carry + ex;
+      carry += tot;
+    }
+    if (threadIdx.x == 0) {
+      ev.sc->walkDone = 0;
+      if (which == 0) {
+        ev.sc->nPT5Total = carry;
+        *ev.pt5.totOccupancyPixelQuintuplets = carry;
+        *ev.pt5.nPixelQuintuplets = carry < kMaxPixelQuintuplets ? carry : kMaxPixelQuintuplets;
+      } else {
+        ev.sc->nPT3Total = carry;
+        *ev.pt3.totOccupancyPixelTriplets = carry;
+        *ev.pt3.nPixelTriplets = carry < kMaxPixelTriplets ? carry : kMaxPixelTriplets;
+      }
+      if ((which == 0 && carry > kMaxPixelQuintuplets) || (which == 1 && carry > kMaxPixelTriplets))
+        atomicOr(&ev.sc->status, kStatusCapOverflow);
+    }
+  }
+
   // Walks the pT5 candidates of one pLS in order; emit selects the pass:
   // count passing candidates, or store those with global rank < cap.
   constexpr int kPixWarps = 4;
@@ -2190,6 +2245,7 @@ namespace lst {
         ev.plsCount[i] = 0;
       pt5Walk<false>(es, ev, i, sPre[wib], sMods[wib]);
     }
+    plsScanByLast(es, ev, 0);
   }
 
   // Register budget: this fallback does work only for events whose candidates
@@ -2212,39 +2268,6 @@ namespace lst {
     }
   }
 
-  // Exclusive scan of the per-pLS pass counts; one block per event.
-  // which = 0: pT5 (cap 15000), 1: pT3 (cap 5000).
-  __global__ void __launch_bounds__(1024) kPLSScan(DeviceES es, const EventView* evs, int which) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    if (!ev.sc->pixFallback)
-      return;
-    const unsigned int n = ev.ls.nSegments[es.pixelModule];
-    unsigned int carry = 0;
-    for (unsigned int base = 0; base < n; base += blockDim.x) {
-      unsigned int i = base + threadIdx.x;
-      unsigned int c = (i < n) ? ev.plsCount[i] : 0u;
-      unsigned int tot;
-      unsigned int ex = blockExclusiveScan(c, tot);
-      if (i < n)
-        ev.plsOffset[i] = carry + ex;
-      carry += tot;
-    }
-    if (threadIdx.x == 0) {
-      if (which == 0) {
-        ev.sc->nPT5Total = carry;
-        *ev.pt5.totOccupancyPixelQuintuplets = carry;
-        *ev.pt5.nPixelQuintuplets = carry < kMaxPixelQuintuplets ? carry : kMaxPixelQuintuplets;
-      } else {
-        ev.sc->nPT3Total = carry;
-        *ev.pt3.totOccupancyPixelTriplets = carry;
-        *ev.pt3.nPixelTriplets = carry < kMaxPixelTriplets ? carry : kMaxPixelTriplets;
-      }
-      if ((which == 0 && carry > kMaxPixelQuintuplets) || (which == 1 && carry > kMaxPixelTriplets))
-        atomicOr(&ev.sc->status, kStatusCapOverflow);
-    }
-  }
-
   // pT5 duplicate removal (SDL/Kernels.h:356-382): pT5 ix is removed if some
   // jx shares at least 7 of its 14 hit slots and has a lower score (ties: the
   // higher index goes).  The outcome is an OR over jx, and a pair sharing 7
@@ -2264,61 +2287,12 @@ namespace lst {
   constexpr unsigned int kPT5DedupSlots = 8;
   LST_DEV unsigned int pt5HitBucket(unsigned int h) { return (h * 2654435761u) >> (32 - kPT5HitBucketBits); }
 
-  __global__ void kPT5DedupHits(DeviceES es, const EventView* evs) {
-    kernelEntry();
-    const EventView& ev = evs[blockIdx.y];
-    const unsigned int n = *ev.pt5.nPixelQuintuplets;
-    if (ev.sc->pixFallback)
-      return;
-    PixelQuintuplets p = ev.pt5;
-    for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < kPT5DedupSlots * n;
-         t += gridDim.x * blockDim.x) {
-      const unsigned int a = t / kPT5DedupSlots;
-      const unsigned int h = p.hitIndices[14 * a + t % kPT5DedupSlots];
-      const float score1 = p.score[a];
-      for (unsigned int q = ev.pt5HitHead[pt5HitBucket(h)]; q != kPT5HitNone; q = ev.pt5HitNext[q]) {
-        const unsigned int b = q / 14;
-        if (p.hitIndices[q] != h || b == a)
-          continue;
-        const float score2 = p.score[b];
-        if (!(score1 > score2 or ((score1 == score2) and (a > b))))
-          continue;
-        // (56 bytes per pT5: the fourteen indices lie on an 8-byte boundary)
-        const uint2* mine = reinterpret_cast<const uint2*>(p.hitIndices + 14 * size_t(a));
-        const uint2* other = reinterpret_cast<const uint2*>(p.hitIndices + 14 * size_t(b));
-        uint2 o[7];
-#pragma unroll
-        for (int j = 0; j < 7; ++j)
-          o[j] = other[j];
-        int nMatched = 0;
-#pragma unroll
-        for (int i = 0; i < 7; ++i) {
-          const uint2 m = mine[i];
-          bool mx = false, my = false;
-#pragma unroll
-          for (int j = 0; j < 7; ++j) {
-            mx |= m.x == o[j].x || m.x == o[j].y;
-            my |= m.y == o[j].x || m.y == o[j].y;
-          }
-          nMatched += (mx ? 1 : 0) + (my ? 1 : 0);
-        }
-        if (nMatched >= 7) {
-          p.isDup[a] = 1;
-          break;
-        }
-      }
-    }
-  }
-
+  // Every pair, in tiles staged in shared memory (a block of kDedupTile threads).
   constexpr int kDedupTile = 128;
-  __global__ void __launch_bounds__(kDedupTile) kPT5Dedup(DeviceES es, const EventView* evs) {
-    kernelEntry();
+  __device__ __forceinline__ void pt5DedupTiles(const EventView& ev) {
     __shared__ unsigned int sHits[kDedupTile * 14];
     __shared__ float sScore[kDedupTile];
-    const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.pt5.nPixelQuintuplets;
-    if (!ev.sc->pixFallback)
-      return;  // kPT5DedupHits has done this event
     PixelQuintuplets p = ev.pt5;
     for (unsigned int ixBase = blockIdx.x * kDedupTile; ixBase < n; ixBase += gridDim.x * kDedupTile) {
       const unsigned int ix = ixBase + threadIdx.x;
@@ -2367,6 +2341,56 @@ namespace lst {
       }
       if (valid && dup)
         p.isDup[ix] = 1;
+    }
+  }
+
+  __global__ void __launch_bounds__(kDedupTile) kPT5DedupHits(DeviceES es, const EventView* evs) {
+    kernelEntry();
+    const EventView& ev = evs[blockIdx.y];
+    const unsigned int n = *ev.pt5.nPixelQuintuplets;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      pixCountersClear(ev);  // the pixel lists have been read
+    if (ev.sc->pixFallback) {
+      pt5DedupTiles(ev);
+      return;
+    }
+    PixelQuintuplets p = ev.pt5;
+    for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < kPT5DedupSlots * n;
+         t += gridDim.x * blockDim.x) {
+      const unsigned int a = t / kPT5DedupSlots;
+      const unsigned int h = p.hitIndices[14 * a + t % kPT5DedupSlots];
+      const float score1 = p.score[a];
+      for (unsigned int q = ev.pt5HitHead[pt5HitBucket(h)]; q != kPT5HitNone; q = ev.pt5HitNext[q]) {
+        const unsigned int b = q / 14;
+        if (p.hitIndices[q] != h || b == a)
+          continue;
+        const float score2 = p.score[b];
+        if (!(score1 > score2 or ((score1 == score2) and (a > b))))
+          continue;
+        // (56 bytes per pT5: the fourteen indices lie on an 8-byte boundary)
+        const uint2* mine = reinterpret_cast<const uint2*>(p.hitIndices + 14 * size_t(a));
+        const uint2* other = reinterpret_cast<const uint2*>(p.hitIndices + 14 * size_t(b));
+        uint2 o[7];
+#pragma unroll
+        for (int j = 0; j < 7; ++j)
+          o[j] = other[j];
+        int nMatched = 0;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+          const uint2 m = mine[i];
+          bool mx = false, my = false;
+#pragma unroll
+          for (int j = 0; j < 7; ++j) {
+            mx |= m.x == o[j].x || m.x == o[j].y;
+            my |= m.y == o[j].x || m.y == o[j].y;
+          }
+          nMatched += (mx ? 1 : 0) + (my ? 1 : 0);
+        }
+        if (nMatched >= 7) {
+          p.isDup[a] = 1;
+          break;
+        }
+      }
     }
   }
 
@@ -2523,6 +2547,7 @@ namespace lst {
         ev.plsCount[i] = 0;
       pt3Walk<false>(es, ev, i, sPre[wib], sMods[wib]);
     }
+    plsScanByLast(es, ev, 1);
   }
 
   // Register budget: this fallback does work only for events whose candidates
@@ -2902,6 +2927,8 @@ namespace lst {
   __global__ void kPT3Dedup(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      pixCountersClear(ev);  // the pixel lists have been read
     const unsigned int n = *ev.pt3.nPixelTriplets;
     PixelTriplets p = ev.pt3;
     const unsigned int wpb = blockDim.x >> 5;
