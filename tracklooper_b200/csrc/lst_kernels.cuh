@@ -3278,10 +3278,14 @@ namespace lst {
       carry += tot;
     }
     if (threadIdx.x == 0) {
-      unsigned int accepted = carry < kMaxNonPixelTrackCandidates ? carry : kMaxNonPixelTrackCandidates;
+      // (the store's end bounds a stage that is run again on the same event, which
+      // appends to its candidates)
+      const unsigned int begin = *ev.tc.nTrackCandidates;
+      const unsigned int room = begin < kMaxTrackCandidates ? kMaxTrackCandidates - begin : 0u;
+      const unsigned int accepted = min(carry, min(kMaxNonPixelTrackCandidates, room));
       if (accepted < carry)
         atomicOr(&ev.sc->status, kStatusTCTruncated);
-      ev.sc->t5TCStart = *ev.tc.nTrackCandidates;
+      ev.sc->t5TCStart = begin;
       *ev.tc.nTrackCandidates += accepted;
       *ev.tc.nTrackCandidatesT5 += accepted;
     }
@@ -3309,7 +3313,7 @@ namespace lst {
         f = !(q.isDup[qi] or q.partOfPT5[qi]) && q.TightCutFlag[qi];
       unsigned int tot;
       unsigned int r = rank + warpRank(f, tot);
-      if (f && r < kMaxNonPixelTrackCandidates)
+      if (f && r < kMaxNonPixelTrackCandidates && start + r < kMaxTrackCandidates)
         storeTC(tc, 4, qi, qi, &q.logicalLayers[5 * qi], &q.lowerModuleIndices[5 * qi], &q.hitIndices[10 * qi], -1,
                 q.regressionG[qi], q.regressionF[qi], q.regressionRadius[qi], start + r, qi);
       rank += tot;
@@ -3564,8 +3568,11 @@ namespace lst {
     TrackCandidates tc = ev.tc;
     const Segments& s = ev.ls;
     // candidates with idx - nT5TC < kMaxPixelTrackCandidates are stored: `room` of them
+    // (and none past the store's end)
     const unsigned int room =
-        (start - nT5TC < kMaxPixelTrackCandidates) ? kMaxPixelTrackCandidates - (start - nT5TC) : 0u;
+        (start - nT5TC < kMaxPixelTrackCandidates && start < kMaxTrackCandidates)
+            ? min(kMaxPixelTrackCandidates - (start - nT5TC), kMaxTrackCandidates - start)
+            : 0u;
     auto chosen = [&](unsigned int i) { return i < n && s.isQuad[i] && !s.isDup[i]; };
     unsigned int before = 0, counted = 0;  // candidates in the pLS [0, counted)
     for (unsigned int c = blockIdx.x; c < nChunks; c += gridDim.x) {
