@@ -386,14 +386,29 @@ namespace lst {
   // module or pLS is very uneven.  A counter is zero before its kernel runs:
   // kResetEvent clears them all, and the kernel after the one that counts clears
   // its counter again, in case the stage is run again.
-  // The next task of the calling warp from counter *next (the same value on
-  // every lane).
-  __device__ __forceinline__ unsigned int warpNextTask(unsigned int* next) {
-    unsigned int t = 0;
-    if (laneId() == 0)
-      t = atomicAdd(next, 1u);
-    return __shfl_sync(kFullMask, t, 0);
-  }
+  // The tasks of the calling warp: first the one of its own number among the
+  // event's warps, then from counter *next, which numbers the tasks after those
+  // (the same value on every lane).  Without the first, thousands of warps start
+  // with an atomic on one address.
+  struct WarpTasks {
+    unsigned int* next;
+    unsigned int nWarps, own;
+    bool started = false;
+    __device__ __forceinline__ explicit WarpTasks(unsigned int* counter)
+        : next(counter),
+          nWarps(gridDim.x * (blockDim.x >> 5)),
+          own(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) {}
+    __device__ __forceinline__ unsigned int take() {
+      if (!started) {
+        started = true;
+        return own;
+      }
+      unsigned int t = 0;
+      if (laneId() == 0)
+        t = atomicAdd(next, 1u);
+      return nWarps + __shfl_sync(kFullMask, t, 0);
+    }
+  };
 
   // ======================================================== mini-doublets
   // SDL/MiniDoublet.h:896-992: every (lower hit, upper hit) pair of a lower
@@ -527,7 +542,8 @@ namespace lst {
     const int w = threadIdx.x >> 5;
     const unsigned int nTasks = (es.nLowerModules + modulesPerTask - 1u) / modulesPerTask;
     // tasks from the event's counter (zero before the kernel)
-    for (unsigned int task = warpNextTask(&ev.sc->mdNext); task < nTasks; task = warpNextTask(&ev.sc->mdNext))
+    WarpTasks tasks(&ev.sc->mdNext);
+    for (unsigned int task = tasks.take(); task < nTasks; task = tasks.take())
       mdTask(es, ev, task, modulesPerTask, sCount[w]);
   }
 
@@ -665,7 +681,8 @@ namespace lst {
     const EventView& ev = evs[blockIdx.y];
     const int wib = threadIdx.x >> 5;
     // modules from the event's counter (zero before the kernel)
-    for (unsigned int w = warpNextTask(&ev.sc->lsNext); w < es.nLowerModules; w = warpNextTask(&ev.sc->lsNext)) {
+    WarpTasks tasks(&ev.sc->lsNext);
+    for (unsigned int w = tasks.take(); w < es.nLowerModules; w = tasks.take()) {
       __syncwarp();
       lsModule(es, ev, static_cast<uint16_t>(w), sScratch[wib]);
     }
@@ -741,8 +758,8 @@ namespace lst {
     }
   }
 
-  // The same grouping for 32 consecutive modules at once (most modules hold a
-  // few objects): their bins lie side by side in bins[0, sum of the modules'
+  // The same grouping for `group` (up to 32) consecutive modules at once (most
+  // modules hold a few objects): their bins lie side by side in bins[0, sum of the modules'
   // MDs), each object is counted into its module's bin, and a module-relative
   // start is the running count over all bins minus the objects of the
   // group's earlier modules (each object lies in a bin of its own module).
@@ -775,12 +792,13 @@ namespace lst {
   }
 
   template <typename NOf, typename ObjBase, typename FirstMD>
-  __device__ __forceinline__ bool buildByMDGroup(DeviceES const& es, const EventView& ev, unsigned int w0, NOf nOf,
+  __device__ __forceinline__ bool buildByMDGroup(DeviceES const& es, const EventView& ev, unsigned int w0,
+                                                 unsigned int group, NOf nOf,
                                                  ObjBase objBase, FirstMD firstMD, uint16_t* start, uint16_t* count,
                                                  uint16_t* perm, unsigned int* bins, unsigned int* cursor) {
     const unsigned int lane = laneId();
     const unsigned int w = w0 + lane;
-    const bool inRange = w < es.nLowerModules;
+    const bool inRange = lane < group && w < es.nLowerModules;
     const unsigned int n = inRange ? nOf(w) : 0u;
     const unsigned int nMD = (inRange && n > 0) ? ev.md.nMDs[w] : 0u;
     const unsigned int mdBase = inRange ? static_cast<unsigned int>(es.mdOffset[w]) : 0u;
@@ -868,7 +886,7 @@ namespace lst {
   // not fit (or the fallback paths are forced).  Also sets the modules' segment
   // ranges and clears kCreateLS's counter.
   constexpr int kIdxWarps = 4;
-  __global__ void kLSByMD(DeviceES es, const EventView* evs) {
+  __global__ void kLSByMD(DeviceES es, const EventView* evs, unsigned int group) {
     kernelEntry();
     __shared__ unsigned int sBins[kIdxWarps][kByMDGroupBins];
     __shared__ unsigned int sCursor[kIdxWarps][kByMDGroupBins];
@@ -879,16 +897,16 @@ namespace lst {
     const int wib = threadIdx.x >> 5;
     const unsigned int* mdIdx = ev.ls.mdIndices;
     const unsigned int nWarps = gridDim.x * kIdxWarps;
-    for (unsigned int w0 = (blockIdx.x * kIdxWarps + wib) * 32u; w0 < es.nLowerModules; w0 += nWarps * 32u) {
+    for (unsigned int w0 = (blockIdx.x * kIdxWarps + wib) * group; w0 < es.nLowerModules; w0 += nWarps * group) {
       __syncwarp();
       if (!ev.forceWalk &&
           buildByMDGroup(
-              es, ev, w0, [&](unsigned int w) { return static_cast<unsigned int>(ev.ls.nSegments[w]); },
+              es, ev, w0, group, [&](unsigned int w) { return static_cast<unsigned int>(ev.ls.nSegments[w]); },
               [&](unsigned int w) { return static_cast<unsigned int>(es.lsOffset[w]); },
               [&](unsigned int w, unsigned int k) { return mdIdx[2 * (es.lsOffset[w] + k)] - es.mdOffset[w]; },
               ev.mdLSStart, ev.mdLSCount, ev.lsByMD, sBins[wib], sCursor[wib]))
         continue;
-      for (unsigned int w = w0; w < w0 + 32u && w < es.nLowerModules; ++w) {
+      for (unsigned int w = w0; w < w0 + group && w < es.nLowerModules; ++w) {
         __syncwarp();
         const unsigned int n = ev.ls.nSegments[w];
         if (n == 0)
@@ -918,7 +936,7 @@ namespace lst {
 
   // Triplets of each lower module grouped by first MD (after kCreateT3), in
   // the same way, with the modules' triplet ranges and kCreateT3's counter.
-  __global__ void kT3ByMD(DeviceES es, const EventView* evs) {
+  __global__ void kT3ByMD(DeviceES es, const EventView* evs, unsigned int group) {
     kernelEntry();
     __shared__ unsigned int sBins[kIdxWarps][kByMDGroupBins];
     __shared__ unsigned int sCursor[kIdxWarps][kByMDGroupBins];
@@ -930,18 +948,18 @@ namespace lst {
     const unsigned int* segIdx = ev.t3.segmentIndices;
     const unsigned int* mdIdx = ev.ls.mdIndices;
     const unsigned int nWarps = gridDim.x * kIdxWarps;
-    for (unsigned int w0 = (blockIdx.x * kIdxWarps + wib) * 32u; w0 < es.nLowerModules; w0 += nWarps * 32u) {
+    for (unsigned int w0 = (blockIdx.x * kIdxWarps + wib) * group; w0 < es.nLowerModules; w0 += nWarps * group) {
       __syncwarp();
       if (!ev.forceWalk &&
           buildByMDGroup(
-              es, ev, w0, [&](unsigned int w) { return static_cast<unsigned int>(ev.t3.nTriplets[w]); },
+              es, ev, w0, group, [&](unsigned int w) { return static_cast<unsigned int>(ev.t3.nTriplets[w]); },
               [&](unsigned int w) { return static_cast<unsigned int>(ev.rg.tripletModuleIndices[w]); },
               [&](unsigned int w, unsigned int k) {
                 return mdIdx[2 * segIdx[2 * (ev.rg.tripletModuleIndices[w] + k)]] - es.mdOffset[w];
               },
               ev.mdT3Start, ev.mdT3Count, ev.t3ByMD, sBins[wib], sCursor[wib]))
         continue;
-      for (unsigned int w = w0; w < w0 + 32u && w < es.nLowerModules; ++w) {
+      for (unsigned int w = w0; w < w0 + group && w < es.nLowerModules; ++w) {
         __syncwarp();
         const unsigned int n = ev.t3.nTriplets[w];
         if (n == 0)
@@ -957,22 +975,45 @@ namespace lst {
   }
 
   // ============================================================ triplets
+  // Modules of a one-block-per-event scan over the lower modules: each warp takes
+  // a contiguous run of them, kScanSteps x 32 at a time with all loads of a run
+  // issued before the first sum, so that the scan costs one round of loads and one
+  // block scan of the warps' totals per run (13200 modules: one run).
+  constexpr int kScanSteps = 13;
+  constexpr unsigned int kScanRun = 32u * 32u * kScanSteps;  // modules of one run of a 1024-thread block
+
   // Per-module triplet offsets (SDL/Triplet.h:1007-1102); one block per event.
   __global__ void __launch_bounds__(1024) kT3Offsets(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
+    const unsigned int lane = laneId(), wid = threadIdx.x >> 5;
     unsigned int carry = 0;
-    for (unsigned int base = 0; base < es.nLowerModules; base += blockDim.x) {
-      unsigned int i = base + threadIdx.x;
-      unsigned int occ = 0;
-      bool valid = i < es.nLowerModules;
-      if (valid && ev.ls.nSegments[i] != 0)
-        occ = static_cast<unsigned int>(es.t3CapIfUsed[i]);
+    for (unsigned int base = 0; base < es.nLowerModules; base += kScanRun) {
+      const unsigned int i0 = base + wid * 32u * kScanSteps + lane;
+      unsigned int occ[kScanSteps], ex[kScanSteps], sum = 0;
+#pragma unroll
+      for (int k = 0; k < kScanSteps; ++k) {
+        const unsigned int i = i0 + 32u * k;
+        occ[k] = i < es.nLowerModules && ev.ls.nSegments[i] != 0 ? static_cast<unsigned int>(es.t3CapIfUsed[i]) : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < kScanSteps; ++k) {
+        const unsigned int incl = laneInclusiveSum(occ[k]);
+        ex[k] = sum + incl - occ[k];
+        sum += __shfl_sync(kFullMask, incl, 31);
+      }
       unsigned int tot;
-      unsigned int ex = blockExclusiveScan(occ, tot);
-      if (valid) {
-        ev.rg.tripletModuleIndices[i] = static_cast<int>(carry + ex);
-        ev.rg.tripletModuleOccupancy[i] = static_cast<int>(occ);
+      // (the warp's total from its first lane, so that the exclusive sum at that
+      // lane is the total of the warps before it)
+      const unsigned int before =
+          __shfl_sync(kFullMask, blockExclusiveScan(lane == 0 ? sum : 0u, tot), 0);
+#pragma unroll
+      for (int k = 0; k < kScanSteps; ++k) {
+        const unsigned int i = i0 + 32u * k;
+        if (i < es.nLowerModules) {
+          ev.rg.tripletModuleIndices[i] = static_cast<int>(carry + before + ex[k]);
+          ev.rg.tripletModuleOccupancy[i] = static_cast<int>(occ[k]);
+        }
       }
       carry += tot;
     }
@@ -1060,7 +1101,8 @@ namespace lst {
     const EventView& ev = evs[blockIdx.y];
     const int wib = threadIdx.x >> 5;
     // modules from the event's counter (zero before the kernel)
-    for (unsigned int w = warpNextTask(&ev.sc->t3Next); w < es.nLowerModules; w = warpNextTask(&ev.sc->t3Next)) {
+    WarpTasks tasks(&ev.sc->t3Next);
+    for (unsigned int w = tasks.take(); w < es.nLowerModules; w = tasks.take()) {
       __syncwarp();
       t3Module(es, ev, static_cast<uint16_t>(w), sScratch[wib]);
     }
@@ -1081,52 +1123,80 @@ namespace lst {
   constexpr unsigned int kT5SortCap = 1u << 15;    // quintuplets per event listed for the track-candidate stage
   // Eligible T5 seed modules and their offsets (SDL/Quintuplet.h:3117-3213),
   // and the tasks of kT5Eval's warps: up to 32 inner triplets of one module.
-  // Each thread takes a contiguous range of modules, so that one block scan
-  // of the per-thread sums gives every eligible module its place.
+  // One block per event, a run of modules per warp as in kT3Offsets; the three
+  // sums (modules, quintuplet places, tasks) are scanned together.
   __global__ void __launch_bounds__(1024) kT5Eligible(DeviceES es, const EventView* evs, unsigned int innerPerTask) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
-    const unsigned int n = es.nLowerModules;
-    const unsigned int per = (n + blockDim.x - 1) / blockDim.x;
-    const unsigned int i0 = min(threadIdx.x * per, n), i1 = min(i0 + per, n);
-    auto eligible = [&](unsigned int i) { return ev.t3.nTriplets[i] != 0 && es.t5CapIfEligible[i] >= 0; };
-    auto tasksOf = [&](unsigned int i) {
-      const int layer = es.m.layers[i];
-      return layer == 1 || layer == 2 ? (static_cast<unsigned int>(ev.t3.nTriplets[i]) + innerPerTask - 1u) / innerPerTask : 0u;
-    };
-    unsigned int myN = 0, myQ = 0, myT = 0;
-    for (unsigned int i = i0; i < i1; ++i)
-      if (eligible(i)) {
-        ++myN;
-        myQ += static_cast<unsigned int>(es.t5CapIfEligible[i]);
-        myT += tasksOf(i);
+    const unsigned int lane = laneId(), wid = threadIdx.x >> 5;
+    unsigned int runN = 0, runQ = 0, runT = 0;
+    for (unsigned int base = 0; base < es.nLowerModules; base += kScanRun) {
+      const unsigned int i0 = base + wid * 32u * kScanSteps + lane;
+      unsigned int nT3[kScanSteps];
+      int cap[kScanSteps];
+      unsigned int layer12 = 0;  // bit k: module of step k lies in layer 1 or 2
+      unsigned int sumN = 0, sumQ = 0, sumT = 0;
+#pragma unroll
+      for (int k = 0; k < kScanSteps; ++k) {
+        const unsigned int i = i0 + 32u * k;
+        const bool in = i < es.nLowerModules;
+        nT3[k] = in ? static_cast<unsigned int>(ev.t3.nTriplets[i]) : 0u;
+        cap[k] = in ? es.t5CapIfEligible[i] : -1;
+        const int layer = in ? es.m.layers[i] : 0;
+        layer12 |= (layer == 1 || layer == 2) ? 1u << k : 0u;
       }
-    unsigned int totN, totQ, totT;
-    unsigned int runN = blockExclusiveScan(myN, totN);
-    unsigned int runQ = blockExclusiveScan(myQ, totQ);
-    unsigned int runT = blockExclusiveScan(myT, totT);
-    for (unsigned int i = i0; i < i1; ++i) {
-      if (!eligible(i))
-        continue;
-      const unsigned int occ = static_cast<unsigned int>(es.t5CapIfEligible[i]);
-      const unsigned int nTasks = tasksOf(i);
-      for (unsigned int k = 0; k < nTasks; ++k)
-        ev.t5Task[runT++] = (runN << kT5KeyModuleShift) | (k * innerPerTask);
-      ev.rg.indicesOfEligibleT5Modules[runN++] = static_cast<uint16_t>(i);
-      ev.rg.quintupletModuleIndices[i] = static_cast<int>(runQ);
-      ev.rg.quintupletModuleOccupancy[i] = static_cast<int>(occ);
-      runQ += occ;
-      // (the modules' counts are written by the kernels that store the T5s, for
-      // the modules that have any)
-      ev.t5.nQuintuplets[i] = 0;
-      ev.t5.totOccupancyQuintuplets[i] = 0;
+      auto tasksOf = [&](int k) {
+        return (layer12 >> k) & 1u ? (nT3[k] + innerPerTask - 1u) / innerPerTask : 0u;
+      };
+#pragma unroll
+      for (int k = 0; k < kScanSteps; ++k)
+        if (nT3[k] != 0 && cap[k] >= 0) {
+          ++sumN;
+          sumQ += static_cast<unsigned int>(cap[k]);
+          sumT += tasksOf(k);
+        }
+      unsigned int totN, totQ, totT;
+      const unsigned int n0 = laneInclusiveSum(sumN), q0 = laneInclusiveSum(sumQ), t0 = laneInclusiveSum(sumT);
+      const unsigned int bN = blockExclusiveScan(lane == 31 ? n0 : 0u, totN);
+      const unsigned int bQ = blockExclusiveScan(lane == 31 ? q0 : 0u, totQ);
+      const unsigned int bT = blockExclusiveScan(lane == 31 ? t0 : 0u, totT);
+      // (before lane 31's value is added, every lane of the warp has the total of
+      // the warps before it)
+      unsigned int posN = runN + bN, posQ = runQ + bQ, posT = runT + bT;
+#pragma unroll
+      for (int k = 0; k < kScanSteps; ++k) {
+        const unsigned int i = i0 + 32u * k;
+        const bool on = nT3[k] != 0 && cap[k] >= 0;
+        const unsigned int occ = on ? static_cast<unsigned int>(cap[k]) : 0u, nTasks = on ? tasksOf(k) : 0u;
+        const unsigned int mask = __ballot_sync(kFullMask, on);
+        const unsigned int inclQ = laneInclusiveSum(occ), inclT = laneInclusiveSum(nTasks);
+        if (on) {
+          const unsigned int pos = posN + __popc(mask & lanesBelowMask());
+          const unsigned int first = posT + inclT - nTasks;
+          for (unsigned int t = 0; t < nTasks; ++t)
+            ev.t5Task[first + t] = (pos << kT5KeyModuleShift) | (t * innerPerTask);
+          ev.rg.indicesOfEligibleT5Modules[pos] = static_cast<uint16_t>(i);
+          ev.rg.quintupletModuleIndices[i] = static_cast<int>(posQ + inclQ - occ);
+          ev.rg.quintupletModuleOccupancy[i] = static_cast<int>(occ);
+          // (the modules' counts are written by the kernels that store the T5s, for
+          // the modules that have any)
+          ev.t5.nQuintuplets[i] = 0;
+          ev.t5.totOccupancyQuintuplets[i] = 0;
+        }
+        posN += __popc(mask);
+        posQ += __shfl_sync(kFullMask, inclQ, 31);
+        posT += __shfl_sync(kFullMask, inclT, 31);
+      }
+      runN += totN;
+      runQ += totQ;
+      runT += totT;
     }
     if (threadIdx.x == 0) {
-      *ev.rg.nEligibleT5Modules = static_cast<uint16_t>(totN);
-      *ev.rg.device_nTotalQuints = totQ;
-      ev.sc->t5Tasks = totT;
+      *ev.rg.nEligibleT5Modules = static_cast<uint16_t>(runN);
+      *ev.rg.device_nTotalQuints = runQ;
+      ev.sc->t5Tasks = runT;
       ev.sc->t5InnerPerTask = innerPerTask;
-      ev.sc->t5Overflow = totN > kT5KeyModules ? 1u : 0u;
+      ev.sc->t5Overflow = runN > kT5KeyModules ? 1u : 0u;
       ev.sc->t5Next = 0;
       ev.sc->t5StagedCount = 0;
       ev.sc->t5PassCount = 0;
@@ -1362,6 +1432,7 @@ namespace lst {
     T5Scratch& sc = sScratch[threadIdx.x >> 5];
     const Triplets& t3 = ev.t3;
     const unsigned int nTasks = ev.sc->t5Tasks, innerPerTask = ev.sc->t5InnerPerTask;
+    WarpTasks tasks(&ev.sc->t5Next);
     const unsigned int lane = laneId();
     bool more = true;                // the event may have tasks left
     unsigned int module = 0, inner0 = 0, t3Base = 0;  // the current task: module position, first inner triplet
@@ -1401,7 +1472,7 @@ namespace lst {
           }
           n0 += __popc(ok);
         } else if (more) {
-          const unsigned int task = warpNextTask(&ev.sc->t5Next);
+          const unsigned int task = tasks.take();
           more = task < nTasks;
           if (!more)
             break;
@@ -1649,11 +1720,12 @@ namespace lst {
   constexpr int kT5RankThreads = 128;
   __global__ void __launch_bounds__(kT5RankThreads) kT5RankEmit(DeviceES es, const EventView* evs) {
     kernelEntry();
-    __shared__ unsigned int sKey[kT5RankCap];
+    __shared__ __align__(16) unsigned int sKey[kT5RankCap];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.sc->t5PassCount;
     if (t5NeedsWalk(ev) || blockIdx.x * kT5RankThreads >= n)
       return;
+    const unsigned int n4 = n & ~3u;  // four keys a read
     for (unsigned int j = threadIdx.x; j < n; j += kT5RankThreads)
       sKey[j] = ev.t5PassC[j];
     __syncthreads();
@@ -1662,11 +1734,21 @@ namespace lst {
     for (unsigned int q = blockIdx.x * kT5RankThreads + threadIdx.x; q < n; q += gridDim.x * kT5RankThreads) {
       const unsigned int key = sKey[q], w = key >> kT5KeyModuleShift, base = w << kT5KeyModuleShift;
       unsigned int r = 0, count = 0;
-      for (unsigned int j = 0; j < n; ++j) {
-        const unsigned int d = sKey[j] - base;  // wraps to a large value below the module's keys
+      auto add = [&](unsigned int k) {
+        const unsigned int d = k - base;  // wraps to a large value below the module's keys
         r += d < key - base ? 1u : 0u;
         count += d < (1u << kT5KeyModuleShift) ? 1u : 0u;
+      };
+#pragma unroll 2
+      for (unsigned int j = 0; j < n4; j += 4) {
+        const uint4 k = *reinterpret_cast<const uint4*>(sKey + j);
+        add(k.x);
+        add(k.y);
+        add(k.z);
+        add(k.w);
       }
+      for (unsigned int j = n4; j < n; ++j)
+        add(sKey[j]);
       const uint16_t lm1 = ev.rg.indicesOfEligibleT5Modules[w];
       const int cap = ev.rg.quintupletModuleOccupancy[lm1];
       if (int(r) < cap) {
@@ -2022,9 +2104,35 @@ namespace lst {
     for (int b = threadIdx.x; b <= kPLSBins; b += blockDim.x)
       sCount[b] = 0;
     __syncthreads();
-    for (unsigned int i = threadIdx.x; i < nPix; i += blockDim.x)
-      if (plsCleanEligible(s, i, true))
-        atomicAdd(&sCount[plsEtaBin(s.eta[i])], 1u);
+    // The eligible pLS among 8 of this thread's at a time, all loads of a round
+    // issued together (a round of one pLS per thread waited for each load).
+    constexpr int kRound = 8;
+    auto round = [&](unsigned int i0, float* eta, float* phi) {
+      unsigned int on = 0;
+      int8_t quad[kRound], dup[kRound];
+#pragma unroll
+      for (int k = 0; k < kRound; ++k) {
+        const unsigned int i = i0 + k * 1024u;
+        const bool in = i < nPix;
+        quad[k] = in ? s.isQuad[i] : 0;
+        dup[k] = in ? s.isDup[i] : 1;
+        eta[k] = in ? s.eta[i] : 0.f;
+        if (phi)
+          phi[k] = in ? s.phi[i] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < kRound; ++k)
+        on |= quad[k] && !(dup[k] & 1) ? 1u << k : 0u;
+      return on;
+    };
+    for (unsigned int i0 = threadIdx.x; i0 < nPix; i0 += kRound * 1024u) {
+      float eta[kRound];
+      const unsigned int on = round(i0, eta, nullptr);
+#pragma unroll
+      for (int k = 0; k < kRound; ++k)
+        if ((on >> k) & 1u)
+          atomicAdd(&sCount[plsEtaBin(eta[k])], 1u);
+    }
     __syncthreads();
     unsigned int c = threadIdx.x <= kPLSBins ? sCount[threadIdx.x] : 0u;
     unsigned int tot;
@@ -2036,15 +2144,19 @@ namespace lst {
     if (threadIdx.x == 0)
       ev.plsBinStart[kPLSBins + 1] = tot;
     __syncthreads();
-    for (unsigned int i = threadIdx.x; i < nPix; i += blockDim.x) {
-      if (!plsCleanEligible(s, i, true))
-        continue;
-      PLSRec r;
-      r.eta = s.eta[i];
-      r.phi = s.phi[i];
-      r.index = i;
-      r.pad = 0;
-      ev.plsRec[atomicAdd(&sCursor[plsEtaBin(r.eta)], 1u)] = r;
+    for (unsigned int i0 = threadIdx.x; i0 < nPix; i0 += kRound * 1024u) {
+      float eta[kRound], phi[kRound];
+      const unsigned int on = round(i0, eta, phi);
+#pragma unroll
+      for (int k = 0; k < kRound; ++k)
+        if ((on >> k) & 1u) {
+          PLSRec r;
+          r.eta = eta[k];
+          r.phi = phi[k];
+          r.index = i0 + k * 1024u;
+          r.pad = 0;
+          ev.plsRec[atomicAdd(&sCursor[plsEtaBin(r.eta)], 1u)] = r;
+        }
     }
   }
 
@@ -2644,6 +2756,7 @@ namespace lst {
     const unsigned int lane = laneId();
     const unsigned int nWarps = gridDim.x * (blockDim.x >> 5);
     const unsigned int perTask = min(32u, max(1u, nPLS / (2u * nWarps)));
+    WarpTasks tasks(&ev.sc->pixNext);
     bool more = true;                  // the event may have tasks left
     unsigned int task = 0, left = 0;   // the current task's first pLS and the lanes of those not yet grouped
     unsigned int size = 0, index = 0;  // this lane's pLS of the task: its pixel-map slice
@@ -2736,7 +2849,7 @@ namespace lst {
             __syncwarp();
             f0 = 0;
           } else if (more) {
-            task = warpNextTask(&ev.sc->pixNext) * perTask;
+            task = tasks.take() * perTask;
             more = task < nPLS;
             const unsigned int i = task + lane;
             size = 0;
@@ -2837,7 +2950,7 @@ namespace lst {
   template <int K>
   __global__ void __launch_bounds__(kPixRankThreads) kPixRankEmit(DeviceES es, const EventView* evs) {
     kernelEntry();
-    __shared__ unsigned int sKey[kPixPassCap];
+    __shared__ __align__(16) unsigned int sKey[kPixPassCap];
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = ev.sc->pixPassCount;
     const unsigned int capOut = K == 5 ? kMaxPixelQuintuplets : kMaxPixelTriplets;
@@ -2848,8 +2961,9 @@ namespace lst {
     }
     if (blockIdx.x != 0 && blockIdx.x * blockDim.x >= n)
       return;
-    for (unsigned int j = threadIdx.x; j < n; j += blockDim.x)
-      sKey[j] = ev.pixPassC[j];
+    const unsigned int n4 = (n + 3u) & ~3u;  // (four keys a read; the last ones never rank below)
+    for (unsigned int j = threadIdx.x; j < n4; j += blockDim.x)
+      sKey[j] = j < n ? ev.pixPassC[j] : 0xffffffffu;
     __syncthreads();
     const unsigned int plsBase = es.lsOffset[es.nLowerModules];
     Segments ls = ev.ls;
@@ -2858,8 +2972,11 @@ namespace lst {
     for (unsigned int sIdx = blockIdx.x * blockDim.x + threadIdx.x; sIdx < n; sIdx += gridDim.x * blockDim.x) {
       const unsigned int key = sKey[sIdx];
       unsigned int rank = 0;
-      for (unsigned int j = 0; j < n; ++j)
-        rank += sKey[j] < key ? 1u : 0u;
+#pragma unroll 4
+      for (unsigned int j = 0; j < n4; j += 4) {
+        const uint4 k = *reinterpret_cast<const uint4*>(sKey + j);
+        rank += (k.x < key ? 1u : 0u) + (k.y < key ? 1u : 0u) + (k.z < key ? 1u : 0u) + (k.w < key ? 1u : 0u);
+      }
       if (rank >= capOut)
         continue;
       const unsigned int obj = ev.pixPassObj[sIdx];
