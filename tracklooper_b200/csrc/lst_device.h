@@ -78,7 +78,7 @@ namespace lst {
     unsigned int mdNext;          // next task for kCreateMD's warps
     unsigned int lsNext;          // next lower module for kCreateLS's warps
     unsigned int pixNext; // next task (a few pLS) for kPixMid's warps
-    unsigned int t3Next;          // next lower module for kCreateT3's warps
+    unsigned int t3Next;          // next task for kCreateT3's blocks
   };
 
   // All device pointers of one event.

@@ -517,6 +517,13 @@ namespace {
                                                    static_cast<size_t>(std::max(count, 1))));
     return dim3(static_cast<unsigned int>(std::min(want, cap)), count);
   }
+  // Tuned kernel k, a block per task.
+  dim3 tunedBlockGrid(const lst_event* ev, int k, size_t nTasks, int count) {
+    const LaunchShape& sh = ev->shape[k];
+    const size_t cap = std::max<size_t>(1, ceilDiv(static_cast<size_t>(sh.perSM) * ev->nSM,
+                                                   static_cast<size_t>(std::max(count, 1))));
+    return dim3(static_cast<unsigned int>(std::min(std::max<size_t>(1, nTasks), cap)), count);
+  }
   // Tuned kernel k striding over a candidate list whose length only the device knows.
   dim3 tunedFlatGrid(const lst_event* ev, int k, int count) {
     const LaunchShape& sh = ev->shape[k];
@@ -556,11 +563,17 @@ namespace {
         LST_LAUNCH(lst::kCreateLS, tunedWarpGrid(ev, kTuLS, nLower, count), tunedThreads(ev, kTuLS), d, v);
         LST_LAUNCH(lst::kLSByMD, warpGrid(ceilDiv(nLower, group), lst::kIdxWarps, count), 32 * lst::kIdxWarps, d, v, group);
         break;
-      case LST_STAGE_TRIPLETS:
+      case LST_STAGE_TRIPLETS: {
+        // modules per block task: 16, and 8 for a few events, which then make 1660
+        // tasks each (one event: 41 us, with 4 43, with 16 64; 64 events at 16
+        // blocks per SM: 770, with 8 930, with 32 720; 8 events: 115, 134, 150)
+        const unsigned int t3Modules = count >= 4 ? 16u : 8u;
         LST_LAUNCH(lst::kT3Offsets, one, 1024, d, v);
-        LST_LAUNCH(lst::kCreateT3, tunedWarpGrid(ev, kTuT3, nLower, count), tunedThreads(ev, kTuT3), d, v);
+        LST_LAUNCH(lst::kCreateT3, tunedBlockGrid(ev, kTuT3, ceilDiv(nLower, t3Modules), count), tunedThreads(ev, kTuT3),
+                   d, v, t3Modules);
         LST_LAUNCH(lst::kT3ByMD, warpGrid(ceilDiv(nLower, group), lst::kIdxWarps, count), 32 * lst::kIdxWarps, d, v, group);
         break;
+      }
       case LST_STAGE_QUINTUPLETS: {
         if (ev->t5Method == LST_T5_DNN && !ev->es->haveDnn)
           return setError("the DNN T5 method needs weights (lst_es_load or lst_es_set_t5dnn_weights)");

@@ -90,6 +90,16 @@ namespace lst {
     return lo;
   }
 
+  __device__ __forceinline__ unsigned int laneInclusiveSum(unsigned int v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int y = __shfl_up_sync(kFullMask, v, o);
+      if (int(laneId()) >= o)
+        v += y;
+    }
+    return v;
+  }
+
   // Block-wide exclusive scan (blockDim.x a multiple of 32, <= 1024).
   __device__ __forceinline__ unsigned int blockExclusiveScan(unsigned int v, unsigned int& total) {
     __shared__ unsigned int sWarp[32];
@@ -410,6 +420,71 @@ namespace lst {
     }
   };
 
+  // The same for the calling block's tasks.  (The barriers also end the use of
+  // the shared memory of the task before.)
+  struct BlockTasks {
+    unsigned int* next;
+    bool started = false;
+    __device__ __forceinline__ explicit BlockTasks(unsigned int* counter) : next(counter) {}
+    __device__ __forceinline__ unsigned int take() {
+      if (!started) {
+        started = true;
+        return blockIdx.x;
+      }
+      __shared__ unsigned int sTask;
+      __syncthreads();
+      if (threadIdx.x == 0)
+        sTask = gridDim.x + atomicAdd(next, 1u);
+      __syncthreads();
+      return sTask;
+    }
+  };
+
+  // A block's queue of candidates, in order: the calling thread's place (if it
+  // adds one), and the queue's new length.  Every thread calls it; the entries
+  // may be written when it returns and read after a barrier.
+  __device__ __forceinline__ unsigned int blockQueuePlace(bool add, unsigned int* warpCount, unsigned int& queued) {
+    unsigned int n;
+    unsigned int at = queued + warpRank(add, n);
+    const unsigned int wid = threadIdx.x >> 5;
+    if (laneId() == 0)
+      warpCount[wid] = n;
+    __syncthreads();
+    for (unsigned int w = 0; w < blockDim.x >> 5; ++w) {
+      const unsigned int c = warpCount[w];
+      at += w < wid ? c : 0u;
+      queued += c;
+    }
+    return at;
+  }
+
+  // The rank of a passing candidate among its module's, over the block's tasks of
+  // up to 32 modules (module j's count so far in count[j]).  passing[] holds 32
+  // words per warp.  Every thread calls it, then blockRankDone.
+  __device__ __forceinline__ unsigned int blockModuleRank(bool ok, unsigned int j, unsigned int* passing,
+                                                          const unsigned int* count) {
+    const unsigned int wid = threadIdx.x >> 5;
+    passing[32u * wid + laneId()] = 0;
+    __syncwarp();
+    const unsigned int peers = __match_any_sync(kFullMask, ok ? j : 32u + laneId());
+    const unsigned int rank = __popc(peers & lanesBelowMask());
+    if (ok && rank == 0)
+      passing[32u * wid + j] = __popc(peers);
+    __syncthreads();
+    unsigned int r = count[j] + rank;
+    for (unsigned int w = 0; w < wid; ++w)
+      r += passing[32u * w + j];
+    return r;
+  }
+  // Ends with a barrier.
+  __device__ __forceinline__ void blockRankDone(const unsigned int* passing, unsigned int* count) {
+    __syncthreads();
+    if (threadIdx.x < 32)
+      for (unsigned int w = 0; w < blockDim.x >> 5; ++w)
+        count[threadIdx.x] += passing[32u * w + threadIdx.x];
+    __syncthreads();
+  }
+
   // ======================================================== mini-doublets
   // SDL/MiniDoublet.h:896-992: every (lower hit, upper hit) pair of a lower
   // module is a candidate; passing ones are stored in the module's arena at
@@ -516,7 +591,7 @@ namespace lst {
 #define LST_LB_LS_B 12
 #endif
 #ifndef LST_LB_T3_B
-#define LST_LB_T3_B 10
+#define LST_LB_T3_B 14
 #endif
 #ifndef LST_LB_EVAL_B
 #define LST_LB_EVAL_B 10
@@ -781,16 +856,6 @@ namespace lst {
     }
     return owner;
   }
-  __device__ __forceinline__ unsigned int laneInclusiveSum(unsigned int v) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned int y = __shfl_up_sync(kFullMask, v, o);
-      if (int(laneId()) >= o)
-        v += y;
-    }
-    return v;
-  }
-
   template <typename NOf, typename ObjBase, typename FirstMD>
   __device__ __forceinline__ bool buildByMDGroup(DeviceES const& es, const EventView& ev, unsigned int w0,
                                                  unsigned int group, NOf nOf,
@@ -1021,91 +1086,176 @@ namespace lst {
       *ev.rg.device_nTotalTrips = carry;
   }
 
-  // One warp per inner-inner lower module walking (inner segment, outer
-  // segment of the middle module) in order (SDL/Triplet.h:874-1005).
+  // Triplets (SDL/Triplet.h:874-1005): a block walks (inner segment, outer
+  // segment of the middle module) of several inner lower modules in order.
   //
-  // The inner segments are taken kT3Chunk at a time.  For each the warp
-  // keeps in shared memory the prefix of its candidates and where its outer
-  // segments are listed (the MD-keyed segment index of the middle module),
-  // so that a candidate reaches its outer segment with one global load.
+  // Most modules hold a few inner segments and some twenty candidates, the
+  // heaviest thousands.  A task is therefore up to kT3TaskModules modules, whose
+  // inner segments are dealt out across the module boundaries, a thread each, so
+  // that the chain of a dozen dependent loads to a triplet is not spent on one
+  // module's few candidates; and a task is a block's rather than a warp's, so that
+  // a heavy module does not outlast the rest of the kernel in one warp.  For each
+  // inner segment shared memory holds the prefix of its candidates and where its
+  // outer segments are listed (the MD-keyed segment index of the middle module),
+  // so that a candidate reaches its outer segment with one global load.  Only
+  // outer segments whose inner MD is the inner segment's outer MD can pass (the
+  // first test of the reference's triplet algorithm), so no others are listed;
+  // they come in storage order, and candidates keep the reference's (inner,
+  // outer) order.
+  //
+  // Three quarters of the candidates end at the r-z residual (241k per PU200
+  // event: 93k have layers that never pass, 86k a residual too large), so a
+  // candidate takes that test first and the ones that pass wait in a queue,
+  // in order, until there is one for every thread for the rest of the tests.  A
+  // passing triplet's place is its module's running count plus the passing
+  // candidates of the same module before it.
+  //
+  // Bound by the latency of the gathers (long scoreboard and the barriers that
+  // wait for them; issue slots half used).  A warp per module, all tests in one
+  // pass: 64 PU200 events 1120 us, 8 events 183, one 86; so 520 (with the blocks
+  // per SM of the default shape; 760 at the same 16), 115 and 38.  A warp per
+  // task of 8 modules: 636 at 16 blocks per SM, but 180 for 8 events and 66 for
+  // one, where single warps with heavy modules set the length.
   constexpr int kT3Warps = 4;
-  constexpr int kT3Chunk = 128;
+  constexpr unsigned int kT3Threads = 32 * kT3Warps;  // threads per block the kernel is launched with (at most)
+  constexpr unsigned int kT3TaskModules = 32;         // modules per task (at most, a lane each)
   struct T3Scratch {
-    unsigned int pre[kT3Chunk + 1];
-    unsigned int listStart[kT3Chunk];  // first entry of the inner segment's outer segments in lsByMD
-    unsigned int outerBase[kT3Chunk];  // first segment of the middle module
+    unsigned int pre[kT3Threads + 1];
+    unsigned int innerSeg[kT3Threads];
+    unsigned int listStart[kT3Threads];  // first entry of the inner segment's outer segments in lsByMD
+    unsigned int outerBase[kT3Threads];  // first segment of the middle module
+    unsigned int modulePre[kT3TaskModules + 1];  // prefix of the task's inner segments over its modules
+    unsigned int segBase[kT3TaskModules], flags[kT3TaskModules], count[kT3TaskModules];
+    unsigned int passing[32 * kT3Warps];  // per warp and module, of the candidates in hand
+    unsigned int warpCount[kT3Warps];
+    uint2 queue[2 * kT3Threads];           // (inner, outer) segments that passed the r-z test
+    uint8_t queueModule[2 * kT3Threads];   //   and the number of the module in the task
+    uint8_t module[kT3Threads];
   };
-  __device__ __forceinline__ void t3Module(DeviceES const& es, const EventView& ev, uint16_t lm1, T3Scratch& sc) {
+  __device__ __forceinline__ void t3Task(DeviceES const& es, const EventView& ev, unsigned int firstModule,
+                                         unsigned int nModules, T3Scratch& sc) {
     const Modules& m = es.m;
-    if (m.nConnectedModules[lm1] == 0)
-      return;
-    const unsigned int nInner = ev.ls.nSegments[lm1];
-    if (nInner == 0)
-      return;
-    const unsigned int segBase = es.lsOffset[lm1];
+    const unsigned int lane = laneId(), wid = threadIdx.x >> 5, nThreads = blockDim.x;
     const Segments& ls = ev.ls;
-    const int cap = ev.rg.tripletModuleOccupancy[lm1];
-    const unsigned int base = ev.rg.tripletModuleIndices[lm1];
+    const MDRec* rec = ev.md.rec;
+    // the lane's module (every warp has all of the task's)
+    const unsigned int own = firstModule + lane;
+    const bool valid = lane < nModules && own < es.nLowerModules && m.nConnectedModules[own] != 0;
+    const unsigned int nInnerOwn = valid ? static_cast<unsigned int>(ls.nSegments[own]) : 0u;
+    const int capOwn = valid ? ev.rg.tripletModuleOccupancy[own] : 0;
+    const unsigned int baseOwn = valid ? static_cast<unsigned int>(ev.rg.tripletModuleIndices[own]) : 0u;
+    const unsigned int incl = laneInclusiveSum(nInnerOwn);
+    const unsigned int nInner = __shfl_sync(kFullMask, incl, 31);
+    if (wid == 0) {
+      sc.segBase[lane] = valid ? static_cast<unsigned int>(es.lsOffset[own]) : 0u;
+      sc.flags[lane] = valid ? es.lsCuts[own].flags : 0u;
+      sc.count[lane] = 0;
+      sc.modulePre[lane + 1] = incl;
+      if (lane == 0)
+        sc.modulePre[0] = 0;
+    }
+    __syncthreads();
     Triplets t3 = ev.t3;
-    unsigned int count = 0;
-    for (unsigned int c0 = 0; c0 < nInner; c0 += kT3Chunk) {
-      const int n = int(min(nInner - c0, unsigned(kT3Chunk)));
-      __syncwarp();  // the previous chunk's scratch has been read
-      // Only outer segments whose inner MD is the inner segment's outer MD
-      // can pass (the first test of the reference's triplet algorithm); they
-      // are enumerated through the MD-keyed segment index in storage order,
-      // so candidates keep the reference's (inner, outer) order.
-      const unsigned int total = warpPrefix(sc.pre, n, [&](int i) {
-        const unsigned int seg = segBase + c0 + unsigned(i);
+    unsigned int queued = 0;
+    for (unsigned int c0 = 0; c0 < nInner; c0 += nThreads) {
+      const int n = int(min(nInner - c0, nThreads));
+      const bool lastChunk = c0 + nThreads >= nInner;
+      unsigned int nOuter = 0;
+      if (int(threadIdx.x) < n) {
+        const unsigned int g = c0 + threadIdx.x;
+        const int j = findSlot(sc.modulePre, kT3TaskModules, g);
+        const unsigned int seg = sc.segBase[j] + (g - sc.modulePre[j]);
         const uint16_t middle = ls.outerLowerModuleIndices[seg];
-        if (ls.nSegments[middle] == 0)
-          return 0u;
         const unsigned int mdMid = ls.mdIndices[2 * seg + 1];
         const unsigned int outerBase = es.lsOffset[middle];
-        sc.outerBase[i] = outerBase;
-        sc.listStart[i] = outerBase + ev.mdLSStart[mdMid];
-        return static_cast<unsigned int>(ev.mdLSCount[mdMid]);
-      });
-      for (unsigned int start = 0; start < total; start += 32) {
-        unsigned int f = start + laneId();
-        bool ok = false;
-        T3Values v;
-        unsigned int innerSeg = 0, outerSeg = 0;
-        uint16_t middle = 0, outerOuter = 0;
-        if (f < total) {
-          int i = findSlot(sc.pre, n, f);
-          innerSeg = segBase + c0 + unsigned(i);
-          middle = ls.outerLowerModuleIndices[innerSeg];
-          outerSeg = sc.outerBase[i] + ev.lsByMD[sc.listStart[i] + (f - sc.pre[i])];
-          outerOuter = ls.outerLowerModuleIndices[outerSeg];
-          ok = t3Select(m, ev.md, ls, lm1, middle, outerOuter, innerSeg, outerSeg, v);
+        const unsigned int listStart = ev.mdLSStart[mdMid], listed = ev.mdLSCount[mdMid];
+        sc.innerSeg[threadIdx.x] = seg;
+        sc.module[threadIdx.x] = static_cast<uint8_t>(j);
+        sc.outerBase[threadIdx.x] = outerBase;
+        if (ls.nSegments[middle] != 0) {  // (the index is written for these only)
+          sc.listStart[threadIdx.x] = outerBase + listStart;
+          nOuter = listed;
         }
-        unsigned int tot;
-        unsigned int r = count + warpRank(ok, tot);
-        if (ok && int(r) < cap)
-          storeT3(m, ev.md, ls, t3, innerSeg, outerSeg, lm1, middle, outerOuter, v, base + r);
-        count += tot;
       }
+      unsigned int total;
+      const unsigned int before = blockExclusiveScan(nOuter, total);
+      if (int(threadIdx.x) < n)
+        sc.pre[threadIdx.x] = before;
+      if (threadIdx.x == 0)
+        sc.pre[n] = total;
+      __syncthreads();
+      for (unsigned int start = 0; start < total || (lastChunk && queued > 0); start += nThreads) {
+        const unsigned int f = start + threadIdx.x;
+        bool pass = false;
+        unsigned int innerSeg = 0, outerSeg = 0, module = 0;
+        if (f < total) {
+          const int i = findSlot(sc.pre, n, f);
+          innerSeg = sc.innerSeg[i];
+          module = sc.module[i];
+          outerSeg = sc.outerBase[i] + ev.lsByMD[sc.listStart[i] + (f - sc.pre[i])];
+          const float cut =
+              t3RZCut(cutLayer(sc.flags[module]), cutLayer(es.lsCuts[ls.outerLowerModuleIndices[innerSeg]].flags),
+                      cutLayer(es.lsCuts[ls.outerLowerModuleIndices[outerSeg]].flags));
+          if (cut > 0) {
+            const MDRec& in = rec[ls.mdIndices[2 * innerSeg]];
+            const MDRec& mid = rec[ls.mdIndices[2 * innerSeg + 1]];
+            const MDRec& out = rec[ls.mdIndices[2 * outerSeg + 1]];
+            pass = t3PassRZ(in.rt, in.z, mid.rt, mid.z, out.rt, out.z, cut);
+          }
+        }
+        const unsigned int at = blockQueuePlace(pass, sc.warpCount, queued);
+        if (pass) {
+          sc.queue[at] = make_uint2(innerSeg, outerSeg);
+          sc.queueModule[at] = static_cast<uint8_t>(module);
+        }
+        __syncthreads();
+        const bool flush = lastChunk && start + nThreads >= total;
+        while (queued >= nThreads || (flush && queued > 0)) {
+          bool ok = false;
+          T3Values v;
+          uint16_t middle = 0, outerOuter = 0;
+          const uint2 segs = sc.queue[threadIdx.x], moved = sc.queue[nThreads + threadIdx.x];
+          const unsigned int j = threadIdx.x < queued ? sc.queueModule[threadIdx.x] : 0u;
+          const uint8_t movedModule = sc.queueModule[nThreads + threadIdx.x];
+          if (threadIdx.x < queued) {
+            middle = ls.outerLowerModuleIndices[segs.x];
+            outerOuter = ls.outerLowerModuleIndices[segs.y];
+            ok = t3Rest(sc.flags[j], es.lsCuts[middle].flags, es.lsCuts[outerOuter].flags, m.ptCut,
+                        rec[ls.mdIndices[2 * segs.x]], rec[ls.mdIndices[2 * segs.x + 1]],
+                        rec[ls.mdIndices[2 * segs.y + 1]], ls, segs.x, v);
+          }
+          const int cap = __shfl_sync(kFullMask, capOwn, j);
+          const unsigned int base = __shfl_sync(kFullMask, baseOwn, j);
+          const unsigned int r = blockModuleRank(ok, j, sc.passing, sc.count);
+          if (ok && int(r) < cap)
+            storeT3(m, ev.md, ls, t3, segs.x, segs.y, static_cast<uint16_t>(firstModule + j), middle, outerOuter, v,
+                    base + r);
+          sc.queue[threadIdx.x] = moved;
+          sc.queueModule[threadIdx.x] = movedModule;
+          queued -= min(queued, nThreads);
+          blockRankDone(sc.passing, sc.count);
+        }
+      }
+      __syncthreads();  // the chunk's scratch has been read
     }
-    if (laneId() == 0) {
-      t3.nTriplets[lm1] = (int(count) < cap) ? count : (cap > 0 ? unsigned(cap) : 0u);
-      t3.totOccupancyTriplets[lm1] = count;
-      if (int(count) > cap)
+    if (wid == 0 && nInnerOwn > 0) {
+      const unsigned int n = sc.count[lane];
+      t3.nTriplets[own] = (int(n) < capOwn) ? n : (capOwn > 0 ? unsigned(capOwn) : 0u);
+      t3.totOccupancyTriplets[own] = n;
+      if (int(n) > capOwn)
         atomicOr(&ev.sc->status, kStatusCapOverflow);
     }
   }
 
-  __global__ void __launch_bounds__(LST_LB_T3) kCreateT3(DeviceES es, const EventView* evs) {
+  __global__ void __launch_bounds__(LST_LB_T3) kCreateT3(DeviceES es, const EventView* evs, unsigned int modulesPerTask) {
     kernelEntry();
-    __shared__ T3Scratch sScratch[kT3Warps];
+    __shared__ T3Scratch sc;
     const EventView& ev = evs[blockIdx.y];
-    const int wib = threadIdx.x >> 5;
-    // modules from the event's counter (zero before the kernel)
-    WarpTasks tasks(&ev.sc->t3Next);
-    for (unsigned int w = tasks.take(); w < es.nLowerModules; w = tasks.take()) {
-      __syncwarp();
-      t3Module(es, ev, static_cast<uint16_t>(w), sScratch[wib]);
-    }
+    const unsigned int nTasks = (es.nLowerModules + modulesPerTask - 1u) / modulesPerTask;
+    // tasks from the event's counter (zero before the kernel)
+    BlockTasks tasks(&ev.sc->t3Next);
+    for (unsigned int task = tasks.take(); task < nTasks; task = tasks.take())
+      t3Task(es, ev, task * modulesPerTask, modulesPerTask, sc);
   }
 
   // ========================================================= quintuplets

@@ -140,7 +140,8 @@ namespace lst {
     kCutMovesLower = 16,    // shiftMovesLower
     kCutEndcap = 32,
     kCutEndcapTwoS = 64,
-    kCutInnerLayers = 128   // layers 1 and 2
+    kCutInnerLayers = 128,  // layers 1 and 2
+    kCutLayerShift = 8      // from this bit on: sdlLayers
   };
 
   LST_HD unsigned int cutFlags(const Modules& m, uint16_t mi) {
@@ -148,8 +149,10 @@ namespace lst {
     return (barrel ? kCutBarrel : 0u) | (barrel and m.sides[mi] == Center ? kCutCenter : 0u) |
            (m.moduleType[mi] == PS ? kCutPS : 0u) | (m.moduleLayerType[mi] == Pixel ? kCutLowerIsPixel : 0u) |
            (shiftMovesLower(m, mi) ? kCutMovesLower : 0u) | (endcap ? kCutEndcap : 0u) |
-           (endcap and m.moduleType[mi] == TwoS ? kCutEndcapTwoS : 0u) | (m.layers[mi] <= 2 ? kCutInnerLayers : 0u);
+           (endcap and m.moduleType[mi] == TwoS ? kCutEndcapTwoS : 0u) | (m.layers[mi] <= 2 ? kCutInnerLayers : 0u) |
+           (static_cast<unsigned int>(m.sdlLayers[mi]) << kCutLayerShift);
   }
+  LST_HD int cutLayer(unsigned int flags) { return static_cast<int>(flags >> kCutLayerShift); }
 
   LST_HD MDCut mdCut(const Modules& m, uint16_t mi) {
     unsigned int iL = m.layers[mi] - 1;

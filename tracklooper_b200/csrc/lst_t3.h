@@ -6,50 +6,38 @@
 
 namespace lst {
 
-  // r-z residual of the middle hit against the line through the outer two
-  // (SDL/Triplet.h:241-299); layers use the sdlLayers numbering.
-  LST_HD bool t3PassRZ(const Modules& m,
-                       const MiniDoublets& md,
-                       uint16_t lm1,
-                       uint16_t lm2,
-                       uint16_t lm3,
-                       unsigned int md1,
-                       unsigned int md2,
-                       unsigned int md3) {
-    const float r1 = md.rec[md1].rt, r2 = md.rec[md2].rt, r3 = md.rec[md3].rt;
-    const float z1 = md.rec[md1].z, z2 = md.rec[md2].z, z3 = md.rec[md3].z;
-    const int layer1 = m.sdlLayers[lm1], layer2 = m.sdlLayers[lm2], layer3 = m.sdlLayers[lm3];
+  // Largest r-z residual of the middle hit against the line through the outer
+  // two, by the three modules' layers in the sdlLayers numbering
+  // (SDL/Triplet.h:241-299); 0 for the layers that never pass.
+  LST_HD float t3RZCut(int layer1, int layer2, int layer3) {
+    const int key = (layer1 << 10) | (layer2 << 5) | layer3;
+    switch (key) {
+      case (12 << 10) | (13 << 5) | 14:
+      case (13 << 10) | (14 << 5) | 15:
+      case (14 << 10) | (15 << 5) | 16:
+        return 0.f;
+      case (1 << 10) | (2 << 5) | 3:
+        return 0.53f;
+      case (2 << 10) | (3 << 5) | 4:
+        return 1.21f;
+      case (3 << 10) | (4 << 5) | 5:
+        return 2.7f;
+      case (4 << 10) | (5 << 5) | 6:
+        return 3.06f;
+      case (1 << 10) | (2 << 5) | 7:
+      case (1 << 10) | (7 << 5) | 8:
+      case (2 << 10) | (3 << 5) | 7:
+      case (2 << 10) | (7 << 5) | 8:
+      case (7 << 10) | (8 << 5) | 9:
+      case (8 << 10) | (9 << 5) | 10:
+      case (9 << 10) | (10 << 5) | 11:
+        return 1.f;
+    }
+    return 5.f;
+  }
+  LST_HD bool t3PassRZ(float r1, float z1, float r2, float z2, float r3, float z3, float cut) {
     const float residual = z2 - ((z3 - z1) / (r3 - r1) * (r2 - r1) + z1);
-    const float ar = fabs_(residual);
-    if (layer1 == 12 and layer2 == 13 and layer3 == 14)
-      return false;
-    if (layer1 == 1 and layer2 == 2 and layer3 == 3)
-      return ar < 0.53f;
-    if (layer1 == 1 and layer2 == 2 and layer3 == 7)
-      return ar < 1;
-    if (layer1 == 13 and layer2 == 14 and layer3 == 15)
-      return false;
-    if (layer1 == 14 and layer2 == 15 and layer3 == 16)
-      return false;
-    if (layer1 == 1 and layer2 == 7 and layer3 == 8)
-      return ar < 1;
-    if (layer1 == 2 and layer2 == 3 and layer3 == 4)
-      return ar < 1.21f;
-    if (layer1 == 2 and layer2 == 3 and layer3 == 7)
-      return ar < 1.f;
-    if (layer1 == 2 and layer2 == 7 and layer3 == 8)
-      return ar < 1.f;
-    if (layer1 == 3 and layer2 == 4 and layer3 == 5)
-      return ar < 2.7f;
-    if (layer1 == 4 and layer2 == 5 and layer3 == 6)
-      return ar < 3.06f;
-    if (layer1 == 7 and layer2 == 8 and layer3 == 9)
-      return ar < 1;
-    if (layer1 == 8 and layer2 == 9 and layer3 == 10)
-      return ar < 1;
-    if (layer1 == 9 and layer2 == 10 and layer3 == 11)
-      return ar < 1;
-    return ar < 5;
+    return fabs_(residual) < cut;
   }
 
   LST_HD float segmentDr(const MiniDoublets& md, unsigned int a, unsigned int b) {
@@ -57,203 +45,120 @@ namespace lst {
                  (md.rec[b].y - md.rec[a].y) * (md.rec[b].y - md.rec[a].y));
   }
 
-  // Barrel-barrel-barrel pointing and first beta cut (SDL/Triplet.h:301-402).
-  LST_HD_BIG bool t3PointingBBB(const Modules& m,
-                            const MiniDoublets& md,
-                            const Segments& s,
-                            uint16_t lm1,
-                            uint16_t lm3,
-                            unsigned int md1,
-                            unsigned int md2,
-                            unsigned int md3,
-                            unsigned int innerSeg,
-                            float& betaIn) {
-    bool isPSIn = (m.moduleType[lm1] == PS);
-    bool isPSOut = (m.moduleType[lm3] == PS);
-    float rtIn = md.rec[md1].rt, rtMid = md.rec[md2].rt, rtOut = md.rec[md3].rt;
-    float zIn = md.rec[md1].z, zMid = md.rec[md2].z, zOut = md.rec[md3].z;
-    float alpha1GeVOut = md.rec[md3].slope;
-    float rtRatio_OutIn = rtOut / rtIn;
-    float dzDrtScale = md.rec[md3].tanSlope / alpha1GeVOut;
-    float zpitchIn = (isPSIn ? kPixelPSZpitch : kStrip2SZpitch);
-    float zpitchOut = (isPSOut ? kPixelPSZpitch : kStrip2SZpitch);
-    const float zHi =
-        zIn + (zIn + kDeltaZLum) * (rtRatio_OutIn - 1.f) * (zIn < 0.f ? 1.f : dzDrtScale) + (zpitchIn + zpitchOut);
-    const float zLo =
-        zIn + (zIn - kDeltaZLum) * (rtRatio_OutIn - 1.f) * (zIn > 0.f ? 1.f : dzDrtScale) - (zpitchIn + zpitchOut);
-    if (!((zOut >= zLo) && (zOut <= zHi)))
+  // Pointing of the triplet and its first beta cut: barrel-barrel-barrel
+  // (SDL/Triplet.h:301-402), barrel-barrel-endcap / barrel-endcap-endcap
+  // (SDL/Triplet.h:404-531) and endcap-endcap-endcap (SDL/Triplet.h:533-658) in
+  // one body: a warp holds candidates of all three, and the parts they share
+  // (the extrapolation error, the atan2, the arcsine) run once for all of them.
+  // f1, f2, f3: the modules' MDCutFlags.
+  LST_HD bool t3Pointing(unsigned int f1,
+                         unsigned int f2,
+                         unsigned int f3,
+                         float ptCut,
+                         const MDRec& in,
+                         const MDRec& mid,
+                         const MDRec& out,
+                         const Segments& s,
+                         unsigned int innerSeg,
+                         float& betaIn) {
+    const bool eee = (f1 & f2 & f3 & kCutEndcap) != 0;
+    const bool bbb = (f1 & f2 & f3 & kCutBarrel) != 0;
+    // (the second module of a barrel-endcap triplet lies on either side)
+    if (!(bbb or eee or ((f1 & kCutBarrel) and (f2 & (kCutBarrel | kCutEndcap)) and (f3 & kCutEndcap))))
       return false;
-
-    float drt_OutIn = (rtOut - rtIn);
-    float r3In = fsqrt(zIn * zIn + rtIn * rtIn);
-    float drt_InSeg = rtMid - rtIn;
-    float dz_InSeg = zMid - zIn;
-    float dr3_InSeg = fsqrt(rtMid * rtMid + zMid * zMid) - fsqrt(rtIn * rtIn + zIn * zIn);
-    float coshEta = dr3_InSeg / drt_InSeg;
-    float dzErr = (zpitchIn + zpitchOut) * (zpitchIn + zpitchOut) * 2.f;
-    float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rtOut - rtIn) / 50.f) * fsqrt(r3In / rtIn);
-    float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    dzErr += sdlMuls * sdlMuls * drt_OutIn * drt_OutIn / 3.f * coshEta * coshEta;
-    dzErr = fsqrt(dzErr);
-    const float dzMean = dz_InSeg / drt_InSeg * drt_OutIn;
-    const float zWindow = dzErr / drt_InSeg * drt_OutIn + (zpitchIn + zpitchOut);
-    const float zLoPointed = zIn + dzMean * (zIn > 0.f ? 1.f : dzDrtScale) - zWindow;
-    const float zHiPointed = zIn + dzMean * (zIn < 0.f ? 1.f : dzDrtScale) + zWindow;
-    bool pass = ((zOut >= zLoPointed) && (zOut <= zHiPointed));
-
-    float alpha_InLo = s.dPhiChanges[innerSeg];
-    float tl_axis_x = md.rec[md3].x - md.rec[md1].x;
-    float tl_axis_y = md.rec[md3].y - md.rec[md1].y;
-    betaIn = alpha_InLo - phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.rec[md1].phi);
-    float drt_tl_axis = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    const float rt_InSeg = segmentDr(md, md1, md2);
-    float betaInCut = fasin(fmin_((-rt_InSeg + drt_tl_axis) * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / drt_InSeg);
-    return pass and (fabs_(betaIn) < betaInCut);
-  }
-
-  // Barrel-barrel-endcap / barrel-endcap-endcap (SDL/Triplet.h:404-531).
-  LST_HD_BIG bool t3PointingBBE(const Modules& m,
-                            const MiniDoublets& md,
-                            const Segments& s,
-                            uint16_t lm1,
-                            uint16_t lm3,
-                            unsigned int md1,
-                            unsigned int md2,
-                            unsigned int md3,
-                            unsigned int innerSeg,
-                            float& betaIn) {
-    bool isPSIn = (m.moduleType[lm1] == PS);
-    bool isPSOut = (m.moduleType[lm3] == PS);
-    float rtIn = md.rec[md1].rt, rtMid = md.rec[md2].rt, rtOut = md.rec[md3].rt;
-    float zIn = md.rec[md1].z, zMid = md.rec[md2].z, zOut = md.rec[md3].z;
-    float alpha1GeV_OutLo = md.rec[md3].slope;
-    float dzDrtScale = md.rec[md3].tanSlope / alpha1GeV_OutLo;
-    float zpitchIn = (isPSIn ? kPixelPSZpitch : kStrip2SZpitch);
-    float zpitchOut = (isPSOut ? kPixelPSZpitch : kStrip2SZpitch);
-    float zGeom = zpitchIn + zpitchOut;
-    if (!(zIn * zOut > 0))
-      return false;
-    float dLum = signTransfer(kDeltaZLum, zIn);
-    bool isOutSgInnerMDPS = m.moduleType[lm3] == PS;
-    float rtGeom1 = isOutSgInnerMDPS ? kPixelPSZpitch : kStrip2SZpitch;
-    float zGeom1 = signTransfer(zGeom, zIn);
-    float rtLo = rtIn * (1.f + (zOut - zIn - zGeom1) / (zIn + zGeom1 + dLum) / dzDrtScale) - rtGeom1;
-    float zInForHi = zIn - zGeom1 - dLum;
-    if (zInForHi * zIn < 0) {
-      zInForHi = signTransfer(0.1f, zIn);
+    const bool isPSIn = (f1 & kCutPS) != 0, isPSOut = (f3 & kCutPS) != 0;
+    const float rtIn = in.rt, rtMid = mid.rt, rtOut = out.rt;
+    const float zIn = in.z, zMid = mid.z, zOut = out.z;
+    const float dzDrtScale = out.tanSlope / out.slope;
+    const float zGeom = (isPSIn ? kPixelPSZpitch : kStrip2SZpitch) + (isPSOut ? kPixelPSZpitch : kStrip2SZpitch);
+    const float dz = zOut - zIn;
+    float rtGeom = 0;
+    if (bbb) {
+      const float rtRatio_OutIn = rtOut / rtIn;
+      const float zHi = zIn + (zIn + kDeltaZLum) * (rtRatio_OutIn - 1.f) * (zIn < 0.f ? 1.f : dzDrtScale) + zGeom;
+      const float zLo = zIn + (zIn - kDeltaZLum) * (rtRatio_OutIn - 1.f) * (zIn > 0.f ? 1.f : dzDrtScale) - zGeom;
+      if (!((zOut >= zLo) && (zOut <= zHi)))
+        return false;
+    } else {
+      if (!(zIn * zOut > 0))
+        return false;
+      const float dLum = signTransfer(kDeltaZLum, zIn);
+      float dzLo = dz, dzHi = dz, denLo = zIn + dLum, denHi = zIn - dLum;
+      if (eee)
+        rtGeom = (isPSIn and isPSOut)  ? 2.f * kPixelPSZpitch
+                 : (isPSIn or isPSOut) ? kPixelPSZpitch + kStrip2SZpitch
+                                       : 2.f * kStrip2SZpitch;
+      else {
+        rtGeom = isPSOut ? kPixelPSZpitch : kStrip2SZpitch;
+        const float zGeom1 = signTransfer(zGeom, zIn);
+        dzLo = dz - zGeom1;
+        dzHi = dz + zGeom1;
+        denLo = zIn + zGeom1 + dLum;
+        denHi = zIn - zGeom1 - dLum;
+        if (denHi * zIn < 0)
+          denHi = signTransfer(0.1f, zIn);
+      }
+      const float rtLo = rtIn * (1.f + dzLo / denLo / dzDrtScale) - rtGeom;
+      const float rtHi = rtIn * (1.f + dzHi / denHi) + rtGeom;
+      if (!((rtOut >= rtLo) && (rtOut <= rtHi)))
+        return false;
     }
-    float rtHi = rtIn * (1.f + (zOut - zIn + zGeom1) / zInForHi) + rtGeom1;
-    if (!((rtOut >= rtLo) && (rtOut <= rtHi)))
-      return false;
 
-    float rIn = fsqrt(zIn * zIn + rtIn * rtIn);
-    const float drtSDIn = rtMid - rtIn;
-    const float dzSDIn = zMid - zIn;
-    const float dr3SDIn = fsqrt(rtMid * rtMid + zMid * zMid) - fsqrt(rtIn * rtIn + zIn * zIn);
-    const float coshEta = dr3SDIn / drtSDIn;
-    const float dzOutInAbs = fabs_(zOut - zIn);
-    const float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
-    const float zGeom1_another = kPixelPSZpitch;
-    const float kZ = (zOut - zIn) / dzSDIn;
-    float drtErr =
-        zGeom1_another * zGeom1_another * drtSDIn * drtSDIn / dzSDIn / dzSDIn * (1.f - 2.f * kZ + 2.f * kZ * kZ);
-    // The reference evaluates 0.1f + 0.2 * (...) / 50.f in double here.
-    const float sdlThetaMulsF =
-        0.015f * dsqrt(0.1f + 0.2 * (rtOut - rtIn) / 50.f) * fsqrt(rIn / rtIn);
-    const float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    drtErr += sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta;
-    drtErr = fsqrt(drtErr);
-    bool pass = (kZ >= 0) && (rtOut >= rtLo) && (rtOut <= rtHi);
-
-    float rt_InLo = md.rec[md1].rt;
-    float rt_InOut = md.rec[md2].rt;
-    float sdIn_alpha = s.dPhiChanges[innerSeg];
-    float tl_axis_x = md.rec[md3].x - md.rec[md1].x;
-    float tl_axis_y = md.rec[md3].y - md.rec[md1].y;
-    betaIn = sdIn_alpha - phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.rec[md1].phi);
-    float betaInRHmin = betaIn;
-    float betaInRHmax = betaIn;
-    if (fabs_(betaInRHmin) > fabs_(betaInRHmax)) {
-      float swapTemp = betaInRHmin;
-      betaInRHmin = betaInRHmax;
-      betaInRHmax = swapTemp;
+    const float drtIn = rtMid - rtIn, dzIn = zMid - zIn;
+    if (!bbb and (!eee or (isPSIn and isPSOut))) {
+      const float kZ = dz / dzIn;
+      if (!(kZ >= 0))
+        return false;
     }
-    float sdIn_dr = segmentDr(md, md1, md2);
-    float sdIn_d = rt_InOut - rt_InLo;
-    float dr = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    float betaInCut = fasin(fmin_((-sdIn_dr + dr) * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdIn_d);
-    return pass and (fabs_(betaInRHmin) < betaInCut);
-  }
-
-  // Endcap-endcap-endcap (SDL/Triplet.h:533-658).
-  LST_HD_BIG bool t3PointingEEE(const Modules& m,
-                            const MiniDoublets& md,
-                            const Segments& s,
-                            uint16_t lm1,
-                            uint16_t lm3,
-                            unsigned int md1,
-                            unsigned int md2,
-                            unsigned int md3,
-                            unsigned int innerSeg,
-                            float& betaIn) {
-    float rtIn = md.rec[md1].rt, rtMid = md.rec[md2].rt, rtOut = md.rec[md3].rt;
-    float zIn = md.rec[md1].z, zMid = md.rec[md2].z, zOut = md.rec[md3].z;
-    float alpha1GeV_Out = md.rec[md3].slope;
-    float dzDrtScale = md.rec[md3].tanSlope / alpha1GeV_Out;
-    if (!(zIn * zOut > 0))
-      return false;
-    float dLum = signTransfer(kDeltaZLum, zIn);
-    bool isOutSgOuterMDPS = m.moduleType[lm3] == PS;
-    bool isInSgInnerMDPS = m.moduleType[lm1] == PS;
-    float rtGeom = (isInSgInnerMDPS and isOutSgOuterMDPS)  ? 2.f * kPixelPSZpitch
-                   : (isInSgInnerMDPS or isOutSgOuterMDPS) ? kPixelPSZpitch + kStrip2SZpitch
-                                                           : 2.f * kStrip2SZpitch;
-    float dz = zOut - zIn;
-    const float rtLo = rtIn * (1.f + dz / (zIn + dLum) / dzDrtScale) - rtGeom;
-    const float rtHi = rtIn * (1.f + dz / (zIn - dLum)) + rtGeom;
-    if (!((rtOut >= rtLo) && (rtOut <= rtHi)))
-      return false;
-
-    bool isInSgOuterMDPS = m.moduleType[lm3] == PS;
-    float drtSDIn = rtMid - rtIn;
-    float dzSDIn = zMid - zIn;
-    float dr3SDIn = fsqrt(rtMid * rtMid + zMid * zMid) - fsqrt(rtIn * rtIn + zIn * zIn);
-    float coshEta = dr3SDIn / drtSDIn;
-    float dzOutInAbs = fabs_(zOut - zIn);
-    float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
-    float kZ = (zOut - zIn) / dzSDIn;
-    float sdlThetaMulsF = 0.015f * fsqrt(0.1f + 0.2f * (rtOut - rtIn) / 50.f);
-    float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    float drtErr = fsqrt(kPixelPSZpitch * kPixelPSZpitch * 2.f / (dzSDIn * dzSDIn) * (dzOutInAbs * dzOutInAbs) +
-                         sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta);
-    float drtMean = drtSDIn * dzOutInAbs / fabs_(dzSDIn);
-    float rtWindow = drtErr + rtGeom;
-    float rtLo_point = rtIn + drtMean / dzDrtScale - rtWindow;
-    float rtHi_point = rtIn + drtMean + rtWindow;
-    bool pass = true;
-    if (isInSgInnerMDPS and isInSgOuterMDPS)
-      pass = ((kZ >= 0) && (rtOut >= rtLo_point) && (rtOut <= rtHi_point));
-
-    float rt_InLo = md.rec[md1].rt;
-    float rt_InOut = md.rec[md2].rt;
-    float sdIn_alpha = s.dPhiChanges[innerSeg];
-    float tl_axis_x = md.rec[md3].x - md.rec[md1].x;
-    float tl_axis_y = md.rec[md3].y - md.rec[md1].y;
-    betaIn = sdIn_alpha - phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - md.rec[md1].phi);
-    float sdIn_alphaRHmin = s.dPhiChangeMins[innerSeg];
-    float sdIn_alphaRHmax = s.dPhiChangeMaxs[innerSeg];
-    float betaInRHmin = betaIn + sdIn_alphaRHmin - sdIn_alpha;
-    float betaInRHmax = betaIn + sdIn_alphaRHmax - sdIn_alpha;
-    if (fabs_(betaInRHmin) > fabs_(betaInRHmax)) {
-      float swapTemp = betaInRHmin;
-      betaInRHmin = betaInRHmax;
-      betaInRHmax = swapTemp;
+    if (bbb or (eee and isPSIn and isPSOut)) {
+      const float r3In = fsqrt(zIn * zIn + rtIn * rtIn);
+      const float dr3In = fsqrt(rtMid * rtMid + zMid * zMid) - r3In;
+      const float coshEta = dr3In / drtIn;
+      const float dzAbs = fabs_(dz);
+      float theta = 0.015f * fsqrt(0.1f + 0.2f * (rtOut - rtIn) / 50.f);
+      float lever, err;
+      if (bbb) {
+        theta = theta * fsqrt(r3In / rtIn);
+        lever = rtOut - rtIn;
+        err = zGeom * zGeom * 2.f;
+      } else {
+        lever = dzAbs * coshEta / (coshEta * coshEta - 1.f);
+        err = kPixelPSZpitch * kPixelPSZpitch * 2.f / (dzIn * dzIn) * (dzAbs * dzAbs);
+      }
+      const float sdlMuls = theta * 3.f / ptCut * 4.f;
+      err = fsqrt(err + sdlMuls * sdlMuls * lever * lever / 3.f * coshEta * coshEta);
+      float lo, hi, x;
+      if (bbb) {
+        const float dzMean = dzIn / drtIn * lever;
+        const float window = err / drtIn * lever + zGeom;
+        lo = zIn + dzMean * (zIn > 0.f ? 1.f : dzDrtScale) - window;
+        hi = zIn + dzMean * (zIn < 0.f ? 1.f : dzDrtScale) + window;
+        x = zOut;
+      } else {
+        const float drtMean = drtIn * dzAbs / fabs_(dzIn);
+        const float window = err + rtGeom;
+        lo = rtIn + drtMean / dzDrtScale - window;
+        hi = rtIn + drtMean + window;
+        x = rtOut;
+      }
+      if (!((x >= lo) && (x <= hi)))
+        return false;
     }
-    float sdIn_dr = segmentDr(md, md1, md2);
-    float sdIn_d = rt_InOut - rt_InLo;
-    float dr = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
-    float betaInCut = fasin(fmin_((-sdIn_dr + dr) * k2Rinv1GeVf / m.ptCut, kSinAlphaMax)) + (0.02f / sdIn_d);
-    return pass and (fabs_(betaInRHmin) < betaInCut);
+
+    const float alpha = s.dPhiChanges[innerSeg];
+    const float tl_axis_x = out.x - in.x;
+    const float tl_axis_y = out.y - in.y;
+    betaIn = alpha - phiMpiPi(phiOf(tl_axis_x, tl_axis_y) - in.phi);
+    float beta = betaIn;
+    if (eee) {
+      const float betaMin = betaIn + s.dPhiChangeMins[innerSeg] - alpha;
+      const float betaMax = betaIn + s.dPhiChangeMaxs[innerSeg] - alpha;
+      beta = fabs_(betaMin) > fabs_(betaMax) ? betaMax : betaMin;
+    }
+    const float drAxis = fsqrt(tl_axis_x * tl_axis_x + tl_axis_y * tl_axis_y);
+    const float drIn = fsqrt((mid.x - in.x) * (mid.x - in.x) + (mid.y - in.y) * (mid.y - in.y));
+    const float betaInCut = fasin(fmin_((-drIn + drAxis) * k2Rinv1GeVf / ptCut, kSinAlphaMax)) + (0.02f / drtIn);
+    return fabs_(beta) < betaInCut;
   }
 
   // Circle through three points; radius -1 for collinear points
@@ -278,6 +183,23 @@ namespace lst {
     float betaIn, circleRadius, circleCenterX, circleCenterY;
   };
 
+  // The tests after the r-z residual, and the circle.
+  LST_HD bool t3Rest(unsigned int f1,
+                     unsigned int f2,
+                     unsigned int f3,
+                     float ptCut,
+                     const MDRec& in,
+                     const MDRec& mid,
+                     const MDRec& out,
+                     const Segments& s,
+                     unsigned int innerSeg,
+                     T3Values& v) {
+    if (!t3Pointing(f1, f2, f3, ptCut, in, mid, out, s, innerSeg, v.betaIn))
+      return false;
+    v.circleRadius = circleFrom3(in.x, in.y, mid.x, mid.y, out.x, out.y, v.circleCenterX, v.circleCenterY);
+    return true;
+  }
+
   // SDL/Triplet.h:797-870
   LST_HD bool t3Select(const Modules& m,
                        const MiniDoublets& md,
@@ -293,31 +215,11 @@ namespace lst {
     unsigned int md1 = s.mdIndices[2 * innerSeg];
     unsigned int md2 = s.mdIndices[2 * outerSeg];
     unsigned int md3 = s.mdIndices[2 * outerSeg + 1];
-    if (!t3PassRZ(m, md, lm1, lm2, lm3, md1, md2, md3))
+    const MDRec &in = md.rec[md1], &mid = md.rec[md2], &out = md.rec[md3];
+    const unsigned int f1 = cutFlags(m, lm1), f2 = cutFlags(m, lm2), f3 = cutFlags(m, lm3);
+    if (!t3PassRZ(in.rt, in.z, mid.rt, mid.z, out.rt, out.z, t3RZCut(cutLayer(f1), cutLayer(f2), cutLayer(f3))))
       return false;
-    short sub1 = m.subdets[lm1], sub2 = m.subdets[lm2], sub3 = m.subdets[lm3];
-    bool pass;
-    if (sub1 == Barrel and sub2 == Barrel and sub3 == Barrel)
-      pass = t3PointingBBB(m, md, s, lm1, lm3, md1, md2, md3, innerSeg, v.betaIn);
-    else if (sub1 == Barrel and sub2 == Barrel and sub3 == Endcap)
-      pass = t3PointingBBE(m, md, s, lm1, lm3, md1, md2, md3, innerSeg, v.betaIn);
-    else if (sub1 == Barrel and sub2 == Endcap and sub3 == Endcap)
-      pass = t3PointingBBE(m, md, s, lm1, lm3, md1, md2, md3, innerSeg, v.betaIn);
-    else if (sub1 == Endcap and sub2 == Endcap and sub3 == Endcap)
-      pass = t3PointingEEE(m, md, s, lm1, lm3, md1, md2, md3, innerSeg, v.betaIn);
-    else
-      pass = false;
-    if (!pass)
-      return false;
-    v.circleRadius = circleFrom3(md.rec[md1].x,
-                                 md.rec[md1].y,
-                                 md.rec[md2].x,
-                                 md.rec[md2].y,
-                                 md.rec[md3].x,
-                                 md.rec[md3].y,
-                                 v.circleCenterX,
-                                 v.circleCenterY);
-    return true;
+    return t3Rest(f1, f2, f3, m.ptCut, in, mid, out, s, innerSeg, v);
   }
 
   // SDL/Triplet.h:181-239
