@@ -346,15 +346,33 @@ namespace {
     const char* name;  // as it appears in the launch profile
     int maxWarps;      // the kernel's launch bounds / per-warp shared memory
     int defWarps;
+    int perEvent;      // blocks per SM and event of the default shape (see below), or 0
   };
-  const TuneSpec kTuneSpecs[kTuCount] = {{"kCreateMD", 8, 8},   {"kMDDerived", 8, 8},   {"kCreateLS", 4, 4},
-                                         {"kCreateT3", 4, 4},   {"kT5Eval", 4, 4},      {"kPixEval<5>", 4, 4},
-                                         {"kPixEval<3>", 4, 4}, {"kPixMid<5>", 4, 4},    {"kPixMid<3>", 4, 4}};
-  constexpr int kDefaultBlocksPerSM = 16;
+  const TuneSpec kTuneSpecs[kTuCount] = {
+      {"kCreateMD", 8, 8, 2},    {"kMDDerived", 8, 8, 0},  {"kCreateLS", 4, 4, 4},
+      {"kCreateT3", 4, 4, 4},    {"kT5Eval", 4, 4, 0},     {"kPixEval<5>", 4, 4, 0},
+      {"kPixEval<3>", 4, 4, 0},  {"kPixMid<5>", 4, 4, 0},  {"kPixMid<3>", 4, 4, 2}};
+  constexpr int kDefaultBlocksPerSM = 16, kMostDefaultBlocksPerSM = 64;
   struct LaunchShape {
     int warps = 4;
     int perSM = kDefaultBlocksPerSM;
+    bool chosen = false;  // by the autotuner or the caller
   };
+  // Blocks per SM across a batch of count events.  A grid of 16 per SM holds all
+  // of a large batch's events at once, 37 blocks each for 64 events, and what the
+  // kernels gather again and again (some 6 MB of mini-doublets and segments per
+  // event) falls out of the L2; with more blocks the first ones are those of fewer
+  // events.  64 events, 16 / 32 / 64 / 128 blocks per SM: kCreateLS 1359 / 1181 /
+  // 1136 / 1109 us, kCreateT3 765 / 619 / 576 / 551, kPixMid<3> 1255 / 1142 / 1065
+  // / 1113, kCreateMD 1164 / 1151 / 1131 / 1124; the other kernels gain nothing or
+  // lose (kPixMid<5> 379 / 368 / 377 / 460, kT5Eval 517 / 525 / 562 / 638), and a
+  // few events want 16 (8 events, kPixMid<3>: 180 / 192 / 210 / 255).
+  int blocksPerSM(const LaunchShape& shape, int k, int count) {
+    if (shape.chosen)
+      return shape.perSM;
+    const int want = kTuneSpecs[k].perEvent * std::min(count, kMostDefaultBlocksPerSM);
+    return std::max(kDefaultBlocksPerSM, std::min(want, kMostDefaultBlocksPerSM));
+  }
 }  // namespace
 
 struct lst_event {
@@ -513,21 +531,21 @@ namespace {
   dim3 tunedWarpGrid(const lst_event* ev, int k, size_t nObjects, int count) {
     const LaunchShape& sh = ev->shape[k];
     const size_t want = std::max<size_t>(1, ceilDiv(nObjects, static_cast<size_t>(sh.warps)));
-    const size_t cap = std::max<size_t>(1, ceilDiv(static_cast<size_t>(sh.perSM) * ev->nSM,
+    const size_t cap = std::max<size_t>(1, ceilDiv(static_cast<size_t>(blocksPerSM(sh, k, count)) * ev->nSM,
                                                    static_cast<size_t>(std::max(count, 1))));
     return dim3(static_cast<unsigned int>(std::min(want, cap)), count);
   }
   // Tuned kernel k, a block per task.
   dim3 tunedBlockGrid(const lst_event* ev, int k, size_t nTasks, int count) {
     const LaunchShape& sh = ev->shape[k];
-    const size_t cap = std::max<size_t>(1, ceilDiv(static_cast<size_t>(sh.perSM) * ev->nSM,
+    const size_t cap = std::max<size_t>(1, ceilDiv(static_cast<size_t>(blocksPerSM(sh, k, count)) * ev->nSM,
                                                    static_cast<size_t>(std::max(count, 1))));
     return dim3(static_cast<unsigned int>(std::min(std::max<size_t>(1, nTasks), cap)), count);
   }
   // Tuned kernel k striding over a candidate list whose length only the device knows.
   dim3 tunedFlatGrid(const lst_event* ev, int k, int count) {
     const LaunchShape& sh = ev->shape[k];
-    const size_t blocks = std::max<size_t>(1, ceilDiv(static_cast<size_t>(sh.perSM) * ev->nSM,
+    const size_t blocks = std::max<size_t>(1, ceilDiv(static_cast<size_t>(blocksPerSM(sh, k, count)) * ev->nSM,
                                                       static_cast<size_t>(std::max(count, 1))));
     return dim3(static_cast<unsigned int>(blocks), count);
   }
@@ -2143,10 +2161,12 @@ int lst_event_set_launch_shape(lst_event* ev, int k, int warps_per_block, int bl
                     std::to_string(kTuneSpecs[k].maxWarps) + " warps per block");
   if (blocks_per_sm < 1 || blocks_per_sm > 256)
     return setError("lst_event_set_launch_shape: blocks per SM must be 1..256");
-  if (ev->shape[k].warps != warps_per_block || ev->shape[k].perSM != blocks_per_sm) {
+  LaunchShape& shape = ev->shape[k];
+  if (!shape.chosen || shape.warps != warps_per_block || shape.perSM != blocks_per_sm) {
     dropGraphs(ev);
-    ev->shape[k].warps = warps_per_block;
-    ev->shape[k].perSM = blocks_per_sm;
+    shape.warps = warps_per_block;
+    shape.perSM = blocks_per_sm;
+    shape.chosen = true;
   }
   return 0;
   LST_ABI_CATCH_INT
@@ -2211,8 +2231,8 @@ int lst_autotune(lst_event* ev, int first, int count, const char* cache_path) {
   LaunchShape saved[kTuCount];
   std::copy(ev->shape, ev->shape + kTuCount, saved);
   auto restore = [&]() {
-    for (int k = 0; k < kTuCount; ++k)
-      lst_event_set_launch_shape(ev, k, saved[k].warps, saved[k].perSM);
+    dropGraphs(ev);
+    std::copy(saved, saved + kTuCount, ev->shape);
     ev->profiling = wasProfiling;
     ev->profile.clear();
     ev->poolUsed = 0;
@@ -2282,9 +2302,10 @@ int lst_autotune(lst_event* ev, int first, int count, const char* cache_path) {
     for (size_t t = 1; t < trials.size(); ++t)
       if (best[k][t] < best[k][arg])
         arg = t;
-    if (best[k][arg] >= 1e30)  // never timed: keep the previous shape
-      lst_event_set_launch_shape(ev, k, saved[k].warps, saved[k].perSM);
-    else
+    if (best[k][arg] >= 1e30) {  // never timed: keep the previous shape
+      dropGraphs(ev);
+      ev->shape[k] = saved[k];
+    } else
       lst_event_set_launch_shape(ev, k, trials[arg].w, trials[arg].p);
   }
   if (cache_path && *cache_path) {
