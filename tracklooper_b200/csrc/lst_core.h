@@ -290,8 +290,9 @@ namespace lst {
     // The anchor hit's x, y, z, rt in one 16-byte record: the segment, triplet
     // and pixel kernels gather them together for mini-doublets chosen by index.
     struct MDPos* anchorPos;
-    // Everything the segment cuts read of a mini-doublet, in one 48-byte
-    // record (three 16-byte loads instead of a dozen scattered ones).
+    // Everything the segment, triplet and pixel cuts read of a mini-doublet, in
+    // one 64-byte record (16-byte loads instead of a dozen scattered ones; two
+    // whole 32-byte sectors), with the quotients that the cuts form of it.
     struct MDRec* rec;
   };
 
@@ -302,6 +303,7 @@ namespace lst {
   struct alignas(16) MDRec {
     float x, y, z, rt;                         // anchor hit
     float phi, slope, tanSlope, dphichange;    // anchorPhi, slope, tanSlope, dphichanges
+    float dzDrtScale, drtDzScale, pvOff, lum;  // tanSlope / slope, slope / tanSlope, 0.1 / rt, dphi * 15 / dz
     float dphi, dz, highEdgePhi, lowEdgePhi;   // dphis, dzs, anchorHighEdgePhi, anchorLowEdgePhi
   };
 

@@ -47,11 +47,11 @@ namespace lst {
     if (innerBarrel)
       sdLumForInnerMini = in.tilt * dAlpha_Bfield;
     else
-      sdLumForInnerMini = rIn.dphi * 15.0f / rIn.dz;
+      sdLumForInnerMini = rIn.lum;
     if (outerBarrel)
       sdLumForOuterMini = out.tilt * dAlpha_Bfield;
     else
-      sdLumForOuterMini = rOut.dphi * 15.0f / rOut.dz;
+      sdLumForOuterMini = rOut.lum;
 
     // (both resolutions are taken with the inner module's separation)
     float dAlpha_res_inner = in.res * (innerBarrel ? 1.0f : fabs_(rIn.z) / rIn.rt);
@@ -88,8 +88,8 @@ namespace lst {
     float xOut = rOut.x, yOut = rOut.y, zOut = rOut.z, rtOut = rOut.rt;
 
     float sdSlope = rOut.slope;
-    float sdPVoff = 0.1f / rtOut;
-    float dzDrtScale = rOut.tanSlope / sdSlope;
+    float sdPVoff = rOut.pvOff;
+    float dzDrtScale = rOut.dzDrtScale;
     const float zGeom = (in.flags & kCutInnerLayers) ? 2.f * kPixelPSZpitch : 2.f * kStrip2SZpitch;
     float zLo = zIn + (zIn - kDeltaZLum) * (rtOut / rtIn - 1.f) * (zIn > 0.f ? 1.f : dzDrtScale) - zGeom;
     float zHi = zIn + (zIn + kDeltaZLum) * (rtOut / rtIn - 1.f) * (zIn < 0.f ? 1.f : dzDrtScale) + zGeom;
@@ -138,7 +138,7 @@ namespace lst {
       return false;
     float dz = zOut - zIn;
     float dLum = signTransfer(kDeltaZLum, zIn);
-    float drtDzScale = sdSlope / rOut.tanSlope;
+    float drtDzScale = rOut.drtDzScale;
     float rtLo = fmax_(rtIn * (1.f + dz / (zIn + dLum) * drtDzScale) - rtGeom, rtIn - 0.5f * rtGeom);
     float rtHi = rtIn * (zOut - dLum) / (zIn - dLum) + rtGeom;
     if (!((rtOut >= rtLo) && (rtOut <= rtHi)))

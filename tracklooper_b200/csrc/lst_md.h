@@ -251,7 +251,8 @@ namespace lst {
     md.slope[idx] = slope;
     md.tanSlope[idx] = tanSlope;
     md.slope3[idx] = slope3;
-    md.rec[idx] = MDRec{p.x, p.y, p.z, p.rt, phi, slope, tanSlope, dphichange, dphi, dz, highEdgePhi, lowEdgePhi};
+    md.rec[idx] = MDRec{p.x,  p.y, p.z, p.rt, phi, slope, tanSlope, dphichange, tanSlope / slope, slope / tanSlope,
+                        0.1f / p.rt, dphi * 15.0f / dz, dphi, dz, highEdgePhi, lowEdgePhi};
   }
 
   struct MDValues {

@@ -71,8 +71,7 @@ namespace lst {
     float pz = s.pz[pls];
     float etaErr = s.etaErr[pls];
 
-    float alpha1GeV_OutLo = rec3.slope;
-    const float dzDrtScale = rec3.tanSlope / alpha1GeV_OutLo;
+    const float dzDrtScale = rec3.dzDrtScale;
     const float zpitch_InLo = 0.05f;
     const float zpitch_InOut = 0.05f;
     float zpitch_OutLo = (isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch);
@@ -235,7 +234,7 @@ namespace lst {
     if (!(fabs_(betaOut) < betaOutCut))
       return false;
     const float sdlMuls = sdlThetaMulsF * 3.f / m.ptCut * 4.f;
-    const float sdlPVoff = 0.1f / rt_OutLo;
+    const float sdlPVoff = rec3.pvOff;
     float sdlCut = rec3.slope + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
     if (!isEC_lastLayer)
       dPhi = midPointDPhi();

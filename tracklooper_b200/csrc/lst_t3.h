@@ -69,7 +69,7 @@ namespace lst {
     const bool isPSIn = (f1 & kCutPS) != 0, isPSOut = (f3 & kCutPS) != 0;
     const float rtIn = in.rt, rtMid = mid.rt, rtOut = out.rt;
     const float zIn = in.z, zMid = mid.z, zOut = out.z;
-    const float dzDrtScale = out.tanSlope / out.slope;
+    const float dzDrtScale = out.dzDrtScale;
     const float zGeom = (isPSIn ? kPixelPSZpitch : kStrip2SZpitch) + (isPSOut ? kPixelPSZpitch : kStrip2SZpitch);
     const float dz = zOut - zIn;
     float rtGeom = 0;

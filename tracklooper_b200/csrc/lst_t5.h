@@ -127,7 +127,7 @@ namespace lst {
     float rt_InLo = r1.rt, rt_InOut = r2.rt, rt_OutLo = r3.rt;
     float z_InLo = r1.z, z_InOut = r2.z, z_OutLo = r3.z;
     float alpha1GeV_OutLo = r3.slope;
-    float dzDrtScale = r3.tanSlope / alpha1GeV_OutLo;
+    float dzDrtScale = r3.dzDrtScale;
     float zpitch_InLo = (isPS_InLo ? kPixelPSZpitch : kStrip2SZpitch);
     float zpitch_OutLo = (isPS_OutLo ? kPixelPSZpitch : kStrip2SZpitch);
     const float drt_InSeg = rt_InOut - rt_InLo;
@@ -206,7 +206,7 @@ namespace lst {
       }
     }
 
-    const float sdlPVoff = 0.1f / rt_OutLo;
+    const float sdlPVoff = r3.pvOff;
     const float sdlCut = alpha1GeV_OutLo + fsqrt(sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
     const float deltaPhiPos = phiMpiPi(r4.phi - r2.phi);
     if (!(fabs_(deltaPhiPos) <= sdlCut))
