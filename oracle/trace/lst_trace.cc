@@ -209,7 +209,6 @@ namespace {
       md.anchorLowEdgeY = f[k++]; md.anchorLowEdgePhi = f[k++]; md.anchorHighEdgePhi = f[k++]; md.outerX = f[k++];
       md.outerY = f[k++]; md.outerZ = f[k++]; md.outerRt = f[k++]; md.outerPhi = f[k++]; md.outerEta = f[k++];
       md.outerHighEdgeX = f[k++]; md.outerHighEdgeY = f[k++]; md.outerLowEdgeX = f[k++]; md.outerLowEdgeY = f[k++];
-      md.slope = f[k++]; md.tanSlope = f[k++]; md.slope3 = f[k++];
       md.anchorPos = mdPos.data();
       md.rec = mdRec.data();
 

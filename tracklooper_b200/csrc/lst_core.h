@@ -279,20 +279,15 @@ namespace lst {
     float* outerHighEdgeY;
     float* outerLowEdgeX;
     float* outerLowEdgeY;
-    // Derived per mini-doublet from its anchor radius rt (not reference
-    // fields): slope = asin(min(rt k / ptCut, sinAlphaMax)), tanSlope =
-    // tan(slope), slope3 = asin(min(rt k / 3, sinAlphaMax)).  The cut
-    // algorithms evaluate exactly these expressions of a mini-doublet's rt
-    // many times over; stored once, they give the same values.
-    float* slope;
-    float* tanSlope;
-    float* slope3;
     // The anchor hit's x, y, z, rt in one 16-byte record: the segment, triplet
     // and pixel kernels gather them together for mini-doublets chosen by index.
     struct MDPos* anchorPos;
-    // Everything the segment, triplet and pixel cuts read of a mini-doublet, in
-    // one 64-byte record (16-byte loads instead of a dozen scattered ones; two
-    // whole 32-byte sectors), with the quotients that the cuts form of it.
+    // Everything the segment, triplet and tracklet cuts read of a mini-doublet,
+    // in one 64-byte record (16-byte loads instead of a dozen scattered ones; two
+    // whole 32-byte sectors), with values that the cuts form of it many times
+    // over; formed once, by exactly their expressions, they are the same values:
+    // slope = asin(min(rt k / ptCut, sinAlphaMax)), tanSlope = tan(slope),
+    // slope3 = asin(min(rt k / 3, sinAlphaMax)), and quotients.
     struct MDRec* rec;
   };
 
@@ -302,9 +297,10 @@ namespace lst {
 
   struct alignas(16) MDRec {
     float x, y, z, rt;                         // anchor hit
-    float phi, slope, tanSlope, dphichange;    // anchorPhi, slope, tanSlope, dphichanges
-    float dzDrtScale, drtDzScale, pvOff, lum;  // tanSlope / slope, slope / tanSlope, 0.1 / rt, dphi * 15 / dz
-    float dphi, dz, highEdgePhi, lowEdgePhi;   // dphis, dzs, anchorHighEdgePhi, anchorLowEdgePhi
+    float phi, slope, dzDrtScale, dphichange;  // anchorPhi, slope, tanSlope / slope, dphichanges
+    float drtDzScale, lum, highEdgePhi, lowEdgePhi;  // slope / tanSlope, dphis * 15 / dzs, the anchor's edges
+    float pvOff, slope3;                       // 0.1 / rt, slope3
+    unsigned int anchorHit, outerHit;          // anchorHitIndices, outerHitIndices
   };
 
   struct Segments {

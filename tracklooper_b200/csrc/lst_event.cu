@@ -152,9 +152,6 @@ namespace {
 #define LST_CARVE_SCRATCH(field, type, count) v.field = c.take<type>(count);
     LST_SCRATCH_FIELDS(LST_CARVE_SCRATCH)
 #undef LST_CARVE_SCRATCH
-    v.md.slope = c.take<float>(MD);
-    v.md.tanSlope = c.take<float>(MD);
-    v.md.slope3 = c.take<float>(MD);
     v.md.anchorPos = c.take<lst::MDPos>(MD);
     v.md.rec = c.take<lst::MDRec>(MD);
     v.sc = c.take<lst::EventScalars>(1);

@@ -238,21 +238,19 @@ namespace lst {
     shiftStripFinish(c, pre.shiftXa[p], pre.shiftYa[p], xo, yo, xn, yn);
   }
 
-  // The derived per-MD values of MiniDoublets (slope, tanSlope, slope3).
+  // The record of a stored mini-doublet.
   // Also fills the mini-doublet's record of segment-cut inputs (MDRec).
   LST_HD void storeMDDerived(MiniDoublets& md, unsigned int idx, float ptCut) {
     // (loads before stores, as in storeMD)
     const MDPos p = md.anchorPos[idx];
     const float phi = md.anchorPhi[idx], dphichange = md.dphichanges[idx], dphi = md.dphis[idx], dz = md.dzs[idx];
     const float highEdgePhi = md.anchorHighEdgePhi[idx], lowEdgePhi = md.anchorLowEdgePhi[idx];
+    const unsigned int anchorHit = md.anchorHitIndices[idx], outerHit = md.outerHitIndices[idx];
     const float slope = fasin(fmin_(p.rt * k2Rinv1GeVf / ptCut, kSinAlphaMax));
     const float tanSlope = ftan(slope);
     const float slope3 = fasin(fmin_(p.rt * k2Rinv1GeVf / 3.0f, kSinAlphaMax));
-    md.slope[idx] = slope;
-    md.tanSlope[idx] = tanSlope;
-    md.slope3[idx] = slope3;
-    md.rec[idx] = MDRec{p.x,  p.y, p.z, p.rt, phi, slope, tanSlope, dphichange, tanSlope / slope, slope / tanSlope,
-                        0.1f / p.rt, dphi * 15.0f / dz, dphi, dz, highEdgePhi, lowEdgePhi};
+    md.rec[idx] = MDRec{p.x, p.y, p.z, p.rt, phi, slope, tanSlope / slope, dphichange, slope / tanSlope,
+                        dphi * 15.0f / dz, highEdgePhi, lowEdgePhi, 0.1f / p.rt, slope3, anchorHit, outerHit};
   }
 
   struct MDValues {

@@ -206,8 +206,8 @@ namespace lst {
     betaOutRHmax *= betaOutMMSF;
 
     const float dBetaMuls = sdlThetaMulsF * 4.f / fmin_(fabs_(pt_beta), kPtBetaMax);
-    const float alphaInAbsReg = fmax_(fabs_(alpha_InLo), md.slope3[md2]);
-    const float alphaOutAbsReg = fmax_(fabs_(alpha_OutLo), md.slope3[md3]);
+    const float alphaInAbsReg = fmax_(fabs_(alpha_InLo), md.rec[md2].slope3);
+    const float alphaOutAbsReg = fmax_(fabs_(alpha_OutLo), md.rec[md3].slope3);
     const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InUp);
     const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
     const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);

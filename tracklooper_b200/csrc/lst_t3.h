@@ -241,8 +241,8 @@ namespace lst {
     const uint8_t layer1 = m.layers[lm1] + (m.subdets[lm1] == 4) * 6;
     const uint8_t layer2 = m.layers[lm2] + (m.subdets[lm2] == 4) * 6;
     const uint8_t layer3 = m.layers[lm3] + (m.subdets[lm3] == 4) * 6;
-    const unsigned int hits[6] = {md.anchorHitIndices[md1], md.outerHitIndices[md1], md.anchorHitIndices[md2],
-                                  md.outerHitIndices[md2],  md.anchorHitIndices[md3], md.outerHitIndices[md3]};
+    const unsigned int hits[6] = {md.rec[md1].anchorHit, md.rec[md1].outerHit, md.rec[md2].anchorHit,
+                                  md.rec[md2].outerHit,  md.rec[md3].anchorHit, md.rec[md3].outerHit};
     t.segmentIndices[idx * 2] = innerSeg;
     t.segmentIndices[idx * 2 + 1] = outerSeg;
     t.lowerModuleIndices[idx * 3] = lm1;

@@ -297,8 +297,8 @@ namespace lst {
     betaOutRHmax *= betaOutMMSF;
 
     const float dBetaMuls = sdlThetaMulsF * 4.f / fmin_(fabs_(pt_beta), kPtBetaMax);
-    const float alphaInAbsReg = fmax_(fabs_(alpha_InLo), md.slope3[q.md1]);
-    const float alphaOutAbsReg = fmax_(fabs_(alpha_OutLo), md.slope3[q.md3]);
+    const float alphaInAbsReg = fmax_(fabs_(alpha_InLo), md.rec[q.md1].slope3);
+    const float alphaOutAbsReg = fmax_(fabs_(alpha_OutLo), md.rec[q.md3].slope3);
     const float dBetaInLum = lIn < 11 ? 0.0f : fabs_(alphaInAbsReg * kDeltaZLum / z_InLo);
     const float dBetaOutLum = lOut < 11 ? 0.0f : fabs_(alphaOutAbsReg * kDeltaZLum / z_OutLo);
     const float dBetaLum2 = (dBetaInLum + dBetaOutLum) * (dBetaInLum + dBetaOutLum);
