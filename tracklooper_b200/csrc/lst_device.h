@@ -76,7 +76,7 @@ namespace lst {
     unsigned int walkDone;        // blocks of a fallback count kernel that have finished
     unsigned int plsTCDone;       // blocks of kAddPLSTC that have finished
     unsigned int mdNext;          // next task for kCreateMD's warps
-    unsigned int lsNext;          // next lower module for kCreateLS's warps
+    unsigned int lsNext;          // next task for kCreateLS's warps
     unsigned int pixNext; // next task (a few pLS) for kPixMid's warps
     unsigned int t3Next;          // next task for kCreateT3's blocks
   };

@@ -574,10 +574,17 @@ namespace {
                    d, v);
         break;
       }
-      case LST_STAGE_SEGMENTS:
-        LST_LAUNCH(lst::kCreateLS, tunedWarpGrid(ev, kTuLS, nLower, count), tunedThreads(ev, kTuLS), d, v);
+      case LST_STAGE_SEGMENTS: {
+        // modules per warp task: 4 where the tasks still are many times the warps that
+        // the GPU holds (64 events: 953 us, with 1 1142, with 2 1000, with 8 1003);
+        // else 1, so that heavy modules are not put into one task (8 events: 188, with
+        // 2 188, with 4 231; 16 pt0.6 events: 660, 693, 743)
+        const unsigned int lsModules = count >= 32 ? 4u : 1u;
+        LST_LAUNCH(lst::kCreateLS, tunedWarpGrid(ev, kTuLS, ceilDiv(nLower, lsModules), count), tunedThreads(ev, kTuLS),
+                   d, v, lsModules);
         LST_LAUNCH(lst::kLSByMD, warpGrid(ceilDiv(nLower, group), lst::kIdxWarps, count), 32 * lst::kIdxWarps, d, v, group);
         break;
+      }
       case LST_STAGE_TRIPLETS: {
         // modules per block task: 16, and 8 for a few events, which then make 1660
         // tasks each (one event: 41 us, with 4 43, with 16 64; 64 events at 16

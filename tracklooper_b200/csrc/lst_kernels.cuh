@@ -688,79 +688,118 @@ namespace lst {
   }
 
   // ======================================================== line segments
-  // One warp per inner lower module walking (connected module, inner MD,
-  // outer MD) in order (SDL/Segment.h:798-910).
+  // Segments (SDL/Segment.h:798-910): a warp walks (connected module, inner
+  // MD, outer MD) of up to kLSTaskModules inner lower modules in order.  The
+  // (module, connected module) pairs are dealt out over the lanes, kLSChunk at a
+  // time; the warp's shared memory then has the prefix of the candidates over the
+  // pairs, and per pair the connected module, its MD count and first MD, so that
+  // a candidate finds its MDs without a global load.  A passing segment's place
+  // is its module's running count plus the passing lanes of the same module below.
+  //
+  // Bound by the gathers' latency and the L1 (72 % busy with them); a module's
+  // own chain of dependent loads is shared by the task's modules (64 PU200 events:
+  // a module per warp 1142 us, 4 modules 953).  A block per task with a queue
+  // between the window and the rest, as in kCreateT3, has lanes 84 % busy instead
+  // of 64 but loses it at the barriers (1066; one event 70 instead of 50).
   constexpr int kLSWarps = 4;
-  // Per-warp scratch of the walk: the prefix of the candidates over the
-  // connected modules, and per connected module its index, MD count and
-  // first MD, so that a candidate finds its MDs without a global load.
+  constexpr int kLSChunk = 64;
+  constexpr unsigned int kLSTaskModules = 8;  // modules per task (at most)
   struct LSScratch {
-    unsigned int pre[kMaxConnectedModules + 1];
-    unsigned int nOuterMDs[kMaxConnectedModules];
-    unsigned int outerBase[kMaxConnectedModules];
-    uint16_t outer[kMaxConnectedModules];
+    unsigned int pre[kLSChunk + 1];
+    unsigned int outerBase[kLSChunk];
+    unsigned int modulePre[kLSTaskModules + 1];  // prefix of the task's pairs over its modules
+    unsigned int innerBase[kLSTaskModules], nInnerMDs[kLSTaskModules], count[kLSTaskModules];
+    LSCut cut[kLSTaskModules];
+    uint16_t nOuterMDs[kLSChunk];
+    uint16_t outer[kLSChunk];
+    uint8_t module[kLSChunk];
   };
-  __device__ __forceinline__ void lsModule(DeviceES const& es, const EventView& ev, uint16_t lm, LSScratch& sc) {
-    const unsigned int nInnerMDs = ev.md.nMDs[lm];
-    if (nInnerMDs == 0)
-      return;
+  __device__ __forceinline__ void lsTask(DeviceES const& es, const EventView& ev, unsigned int firstModule,
+                                         unsigned int nModules, LSScratch& sc) {
     const Modules& m = es.m;
-    const int nConn = m.nConnectedModules[lm];
-    uint16_t* outer = sc.outer;
-    const unsigned int total = warpPrefix(sc.pre, nConn, [&](int k) {
-      const uint16_t o = m.moduleMap[lm * kMaxConnectedModules + k];
-      const unsigned int n = ev.md.nMDs[o];
-      outer[k] = o;
-      sc.nOuterMDs[k] = n;
-      sc.outerBase[k] = static_cast<unsigned int>(es.mdOffset[o]);
-      return nInnerMDs * n;
-    });
-    const int cap = es.lsCap[lm];
-    const unsigned int base = es.lsOffset[lm];
-    const unsigned int innerBase = es.mdOffset[lm];
-    const LSCut inner = es.lsCuts[lm];
-    Segments ls = ev.ls;
-    unsigned int count = 0;
-    for (unsigned int start = 0; start < total; start += 32) {
-      unsigned int f = start + laneId();
-      bool ok = false;
-      LSValues v;
-      unsigned int innerMD = 0, outerMD = 0;
-      uint16_t outerLM = 0;
-      if (f < total) {
-        int k = findSlot(sc.pre, nConn, f);
-        outerLM = outer[k];
-        unsigned int nOuterMDs = sc.nOuterMDs[k];
-        unsigned int local = f - sc.pre[k];
-        innerMD = innerBase + local / nOuterMDs;
-        outerMD = sc.outerBase[k] + local % nOuterMDs;
-        ok = lsSelect(inner, es.lsCuts[outerLM], m.ptCut, ev.md.rec[innerMD], ev.md.rec[outerMD], v);
-      }
-      unsigned int tot;
-      unsigned int r = count + warpRank(ok, tot);
-      if (ok && int(r) < cap)
-        storeLS(ls, ev.md, innerMD, outerMD, lm, outerLM, v, base + r);
-      count += tot;
+    const unsigned int lane = laneId();
+    const unsigned int own = firstModule + lane;  // the lane's module
+    const bool valid = lane < nModules && own < es.nLowerModules;
+    const unsigned int nMDsOwn = valid ? ev.md.nMDs[own] : 0u;
+    const int capOwn = valid ? es.lsCap[own] : 0;
+    const unsigned int baseOwn = valid ? static_cast<unsigned int>(es.lsOffset[own]) : 0u;
+    const unsigned int nConnOwn = valid ? m.nConnectedModules[own] : 0u;
+    const unsigned int incl = laneInclusiveSum(nMDsOwn != 0 ? nConnOwn : 0u);
+    const unsigned int nPairs = __shfl_sync(kFullMask, incl, 31);
+    if (lane < kLSTaskModules) {
+      sc.innerBase[lane] = valid ? static_cast<unsigned int>(es.mdOffset[own]) : 0u;
+      sc.nInnerMDs[lane] = nMDsOwn;
+      if (valid)
+        sc.cut[lane] = es.lsCuts[own];
+      sc.count[lane] = 0;
+      sc.modulePre[lane + 1] = incl;
     }
-    if (laneId() == 0) {
-      ls.nSegments[lm] = (int(count) < cap) ? count : (cap > 0 ? unsigned(cap) : 0u);
-      ls.totOccupancySegments[lm] = count;
-      if (int(count) > cap)
+    if (lane == 0)
+      sc.modulePre[0] = 0;
+    __syncwarp();
+    Segments ls = ev.ls;
+    for (unsigned int c0 = 0; c0 < nPairs; c0 += kLSChunk) {
+      const int n = int(min(nPairs - c0, unsigned(kLSChunk)));
+      const unsigned int total = warpPrefix(sc.pre, n, [&](int i) {
+        const unsigned int g = c0 + unsigned(i);
+        const int j = findSlot(sc.modulePre, kLSTaskModules, g);
+        const uint16_t o = m.moduleMap[(firstModule + j) * kMaxConnectedModules + (g - sc.modulePre[j])];
+        const unsigned int nOuter = ev.md.nMDs[o];
+        sc.outer[i] = o;
+        sc.nOuterMDs[i] = static_cast<uint16_t>(nOuter);
+        sc.outerBase[i] = static_cast<unsigned int>(es.mdOffset[o]);
+        sc.module[i] = static_cast<uint8_t>(j);
+        return sc.nInnerMDs[j] * nOuter;
+      });
+      for (unsigned int start = 0; start < total; start += 32) {
+        const unsigned int f = start + lane;
+        bool ok = false;
+        LSValues v;
+        unsigned int innerMD = 0, outerMD = 0, j = 0;
+        uint16_t outerLM = 0;
+        if (f < total) {
+          const int k = findSlot(sc.pre, n, f);
+          outerLM = sc.outer[k];
+          j = sc.module[k];
+          const unsigned int nOuterMDs = sc.nOuterMDs[k], local = f - sc.pre[k];
+          innerMD = sc.innerBase[j] + local / nOuterMDs;
+          outerMD = sc.outerBase[k] + local % nOuterMDs;
+          ok = lsSelect(sc.cut[j], es.lsCuts[outerLM], m.ptCut, ev.md.rec[innerMD], ev.md.rec[outerMD], v);
+        }
+        const unsigned int peers = __match_any_sync(kFullMask, ok ? j : 32u + lane);
+        const unsigned int rank = __popc(peers & lanesBelowMask());
+        const int cap = __shfl_sync(kFullMask, capOwn, j);
+        const unsigned int base = __shfl_sync(kFullMask, baseOwn, j);
+        const unsigned int r = sc.count[j] + rank;
+        if (ok && int(r) < cap)
+          storeLS(ls, ev.md, innerMD, outerMD, static_cast<uint16_t>(firstModule + j), outerLM, v, base + r);
+        __syncwarp();
+        if (ok && rank == 0)
+          sc.count[j] += __popc(peers);
+        __syncwarp();
+      }
+      __syncwarp();  // the chunk's scratch has been read
+    }
+    if (nMDsOwn != 0) {
+      const unsigned int n = sc.count[lane];
+      ls.nSegments[own] = (int(n) < capOwn) ? n : (capOwn > 0 ? unsigned(capOwn) : 0u);
+      ls.totOccupancySegments[own] = n;
+      if (int(n) > capOwn)
         atomicOr(&ev.sc->status, kStatusCapOverflow);
     }
+    __syncwarp();
   }
 
-  __global__ void __launch_bounds__(LST_LB_LS) kCreateLS(DeviceES es, const EventView* evs) {
+  __global__ void __launch_bounds__(LST_LB_LS) kCreateLS(DeviceES es, const EventView* evs, unsigned int modulesPerTask) {
     kernelEntry();
     __shared__ LSScratch sScratch[kLSWarps];
     const EventView& ev = evs[blockIdx.y];
     const int wib = threadIdx.x >> 5;
-    // modules from the event's counter (zero before the kernel)
+    const unsigned int nTasks = (es.nLowerModules + modulesPerTask - 1u) / modulesPerTask;
+    // tasks from the event's counter (zero before the kernel)
     WarpTasks tasks(&ev.sc->lsNext);
-    for (unsigned int w = tasks.take(); w < es.nLowerModules; w = tasks.take()) {
-      __syncwarp();
-      lsModule(es, ev, static_cast<uint16_t>(w), sScratch[wib]);
-    }
+    for (unsigned int task = tasks.take(); task < nTasks; task = tasks.take())
+      lsTask(es, ev, task * modulesPerTask, modulesPerTask, sScratch[wib]);
   }
 
   // SDL/Segment.h:1010-1029
