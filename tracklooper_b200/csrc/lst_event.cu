@@ -564,10 +564,7 @@ namespace {
       case LST_STAGE_MINI_DOUBLETS: {
         // modules per warp task: 8 from 4 events per launch, 4 for fewer, so
         // that a single event still makes enough tasks to fill the GPU
-#ifndef LST_MD_MPT
-#define LST_MD_MPT 8u
-#endif
-        const unsigned int mpt = count >= 4 ? LST_MD_MPT : 4u;
+        const unsigned int mpt = count >= 4 ? 8u : 4u;
         LST_LAUNCH(lst::kCreateMD, tunedWarpGrid(ev, kTuMD, ceilDiv(nLower, mpt), count), tunedThreads(ev, kTuMD), d, v,
                    mpt);
         LST_LAUNCH(lst::kMDDerived, tunedWarpGrid(ev, kTuMDDerived, nLower + 1, count), tunedThreads(ev, kTuMDDerived),

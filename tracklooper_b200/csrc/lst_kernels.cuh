@@ -562,7 +562,7 @@ namespace lst {
       if (ok) {
         const unsigned int r = count[j] + rank;
         if (int(r) < capj)
-          storeMD(es.m, h, md, lowerIdx, upperIdx, lm, v, basej + r);
+          storeMDPair(es.m, md, lowerIdx, upperIdx, lm, v, basej + r);
       }
       __syncwarp();
       if (ok && rank == 0)
@@ -585,7 +585,7 @@ namespace lst {
   // the fastest of a sweep over 2..14 blocks on B200 (PU200 batches, launch
   // shapes autotuned for each setting).
 #ifndef LST_LB_MD_B
-#define LST_LB_MD_B 4
+#define LST_LB_MD_B 6
 #endif
 #ifndef LST_LB_LS_B
 #define LST_LB_LS_B 12
@@ -635,13 +635,18 @@ namespace lst {
     }
   }
 
-  // Derived per-MD values for every stored MD (lower modules and the pixel
-  // module).  A warp takes 32 lower modules at a time (a module holds a few
+  // The hits' values of every stored MD, and its record for the later cuts (the
+  // record alone for the pixel module's, which are whole already).  A warp takes 32 lower modules at a time (a module holds a few
   // MDs) and shares their MDs out over its lanes: a lane-level prefix of the
   // modules' counts, and per MD the owning lane by a search over it.
   // The pixel module's mini-doublets (two per pLS, thousands per event) are
   // shared out over all of the event's threads.
   // Also sets the modules' mini-doublet ranges and clears kCreateMD's counter.
+  // Waits for scattered sectors (a warp's 32 mini-doublets lie in a dozen modules'
+  // places of some 25 arrays), with all of a mini-doublet's loads in flight: held
+  // to 64 registers a thread instead of its 122 it took 746 us instead of 646 (64
+  // PU200 events; kCreateMD, which stored all of it, was 1128 and is 477, and this
+  // kernel 177).
   __global__ void kMDDerived(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
@@ -678,7 +683,7 @@ namespace lst {
         const unsigned int ownerN = __shfl_sync(kFullMask, n, owner);
         const unsigned int ownerBase = __shfl_sync(kFullMask, base, owner);
         if (f < total)
-          storeMDDerived(md, ownerBase + (f - (ownerIncl - ownerN)), es.m.ptCut);
+          storeMDRest(es.m, ev.hits, md, static_cast<uint16_t>(w0 + owner), ownerBase + (f - (ownerIncl - ownerN)));
       }
     }
     const unsigned int nPix = md.nMDs[es.nLowerModules];

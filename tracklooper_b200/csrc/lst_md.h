@@ -238,19 +238,24 @@ namespace lst {
     shiftStripFinish(c, pre.shiftXa[p], pre.shiftYa[p], xo, yo, xn, yn);
   }
 
-  // The record of a stored mini-doublet.
-  // Also fills the mini-doublet's record of segment-cut inputs (MDRec).
-  LST_HD void storeMDDerived(MiniDoublets& md, unsigned int idx, float ptCut) {
-    // (loads before stores, as in storeMD)
-    const MDPos p = md.anchorPos[idx];
-    const float phi = md.anchorPhi[idx], dphichange = md.dphichanges[idx], dphi = md.dphis[idx], dz = md.dzs[idx];
-    const float highEdgePhi = md.anchorHighEdgePhi[idx], lowEdgePhi = md.anchorLowEdgePhi[idx];
-    const unsigned int anchorHit = md.anchorHitIndices[idx], outerHit = md.outerHitIndices[idx];
+  // The mini-doublet's record of what the later cuts read (MDRec).
+  LST_HD void storeMDRec(MiniDoublets& md, unsigned int idx, float ptCut, const MDPos& p, float phi, float dphichange,
+                         float dphi, float dz, float highEdgePhi, float lowEdgePhi, unsigned int anchorHit,
+                         unsigned int outerHit) {
     const float slope = fasin(fmin_(p.rt * k2Rinv1GeVf / ptCut, kSinAlphaMax));
     const float tanSlope = ftan(slope);
     const float slope3 = fasin(fmin_(p.rt * k2Rinv1GeVf / 3.0f, kSinAlphaMax));
     md.rec[idx] = MDRec{p.x, p.y, p.z, p.rt, phi, slope, tanSlope / slope, dphichange, slope / tanSlope,
                         dphi * 15.0f / dz, highEdgePhi, lowEdgePhi, 0.1f / p.rt, slope3, anchorHit, outerHit};
+  }
+  // The same of a mini-doublet that storeMD has stored.
+  LST_HD void storeMDDerived(MiniDoublets& md, unsigned int idx, float ptCut) {
+    // (loads before stores, as in storeMDHits)
+    const MDPos p = md.anchorPos[idx];
+    const float phi = md.anchorPhi[idx], dphichange = md.dphichanges[idx], dphi = md.dphis[idx], dz = md.dzs[idx];
+    const float highEdgePhi = md.anchorHighEdgePhi[idx], lowEdgePhi = md.anchorLowEdgePhi[idx];
+    const unsigned int anchorHit = md.anchorHitIndices[idx], outerHit = md.outerHitIndices[idx];
+    storeMDRec(md, idx, ptCut, p, phi, dphichange, dphi, dz, highEdgePhi, lowEdgePhi, anchorHit, outerHit);
   }
 
   struct MDValues {
@@ -430,16 +435,20 @@ namespace lst {
                     pre, lowerIdx, upperIdx, v);
   }
 
-  // Writes a mini-doublet record (SDL/MiniDoublet.h:193-266).  On PS modules
-  // whose lower sensor is the strip sensor the anchor is the upper (pixel) hit.
-  LST_HD void storeMD(const Modules& m,
-                      const Hits& h,
-                      MiniDoublets& md,
-                      unsigned int lowerHitIdx,
-                      unsigned int upperHitIdx,
-                      uint16_t lowerModuleIdx,
-                      const MDValues& v,
-                      unsigned int idx) {
+  // A mini-doublet (SDL/MiniDoublet.h:193-266) is stored in two parts: its hits
+  // and the values of its cuts by the kernel that finds it, where few lanes of a
+  // warp have one, and the values of its hits by the next (kMDDerived), whose
+  // lanes take stored mini-doublets in a row.
+  //
+  // On PS modules whose lower sensor is the strip sensor the anchor is the upper
+  // (pixel) hit.
+  LST_HD void storeMDPair(const Modules& m,
+                          MiniDoublets& md,
+                          unsigned int lowerHitIdx,
+                          unsigned int upperHitIdx,
+                          uint16_t lowerModuleIdx,
+                          const MDValues& v,
+                          unsigned int idx) {
     unsigned int anchor, outer;
     if (m.moduleType[lowerModuleIdx] == PS and m.moduleLayerType[lowerModuleIdx] == Strip) {
       anchor = upperHitIdx;
@@ -448,6 +457,31 @@ namespace lst {
       anchor = lowerHitIdx;
       outer = upperHitIdx;
     }
+    md.moduleIndices[idx] = lowerModuleIdx;
+    md.anchorHitIndices[idx] = anchor;
+    md.outerHitIndices[idx] = outer;
+    md.dphichanges[idx] = v.dphichange;
+    md.dphis[idx] = v.dphi;
+    md.dzs[idx] = v.dz;
+    md.shiftedXs[idx] = v.shiftedX;
+    md.shiftedYs[idx] = v.shiftedY;
+    md.shiftedZs[idx] = v.shiftedZ;
+    md.noShiftedDzs[idx] = v.noShiftedDz;
+    md.noShiftedDphis[idx] = v.noShiftedDphi;
+    md.noShiftedDphiChanges[idx] = v.noShiftedDphiChange;
+  }
+
+  struct MDAnchor {
+    MDPos pos;
+    float phi, highEdgePhi, lowEdgePhi;
+  };
+  LST_HD MDAnchor storeMDHits(const Modules& m,
+                              const Hits& h,
+                              MiniDoublets& md,
+                              unsigned int anchor,
+                              unsigned int outer,
+                              uint16_t lowerModuleIdx,
+                              unsigned int idx) {
     // All loads before the first store: a load after a store that might alias it
     // waits for its turn, some 25 round trips in a row per stored mini-doublet
     // (with the other objects' stores in the same way, the kernels of 64 PU200
@@ -467,19 +501,6 @@ namespace lst {
       hphi = fatan2(hey, hex);
       lphi = fatan2(ley, lex);
     }
-    md.moduleIndices[idx] = lowerModuleIdx;
-    md.anchorHitIndices[idx] = anchor;
-    md.outerHitIndices[idx] = outer;
-    md.dphichanges[idx] = v.dphichange;
-    md.dphis[idx] = v.dphi;
-    md.dzs[idx] = v.dz;
-    md.shiftedXs[idx] = v.shiftedX;
-    md.shiftedYs[idx] = v.shiftedY;
-    md.shiftedZs[idx] = v.shiftedZ;
-    md.noShiftedDzs[idx] = v.noShiftedDz;
-    md.noShiftedDphis[idx] = v.noShiftedDphi;
-    md.noShiftedDphiChanges[idx] = v.noShiftedDphiChange;
-
     md.anchorX[idx] = ax;
     md.anchorY[idx] = ay;
     md.anchorZ[idx] = az;
@@ -504,6 +525,28 @@ namespace lst {
     md.outerHighEdgeY[idx] = ohey;
     md.outerLowEdgeX[idx] = olex;
     md.outerLowEdgeY[idx] = oley;
+    return MDAnchor{MDPos{ax, ay, az, art}, aphi, hphi, lphi};
+  }
+
+  LST_HD void storeMD(const Modules& m,
+                      const Hits& h,
+                      MiniDoublets& md,
+                      unsigned int lowerHitIdx,
+                      unsigned int upperHitIdx,
+                      uint16_t lowerModuleIdx,
+                      const MDValues& v,
+                      unsigned int idx) {
+    storeMDPair(m, md, lowerHitIdx, upperHitIdx, lowerModuleIdx, v, idx);
+    storeMDHits(m, h, md, md.anchorHitIndices[idx], md.outerHitIndices[idx], lowerModuleIdx, idx);
+  }
+
+  // The second part and the record of a mini-doublet that storeMDPair stored.
+  LST_HD void storeMDRest(const Modules& m, const Hits& h, MiniDoublets& md, uint16_t lowerModuleIdx,
+                          unsigned int idx) {
+    const unsigned int anchor = md.anchorHitIndices[idx], outer = md.outerHitIndices[idx];
+    const float dphichange = md.dphichanges[idx], dphi = md.dphis[idx], dz = md.dzs[idx];
+    const MDAnchor a = storeMDHits(m, h, md, anchor, outer, lowerModuleIdx, idx);
+    storeMDRec(md, idx, m.ptCut, a.pos, a.phi, dphichange, dphi, dz, a.highEdgePhi, a.lowEdgePhi, anchor, outer);
   }
 
   // Per-module mini-doublet capacity from the (category, |eta|) occupancy table
