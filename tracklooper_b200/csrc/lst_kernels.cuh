@@ -4237,10 +4237,31 @@ namespace lst {
     }
   }
 
-  // Writes the batch output: hits, len, seedIdx and type, contiguous.
+  // The batch output: hits, len, seedIdx and type, each 256-byte aligned.
+  struct OutputLayout {
+    size_t len, seed, type, end;
+  };
+  LST_HD OutputLayout outputLayout(size_t nHits, size_t nTC) {
+    auto up = [](size_t n) { return (n + 255) & ~size_t(255); };
+    OutputLayout l;
+    l.len = up(4 * nHits);
+    l.seed = up(l.len + 4 * nTC);
+    l.type = up(l.seed + 4 * nTC);
+    l.end = l.type + 2 * nTC;
+    return l;
+  }
+
+  // Writes the batch output, if it fits in `room` bytes.
   __global__ void kOutputGather(const EventView* evs, int count, const unsigned long long* offsets,
-                                unsigned int* outHits, unsigned int* outLen, int* outSeed, short* outType) {
+                                unsigned char* out, size_t room) {
     kernelEntry();
+    const OutputLayout l = outputLayout(offsets[2 * count + 1], offsets[count]);
+    if (l.end > room)
+      return;
+    unsigned int* outHits = reinterpret_cast<unsigned int*>(out);
+    unsigned int* outLen = reinterpret_cast<unsigned int*>(out + l.len);
+    int* outSeed = reinterpret_cast<int*>(out + l.seed);
+    short* outType = reinterpret_cast<short*>(out + l.type);
     const EventView& ev = evs[blockIdx.y];
     const unsigned int n = *ev.tc.nTrackCandidates;
     const unsigned long long tc0 = offsets[blockIdx.y];
@@ -4251,6 +4272,22 @@ namespace lst {
       outSeed[tc0 + i] = ev.tc.pixelSeedIndex[i];
       outType[tc0 + i] = ev.tc.trackCandidateType[i];
     }
+  }
+
+  // The events' offsets, and the batch output if it fits in `room` bytes, to
+  // pinned host memory, 16 bytes a thread.
+  __global__ void kOutputToHost(int count, const unsigned long long* offsets, const unsigned char* out, size_t room,
+                                unsigned long long* hostOffsets, unsigned char* host) {
+    kernelEntry();
+    const unsigned int t = blockIdx.x * blockDim.x + threadIdx.x, nThreads = gridDim.x * blockDim.x;
+    for (unsigned int i = t; i < 2u * (count + 1u); i += nThreads)
+      hostOffsets[i] = offsets[i];
+    const OutputLayout l = outputLayout(offsets[2 * count + 1], offsets[count]);
+    if (l.end > room)
+      return;
+    // (room is a multiple of 16, and so both buffers hold the last part)
+    for (size_t i = t; 16 * i < l.end; i += nThreads)
+      reinterpret_cast<uint4*>(host)[i] = reinterpret_cast<const uint4*>(out)[i];
   }
 
 }  // namespace lst
