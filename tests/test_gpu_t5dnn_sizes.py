@@ -76,3 +76,31 @@ def test_backward(n):
     # added 32 apart and folded; a term carries its product's and dh1's rounding
     chain = 64 * (-(-n // 64) // 592 + 1) + 592 // 32 + 1 + 6 + 34 + 2
     assert (np.abs(grad.cpu().numpy() - want) <= 1.01 * chain * U * size + 1e-30).all()
+
+
+@pytest.mark.parametrize("n", [1, 65, 70001])
+def test_forward_sums_in_order(n):
+    """Unfused 32-bit sums in the order of the inputs, the bias last: every gate as in the plain loop."""
+    import torch
+
+    rng = np.random.default_rng(n + 2)
+    x = rng.standard_normal((n, 38), dtype=np.float32)
+    w = t5dnn.random_weights(n).astype(np.float32)
+    w[t5dnn.B0:t5dnn.W2] = rng.standard_normal(32) * 0.1
+
+    def layer(a, m, b):
+        acc = np.zeros((n, m.shape[1]), np.float32)
+        for k in range(m.shape[0]):
+            acc = acc + a[:, k:k + 1] * m[k]
+        return acc + b
+
+    a1 = np.maximum(layer(x, w[:t5dnn.B0].reshape(38, 32), w[t5dnn.B0:t5dnn.W2]), np.float32(0))
+    a2 = np.maximum(layer(a1, w[t5dnn.W2:t5dnn.B2].reshape(32, 32), w[t5dnn.B2:t5dnn.W4]), np.float32(0))
+    z = layer(a2, w[t5dnn.W4:t5dnn.B4].reshape(32, 1), w[t5dnn.B4])[:, 0]
+    lib = lst.library()
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    got = [torch.empty(s, device="cuda") for s in ((n, 32), (n, 32), (n,))]
+    assert lib.lst_t5dnn_forward(wd.data_ptr(), xd.data_ptr(), n, got[0].data_ptr(), got[1].data_ptr(),
+                                 got[2].data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    for a, b in zip(got, (a1, a2, z)):
+        assert np.array_equal(a.cpu().numpy(), b)

@@ -23,8 +23,18 @@ namespace {
   static_assert(kParams == 2337, "T5 DNN parameter count");
   static_assert(kW0 % 4 == 0 && kW2 % 4 == 0 && kB0 % 4 == 0 && kB2 % 4 == 0 && kW4 % 4 == 0, "16-byte rows");
 
-  // (The file is compiled without contraction; the sums here are of this
-  // project's own order, so they fuse explicitly.)
+  // The file is compiled without contraction.  The forward sums stay unfused, in
+  // the order of the inputs and with the bias last: an activation within a
+  // rounding of zero opens or closes its ReLU gate for the whole gradient of the
+  // sample, and with fused sums other gates would open (262143 samples: one such
+  // gate moved the gradient by 2e-6 of its norm, five times its error in 64 bits).
+  // The gradient sums, which gate nothing, fuse explicitly.
+  __device__ __forceinline__ void mulAdd4(float* acc, float a, const float4& w) {
+    acc[0] += a * w.x;
+    acc[1] += a * w.y;
+    acc[2] += a * w.z;
+    acc[3] += a * w.w;
+  }
   __device__ __forceinline__ void fma4(float* acc, float a, const float4& w) {
     acc[0] = fmaf(a, w.x, acc[0]);
     acc[1] = fmaf(a, w.y, acc[1]);
@@ -48,11 +58,11 @@ namespace {
   // shared memory (coalesced, odd row stride), a layer's 32 sums per sample stay
   // in registers, and a weight row is eight 16-byte broadcasts from shared memory
   // for 32 kSPT multiply-adds.  The activations go out through the warp's own
-  // rows of the staging, whole lines at a time.  Bound by the broadcasts, so large
-  // batches take two samples a thread; below kFwdPairFrom samples, where one
-  // block per SM of that shape would leave SMs idle, one a thread.  262143
-  // samples: 389 us with strided reads and writes and one sum at a time, 129 with
-  // one sample a thread, 99 with two; 8192 samples: 35 us, now 23.
+  // rows of the staging, whole lines at a time.  Bound by the unfused multiplies
+  // and adds and the broadcasts, so large batches take two samples a thread; below
+  // kFwdPairFrom samples, where one block per SM of that shape would leave SMs
+  // idle, one a thread.  262143 samples: 389 us with strided reads and writes and
+  // one sum at a time, now 151; 8192 samples: 35 us, now 25.
   constexpr int kFwdThreads = 64;
   constexpr int kFwdPairFrom = 1 << 16;
   template <int kSPT>
@@ -102,7 +112,7 @@ namespace {
           const float4 wc = w[c];
 #pragma unroll
           for (int p = 0; p < kSPT; ++p)
-            fma4(a1[p] + 4 * c, xk[p], wc);
+            mulAdd4(a1[p] + 4 * c, xk[p], wc);
         }
       }
 #pragma unroll
@@ -137,7 +147,7 @@ namespace {
             const float4 wc = w[c];
 #pragma unroll
             for (int p = 0; p < kSPT; ++p)
-              fma4(a2[p] + 4 * c, a1[p][k], wc);
+              mulAdd4(a2[p] + 4 * c, a1[p][k], wc);
           }
         }
 #pragma unroll
@@ -149,7 +159,7 @@ namespace {
           for (int c = 0; c < kC; ++c) {
             const float v = a2[p][c] + sW[kB2 + half * kC + c];
             const float a = v > 0.f ? v : 0.f;
-            z[p] = fmaf(a, sW[kW4 + half * kC + c], z[p]);
+            z[p] += a * sW[kW4 + half * kC + c];
             own[lane * (kH + 1) + half * kC + c] = a;
           }
         }
