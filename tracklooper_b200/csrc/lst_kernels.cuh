@@ -239,7 +239,8 @@ namespace lst {
 
   // ================================================================ hits
   // SDL/Hit.h:217-269
-  __global__ void __launch_bounds__(256, 4) kHitPrep(DeviceES es, const EventView* evs) {
+  // (64 PU200 events with 3 / 4 / 5 / 6 blocks per SM: 503 / 414 / 407 / 386 us)
+  __global__ void __launch_bounds__(256, 6) kHitPrep(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     const unsigned int nHits = ev.sc->nHits;
@@ -348,10 +349,12 @@ namespace lst {
 
   // ========================================================= pixel segments
   // SDL/Segment.h:1031-1117
-  // Register budget: four 256-thread blocks per SM (at 154 registers a thread
-  // only one fitted, and the kernel waits on gathers).
+  // A thread per mini-doublet, whose stores then lie side by side, and then one per
+  // segment (64 PU200 events: with both of a segment's mini-doublets in its thread
+  // 320 us, now 184).  Register budget: three 256-thread blocks per SM (2: 197 us,
+  // 4: 197, 5: 217).
   // withRanges: sets the modules' hit ranges as well (batched ingest).
-  __global__ void __launch_bounds__(256, 4) kPixelIngest(DeviceES es, const EventView* evs, bool withRanges) {
+  __global__ void __launch_bounds__(256, 3) kPixelIngest(DeviceES es, const EventView* evs, bool withRanges) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
     if (withRanges)
@@ -363,18 +366,26 @@ namespace lst {
     const unsigned int mdBase = es.mdOffset[es.nLowerModules];
     const unsigned int lsBase = es.lsOffset[es.nLowerModules];
     const unsigned int nHits = ev.sc->nHits;
-    for (unsigned int tid = blockIdx.x * blockDim.x + threadIdx.x; tid < nPLS; tid += gridDim.x * blockDim.x) {
-      unsigned int hit[4] = {ev.plsHit0[tid], ev.plsHit1[tid], ev.plsHit2[tid], ev.plsHit3[tid]};
-      // The reference indexes the hit store with these unchecked; an index
-      // outside the event is flagged and replaced by hit 0 (the host rejects
-      // pixel segments for events without hits).
-      for (int k = 0; k < 4; ++k)
-        if (hit[k] >= nHits) {
-          atomicOr(&ev.sc->status, kStatusInvalidInput);
-          hit[k] = 0;
-        }
-      storePixelSegment(
-          es.m, ev.hits, md, ls, pix, mdBase, lsBase, tid, hit[0], hit[1], hit[2], hit[3], ev.plsDPhiChange[tid]);
+    const unsigned int first = blockIdx.x * blockDim.x + threadIdx.x, nThreads = gridDim.x * blockDim.x;
+    // The reference indexes the hit store with a seed's hits unchecked; an index
+    // outside the event is flagged and replaced by hit 0 (the host rejects pixel
+    // segments for events without hits).
+    auto hitOf = [&](unsigned int hit) {
+      if (hit < nHits)
+        return hit;
+      atomicOr(&ev.sc->status, kStatusInvalidInput);
+      return 0u;
+    };
+    // a thread per mini-doublet, then one per segment
+    for (unsigned int k = first; k < 2 * nPLS; k += nThreads) {
+      const unsigned int tid = k >> 1;
+      const unsigned int lower = (k & 1) ? ev.plsHit2[tid] : ev.plsHit0[tid];
+      const unsigned int upper = (k & 1) ? ev.plsHit3[tid] : ev.plsHit1[tid];
+      storePixelMD(es.m, ev.hits, md, pix, mdBase + k, hitOf(lower), hitOf(upper));
+    }
+    for (unsigned int tid = first; tid < nPLS; tid += nThreads) {
+      storePixelLS(es.m, ev.hits, ls, pix, mdBase, lsBase, tid, hitOf(ev.plsHit0[tid]), hitOf(ev.plsHit1[tid]),
+                   hitOf(ev.plsHit2[tid]), hitOf(ev.plsHit3[tid]), ev.plsDPhiChange[tid]);
       ls.partOfPT5[tid] = 0;
       ev.plsPhiP[tid] = phiOf(ls.px[tid], ls.py[tid]);
       ev.plsFlag[tid] = 0;

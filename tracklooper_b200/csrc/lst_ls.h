@@ -225,21 +225,30 @@ namespace lst {
   }
 
   // One pixel line segment: two pixel mini-doublets from the seed's four
-  // pseudo-hits, the rz least-squares score and the seed's circle
-  // (SDL/Segment.h:1031-1117 with SDL/Segment.h:392-453).
-  LST_HD void storePixelSegment(const Modules& m,
-                                const Hits& h,
-                                MiniDoublets& md,
-                                Segments& s,
-                                uint16_t pixelModule,
-                                unsigned int mdBase,
-                                unsigned int lsBase,
-                                unsigned int tid,
-                                unsigned int hit0,
-                                unsigned int hit1,
-                                unsigned int hit2,
-                                unsigned int hit3,
-                                float dPhiChange) {
+  // pseudo-hits (storePixelMD), the rz least-squares score and the seed's circle
+  // (storePixelLS) (SDL/Segment.h:1031-1117 with SDL/Segment.h:392-453).
+  LST_HD void storePixelMD(const Modules& m,
+                           const Hits& h,
+                           MiniDoublets& md,
+                           uint16_t pixelModule,
+                           unsigned int idx,
+                           unsigned int lowerHit,
+                           unsigned int upperHit) {
+    const MDValues zero{0, 0, 0, 0, 0, 0, 0, 0, 0};
+    storeMD(m, h, md, lowerHit, upperHit, pixelModule, zero, idx);
+  }
+  LST_HD void storePixelLS(const Modules& m,
+                           const Hits& h,
+                           Segments& s,
+                           uint16_t pixelModule,
+                           unsigned int mdBase,
+                           unsigned int lsBase,
+                           unsigned int tid,
+                           unsigned int hit0,
+                           unsigned int hit1,
+                           unsigned int hit2,
+                           unsigned int hit3,
+                           float dPhiChange) {
     unsigned int innerMD = mdBase + 2 * tid;
     unsigned int outerMD = mdBase + 2 * tid + 1;
     unsigned int pls = lsBase + tid;
@@ -274,9 +283,6 @@ namespace lst {
         bestIndex = i;
       }
     }
-    MDValues zero{0, 0, 0, 0, 0, 0, 0, 0, 0};
-    storeMD(m, h, md, hit0, hit1, pixelModule, zero, innerMD);
-    storeMD(m, h, md, hit2, hit3, pixelModule, zero, outerMD);
     s.mdIndices[pls * 2] = innerMD;
     s.mdIndices[pls * 2 + 1] = outerMD;
     s.innerLowerModuleIndices[pls] = pixelModule;
@@ -293,6 +299,23 @@ namespace lst {
     s.circleCenterX[tid] = candidateCenterXs[bestIndex];
     s.circleCenterY[tid] = candidateCenterYs[bestIndex];
     s.circleRadius[tid] = circleRadius;
+  }
+  LST_HD void storePixelSegment(const Modules& m,
+                                const Hits& h,
+                                MiniDoublets& md,
+                                Segments& s,
+                                uint16_t pixelModule,
+                                unsigned int mdBase,
+                                unsigned int lsBase,
+                                unsigned int tid,
+                                unsigned int hit0,
+                                unsigned int hit1,
+                                unsigned int hit2,
+                                unsigned int hit3,
+                                float dPhiChange) {
+    storePixelMD(m, h, md, pixelModule, mdBase + 2 * tid, hit0, hit1);
+    storePixelMD(m, h, md, pixelModule, mdBase + 2 * tid + 1, hit2, hit3);
+    storePixelLS(m, h, s, pixelModule, mdBase, lsBase, tid, hit0, hit1, hit2, hit3, dPhiChange);
   }
 
 }  // namespace lst
