@@ -605,7 +605,7 @@ namespace lst {
 #define LST_LB_T3_B 14
 #endif
 #ifndef LST_LB_EVAL_B
-#define LST_LB_EVAL_B 10
+#define LST_LB_EVAL_B 7
 #endif
 #ifndef LST_LB_T5EVAL_B
 #define LST_LB_T5EVAL_B 8
@@ -3096,6 +3096,8 @@ namespace lst {
   }
 
   // The rest of the selection for the queued candidates.
+  // (blocks per SM 6 / 7 / 8 / 10: 64 PU200 events, pT5 + pT3, 241 / 209 / 217 / 238 us;
+  // 8 events 78 / 82 / 84 / 102; 16 pt0.6 events 117 / 124 / 132 / 156)
   template <int K>
   __global__ void __launch_bounds__(LST_LB_EVAL) kPixEval(DeviceES es, const EventView* evs) {
     kernelEntry();
