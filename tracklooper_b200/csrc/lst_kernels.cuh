@@ -215,6 +215,9 @@ namespace lst {
         ev.sc->lsNext = 0;
         ev.sc->t3Next = 0;
         pixCountersClear(ev);
+        // (the track-candidate stage walks this list, also of an event whose
+        // quintuplet stage has not run)
+        ev.sc->t5ListCount = 0;
         ev.sc->walkDone = 0;
         ev.sc->plsTCDone = 0;
         ev.sc->nPT5Total = 0;
