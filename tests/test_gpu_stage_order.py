@@ -70,3 +70,41 @@ def test_candidates_without_the_quintuplet_stage(es, inputs, stages):
     if "pt3" in stages:
         assert got[0]["pt3.nPixelTriplets"][0] > 100
     same(*got)
+
+
+def shuffled(pls, rng):
+    order = rng.permutation(len(pls["hitIndices0"]))
+    return {name: a[order] for name, a in pls.items()}
+
+
+@pytest.mark.parametrize("walk", [False, True])
+@pytest.mark.parametrize("twice", [False, True])
+def test_pixel_segments_after_the_mini_doublets(es, inputs, twice, walk):
+    """Added after createMiniDoublets on a slot that another event has filled, or
+    added in another order first and again then: the candidates of the usual order."""
+    before, inp = inputs
+    got = []
+    for late in (False, True):
+        s = lst.EventSet(es, 1, max(i.n_hits for i in inputs) + 1024)
+        try:
+            s.set_walk(walk)
+            if late:
+                s.add_inputs(0, before)
+                for st in lst.STAGE_ORDER:
+                    s.run_stage(0, st)
+            s.add_hits(0, inp.x, inp.y, inp.z, inp.detId, inp.idxInNtuple)
+            if late:
+                if twice:
+                    s.add_pixel_segments(0, shuffled(inp.pls, np.random.default_rng(5)))
+                s.run_stage(0, "md")
+                s.add_pixel_segments(0, inp.pls)
+            else:
+                s.add_pixel_segments(0, inp.pls)
+                s.run_stage(0, "md")
+            for st in lst.STAGE_ORDER[1:]:
+                s.run_stage(0, st)
+            got.append(stores(s, 0))
+        finally:
+            s.close()
+    assert got[0]["pt5.nPixelQuintuplets"][0] > 100 and got[0]["pt3.nPixelTriplets"][0] > 100
+    same(*got)

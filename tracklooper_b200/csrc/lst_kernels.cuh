@@ -354,8 +354,10 @@ namespace lst {
   // SDL/Segment.h:1031-1117
   // A thread per mini-doublet, whose stores then lie side by side, and then one per
   // segment (64 PU200 events: with both of a segment's mini-doublets in its thread
-  // 320 us, now 184).  Register budget: three 256-thread blocks per SM (2: 197 us,
-  // 4: 197, 5: 217).
+  // 320 us, then 184; 220 since the mini-doublets' records are written here too, so
+  // that they are this event's whenever the segments are added, and no longer by
+  // kMDDerived, which takes 617 instead of 646).  Register budget: three 256-thread
+  // blocks per SM (before the records 184 us; 2: 197, 4: 197, 5: 217).
   // withRanges: sets the modules' hit ranges as well (batched ingest).
   __global__ void __launch_bounds__(256, 3) kPixelIngest(DeviceES es, const EventView* evs, bool withRanges) {
     kernelEntry();
@@ -649,18 +651,17 @@ namespace lst {
     }
   }
 
-  // The hits' values of every stored MD, and its record for the later cuts (the
-  // record alone for the pixel module's, which are whole already).  A warp takes 32 lower modules at a time (a module holds a few
-  // MDs) and shares their MDs out over its lanes: a lane-level prefix of the
-  // modules' counts, and per MD the owning lane by a search over it.
-  // The pixel module's mini-doublets (two per pLS, thousands per event) are
-  // shared out over all of the event's threads.
+  // The hits' values of every MD of the lower modules, and its record for the
+  // later cuts (the pixel module's are whole when kPixelIngest has stored them).
+  // A warp takes 32 lower modules at a time (a module holds a few MDs) and shares
+  // their MDs out over its lanes: a lane-level prefix of the modules' counts, and
+  // per MD the owning lane by a search over it.
   // Also sets the modules' mini-doublet ranges and clears kCreateMD's counter.
   // Waits for scattered sectors (a warp's 32 mini-doublets lie in a dozen modules'
   // places of some 25 arrays), with all of a mini-doublet's loads in flight: held
-  // to 64 registers a thread instead of its 122 it took 746 us instead of 646 (64
-  // PU200 events; kCreateMD, which stored all of it, was 1128 and is 477, and this
-  // kernel 177).
+  // to 64 registers a thread instead of its 122 it took 746 us instead of 646, now
+  // 617 (64 PU200 events; kCreateMD, which stored all of it, was 1128 and is 477, and
+  // this kernel 177).
   __global__ void kMDDerived(DeviceES es, const EventView* evs) {
     kernelEntry();
     const EventView& ev = evs[blockIdx.y];
@@ -700,10 +701,6 @@ namespace lst {
           storeMDRest(es.m, ev.hits, md, static_cast<uint16_t>(w0 + owner), ownerBase + (f - (ownerIncl - ownerN)));
       }
     }
-    const unsigned int nPix = md.nMDs[es.nLowerModules];
-    const unsigned int pixBase = es.mdOffset[es.nLowerModules];
-    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < nPix; k += gridDim.x * blockDim.x)
-      storeMDDerived(md, pixBase + k, es.m.ptCut);
   }
 
   // ======================================================== line segments

@@ -225,7 +225,8 @@ namespace lst {
   }
 
   // One pixel line segment: two pixel mini-doublets from the seed's four
-  // pseudo-hits (storePixelMD), the rz least-squares score and the seed's circle
+  // pseudo-hits (storePixelMD, with their records: the segments may be added
+  // after the mini-doublet stage), the rz least-squares score and the seed's circle
   // (storePixelLS) (SDL/Segment.h:1031-1117 with SDL/Segment.h:392-453).
   LST_HD void storePixelMD(const Modules& m,
                            const Hits& h,
@@ -235,7 +236,14 @@ namespace lst {
                            unsigned int lowerHit,
                            unsigned int upperHit) {
     const MDValues zero{0, 0, 0, 0, 0, 0, 0, 0, 0};
-    storeMD(m, h, md, lowerHit, upperHit, pixelModule, zero, idx);
+    const bool swap = m.moduleType[pixelModule] == PS and m.moduleLayerType[pixelModule] == Strip;
+    const unsigned int anchor = swap ? upperHit : lowerHit, outer = swap ? lowerHit : upperHit;
+    const MDAnchor a = storeMDHits(m, h, md, anchor, outer, pixelModule, idx);
+    storeMDPair(m, md, lowerHit, upperHit, pixelModule, zero, idx);
+    // (the pixel tracklets read the anchor alone; the other values are those of the
+    // cuts between outer-tracker modules)
+    md.rec[idx] = MDRec{a.pos.x, a.pos.y, a.pos.z, a.pos.rt, a.phi, 0, 0, 0, 0, 0, a.highEdgePhi, a.lowEdgePhi, 0, 0,
+                        anchor, outer};
   }
   LST_HD void storePixelLS(const Modules& m,
                            const Hits& h,
