@@ -3569,7 +3569,7 @@ namespace lst {
     const unsigned int wpb = blockDim.x >> 5;
     const unsigned int warp = blockIdx.x * wpb + (threadIdx.x >> 5), nWarps = gridDim.x * wpb;
     const unsigned int n = ev.sc->t5ListCount;
-    if (n <= kT5SortCap) {
+    if (n <= kT5SortCap && !ev.forceWalk) {
       for (unsigned int k = warp; k < n; k += nWarps) {
         const uint2 t = ev.t5List[k];
         t5CrossClean(ev, t.x, t.y);
