@@ -3475,27 +3475,8 @@ namespace lst {
             unsigned int base2 = ev.rg.quintupletModuleIndices[lowmod2];
             for (unsigned int jx1 = 0; jx1 < n2; jx1++) {
               unsigned int jx = base2 + jx1;
-              if (ix == jx)
-                continue;
-              if (q.partOfPT5[jx] || (q.isDup[jx] & 1))
-                continue;
-              float eta2 = q.eta[jx], phi2 = q.phi[jx], score2 = q.score_rphisum[jx];
-              float dEta = fabs_(eta1 - eta2);
-              float dPhi = wrapDPhi(phi1, phi2);
-              if (dEta > 0.1f)
-                continue;
-              if (fabs_(dPhi) > 0.1f)
-                continue;
-              float dR2 = dEta * dEta + dPhi * dPhi;
-              int nMatched = sharedHitsT5(q, ix, jx);
-              if (dR2 < 0.001f || nMatched >= 5) {
-                if (score1 > score2)
-                  ev.t5Flag[ix] = 1;
-                else if (score1 < score2)
-                  ev.t5Flag[jx] = 1;
-                else
-                  ev.t5Flag[ix < jx ? ix : jx] = 1;
-              }
+              if (ix != jx)
+                t5CrossPair(ev, ix, jx, eta1, phi1, score1);
             }
           }
         }
