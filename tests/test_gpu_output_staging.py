@@ -1,0 +1,60 @@
+"""lst_batch_get_output through its pinned staging (256 KiB a slot, 1 MiB at most)
+and past it, against lst_batch_get_output_static, which has no such staging."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tracklooper_b200 import gen, lst
+
+pytestmark = pytest.mark.gpu
+
+FILL = (0xABABABAB, 0xABABABAB, -0x55, -0x55)
+
+
+def call(fn, s, count, tc_capacity, hits_capacity):
+    arrays = [np.full(n, v, dt) for n, v, dt in zip((hits_capacity, tc_capacity, tc_capacity, tc_capacity), FILL,
+                                                    (np.uint32, np.uint32, np.int32, np.int16))]
+    tco, hco = np.zeros(count + 1, np.uint64), np.zeros(count + 1, np.uint64)
+    a, b, c, d = (x.ctypes.data for x in arrays)
+    out = lst.Output(a, hits_capacity, b, c, d, tc_capacity, tco.ctypes.data, hco.ctypes.data)
+    fn.argtypes, fn.restype = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.POINTER(lst.Output)], ctypes.c_int
+    rc = fn(s.handle, 0, count, ctypes.byref(out))
+    return rc, arrays, tco, hco
+
+
+def output_bytes(tco, hco):
+    return 4 * int(hco[-1]) + 10 * int(tco[-1])
+
+
+# (events, slots of the set, whether the output fits the staging)
+CASES = [([(1, 80, 0.0)], 1, True), ([(2, 81, 200.0)], 1, True), ([(2, 920, 400.0)], 1, False),
+         ([(2, 920, 400.0)], 2, True), ([(2, 82, 200.0)] * 5, 5, True), ([(2, 83, 200.0)] * 8, 8, False)]
+
+
+@pytest.fixture(scope="module")
+def es():
+    e = lst.ES(device=0)
+    yield e
+    e.close()
+
+
+@pytest.mark.parametrize("events,slots,fits", CASES)
+def test_either_way_gives_the_output(es, events, slots, fits):
+    inputs = [gen.generate_event(*e) for e in events]
+    n = len(inputs)
+    s = lst.EventSet(es, slots, max(i.n_hits for i in inputs) + 1024)
+    try:
+        s.upload_packed(0, *lst.pack_events(inputs))
+        s.run(0, n)
+        lib = lst.library()
+        rc, want, tco, hco = call(lib.lst_batch_get_output_static, s, n, 31000 * n, 31000 * 14 * n)
+        assert rc == 0 and tco[-1] > 0
+        assert (output_bytes(tco, hco) < min(slots << 18, 1 << 20) - 1024) == fits
+        for _ in range(2):
+            rc, got, t, h = call(lib.lst_batch_get_output, s, n, 31000 * n, 31000 * 14 * n)
+            assert rc == 0 and np.array_equal(t, tco) and np.array_equal(h, hco)
+            for a, b in zip(got, want):
+                assert np.array_equal(a, b)
+    finally:
+        s.close()

@@ -424,7 +424,9 @@ struct lst_event {
   unsigned long long* hOutOffsets = nullptr;  // pinned copy
   unsigned char* dOut = nullptr;
   size_t dOutBytes = 0;
-  unsigned char* hOut = nullptr;  // pinned, kHostOutBytes
+  unsigned char* hOut = nullptr;  // pinned output staging, from the set's first lst_batch_get_output on
+  size_t hOutBytes = 0;
+  bool hOutTried = false;
   unsigned int* dProbeCount = nullptr;
   // launch accounting and optional per-launch timing
   unsigned long long launches = 0;
@@ -459,7 +461,8 @@ namespace {
 namespace {
 
   constexpr unsigned int kThreads = 256;
-  constexpr size_t kHostOutBytes = size_t(1) << 20;  // pinned output staging of lst_batch_get_output
+  // pinned output staging of lst_batch_get_output: per slot, and at most
+  constexpr size_t kHostOutPerSlot = size_t(1) << 18, kHostOutBytes = size_t(1) << 20;
   constexpr unsigned int kResidentBlocks = 148 * 8;
 
   // Blocks per event for a grid-stride kernel over n items.
@@ -1068,7 +1071,6 @@ int lst_event_create(lst_es* es, int n_slots, uint32_t max_hits, void* stream, l
   LST_CUDA(cudaMallocHost(&ev->hCounts, sizeof(lst_counts) * n_slots));
   LST_CUDA(cudaMalloc(&ev->dOutOffsets, sizeof(unsigned long long) * 2 * (n_slots + 1)));
   LST_CUDA(cudaMallocHost(&ev->hOutOffsets, sizeof(unsigned long long) * 2 * (n_slots + 1)));
-  LST_CUDA(cudaMallocHost(&ev->hOut, kHostOutBytes));
   // Start every slot empty.
   int rc = runReset(ev.get(), 0, n_slots);
   if (rc)
@@ -1786,10 +1788,15 @@ int lst_batch_get_output(lst_event* ev, int first, int count, lst_output* out) {
     out->event_hit_offsets[0] = 0;
     return 0;
   }
-  // A small output (up to kHostOutBytes, some seven PU200 events) is written to
-  // pinned host memory by the kernels and copied from there: one wait for the
-  // stream instead of two and no copy calls (one muon: 47 us of the call's host
-  // time before).  A larger one is copied straight to the caller's arrays.
+  // A small output (up to 256 KiB a slot of the set, a PU200 event has 170 kB, and
+  // 1 MiB in all) is written to pinned host memory by the kernels and copied from
+  // there: one wait for the stream instead of two and no copy calls (this call
+  // alone, to pinned or pageable arrays: one muon 22 us instead of 41 or 63, one
+  // PU200 event 49 instead of 58 or 93, four 78 instead of 68 or 132).  A larger
+  // one is copied straight to the caller's arrays.  The staging is made by the
+  // set's first call and not with the set, and by its slots: page-locking costs
+  // 0.75 ms a MiB, and with 1 MiB each, sets of one slot took 1.75 ms to make
+  // instead of 0.5.  Without it (no memory to lock) every output is copied.
   cudaStream_t s = ev->stream;
   const lst::EventView* v = ev->dv + first;
   auto ensureStaging = [&](size_t bytes) -> int {
@@ -1807,11 +1814,21 @@ int lst_batch_get_output(lst_event* ev, int first, int count, lst_output* out) {
   rc = ensureStaging(kHostOutBytes);
   if (rc)
     return rc;
+  if (!ev->hOutTried) {
+    ev->hOutTried = true;
+    const size_t bytes = std::min(kHostOutBytes, kHostOutPerSlot * static_cast<size_t>(ev->nSlots));
+    if (cudaMallocHost(&ev->hOut, bytes) == cudaSuccess) {
+      ev->hOutBytes = bytes;
+    } else {
+      cudaGetLastError();
+      ev->hOut = nullptr;
+    }
+  }
   const dim3 gatherGrid(blocksFor(lst::kMaxTrackCandidates, count), count);
   LST_LAUNCH(lst::kOutputSizes, dim3(1, count), 1024, v);
   LST_LAUNCH(lst::kOutputEventOffsets, 1, 1024, v, count, ev->dOutOffsets);
   LST_LAUNCH(lst::kOutputGather, gatherGrid, kThreads, v, count, ev->dOutOffsets, ev->dOut, ev->dOutBytes);
-  LST_LAUNCH(lst::kOutputToHost, 32, kThreads, count, ev->dOutOffsets, ev->dOut, kHostOutBytes, ev->hOutOffsets,
+  LST_LAUNCH(lst::kOutputToHost, 32, kThreads, count, ev->dOutOffsets, ev->dOut, ev->hOutBytes, ev->hOutOffsets,
              ev->hOut);
   LST_CUDA(cudaStreamSynchronize(s));
   const unsigned long long* tcOff = ev->hOutOffsets;
@@ -1829,7 +1846,7 @@ int lst_batch_get_output(lst_event* ev, int first, int count, lst_output* out) {
   if (!out->hits || !out->len || !out->seedIdx || !out->type)
     return setError("lst_batch_get_output: null output array");
   const lst::OutputLayout l = lst::outputLayout(nHits, nTC);
-  if (l.end <= kHostOutBytes) {
+  if (l.end <= ev->hOutBytes) {
     std::memcpy(out->hits, ev->hOut, nHits * sizeof(unsigned int));
     std::memcpy(out->len, ev->hOut + l.len, nTC * sizeof(unsigned int));
     std::memcpy(out->seedIdx, ev->hOut + l.seed, nTC * sizeof(int));
