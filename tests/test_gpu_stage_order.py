@@ -108,3 +108,35 @@ def test_pixel_segments_after_the_mini_doublets(es, inputs, twice, walk):
             s.close()
     assert got[0]["pt5.nPixelQuintuplets"][0] > 100 and got[0]["pt3.nPixelTriplets"][0] > 100
     same(*got)
+
+
+def test_candidates_again_and_again(es, inputs):
+    """The track-candidate stage run on one event until its candidates fill the
+    store (it appends to them): they end there, the first ones stay, the event in
+    the next slot too, and a reset gives the first run's candidates again."""
+    s = lst.EventSet(es, 2, max(i.n_hits for i in inputs) + 1024)
+    try:
+        for slot, inp in enumerate(inputs):
+            s.add_inputs(slot, inp)
+            for st in lst.STAGE_ORDER:
+                s.run_stage(slot, st)
+        first, other = stores(s, 0), stores(s, 1)
+        n = int(first["tc.nTrackCandidates"][0])
+        last = n
+        for _ in range(24):
+            s.run_stage(0, "tc")
+            now = int(s.field(0, "tc.nTrackCandidates")[0])
+            assert last <= now <= ROOM["tc"]
+            last = now
+        assert last >= 30000 and s.counts(0)["status"] & lst.STATUS_TC_TRUNCATED
+        again = stores(s, 0)
+        for name, x in first.items():
+            if name.startswith("tc.") and name != "tc.nTrackCandidates":
+                assert again[name][:n].tobytes() == x.tobytes(), name
+        same(other, stores(s, 1))
+        s.add_inputs(0, inputs[0])
+        for st in lst.STAGE_ORDER:
+            s.run_stage(0, st)
+        same(first, stores(s, 0))
+    finally:
+        s.close()
