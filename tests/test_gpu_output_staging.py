@@ -58,3 +58,25 @@ def test_either_way_gives_the_output(es, events, slots, fits):
                 assert np.array_equal(a, b)
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("events,slots,fits", CASES)
+@pytest.mark.parametrize("tc_short,hits_short", [(1, 0), (0, 1), (1 << 20, 1 << 20)])
+def test_too_small_arrays_stay_as_they_were(es, events, slots, fits, tc_short, hits_short):
+    """Refused, with the offsets filled and nothing else written."""
+    inputs = [gen.generate_event(*e) for e in events]
+    n = len(inputs)
+    s = lst.EventSet(es, slots, max(i.n_hits for i in inputs) + 1024)
+    try:
+        s.upload_packed(0, *lst.pack_events(inputs))
+        s.run(0, n)
+        fn = lst.library().lst_batch_get_output
+        rc, _, tco, hco = call(fn, s, n, 31000 * n, 31000 * 14 * n)
+        assert rc == 0
+        rc, got, t, h = call(fn, s, n, max(int(tco[-1]) - tc_short, 0), max(int(hco[-1]) - hits_short, 0))
+        assert rc == -1 and b"capacity too small" in lst.library().lst_last_error()
+        assert np.array_equal(t, tco) and np.array_equal(h, hco)
+        for a, v in zip(got, FILL):
+            assert (a == a.dtype.type(v)).all()
+    finally:
+        s.close()
