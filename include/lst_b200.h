@@ -391,7 +391,11 @@ int lst_event_get_profile(lst_event* ev, lst_kernel_time* out, int capacity, int
  * divisions, SDL/Event.cc).  The kernels that do most of the work take their
  * launch shape from the event set: warps per block and resident blocks per
  * SM across the batch (each event gets blocks_per_sm x SMs / events blocks).
- * Object lists do not depend on the shape. */
+ * Object lists do not depend on the shape.  A shape that was set (by hand, by
+ * the autotuner or from its cache) is used as it is; the default ones of some
+ * kernels have more blocks per SM the more events a launch has (16 for one
+ * event, 64 for many).  lst_event_get_launch_shape tells the shape in effect
+ * for a launch of all the set's slots. */
 int lst_tune_kernel_count(void);
 const char* lst_tune_kernel_name(int k);
 int lst_event_set_launch_shape(lst_event* ev, int k, int warps_per_block, int blocks_per_sm);

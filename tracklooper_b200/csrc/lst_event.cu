@@ -2109,11 +2109,12 @@ namespace {
     return key;
   }
 
-  std::string shapesLine(const lst_event* ev) {
+  // The shapes of a launch of count events.
+  std::string shapesLine(const lst_event* ev, int count) {
     std::string line;
     for (int k = 0; k < kTuCount; ++k)
       line += " " + std::string(kTuneSpecs[k].name) + "=" + std::to_string(ev->shape[k].warps) + "x" +
-              std::to_string(ev->shape[k].perSM);
+              std::to_string(blocksPerSM(ev->shape[k], k, count));
     return line;
   }
 
@@ -2203,7 +2204,7 @@ int lst_event_get_launch_shape(const lst_event* ev, int k, int* warps_per_block,
   if (k < 0 || k >= kTuCount)
     return setError("lst_event_get_launch_shape: no tunable kernel " + std::to_string(k));
   *warps_per_block = ev->shape[k].warps;
-  *blocks_per_sm = ev->shape[k].perSM;
+  *blocks_per_sm = blocksPerSM(ev->shape[k], k, ev->nSlots);
   return 0;
   LST_ABI_CATCH_INT
 }
@@ -2342,7 +2343,7 @@ int lst_autotune(lst_event* ev, int first, int count, const char* cache_path) {
         if (!line.empty() && line.compare(0, key.size() + 1, key + " ") != 0)
           lines.push_back(line);
     }
-    lines.push_back(key + shapesLine(ev));
+    lines.push_back(key + shapesLine(ev, count));
     const std::string tmp = std::string(cache_path) + ".tmp";
     {
       std::ofstream out(tmp, std::ios::trunc);

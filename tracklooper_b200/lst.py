@@ -598,7 +598,7 @@ class EventSet:
 
     # -- launch shapes and the autotuner
     def launch_shapes(self) -> dict:
-        """{kernel: (warps per block, blocks per SM)} of the tunable kernels."""
+        """{kernel: (warps per block, blocks per SM)} of the tunable kernels, for a launch of all slots."""
         lib = library()
         out = {}
         for k in range(lib.lst_tune_kernel_count()):
