@@ -329,7 +329,8 @@ int lst_event_prepare_input(lst_event* ev, int slot, const lst_seed_input* in);
 /* Track-candidate output of LST::getOutput (SDL/LST.cc:367-427) for slots
  * [first, first + count), flattened over the events: candidate k of the batch
  * has type[k], seedIdx[k] (pixelSeedIndex) and len[k] input-ntuple hit
- * indices, stored back to back in hits[].  Event i owns candidates
+ * indices, stored back to back in hits[].  All arrays are host memory, pinned
+ * or not.  Event i owns candidates
  * [event_tc_offsets[i], event_tc_offsets[i + 1]) and hits
  * [event_hit_offsets[i], event_hit_offsets[i + 1]); both offset arrays hold
  * count + 1 entries and are always filled.  If tc_capacity or hits_capacity

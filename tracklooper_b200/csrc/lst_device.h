@@ -121,7 +121,7 @@ namespace lst {
     unsigned int* t5CandPre;    // per inner triplet: its first candidate within the module
     unsigned int* t5ModCand;    // per eligible module: candidates
     unsigned int* t5ModOff;     // per eligible module: first candidate of the event
-    unsigned int* t5Task;       // tasks of kT5Eval's warps: module position and 32-triplet chunk
+    unsigned int* t5Task;       // tasks of kT5Eval's warps: module position and first inner triplet
     struct T5Staged* t5Staged;  // quintuplet candidates that pass the tracklet tests
     T5Values* t5PassValues;     // selection values of passing candidates
     unsigned int* t5PassC;      //   their key
@@ -137,8 +137,8 @@ namespace lst {
     unsigned int* t5Order;      // quintuplets sorted by eta bin (their index)
     uint16_t* t5OrderPos;       //   and their module's position in the eligible-module list
     unsigned int* t5BinStart;   // start of each eta bin in t5Order (bins + 2 entries)
-    unsigned int* candQueueObj; // and the object of a queued pixel candidate
-    unsigned int* candQueue;    // candidates passing a pre-selection (T5, then pT5 / pT3), any order
+    unsigned int* candQueue;    // keys of the pT5 / pT3 candidates that pass the opening tests, any order
+    unsigned int* candQueueObj; //   and their object
     struct TCCleanInfo* tcCleanInfo;  // per track candidate: the pLS cross-cleaning record
     struct PLSRec* plsRec;      // pass-2 pLS records sorted by eta bin
     uint2* seedChunk;           // per chunk of seeds: kept seeds and their pseudo-hits

@@ -316,7 +316,7 @@ namespace {
     std::memcpy(&w, es->dnn.data(), sizeof(w));
     LST_CUDA(cudaSetDevice(es->device));
     LST_CUDA(cudaMemcpyToSymbol(lst::c_t5dnn, &w, sizeof(w)));
-  LST_CUDA(cudaMemcpyToSymbol(lst::g_t5dnn, &w, sizeof(w)));
+    LST_CUDA(cudaMemcpyToSymbol(lst::g_t5dnn, &w, sizeof(w)));
     LST_CUDA(cudaDeviceSynchronize());
     es->haveDnn = true;
     return 0;
@@ -602,10 +602,10 @@ namespace {
         if (ev->t5Method == LST_T5_DNN && !ev->es->haveDnn)
           return setError("the DNN T5 method needs weights (lst_es_load or lst_es_set_t5dnn_weights)");
         bool useDnn = ev->t5Method == LST_T5_DNN;
-
         // 8 inner triplets per warp task: the candidates are very uneven, and with
-        // 32 the heaviest task set kT5Eval's length (8 PU200 events: 350 us, with 8
-        // 204, with 4 191; 64 events: 1057, 1019, 1065)
+        // more the heaviest task sets kT5Eval's length (with 32 / 16 / 8 / 4: one PU200
+        // event 68 / 55 / 41 / 39 us, 8 events 245 / 157 / 126 / 122, 64 events 538 /
+        // 527 / 512 / 551, 16 pt0.6 events 700 / 560 / 510 / 505)
         LST_LAUNCH(lst::kT5Eligible, one, 1024, d, v, 8u);
         LST_LAUNCH(lst::kT5Eval, tunedFlatGrid(ev, kTuT5Eval, count), tunedThreads(ev, kTuT5Eval), d, v);
         LST_LAUNCH(lst::kT5Classify, dim3(blocksFor(lst::kT5RankCap, count, lst::kT5ClassifyThreads), count),

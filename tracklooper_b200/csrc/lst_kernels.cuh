@@ -31,11 +31,11 @@ namespace lst {
   // First statement of every kernel that LST_LAUNCH launches.  Those launches let
   // a kernel's blocks in as soon as the last block of the stream's previous kernel
   // has exited (programmatic dependent launch), so that the launch overlaps the
-  // previous kernel's completion: a step is some 65 kernels, most of them a few
-  // microseconds long.  The wait returns when the previous kernel has completed
-  // and its writes are visible; since every block of every kernel waits here
-  // before it does anything (or exits), that holds for all kernels before it as
-  // well.  One muon's lst_run 437 -> 289 us, five PU30 events 865 -> 750, one
+  // previous kernel's completion: a batch is 44 kernels from its unpacking to its
+  // candidates, most of them a few microseconds long.  The wait returns when the
+  // previous kernel has completed and its writes are visible; since every block of
+  // every kernel waits here before it does anything (or exits), that holds for all
+  // kernels before it as well.  One muon's lst_run 437 -> 289 us, five PU30 events 865 -> 750, one
   // PU200 event 1734 -> 1582, 64 PU200 events unchanged.  Letting the next kernel
   // in at the start of the previous one brought no more, and blocks waiting
   // behind a one-block kernel kept other streams' kernels off the SMs (two event
@@ -1002,8 +1002,8 @@ namespace lst {
   }
 
   // Segments of each lower module grouped by inner MD (after kCreateLS): a
-  // warp takes 32 modules at a time, module by module where their bins do
-  // not fit (or the fallback paths are forced).  Also sets the modules' segment
+  // warp takes `group` modules at a time (32; 8 for a few events), module by
+  // module where their bins do not fit (or the fallback paths are forced).  Also sets the modules' segment
   // ranges and clears kCreateLS's counter.
   constexpr int kIdxWarps = 4;
   __global__ void kLSByMD(DeviceES es, const EventView* evs, unsigned int group) {
@@ -1327,7 +1327,7 @@ namespace lst {
   constexpr unsigned int kT5RankCap = 8192;        // passing candidates per event
   constexpr unsigned int kT5SortCap = 1u << 15;    // quintuplets per event listed for the track-candidate stage
   // Eligible T5 seed modules and their offsets (SDL/Quintuplet.h:3117-3213),
-  // and the tasks of kT5Eval's warps: up to 32 inner triplets of one module.
+  // and the tasks of kT5Eval's warps: innerPerTask (up to 32) inner triplets of one module.
   // One block per event, a run of modules per warp as in kT3Offsets; the three
   // sums (modules, quintuplet places, tasks) are scanned together.
   __global__ void __launch_bounds__(1024) kT5Eligible(DeviceES es, const EventView* evs, unsigned int innerPerTask) {
@@ -1577,7 +1577,7 @@ namespace lst {
   }
 
   // The T5 selection up to the classifier (SDL/Quintuplet.h:2508-2920).  A warp
-  // takes a task of up to 32 inner triplets of one module: its lanes fetch where
+  // takes a task of a few inner triplets (up to 32) of one module: its lanes fetch where
   // their outer triplets are listed (those that start at the inner triplet's
   // third mini-doublet), and the candidates are tested 32 at a time.  Each long
   // test runs when the warp's own queue for it, in shared memory, holds a warp
@@ -2895,8 +2895,8 @@ namespace lst {
   // the global rank of a passing candidate is the number of passing candidates
   // with a smaller key.  kPixMid walks all candidates and queues those that
   // pass the opening tests, kPixEval runs the rest of the selection on them,
-  // and one block per event ranks the passing ones and stores the first 15000
-  // (pT5) / 5000 (pT3).  Events that overflow the lists (or a pLS with more
+  // and kPixRankEmit ranks the passing ones and stores the first 15000 (pT5) /
+  // 5000 (pT3).  Events that overflow the lists (or a pLS with more
   // than 2^16 candidates) take the per-pLS count/emit walk instead.
   constexpr unsigned int kPixPassCap = 8192;
   constexpr unsigned int kPixKeyCandidates = 1u << 16;  // candidates of one pLS that a key can number
@@ -3367,16 +3367,15 @@ namespace lst {
   }
 
   // Cross-module T5 duplicate removal before TC building
-  // (SDL/Kernels.h:251-323); one warp per eligible module, marks t5Flag.
-  // Cross-module T5 cleaning (SDL/Kernels.h:251-323).  The reference visits
+  // (SDL/Kernels.h:251-323), which marks t5Flag.  The reference visits
   // the ordered pairs (ix in module A, jx in module B) with A's position in
   // the eligible-module list not after B's and ix != jx; a pair whose
-  // |deta| > 0.1 is skipped at the first test, and marks are only ever set.  kT5Bin counting-sorts the event's
-  // quintuplets into the pLS-cleaning eta bins (one block per event), and
-  // kT5DedupBinned gives each quintuplet a thread that visits the same ordered
-  // pairs among the bins within reach (and the non-finite bin, which meets
-  // every quintuplet, as does a quintuplet of non-finite eta).  Events with
-  // more quintuplets than kT5SortCap keep the module-pair walk.
+  // |deta| > 0.1 is skipped at the first test, and marks are only ever set.
+  // kT5Bin counting-sorts the event's quintuplets into the pLS-cleaning eta bins
+  // (one block per event), and kT5DedupBinned gives each quintuplet a warp that
+  // visits the same ordered pairs among the bins within reach (and the non-finite
+  // bin, which meets every quintuplet, as does a quintuplet of non-finite eta).
+  // Events with more quintuplets than kT5SortCap keep the module-pair walk.
   __global__ void __launch_bounds__(1024) kT5Bin(DeviceES es, const EventView* evs) {
     kernelEntry();
     __shared__ unsigned int sCount[kPLSBins + 1];
