@@ -1,6 +1,8 @@
-"""lst_batch_get_output through its pinned staging (256 KiB a slot, 1 MiB at most)
-and past it, against lst_batch_get_output_static, which has no such staging."""
+"""lst_batch_get_output through its pinned staging (up to 1 MiB) and past it, against
+lst_batch_get_output_static, which has no such staging; and by more threads at a
+time than the event setup has staging buffers."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -28,7 +30,7 @@ def output_bytes(tco, hco):
 
 
 # (events, slots of the set, whether the output fits the staging)
-CASES = [([(1, 80, 0.0)], 1, True), ([(2, 81, 200.0)], 1, True), ([(2, 920, 400.0)], 1, False),
+CASES = [([(1, 80, 0.0)], 1, True), ([(2, 81, 200.0)], 1, True), ([(2, 920, 400.0)], 1, True),
          ([(2, 920, 400.0)], 2, True), ([(2, 82, 200.0)] * 5, 5, True), ([(2, 83, 200.0)] * 8, 8, False)]
 
 
@@ -50,7 +52,7 @@ def test_either_way_gives_the_output(es, events, slots, fits):
         lib = lst.library()
         rc, want, tco, hco = call(lib.lst_batch_get_output_static, s, n, 31000 * n, 31000 * 14 * n)
         assert rc == 0 and tco[-1] > 0
-        assert (output_bytes(tco, hco) < min(slots << 18, 1 << 20) - 1024) == fits
+        assert (output_bytes(tco, hco) < (1 << 20) - 1024) == fits
         for _ in range(2):
             rc, got, t, h = call(lib.lst_batch_get_output, s, n, 31000 * n, 31000 * 14 * n)
             assert rc == 0 and np.array_equal(t, tco) and np.array_equal(h, hco)
@@ -80,3 +82,40 @@ def test_too_small_arrays_stay_as_they_were(es, events, slots, fits, tc_short, h
             assert (a == a.dtype.type(v)).all()
     finally:
         s.close()
+
+
+def test_more_threads_than_buffers(es):
+    """Each thread with a set of its own, one event after the other."""
+    n, rounds = 12, 8
+    inputs = [gen.generate_event(*((3, 90 + i, 20.0) if i % 3 else (2, 90 + i, 200.0))) for i in range(n)]
+    sets = [lst.EventSet(es, 1, max(i.n_hits for i in inputs) + 1024) for _ in range(n)]
+    fn = lst.library().lst_batch_get_output
+    try:
+        want, got, gate = [], [[] for _ in range(n)], threading.Barrier(n)
+        for inp in inputs:
+            sets[0].upload_packed(0, *lst.pack_events([inp]))
+            sets[0].run(0, 1)
+            want.append(call(fn, sets[0], 1, 31000, 31000 * 14))
+
+        def work(i):
+            for k in range(rounds):
+                sets[i].upload_packed(0, *lst.pack_events([inputs[(i + k) % n]]))
+                gate.wait(60)
+                sets[i].run(0, 1)
+                got[i].append(call(fn, sets[i], 1, 31000, 31000 * 14))
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(n)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for i in range(n):
+            assert len(got[i]) == rounds
+            for k, (rc, arrays, tco, hco) in enumerate(got[i]):
+                w = want[(i + k) % n]
+                assert rc == 0 and np.array_equal(tco, w[2]) and np.array_equal(hco, w[3])
+                for a, b in zip(arrays, w[1]):
+                    assert np.array_equal(a, b)
+    finally:
+        for s in sets:
+            s.close()

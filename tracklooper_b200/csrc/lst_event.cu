@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <fstream>
@@ -204,6 +205,11 @@ namespace {
 }  // namespace
 
 // ------------------------------------------------------------------ ES
+// Pinned output staging of lst_batch_get_output: bytes of a buffer, buffers of an
+// event setup.
+constexpr size_t kHostOutBytes = size_t(1) << 20;
+constexpr unsigned int kHostOutBuffers = 8;
+
 struct lst_es {
   int device = 0;
   lst::EsHost host;
@@ -213,9 +219,36 @@ struct lst_es {
   bool haveDnn = false;
   unsigned int nEligibleMax = 0;  // lower modules that can seed T5s
   std::vector<float> dnn;
+  unsigned char* hostOut = nullptr;  // kHostOutBuffers buffers, one after the other, or null
+  std::atomic<unsigned int> hostOutFree{0};  // bit i: buffer i is free
 };
 
 namespace {
+
+  // One of the event setup's output buffers for the duration of a call, or none
+  // if all are in use (by calls of other threads) or could not be locked.
+  class HostOut {
+  public:
+    explicit HostOut(lst_es* es) : es_(es) {
+      unsigned int free = es->hostOutFree.load(std::memory_order_relaxed);
+      while (free != 0 &&
+             !es->hostOutFree.compare_exchange_weak(free, free & (free - 1), std::memory_order_acquire,
+                                                    std::memory_order_relaxed)) {
+      }
+      bit_ = free & (~free + 1);
+      for (unsigned int b = bit_; b > 1; b >>= 1)
+        ++index_;
+    }
+    ~HostOut() { es_->hostOutFree.fetch_or(bit_, std::memory_order_release); }
+    HostOut(const HostOut&) = delete;
+    HostOut& operator=(const HostOut&) = delete;
+    unsigned char* data() const { return bit_ ? es_->hostOut + index_ * kHostOutBytes : nullptr; }
+    size_t room() const { return bit_ ? kHostOutBytes : 0; }
+
+  private:
+    lst_es* es_;
+    unsigned int bit_ = 0, index_ = 0;
+  };
 
   template <typename T>
   const T* upload(Carver& c, const std::vector<T>& v, std::vector<std::pair<void*, const void*>>& copies,
@@ -424,9 +457,6 @@ struct lst_event {
   unsigned long long* hOutOffsets = nullptr;  // pinned copy
   unsigned char* dOut = nullptr;
   size_t dOutBytes = 0;
-  unsigned char* hOut = nullptr;  // pinned output staging, from the set's first lst_batch_get_output on
-  size_t hOutBytes = 0;
-  bool hOutTried = false;
   unsigned int* dProbeCount = nullptr;
   // launch accounting and optional per-launch timing
   unsigned long long launches = 0;
@@ -461,8 +491,6 @@ namespace {
 namespace {
 
   constexpr unsigned int kThreads = 256;
-  // pinned output staging of lst_batch_get_output: per slot, and at most
-  constexpr size_t kHostOutPerSlot = size_t(1) << 18, kHostOutBytes = size_t(1) << 20;
   constexpr unsigned int kResidentBlocks = 148 * 8;
 
   // Blocks per event for a grid-stride kernel over n items.
@@ -880,6 +908,13 @@ int lst_es_load_ex(const char* geometry_dir, const char* t5dnn_weights_path, int
       return rc;
     }
   }
+  // (without memory to lock, outputs are copied as large ones are)
+  if (cudaMallocHost(&es->hostOut, kHostOutBuffers * kHostOutBytes) == cudaSuccess) {
+    es->hostOutFree = (1u << kHostOutBuffers) - 1u;
+  } else {
+    cudaGetLastError();
+    es->hostOut = nullptr;
+  }
   staticOutputDeviceRetain(device);
   *out = es.release();
   return 0;
@@ -970,6 +1005,7 @@ void lst_es_free(lst_es* es) {
   if (es->arena) {
     cudaSetDevice(es->device);
     cudaFree(es->arena);
+    cudaFreeHost(es->hostOut);
     staticOutputDeviceRelease(es->device);
   }
   delete es;
@@ -1108,7 +1144,6 @@ void lst_event_destroy(lst_event* ev) {
   cudaFreeHost(ev->hCounts);
   cudaFree(ev->dOutOffsets);
   cudaFreeHost(ev->hOutOffsets);
-  cudaFreeHost(ev->hOut);
   for (cudaEvent_t e : ev->eventPool)
     cudaEventDestroy(e);
   for (auto& g : ev->graphs)
@@ -1788,15 +1823,14 @@ int lst_batch_get_output(lst_event* ev, int first, int count, lst_output* out) {
     out->event_hit_offsets[0] = 0;
     return 0;
   }
-  // A small output (up to 256 KiB a slot of the set, a PU200 event has 170 kB, and
-  // 1 MiB in all) is written to pinned host memory by the kernels and copied from
-  // there: one wait for the stream instead of two and no copy calls (this call
-  // alone, to pinned or pageable arrays: one muon 22 us instead of 41 or 63, one
-  // PU200 event 49 instead of 58 or 93, four 78 instead of 68 or 132).  A larger
-  // one is copied straight to the caller's arrays.  The staging is made by the
-  // set's first call and not with the set, and by its slots: page-locking costs
-  // 0.75 ms a MiB, and with 1 MiB each, sets of one slot took 1.75 ms to make
-  // instead of 0.5.  Without it (no memory to lock) every output is copied.
+  // A small output (up to kHostOutBytes, some six PU200 events) is written to
+  // pinned host memory by the kernels and copied from there: one wait for the
+  // stream instead of two and no copy calls (this call alone, to pinned or pageable
+  // arrays: one muon 22 us instead of 41 or 63, one PU200 event 49 instead of 58 or
+  // 93, four 78 instead of 68 or 132).  A larger one, or one that finds all buffers
+  // in use, is copied straight to the caller's arrays.  The buffers are the event
+  // setup's, locked when it is loaded: with one of its own, a set took 1.75 ms to
+  // make instead of 0.5, and locked by its first output, that output 3 ms more.
   cudaStream_t s = ev->stream;
   const lst::EventView* v = ev->dv + first;
   auto ensureStaging = [&](size_t bytes) -> int {
@@ -1814,22 +1848,13 @@ int lst_batch_get_output(lst_event* ev, int first, int count, lst_output* out) {
   rc = ensureStaging(kHostOutBytes);
   if (rc)
     return rc;
-  if (!ev->hOutTried) {
-    ev->hOutTried = true;
-    const size_t bytes = std::min(kHostOutBytes, kHostOutPerSlot * static_cast<size_t>(ev->nSlots));
-    if (cudaMallocHost(&ev->hOut, bytes) == cudaSuccess) {
-      ev->hOutBytes = bytes;
-    } else {
-      cudaGetLastError();
-      ev->hOut = nullptr;
-    }
-  }
+  const HostOut staging(ev->es);
   const dim3 gatherGrid(blocksFor(lst::kMaxTrackCandidates, count), count);
   LST_LAUNCH(lst::kOutputSizes, dim3(1, count), 1024, v);
   LST_LAUNCH(lst::kOutputEventOffsets, 1, 1024, v, count, ev->dOutOffsets);
   LST_LAUNCH(lst::kOutputGather, gatherGrid, kThreads, v, count, ev->dOutOffsets, ev->dOut, ev->dOutBytes);
-  LST_LAUNCH(lst::kOutputToHost, 32, kThreads, count, ev->dOutOffsets, ev->dOut, ev->hOutBytes, ev->hOutOffsets,
-             ev->hOut);
+  LST_LAUNCH(lst::kOutputToHost, 32, kThreads, count, ev->dOutOffsets, ev->dOut, staging.room(), ev->hOutOffsets,
+             staging.data());
   LST_CUDA(cudaStreamSynchronize(s));
   const unsigned long long* tcOff = ev->hOutOffsets;
   const unsigned long long* hitOff = ev->hOutOffsets + count + 1;
@@ -1846,11 +1871,12 @@ int lst_batch_get_output(lst_event* ev, int first, int count, lst_output* out) {
   if (!out->hits || !out->len || !out->seedIdx || !out->type)
     return setError("lst_batch_get_output: null output array");
   const lst::OutputLayout l = lst::outputLayout(nHits, nTC);
-  if (l.end <= ev->hOutBytes) {
-    std::memcpy(out->hits, ev->hOut, nHits * sizeof(unsigned int));
-    std::memcpy(out->len, ev->hOut + l.len, nTC * sizeof(unsigned int));
-    std::memcpy(out->seedIdx, ev->hOut + l.seed, nTC * sizeof(int));
-    std::memcpy(out->type, ev->hOut + l.type, nTC * sizeof(short));
+  if (l.end <= staging.room()) {
+    const unsigned char* host = staging.data();
+    std::memcpy(out->hits, host, nHits * sizeof(unsigned int));
+    std::memcpy(out->len, host + l.len, nTC * sizeof(unsigned int));
+    std::memcpy(out->seedIdx, host + l.seed, nTC * sizeof(int));
+    std::memcpy(out->type, host + l.type, nTC * sizeof(short));
     return 0;
   }
   if (l.end > ev->dOutBytes) {
