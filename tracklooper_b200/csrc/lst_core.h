@@ -287,7 +287,8 @@ namespace lst {
     // whole 32-byte sectors), with values that the cuts form of it many times
     // over; formed once, by exactly their expressions, they are the same values:
     // slope = asin(min(rt k / ptCut, sinAlphaMax)), tanSlope = tan(slope),
-    // slope3 = asin(min(rt k / 3, sinAlphaMax)), and quotients.
+    // slope3 = asin(min(rt k / 3, sinAlphaMax)), and quotients.  (Of a pixel
+    // mini-doublet the anchor and the hits alone: the derived values are 0.)
     struct MDRec* rec;
   };
 
